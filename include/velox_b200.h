@@ -112,6 +112,11 @@ int vx_amax(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, float
 int vx_sf_from_natural(int fmt, const void* scales, int64_t R, int64_t K, void* scales_sf,
                        void* stream);
 
+/* The scales of both operands of one GEMM (same K) in one launch: vx_sf_from_natural(fmt_a, ...) and
+ * vx_sf_from_natural(fmt_b, ...). */
+int vx_sf_from_natural_pair(int fmt_a, const void* scales_a, int64_t Ra, void* sf_a, int fmt_b, const void* scales_b,
+                            int64_t Rb, void* sf_b, int64_t K, void* stream);
+
 /* Block-scaled GEMM  D[M,N] = epilogue( A[M,K] . B[N,K]^T ).
  * Replaces velox_dgx_mxfp4_gemm / velox_dgx_mxfp4_blkscale_gemm
  * (veloxvoice/kernels/csrc/dgx/dgx_mxfp4_gemm.cu:61-111,135-180; Python wrappers
@@ -147,7 +152,7 @@ typedef struct vx_gemm_desc {
   const float* out_amax;/* FP4 NV16 output: f32[1] static tensor amax */
   int32_t heads;        /* BIAS_QKVPACK / VX_GEMM_OUT_HEADS: number of attention heads */
   int32_t head_dim;     /*   columns per head (multiple of 32) */
-  const void* pos_u;    /* BIAS_QKVPACK: bf16 [heads, head_dim] positional biases */
+  const void* pos_u;    /* BIAS_QKVPACK: bf16 (VX_GEMM_POS_F32: fp32) [heads, head_dim] positional biases */
   const void* pos_v;
   float qk_scale;       /* BIAS_QKVPACK: scale applied to q + bias */
   int32_t head_col_off; /* VX_GEMM_OUT_HEADS: first column inside the head row (0 or head_dim) */
@@ -173,15 +178,26 @@ int vx_glu_tile(int fmt);
                                   out[n / head_dim][m][head_col_off + n % head_dim]; N = heads * head_dim.
                                   With head_col_off = head_dim and out = the k2 third of a BIAS_QKVPACK
                                   buffer this is where lp(pos_emb) belongs (torch_conformer.py:472,507) */
+#define VX_GEMM_POS_F32 64     /* BIAS_QKVPACK: pos_u / pos_v are fp32, rounded to bf16 on use */
+#define VX_GEMM_CONST_B 128    /* B (codes, scales) is a constant that was packed by vx_quantize_pack from fp32, or with
+                                  natural-layout scales: its loads may start under the tail of the previous launch */
 
 int vx_bsgemm(const vx_gemm_desc* desc, void* stream);
+
+/* One linear of the reference's per-row-scaled lane: out f32 [M, N] = dequant(quantize(x)) . W^T (+ bias), i.e.
+ * vx_quantize_pack(ROWSCALE) of the activation rows and vx_bsgemm (NONE / BIAS, fp32 out).  Replaces
+ * DenseLinear.forward (veloxvoice/models/wenet/torch_conformer.py:251-266: pad copy, cast, quantizer, GEMM, slice, bias add).
+ *   w_codes u8 [N, K/2] (row stride ldw bytes), w_scales u8 [N]: the packed weight, a constant as for VX_GEMM_CONST_B;
+ *   scratch at least M * (K/2 + 1) bytes, 16-byte aligned: the quantized activation. */
+int vx_rowscale_linear(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const void* w_codes, int64_t ldw,
+                       const void* w_scales, int64_t N, const float* bias, void* scratch, float* out, int64_t ldo, void* stream);
 
 /* The residual GEMM that ends a Conformer module together with the LayerNorm + quantizer that opens the
  * next one, in one launch: replaces vx_bsgemm(BIAS_RESIDUAL, bf16) followed by vx_ln_quantize_pack(fmt = MX32)
  * -- in the reference a GEMM, a bias / residual add, a LayerNorm launch and a quantizer launch
  * (veloxvoice/models/wenet/torch_conformer.py:706, 251-262; velox_layernorm.cu:13-58).
  *   desc       as for vx_bsgemm with fmt = MX32, N = 512, K % 256 == 0, epilogue = BIAS_RESIDUAL, bf16 output and
- *              bf16 residual (rows 16-byte aligned; out may alias residual), flags = 0;
+ *              bf16 residual (rows 16-byte aligned; out may alias residual), flags = 0 or VX_GEMM_CONST_B;
  *   out        x = bf16(alpha (A B^T + bias) + residual), stored as by vx_bsgemm;
  *   codes / scales_sf   MX32 codes u8 [M, 256] (row stride ldc bytes) and SF atoms (vx_sf_bytes(MX32, M, 512)) of
  *              LayerNorm(x as stored; gamma, beta, eps) -- the same bits as vx_ln_quantize_pack on x.
@@ -260,6 +276,14 @@ int vx_power_mel_log(const void* spec, int64_t T, int64_t F, int64_t ld_spec, co
 int vx_ctc_topk_threshold(const void* lse_partials, int64_t N, int64_t M, int k, float* threshold, void* stream);
 int vx_ctc_topk_finish(const void* candidates, const int32_t* count, int capacity, const void* lse_partials, int64_t N,
                        int64_t M, int k, int32_t* ids, float* logp, int32_t* overflow, void* stream);
+
+/* The same top-k through bf16 logits that exist for a block of rows at a time: per block one launch of the head into
+ * `logits` (scratch, bf16 [rows][N rounded up to 8], `rows` = a multiple of 128 or >= M) and one kernel that reads it back
+ * while it is in L2 (vx_ctc_topk_rows(N): rows per block for that).  desc: operands, scales and bias of the head (fmt
+ * ROWSCALE, MX32 or NV16); its output side is ignored.  Writes logp f32 [M, k] = logit - logsumexp and ids i64 [M, k],
+ * largest first, equal logits by ascending column, for any number of equal logits.  k <= 16. */
+int64_t vx_ctc_topk_rows(int64_t N);
+int vx_ctc_topk(const vx_gemm_desc* desc, int k, void* logits, int64_t rows, float* logp, int64_t* ids, void* stream);
 
 /* Attention fold pack in one pass: replaces velox_qkv_pack
  * (veloxvoice/kernels/csrc/velox_qkv_pack.cu:34-97; Python wrapper qkv_pack in

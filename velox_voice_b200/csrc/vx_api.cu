@@ -32,6 +32,18 @@ bool pdl_enabled() {
   return on;
 }
 
+int sm_count() {
+  static int cache[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (!cache[dev]) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cache[dev] = n;
+  }
+  return cache[dev];
+}
+
 int* device_status_ptr() {
   // cudaGetSymbolAddress answers for the CURRENT device; looked up once per device.
   static int* cache[64] = {};

@@ -117,6 +117,7 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
 __global__ void __launch_bounds__(AT_THREADS, 1)
 relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
+  pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* const base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* const q_s = base;
@@ -156,6 +157,7 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bar.tmem_base;
+  pdl_wait();  // set-up done: from here on the kernel touches what the previous kernel of the stream produced
 
   if (warp == 0) {
     // =========================== TMA producer ===========================
@@ -396,7 +398,6 @@ extern "C" int vx_relpos_attention(const void* q2, const void* k2, const void* v
     if (dev_cached) attr_done.fetch_or(1ull << dev, std::memory_order_release);
   }
   const dim3 grid(static_cast<unsigned>((T + AT_BM - 1) / AT_BM), static_cast<unsigned>(heads));
-  relpos_attn_kernel<<<grid, AT_THREADS, AT_SMEM, static_cast<cudaStream_t>(stream)>>>(tq, tk, tv, p);
-  VX_CUDA_OK(cudaGetLastError());
+  VX_CUDA_OK(launch_dependent(relpos_attn_kernel, grid, dim3(AT_THREADS), AT_SMEM, static_cast<cudaStream_t>(stream), tq, tk, tv, p));
   return 0;
 }

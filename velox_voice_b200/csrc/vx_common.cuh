@@ -14,6 +14,9 @@ int fail(int code, const char* fmt, ...);
 // Device status word shared by all kernels (bounded waits report here).
 int* device_status_ptr();
 
+// Multiprocessors of the current device (asked once per device).
+int sm_count();
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Block size along K of one scale; 0 = whole row.
@@ -47,6 +50,13 @@ bool pdl_enabled();
 // Launch of a kernel that executes pdl_wait() before its first dependent access: its blocks may be
 // scheduled while the previous kernel of the stream drains, so launch latency and the kernel's own
 // set-up (barriers, tensor memory, constant operands) overlap the predecessor's tail.
+//
+// What a kernel may read before its pdl_wait(): only what no kernel that triggers early (pdl_launch_dependents) wrote in
+// the launch before it, nor -- since a kernel may trigger before its own wait -- in the launches before that.  LayerNorm
+// parameters, biases and the filterbank come from torch kernels, which never trigger early.  Weights come from the
+// quantizers: those that pack weights (quant_kernel, and rows2_kernel when it writes natural-layout scales) do not
+// trigger, and the GEMMs read weights ahead only when the caller says that they are constants (VX_GEMM_CONST_B), not
+// for an operand that the previous launch may just have produced.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                     Args&&... args) {

@@ -117,6 +117,7 @@ struct GemmParams {
   const float* fb;        // FP8: f32 [N, K/128]
   // epilogue
   // shared-memory plan
+  int b_const;            // 1: B was not written by the launches just before this one: it may be loaded ahead of the wait
   int b_resident;         // 1: the CTA keeps its B tile (all K stages) in shared memory
   int sfb_resident;       // 1: B streams, but its scale factors are copied to tensor memory once
                           //    (the CTA owns one n-block, as with b_resident)
@@ -142,8 +143,9 @@ struct GemmParams {
   const float* out_amax;
   // head-major bf16 output (attention fold pack)
   int heads, head_dim, head_col_off;
-  const __nv_bfloat16* pos_u;
-  const __nv_bfloat16* pos_v;
+  const void* pos_u;      // bf16, or fp32 with pos_f32
+  const void* pos_v;
+  int pos_f32;
   float qk_scale;
   float2* lse_part;       // ARGMAX: per (64-column group, row) running (max, sum of exp) or nullptr
   const float* topk_thr;  // ARGMAX + lse_part: per-row threshold of the candidate pass, or nullptr
@@ -712,6 +714,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
       };
       uint8_t* const sfb_stage = sm.arena + (nslots - 1) * slot_bytes + a_slot;
       bool sfb_pending = sfb_res;
+      if (!p.b_const) pdl_wait();
       if (resident) {
         mbar_expect_tx(&sm.b_full, p.k_stages * b_tx(nb0));
         for (int ks = 0; ks < p.k_stages; ++ks) load_b(sm.arena + ks * b_slot, nb0, ks, &sm.b_full);
@@ -729,7 +732,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
                         p.sfb + (static_cast<int64_t>(nb0 * NRT + rt) * p.sf_kg) * 512 + ks * sf_stage, APS * 512,
                         &sm.b_full);
       }
-      pdl_wait();
+      if (p.b_const) pdl_wait();
       int mb = mb0, nb = nb0;
       const int G = p.group, k_groups = p.k_stages / G, ngs = nslots / G;
       for (int i = 0; i < my_tiles && ok; ++i) {
@@ -945,8 +948,8 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     uint32_t group = 0;
     bool ok = true;
     float g_ab = 1.0f, g_out = 1.0f;
-    if (p.a_amax && p.b_amax) g_ab = nv16_global(__ldg(p.a_amax)) * nv16_global(__ldg(p.b_amax));
-    if (p.out_amax) g_out = nv16_global(__ldg(p.out_amax));
+    if (p.a_amax && p.b_amax) g_ab = nv16_global(*p.a_amax) * nv16_global(*p.b_amax);
+    if (p.out_amax) g_out = nv16_global(*p.out_amax);
     const int kb_count = FP8 ? p.k_stages : 0;
     uint8_t* const stage0 = sm.staging[ew & 15];
     // TMA residual: the two halves of the staging buffer alternate per 32-column chunk.  The
@@ -1112,12 +1115,12 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           __syncwarp();
           const int64_t ncol = static_cast<int64_t>(nb) * BNT + col_base + lane;
           const float* src = p.fb + ncol * kb_count;
-          for (int kb = 0; kb < kb_count; ++kb) sb_tab[kb * 32 + lane] = ncol < p.N ? __ldg(src + kb) : 0.0f;
+          for (int kb = 0; kb < kb_count; ++kb) sb_tab[kb * 32 + lane] = ncol < p.N ? src[kb] : 0.0f;
           if constexpr (GLU) {
             if (has_work) {
               const int64_t gcol = ncol + GATE_OFF;
               const float* gsrc = p.fb + gcol * kb_count;
-              for (int kb = 0; kb < kb_count; ++kb) sb_gate[kb * 32 + lane] = gcol < p.N ? __ldg(gsrc + kb) : 0.0f;
+              for (int kb = 0; kb < kb_count; ++kb) sb_gate[kb * 32 + lane] = gcol < p.N ? gsrc[kb] : 0.0f;
             }
           }
           __syncwarp();
@@ -1127,7 +1130,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < 32; ++i) { z[0][i] = 0.0f; gate[i] = 0.0f; }
         const float* sa_row = p.fa + row * kb_count;
-        float sa_next = row_ok ? __ldg(sa_row) : 0.0f;
+        float sa_next = row_ok ? *sa_row : 0.0f;
         for (int kb0 = 0; kb0 < kb_count && ok; kb0 += FP8_ACCS) {
           // one round: up to four K blocks, block u in accumulator u, published together
           const int nkb = kb_count - kb0 < FP8_ACCS ? kb_count - kb0 : FP8_ACCS;
@@ -1141,7 +1144,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           for (int u = 0; u < nkb; ++u) {
             const int kb = kb0 + u;
             const float sa = sa_next;
-            if (kb + 1 < kb_count && row_ok) sa_next = __ldg(sa_row + kb + 1);
+            if (kb + 1 < kb_count && row_ok) sa_next = sa_row[kb + 1];
             const uint64_t sa2 = pack_f32x2(sa, sa);
             // acc[i] += r[i] * (sa * table[i]).  The scale products are a packed fp32x2
             // multiply (both operands come as pairs: sb from shared memory, sa duplicated); the
@@ -1246,9 +1249,9 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           if constexpr (!FP8) {
             if (sf_unit) {
               // reference order: raw * row_scale * col_scale
-              const float row_scale = row_ok ? ue8m0_to_float(__ldg(p.row_scale_u8 + row)) : 0.0f;
+              const float row_scale = row_ok ? ue8m0_to_float(p.row_scale_u8[row]) : 0.0f;
               const int64_t ncol = acc_col0 + lane;
-              const float csv = ncol < p.N ? ue8m0_to_float(__ldg(p.col_scale_u8 + ncol)) : 0.0f;
+              const float csv = ncol < p.N ? ue8m0_to_float(p.col_scale_u8[ncol]) : 0.0f;
 #pragma unroll
               for (int i = 0; i < 32; ++i) z[h][i] = z[h][i] * row_scale * __shfl_sync(0xffffffffu, csv, i);
             } else if (kind_vec4(KIND) && p.a_amax) {
@@ -1304,8 +1307,18 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
                 *reinterpret_cast<uint4*>(buf + lane * 64 + ((v4 ^ ((lane >> 1) & 3)) << 4)) = u;
               }
             };
-            // bias vector (32 bf16, the same for every lane) -> fp32
-            auto load_bias32 = [&](const __nv_bfloat16* src, float (&b)[32]) {
+            // bias vector (32 bf16, or 32 fp32 rounded to bf16; the same for every lane) -> fp32
+            auto load_bias32 = [&](const void* base, float (&b)[32]) {
+              if (p.pos_f32) {
+                const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(base) + within);
+#pragma unroll
+                for (int v4 = 0; v4 < 8; ++v4) {
+                  const float4 w = __ldg(src + v4);
+                  b[4 * v4] = rnd(w.x); b[4 * v4 + 1] = rnd(w.y); b[4 * v4 + 2] = rnd(w.z); b[4 * v4 + 3] = rnd(w.w);
+                }
+                return;
+              }
+              const __nv_bfloat16* src = static_cast<const __nv_bfloat16*>(base) + within;
 #pragma unroll
               for (int v4 = 0; v4 < 4; ++v4) {
                 const uint4 w = __ldg(reinterpret_cast<const uint4*>(src) + v4);
@@ -1323,11 +1336,11 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
             uint8_t* const buf_b = stage0 + STAGING_BYTES / 2;
             if (part == 0) {
               float b[32], o[32];
-              load_bias32(p.pos_u + within, b);
+              load_bias32(p.pos_u, b);
 #pragma unroll
               for (int i = 0; i < 32; ++i) o[i] = __fmul_rn(rnd(__fadd_rn(rnd(z[h][i]), b[i])), p.qk_scale);
               stage_bf16(buf_a, o);
-              load_bias32(p.pos_v + within, b);
+              load_bias32(p.pos_v, b);
 #pragma unroll
               for (int i = 0; i < 32; ++i) o[i] = __fmul_rn(rnd(__fadd_rn(rnd(z[h][i]), b[i])), p.qk_scale);
               stage_bf16(buf_b, o);
@@ -1391,7 +1404,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
               if (TOPK && row_ok) {
                 // candidate pass of the top-k: append every logit of this chunk that reaches the row's threshold
                 // (few chunks of a row hold one; the chunk maximum decides whether to look at all)
-                const float thr = __ldg(p.topk_thr + row);
+                const float thr = p.topk_thr[row];
                 if (cm >= thr) {
 #pragma unroll
                   for (int i = 0; i < 32; ++i) {
@@ -1508,8 +1521,9 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
 }
 
 // keys of the ARGMAX epilogue -> column ids (and the winning bf16 logit as fp32)
-__global__ void argmax_ids_kernel(const unsigned long long* __restrict__ keys, int64_t M,
-                                  int32_t* __restrict__ ids, float* __restrict__ max_out) {
+__global__ void argmax_ids_kernel(const unsigned long long* keys, int64_t M, int32_t* ids, float* max_out) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= M) return;
   const unsigned long long k = keys[i];
@@ -1823,6 +1837,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, 
            GemmParams& p, bool allow_resident, cudaStream_t st) {
   int dev = 0, sms = 0;
   VX_CUDA_OK(cudaGetDevice(&dev));
+  sms = sm_count();
   // The dynamic shared-memory opt-in belongs to the (function, device) pair: once per device
   // and template instance (a process may drive several GPUs).
   static std::atomic<uint64_t> attr_done{0};
@@ -1832,12 +1847,6 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, 
                                                static_cast<int>(kSmemBytes));
     if (e != cudaSuccess) return fail(static_cast<int>(e), "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     if (dev_cached) attr_done.fetch_or(1ull << dev, std::memory_order_release);
-  }
-  static int sm_cache[64] = {};
-  if (dev >= 0 && dev < 64 && sm_cache[dev]) sms = sm_cache[dev];
-  else {
-    VX_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (dev >= 0 && dev < 64) sm_cache[dev] = sms;
   }
   // shared-memory plan: keep B resident when all of its K stages fit beside a useful ring
   constexpr int BNT = kind_bn(KIND);
@@ -1972,7 +1981,7 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
   const bool qkvpack = epi == VX_EPI_BIAS_QKVPACK;
   const bool out_heads = (d->flags & VX_GEMM_OUT_HEADS) != 0;
   constexpr int32_t kKnownFlags = VX_GEMM_DIRECT_STORE | VX_GEMM_STREAM_B | VX_GEMM_WIDE_TILES | VX_GEMM_NARROW_TILES |
-                                  VX_GEMM_OUT_HEADS;
+                                  VX_GEMM_OUT_HEADS | VX_GEMM_POS_F32 | VX_GEMM_CONST_B;
   if (d->flags & ~kKnownFlags) return fail(-1, "unknown bits in flags (0x%x)", d->flags & ~kKnownFlags);
   if (qkvpack && fmt == VX_FMT_ROWSCALE)
     return fail(-1, "BIAS_QKVPACK is not available for the per-row-scaled format (use a block-scaled format or FP8)");
@@ -1984,7 +1993,7 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
     if (qkvpack) {
       if (N != 3ll * d->heads * d->head_dim) return fail(-1, "BIAS_QKVPACK needs N = 3 * heads * head_dim");
       if (!d->pos_u || !d->pos_v || !aligned16(d->pos_u) || !aligned16(d->pos_v))
-        return fail(-1, "BIAS_QKVPACK needs pos_u / pos_v (bf16, 16-byte aligned)");
+        return fail(-1, "BIAS_QKVPACK needs pos_u / pos_v (bf16 or fp32, 16-byte aligned)");
       if (out_heads) return fail(-1, "VX_GEMM_OUT_HEADS does not combine with BIAS_QKVPACK");
     } else {
       if (epi != VX_EPI_NONE && epi != VX_EPI_BIAS) return fail(-1, "VX_GEMM_OUT_HEADS supports NONE / BIAS");
@@ -2026,13 +2035,7 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
     // a tile -- a narrow tile costs about 0.55 of a wide one.  88 row blocks, N = 512: the wide tiling
     // takes 2 rounds on 74 groups, the narrow one 3 half-size rounds on 37.
     if (!narrow && epi != VX_EPI_BIAS_SWISH && epi != VX_EPI_BIAS_GLU) {
-      static int sm_cache[64] = {};
-      int sms = 148, dev = 0;
-      if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
-        if (!sm_cache[dev] && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
-          sm_cache[dev] = sms;
-        if (sm_cache[dev]) sms = sm_cache[dev];
-      }
+      const int sms = sm_count();
       const int64_t mt = (M + BM - 1) / BM, ntw = (N + 255) / 256, ntn = (N + 127) / 128;
       auto rounds = [&](int64_t nt) {
         int64_t groups = nt <= sms ? sms / nt : 1;
@@ -2084,13 +2087,15 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
   p.bias = d->bias;
   p.residual = d->residual; p.residual_dtype = d->residual_dtype; p.ldr = d->ldr; p.alpha = d->alpha;
   p.status = cached_status_ptr();
+  p.b_const = !fp8 && (d->flags & VX_GEMM_CONST_B) != 0;
 
   if (qkvpack || out_heads) {
     p.heads = d->heads;
     p.head_dim = d->head_dim;
     p.head_col_off = qkvpack ? 0 : d->head_col_off;
-    p.pos_u = static_cast<const __nv_bfloat16*>(d->pos_u);
-    p.pos_v = static_cast<const __nv_bfloat16*>(d->pos_v);
+    p.pos_u = d->pos_u;
+    p.pos_v = d->pos_v;
+    p.pos_f32 = (d->flags & VX_GEMM_POS_F32) != 0;
     p.qk_scale = d->qk_scale;
   } else if (argmax) {
     p.out_dtype = VX_F32;
@@ -2179,9 +2184,8 @@ int vx_argmax_ids(const void* keys, int64_t M, int32_t* ids, float* max_out, voi
   if (M == 0) return 0;
   if (!keys || !ids) return fail(-1, "keys and ids must not be NULL");
   const int grid = static_cast<int>((M + 255) / 256);
-  argmax_ids_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const unsigned long long*>(keys), M, ids, max_out);
-  VX_CUDA_OK(cudaGetLastError());
+  VX_CUDA_OK(launch_dependent(argmax_ids_kernel, dim3(grid), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                              static_cast<const unsigned long long*>(keys), M, ids, max_out));
   return 0;
 }
 

@@ -66,6 +66,7 @@ constexpr uint32_t LN_TM_ACC = 0, LN_TM_XP = 256, LN_TM_SFA = 384, LN_TM_SFB = 4
 struct LnParams {
   int64_t M, K;
   int m_tiles, k_stages;
+  int b_const;     // 1: B may be loaded ahead of the wait for the previous launch (VX_GEMM_CONST_B)
   int b_resident;  // 1: the CTA keeps its half of B (all K stages) in shared memory
   const uint8_t* sfa;
   const uint8_t* sfb;
@@ -225,11 +226,12 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           bulk_load(dst + LN_B_TILE + rt * 1024,
                     p.sfb + (static_cast<int64_t>(rank * 2 + rt) * p.sf_kg) * 512 + static_cast<int64_t>(ks) * 1024, 1024, bar);
       };
-      if (resident) {  // weights: constants of the model, loaded before the wait for the previous kernel
+      if (!p.b_const) pdl_wait();
+      if (resident) {  // constant weights are loaded before the wait for the previous kernel
         mbar_expect_tx(&sm.b_full, p.k_stages * LN_B_SLOT);
         for (int ks = 0; ks < p.k_stages; ++ks) load_b(sm.arena + ks * LN_B_SLOT, ks, &sm.b_full);
       }
-      pdl_wait();
+      if (p.b_const) pdl_wait();
       int mb = cluster;
       for (int i = 0; i < my_tiles && ok; ++i, mb += nclusters) {
         const uint8_t* sfa_row = p.sfa + (static_cast<int64_t>(mb) * p.sf_kg) * 512;
@@ -585,7 +587,7 @@ int launch_residual_ln(const vx_gemm_desc* d, const float* gamma, const float* b
     return fail(-1, "%s needs fmt = MX32, N = 512 and K a multiple of 256 (see vx_bsgemm_residual_ln_supported)", who);
   const int64_t M = d->M, K = d->K;
   if (M < 0) return fail(-1, "negative shape");
-  if (d->epilogue != VX_EPI_BIAS_RESIDUAL || d->out_dtype != VX_BF16 || d->residual_dtype != VX_BF16 || d->flags != 0)
+  if (d->epilogue != VX_EPI_BIAS_RESIDUAL || d->out_dtype != VX_BF16 || d->residual_dtype != VX_BF16 || (d->flags & ~VX_GEMM_CONST_B))
     return fail(-1, "%s: epilogue BIAS_RESIDUAL with bf16 output and bf16 residual, no flags", who);
   if (M == 0) return 0;
   const int64_t row_bytes = K / 2;
@@ -608,6 +610,7 @@ int launch_residual_ln(const vx_gemm_desc* d, const float* gamma, const float* b
   p.M = M; p.K = K;
   p.m_tiles = static_cast<int>((M + LN_BM - 1) / LN_BM);
   p.k_stages = static_cast<int>(K / 256);
+  p.b_const = (d->flags & VX_GEMM_CONST_B) != 0;
   p.b_resident = p.k_stages <= LN_RESIDENT_MAX_STAGES;
   p.sfa = static_cast<const uint8_t*>(d->a_scales);
   p.sfb = static_cast<const uint8_t*>(d->b_scales);
@@ -635,13 +638,9 @@ int launch_residual_ln(const vx_gemm_desc* d, const float* gamma, const float* b
   rc = make_tmap_2d(&to, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d->out, M, LN_D, d->ldo * 2, 64, 32);
   if (rc) return rc;
 
-  static int sm_cache[64] = {};
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
-    if (!sm_cache[dev] && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
-      sm_cache[dev] = sms;
-    if (sm_cache[dev]) sms = sm_cache[dev];
-  }
+  const int sms = sm_count();
+  int dev = 0;
+  VX_CUDA_OK(cudaGetDevice(&dev));
   int clusters = sms / 2;
   if (clusters > p.m_tiles) clusters = p.m_tiles;
   if (clusters < 1) clusters = 1;

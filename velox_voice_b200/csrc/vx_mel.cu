@@ -92,6 +92,7 @@ struct MelBarriers {
 };
 
 __global__ void __launch_bounds__(MEL_THREADS, 1) power_mel_log_kernel(const MelParams p) {
+  pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* const ring = base;                                  // p.ring x 16 KB
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(MEL_THREADS, 1) power_mel_log_kernel(const Mel
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bar.tmem_base;
+  pdl_wait();  // the filterbank is a constant of the front-end; the spectrum and the output are not
 
   if (warp >= 4 && warp < 4 + MEL_LOADERS) {
     // =========================== loaders ===========================
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(MEL_THREADS, 1) power_mel_log_kernel(const Mel
 #pragma unroll
       for (int r = 0; r < 16; ++r) {
         const int64_t row = row0 + r;
-        c[r] = (n < items && row < p.T && f < p.F) ? __ldg(p.spec + row * p.ld_spec + f) : make_float2(0.0f, 0.0f);
+        c[r] = (n < items && row < p.T && f < p.F) ? p.spec[row * p.ld_spec + f] : make_float2(0.0f, 0.0f);
       }
     };
     auto publish = [&](uint32_t s, const float2 (&c)[16]) {
@@ -298,9 +300,9 @@ extern "C" int vx_power_mel_log(const void* spec, int64_t T, int64_t F, int64_t 
     return fail(-1, "filterbank of %lld x %lld does not fit in shared memory (%zu bytes needed, %d available)", (long long)M,
                 (long long)F, smem, MEL_MAX_SMEM);
   p.status = device_status_ptr();
-  int dev = 0, sms = 0;
+  int dev = 0;
   VX_CUDA_OK(cudaGetDevice(&dev));
-  VX_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int sms = sm_count();
   static std::atomic<uint64_t> attr_done{0};
   const bool dev_cached = dev >= 0 && dev < 64;
   if (!dev_cached || !(attr_done.load(std::memory_order_acquire) & (1ull << dev))) {
@@ -308,7 +310,6 @@ extern "C" int vx_power_mel_log(const void* spec, int64_t T, int64_t F, int64_t 
     if (dev_cached) attr_done.fetch_or(1ull << dev, std::memory_order_release);
   }
   const int grid = p.tiles < sms ? p.tiles : sms;
-  power_mel_log_kernel<<<grid, MEL_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(p);
-  VX_CUDA_OK(cudaGetLastError());
+  VX_CUDA_OK(launch_dependent(power_mel_log_kernel, dim3(grid), dim3(MEL_THREADS), smem, static_cast<cudaStream_t>(stream), p));
   return 0;
 }

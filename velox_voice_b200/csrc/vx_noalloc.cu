@@ -73,9 +73,7 @@ extern "C" int vx_blkscale_gemm_noalloc(const void* pack_a, const void* pack_b, 
   uint8_t* sfb = scratch + VX_NOALLOC_SF_MAX_BYTES;
   // the relayout clears the bytes it owns (padding rows / K groups must read as zero), so the
   // previous call's contents never leak into this one
-  rc = vx_sf_from_natural(VX_FMT_BLK16_A, scale_a, M, K, sfa, stream);
-  if (rc) return rc;
-  rc = vx_sf_from_natural(VX_FMT_BLK16_B, scale_b, N, K, sfb, stream);
+  rc = vx_sf_from_natural_pair(VX_FMT_BLK16_A, scale_a, M, sfa, VX_FMT_BLK16_B, scale_b, N, sfb, K, stream);
   if (rc) return rc;
   vx_gemm_desc d = {};
   d.struct_size = static_cast<int32_t>(sizeof(vx_gemm_desc));

@@ -230,6 +230,8 @@ __device__ __forceinline__ void tc_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[3
 // predecessor reads or writes (the wait returns once the predecessor grid has completed and its
 // memory is visible).  pdl_launch_dependents() lets the successor's blocks be scheduled as soon as
 // this grid's blocks have all issued it (or exited).  Both are no-ops in a plain launch.
+// What a predecessor may have written is read with PLAIN loads behind pdl_wait(): a read-only load (__ldg, or one the
+// compiler derives from const __restrict__) may be moved above the wait.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

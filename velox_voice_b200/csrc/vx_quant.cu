@@ -46,6 +46,7 @@ struct QuantParams {
   void* y;
   int y_bf16;
   int64_t ldy;
+  int early;    // 1: an activation, let the next launch start under this one's tail (see launch_dependent)
   int* status;  // device status word (bounded waits of the bulk-copy row rings report here)
 };
 
@@ -79,7 +80,7 @@ template <> struct Raw8<float> {
 };
 
 __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
-  const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -88,8 +89,8 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
   }
 }
 __device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-  const float4 b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  const float4 b = *(reinterpret_cast<const float4*>(p) + 1);
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
   v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
@@ -240,8 +241,10 @@ __global__ void __launch_bounds__(256, VX_QUANT_MIN_BLOCKS) quant_kernel(const Q
   const I nunits = static_cast<I>(p.M) / RP;
   const int nchunks = static_cast<int>((static_cast<I>(p.K) + 255) >> 8);
   const T* x = static_cast<const T*>(p.x);
+  pdl_wait();
+  if (p.early) pdl_launch_dependents();  // not by default: this kernel packs weights, which GEMMs read ahead of their wait
   float g = 1.0f;
-  if constexpr (FMT == VX_FMT_NV16) g = nv16_global(__ldg(p.amax));
+  if constexpr (FMT == VX_FMT_NV16) g = nv16_global(*p.amax);
   const I u_first = static_cast<I>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
 
   if constexpr (TMA) {
@@ -385,8 +388,7 @@ __global__ void __launch_bounds__(256, lnq_min_blocks(CH)) ln_quant_kernel(const
   const T* x = static_cast<const T*>(p.x);
   const float k_f = static_cast<float>(p.K);
   const int npass = p.gamma2 ? 2 : 1;
-  float g = 1.0f;
-  if constexpr (FMT == VX_FMT_NV16) g = nv16_global(__ldg(p.amax));
+  pdl_launch_dependents();
 
   // [pass][gamma | beta][16-byte piece: chunk * 2 + half][lane]
   __shared__ float4 gb_s[2][2][CH * 2][32];
@@ -399,6 +401,9 @@ __global__ void __launch_bounds__(256, lnq_min_blocks(CH)) ln_quant_kernel(const
     gb_s[which >> 1][which & 1][piece][l] = val;
   }
   __syncthreads();
+  pdl_wait();
+  float g = 1.0f;
+  if constexpr (FMT == VX_FMT_NV16) g = nv16_global(*p.amax);
 
   const I u_first = static_cast<I>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   // LayerNorm(s) + quantization of unit u, whose RP rows arrive converted in v
@@ -605,7 +610,8 @@ __global__ void __launch_bounds__(256, LN ? VX_R2_MIN_BLOCKS_LN : VX_R2_MIN_BLOC
   const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(p.x);
   const int ldx = static_cast<int>(p.ldx), ldc = static_cast<int>(p.ldc), ldy = static_cast<int>(p.ldy);
   const int npass = LN ? (p.gamma2 ? 2 : 1) : 0;
-  pdl_launch_dependents();
+  // (natural-layout scales: weights are packed that way, see launch_dependent; FP8 GEMMs read nothing ahead)
+  if (FMT == VX_FMT_FP8_1X128 || !p.scales) pdl_launch_dependents();
 
   __shared__ __align__(128) uint8_t ring_s[8 * VX_R2_RING * kR2SlotBytes];
   __shared__ uint64_t full_s[8 * VX_R2_RING];
@@ -632,7 +638,7 @@ __global__ void __launch_bounds__(256, LN ? VX_R2_MIN_BLOCKS_LN : VX_R2_MIN_BLOC
   // the previous kernel of the stream produced
   pdl_wait();
   float g = 1.0f;
-  if constexpr (FMT == VX_FMT_NV16) g = nv16_global(__ldg(p.amax));
+  if constexpr (FMT == VX_FMT_NV16) g = nv16_global(*p.amax);
 
   auto issue = [&](int slot, int u) {
     if (lane == 0) {
@@ -852,56 +858,91 @@ bool launch_rows2(const QuantParams& p, bool ln, cudaStream_t st) {
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) amax_kernel(const T* x, int64_t M, int64_t K, int64_t ldx,
-                                                   float* out) {
-  const int64_t per_row = K >> 3;
-  const int64_t total = M * per_row;
+// max |x|.  Each thread keeps four 16-byte loads in flight; dense tensors (ldx == K) are walked as one long row.  Bound by
+// HBM.  ONE_BLOCK: a tensor small enough for one block, which then writes the result itself (no cleared accumulator).
+template <typename T, bool ONE_BLOCK>
+__global__ void __launch_bounds__(ONE_BLOCK ? 1024 : 256) amax_kernel(const T* x, int64_t rows, int64_t row_vecs, int64_t ldx, float* out) {
+  constexpr int EV = 16 / sizeof(T);  // elements per 16-byte vector
+  pdl_launch_dependents();
+  pdl_wait();
   float a = 0.0f;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t r = i / per_row, k0 = (i - r * per_row) << 3;
-    float t[8];
-    load8(x + r * ldx + k0, t);
-    a = fmaxf(a, amax8(t));
+  auto take = [&](const uint4& u) {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if constexpr (sizeof(T) == 2) a = max3(a, fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xffff0000u)));
+      else a = fmaxf(a, fabsf(__uint_as_float(w[i])));
+    }
+  };
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x, step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  if (rows == 1) {
+    const uint4* v = reinterpret_cast<const uint4*>(x);
+    int64_t i = t0;
+    for (; i + 3 * step < row_vecs; i += 4 * step) {
+      const uint4 u0 = v[i], u1 = v[i + step], u2 = v[i + 2 * step], u3 = v[i + 3 * step];
+      take(u0); take(u1); take(u2); take(u3);
+    }
+    for (; i < row_vecs; i += step) take(v[i]);
+  } else {
+    const int64_t total = rows * row_vecs;
+    for (int64_t i = t0; i < total; i += step) {
+      const int64_t r = i / row_vecs;
+      take(*reinterpret_cast<const uint4*>(x + r * ldx + (i - r * row_vecs) * EV));
+    }
   }
   a = warp_max(a);
-  // non-negative floats order like their bit patterns
-  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned int*>(out), __float_as_uint(a));
+  if constexpr (ONE_BLOCK) {
+    __shared__ float part[32];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      a = warp_max(part[threadIdx.x]);
+      if (threadIdx.x == 0) *out = a;
+    }
+  } else {
+    // non-negative floats order like their bit patterns
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned int*>(out), __float_as_uint(a));
+  }
 }
 
-// natural scale layout -> SF atoms.  One thread per (row, k-group).
-__global__ void sf_relayout_kernel(int fmt, const uint8_t* __restrict__ s, int64_t R, int64_t nkb,
-                                   uint8_t* __restrict__ sf, int64_t sf_kg) {
-  const int64_t ngroups = (nkb + 3) >> 2;
-  const int64_t total = R * ngroups;
+// natural scale layout -> SF atoms, both operands of a GEMM in one launch.  One thread per 4-byte word of the atoms, in
+// the order the words lie in memory, padding rows and k-groups (zero) included: nothing is cleared beforehand.
+struct RelayoutSide {
+  const uint8_t* s;
+  uint8_t* sf;
+  int64_t R, words;  // rows, 4-byte words of all atoms
+  int fmt;
+};
+__global__ void __launch_bounds__(256) sf_relayout_kernel(RelayoutSide a, RelayoutSide b, int nkb, int sf_kg) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t total = a.words + b.words;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t row = i % R, kg = i / R;
-    uint32_t w = 0;
-    for (int j = 0; j < 4; ++j) {
-      const int64_t kb = kg * 4 + j;
-      if (kb >= nkb) break;
-      uint32_t b;
-      if (fmt == VX_FMT_BLK16_A) b = s[kb * (R >> 1) + (row >> 1)];
-      else if (fmt == VX_FMT_BLK16_B) b = s[kb * R + row];
-      else b = s[row * nkb + kb];
-      w |= b << (8 * j);
+    const bool first = i < a.words;
+    const RelayoutSide& p = first ? a : b;
+    const int64_t at = first ? i : i - a.words;
+    const int64_t atom = at >> 7;
+    const int w = static_cast<int>(at & 127);
+    const int64_t tile = atom / sf_kg;
+    const int kg = static_cast<int>(atom - tile * sf_kg);
+    const int64_t row = tile * 128 + (w >> 2) + (w & 3) * 32;
+    uint32_t v = 0;
+    if (row < p.R) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int kb = kg * 4 + j;
+        if (kb < nkb) {
+          uint32_t x;
+          if (p.fmt == VX_FMT_BLK16_A) x = p.s[kb * (p.R >> 1) + (row >> 1)];
+          else if (p.fmt == VX_FMT_BLK16_B) x = p.s[kb * p.R + row];
+          else x = p.s[row * nkb + kb];
+          v |= x << (8 * j);
+        }
+      }
     }
-    *reinterpret_cast<uint32_t*>(sf + sf_offset(row, kg, sf_kg)) = w;
+    reinterpret_cast<uint32_t*>(p.sf)[at] = v;
   }
-}
-
-int sm_count() {
-  static int cache[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!cache[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cache[dev] = n;
-  }
-  return cache[dev];
 }
 
 int grid_for_rows(int64_t units, int blocks_per_sm) {
@@ -916,28 +957,23 @@ template <typename T, int FMT, typename I, bool FAST>
 void launch_quant_idx(const QuantParams& p, bool ln, cudaStream_t st) {
   constexpr int RP = (FMT == VX_FMT_BLK16_A) ? 2 : 1;
   const int ch = p.K <= 512 ? 2 : (p.K <= 1024 ? 4 : 8);
-  const int grid = grid_for_rows(p.M / RP, ln ? lnq_min_blocks(ch) * (ch > 2 ? 2 : 1) : VX_QUANT_MIN_BLOCKS);
+  const dim3 grid(grid_for_rows(p.M / RP, ln ? lnq_min_blocks(ch) * (ch > 2 ? 2 : 1) : VX_QUANT_MIN_BLOCKS));
   // bf16 rows of up to 512 elements, one row per unit: rows come through the per-warp bulk-copy rings
   constexpr bool tma_ok = sizeof(T) == 2 && RP == 1;
   const bool tma = tma_ok && p.K <= 512;
+  auto go = [&](auto* kernel) { launch_dependent(kernel, grid, dim3(256), 0, st, p); };
   if (!ln) {
     if constexpr (tma_ok && FMT != VX_FMT_ROWSCALE) {
-      if (tma) {
-        quant_kernel<T, FMT, I, FAST, true><<<grid, 256, 0, st>>>(p);
-        return;
-      }
+      if (tma) return go(quant_kernel<T, FMT, I, FAST, true>);
     }
-    quant_kernel<T, FMT, I, FAST><<<grid, 256, 0, st>>>(p);
+    go(quant_kernel<T, FMT, I, FAST>);
   } else if (p.K <= 512) {
-    if constexpr (tma_ok) {
-      ln_quant_kernel<T, FMT, 2, I, FAST, true><<<grid, 256, 0, st>>>(p);
-      return;
-    }
-    ln_quant_kernel<T, FMT, 2, I, FAST><<<grid, 256, 0, st>>>(p);
+    if constexpr (tma_ok) go(ln_quant_kernel<T, FMT, 2, I, FAST, true>);
+    else go(ln_quant_kernel<T, FMT, 2, I, FAST>);
   } else if (p.K <= 1024) {
-    ln_quant_kernel<T, FMT, 4, I, FAST><<<grid, 256, 0, st>>>(p);
+    go(ln_quant_kernel<T, FMT, 4, I, FAST>);
   } else {
-    ln_quant_kernel<T, FMT, 8, I, FAST><<<grid, 256, 0, st>>>(p);
+    go(ln_quant_kernel<T, FMT, 8, I, FAST>);
   }
 }
 
@@ -984,7 +1020,7 @@ int quantize_common(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ld
                     void* codes, int64_t ldc, void* scales, void* scales_sf, const float* amax,
                     bool ln, const float* gamma, const float* beta, float eps, void* y,
                     int y_dtype, int64_t ldy, void* stream, const float* gamma2 = nullptr,
-                    const float* beta2 = nullptr) {
+                    const float* beta2 = nullptr, bool early = false) {
   if (!fmt_valid(fmt)) return fail(-1, "unknown format %d", fmt);
   if (x_dtype != VX_F32 && x_dtype != VX_BF16) return fail(-1, "x_dtype must be VX_F32 or VX_BF16");
   if (M < 0 || K < 0) return fail(-1, "negative shape");
@@ -1028,6 +1064,7 @@ int quantize_common(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ld
   p.scales = scales; p.sf = static_cast<uint8_t*>(scales_sf);
   p.sf_kg = sf_kgroups(fmt, K);
   p.status = device_status_ptr();
+  p.early = early;
   p.amax = amax; p.gamma = gamma; p.beta = beta; p.gamma2 = gamma2; p.beta2 = beta2; p.eps = eps; p.y = y; p.y_bf16 = (y_dtype == VX_BF16); p.ldy = ldy;
   if (scales_sf) {
     // k-groups beyond K must read as zero scale factors (rows beyond M: cleared by the kernel)
@@ -1076,48 +1113,95 @@ int vx_ln2_quantize_pack(const void* x, int x_dtype, int64_t M, int64_t K, int64
                              gamma1, beta1, eps, y, y_dtype, ldy, stream, gamma2, beta2);
 }
 
+int vx_rowscale_linear(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const void* w_codes, int64_t ldw,
+                       const void* w_scales, int64_t N, const float* bias, void* scratch, float* out, int64_t ldo, void* stream) {
+  using namespace vx;
+  if (M < 0 || N < 0 || K <= 0) return fail(-1, "bad shape M=%lld N=%lld K=%lld", (long long)M, (long long)N, (long long)K);
+  if (M == 0 || N == 0) return 0;
+  if (!scratch || !aligned16(scratch)) return fail(-1, "scratch must be 16-byte aligned");
+  uint8_t* const codes = static_cast<uint8_t*>(scratch);
+  uint8_t* const scales = codes + M * (K / 2);
+  int rc = quantize_common(x, x_dtype, M, K, ldx, VX_FMT_ROWSCALE, codes, K / 2, scales, nullptr, nullptr, false, nullptr, nullptr, 0.f,
+                           nullptr, 0, 0, stream, nullptr, nullptr, true);
+  if (rc) return rc;
+  vx_gemm_desc d{};
+  d.struct_size = static_cast<int32_t>(sizeof(d));
+  d.fmt = VX_FMT_ROWSCALE;
+  d.M = M; d.N = N; d.K = K;
+  d.a_codes = codes; d.lda = K / 2;
+  d.b_codes = w_codes; d.ldb = ldw;
+  d.a_scales = scales; d.b_scales = w_scales;
+  d.epilogue = bias ? VX_EPI_BIAS : VX_EPI_NONE;
+  d.bias = bias;
+  d.out_dtype = VX_F32; d.out = out; d.ldo = ldo;
+  d.flags = VX_GEMM_CONST_B;
+  return vx_bsgemm(&d, stream);
+}
+
 int vx_amax(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, float* amax_out,
             void* stream) {
   using namespace vx;
   if (x_dtype != VX_F32 && x_dtype != VX_BF16) return fail(-1, "x_dtype must be VX_F32 or VX_BF16");
   if (!amax_out) return fail(-1, "amax_out must not be NULL");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  VX_CUDA_OK(cudaMemsetAsync(amax_out, 0, sizeof(float), st));
-  if (M <= 0 || K <= 0) return 0;
+  if (M <= 0 || K <= 0) {
+    VX_CUDA_OK(cudaMemsetAsync(amax_out, 0, sizeof(float), st));
+    return 0;
+  }
   const int64_t esz = x_dtype == VX_BF16 ? 2 : 4;
   if (!x || K % 8 != 0 || !aligned16(x) || (ldx * esz) % 16 != 0 || ldx < K)
     return fail(-1, "x must be 16-byte aligned rows with K %% 8 == 0");
-  const int64_t threads = M * (K >> 3);
-  int grid = static_cast<int>((threads + 255) / 256);
-  if (grid > 148 * 8) grid = 148 * 8;
-  if (x_dtype == VX_BF16)
-    amax_kernel<<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), M, K, ldx, amax_out);
-  else
-    amax_kernel<<<grid, 256, 0, st>>>(static_cast<const float*>(x), M, K, ldx, amax_out);
-  VX_CUDA_OK(cudaGetLastError());
+  const bool dense = ldx == K || M == 1;
+  const int64_t rows = dense ? 1 : M, row_vecs = (dense ? M * K : K) * esz / 16, vecs = rows * row_vecs;
+  // one block up to 128 KB: eight vectors per thread, about the latency of the launch it saves
+  const bool one = vecs <= 8192;
+  auto go = [&](auto* kernel, const auto* xt, int grid, int threads) {
+    return launch_dependent(kernel, dim3(grid), dim3(threads), 0, st, xt, rows, row_vecs, ldx, amax_out);
+  };
+  if (!one) VX_CUDA_OK(cudaMemsetAsync(amax_out, 0, sizeof(float), st));
+  int64_t blocks = (vecs + 1023) / 1024;
+  if (blocks > sm_count() * 8) blocks = sm_count() * 8;
+  const int grid = one ? 1 : static_cast<int>(blocks), threads = one ? 1024 : 256;
+  if (x_dtype == VX_BF16) {
+    const auto* xt = static_cast<const __nv_bfloat16*>(x);
+    VX_CUDA_OK(one ? go(amax_kernel<__nv_bfloat16, true>, xt, grid, threads) : go(amax_kernel<__nv_bfloat16, false>, xt, grid, threads));
+  } else {
+    const auto* xt = static_cast<const float*>(x);
+    VX_CUDA_OK(one ? go(amax_kernel<float, true>, xt, grid, threads) : go(amax_kernel<float, false>, xt, grid, threads));
+  }
   return 0;
 }
 
-int vx_sf_from_natural(int fmt, const void* scales, int64_t R, int64_t K, void* scales_sf,
-                       void* stream) {
+int vx_sf_from_natural_pair(int fmt_a, const void* scales_a, int64_t Ra, void* sf_a, int fmt_b, const void* scales_b,
+                            int64_t Rb, void* sf_b, int64_t K, void* stream) {
   using namespace vx;
-  if (!fmt_has_sf(fmt)) return fail(-1, "format %d has no SF-atom layout", fmt);
-  if (R <= 0 || K <= 0) return 0;
-  if (!scales || !scales_sf || (reinterpret_cast<uintptr_t>(scales_sf) & 15))
-    return fail(-1, "scales / scales_sf must be non-NULL, scales_sf 16-byte aligned");
-  const int blk = fmt_block(fmt);
-  if (K % blk != 0) return fail(-1, "K must be a multiple of %d", blk);
-  if (fmt == VX_FMT_BLK16_A && (R & 1)) return fail(-1, "BLK16_A needs an even row count");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  VX_CUDA_OK(cudaMemsetAsync(scales_sf, 0, static_cast<size_t>(vx_sf_bytes(fmt, R, K)), st));
-  const int64_t nkb = K / blk;
-  const int64_t total = R * ((nkb + 3) / 4);
-  int grid = static_cast<int>((total + 255) / 256);
-  if (grid > 148 * 16) grid = 148 * 16;
-  sf_relayout_kernel<<<grid, 256, 0, st>>>(fmt, static_cast<const uint8_t*>(scales), R, nkb,
-                                           static_cast<uint8_t*>(scales_sf), sf_kgroups(fmt, K));
-  VX_CUDA_OK(cudaGetLastError());
+  if (K <= 0) return 0;
+  RelayoutSide side[2] = {};
+  const int fmts[2] = {fmt_a, fmt_b};
+  const void* const src[2] = {scales_a, scales_b};
+  void* const dst[2] = {sf_a, sf_b};
+  const int64_t rows[2] = {Ra, Rb};
+  for (int i = 0; i < 2; ++i) {
+    if (!fmt_has_sf(fmts[i])) return fail(-1, "format %d has no SF-atom layout", fmts[i]);
+    if (rows[i] <= 0) continue;
+    if (!src[i] || !dst[i] || (reinterpret_cast<uintptr_t>(dst[i]) & 15))
+      return fail(-1, "scales / scales_sf must be non-NULL, scales_sf 16-byte aligned");
+    if (fmt_block(fmts[i]) != fmt_block(fmt_a)) return fail(-1, "both operands need the same scale block");
+    if (K % fmt_block(fmts[i]) != 0) return fail(-1, "K must be a multiple of %d", fmt_block(fmts[i]));
+    if (fmts[i] == VX_FMT_BLK16_A && (rows[i] & 1)) return fail(-1, "BLK16_A needs an even row count");
+    side[i] = {static_cast<const uint8_t*>(src[i]), static_cast<uint8_t*>(dst[i]), rows[i], vx_sf_bytes(fmts[i], rows[i], K) / 4, fmts[i]};
+  }
+  const int64_t words = side[0].words + side[1].words;
+  if (words == 0) return 0;
+  int64_t grid = (words + 255) / 256;
+  if (grid > 148 * 8) grid = 148 * 8;
+  VX_CUDA_OK(launch_dependent(sf_relayout_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, static_cast<cudaStream_t>(stream), side[0],
+                              side[1], static_cast<int>(K / fmt_block(fmt_a)), static_cast<int>(sf_kgroups(fmt_a, K))));
   return 0;
+}
+
+int vx_sf_from_natural(int fmt, const void* scales, int64_t R, int64_t K, void* scales_sf, void* stream) {
+  return vx_sf_from_natural_pair(fmt, scales, R, scales_sf, fmt, nullptr, 0, nullptr, K, stream);
 }
 
 }  // extern "C"

@@ -1,0 +1,208 @@
+// Top-k of the CTC log-probabilities through bf16 logits that never leave the L2 cache.
+//
+// The prefix beam search takes torch.topk(log_softmax(ctc_lo(x)), k).  The head's GEMM writes the bf16 logits of a block
+// of rows (vx_ctc_topk_rows, about 60 MB: half of the L2) into a scratch buffer, and the kernel below reads them back from
+// L2, one warp per row: log-sum-exp and the k largest values in two passes over the row.  Against the route without
+// logits (two launches of the head, the second with a candidate test in its epilogue, a threshold kernel, a finish
+// kernel and a host check for overflowed candidate lists) that is half the matrix work and no synchronisation.
+
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "vx_common.cuh"
+#include "vx_ptx.cuh"
+#include "vx_quant_math.cuh"
+
+namespace vx {
+namespace {
+
+constexpr int TK_WARPS = 8;
+constexpr int TK_CAND = 128;  // candidate list of a row; more (many equal logits): exact rescans instead
+
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// order-preserving bits of a bf16 value held as fp32, lowest column first among equals
+__device__ __forceinline__ unsigned long long topk_key(float z, int col) {
+  const uint32_t x = __float_as_uint(z);
+  const uint32_t u = x ^ (static_cast<uint32_t>(static_cast<int32_t>(x) >> 31) | 0x80000000u);
+  return (static_cast<unsigned long long>(u) << 32) | (0xffffffffu - static_cast<uint32_t>(col));
+}
+__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w > v ? w : v;
+  }
+  return v;
+}
+__device__ __forceinline__ void unpack8(const uint4& u, float (&z)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    z[2 * i] = __uint_as_float(w[i] << 16);
+    z[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+
+// One warp per row.  Pass 1: every lane's running (max, sum of 2^((z - max) log2 e)) over its 16-byte pieces, merged into the
+// row's log-sum-exp.  The k-th largest of the 32 lane maxima is a threshold that at least k logits reach and each of the k
+// largest does; pass 2 (the row again, from L1) collects what reaches it -- a few more than k -- and the k largest of the
+// list are taken in order.  Bound by instruction issue: about 900 warp instructions per row of 5,538.
+__global__ void __launch_bounds__(TK_WARPS * 32) topk_rows_kernel(const __nv_bfloat16* logits, int64_t ld, int N, int M,
+                                                                  int k, float* logp, int64_t* ids) {
+  __shared__ unsigned long long cand_s[TK_WARPS][TK_CAND];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int row = static_cast<int>(blockIdx.x) * TK_WARPS + w;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (row >= M) return;
+  constexpr float L2E = 1.4426950408889634f;
+  const uint4* const src = reinterpret_cast<const uint4*>(logits + static_cast<int64_t>(row) * ld);
+  const int pieces = (N + 7) >> 3;
+  auto load = [&](int c, float (&z)[8]) {
+    unpack8(src[c], z);
+    if (8 * c + 8 > N) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (8 * c + i >= N) z[i] = -INFINITY;
+    }
+  };
+  float m = -INFINITY, s = 0.0f;
+#pragma unroll 4
+  for (int c = lane; c < pieces; c += 32) {
+    float z[8];
+    load(c, z);
+    float cm = max3(z[0], z[1], z[2]);
+    cm = max3(cm, z[3], z[4]);
+    cm = max3(cm, z[5], z[6]);
+    cm = max3(cm, z[7], m);
+    if (cm > m) {
+      s *= ex2_approx((m - cm) * L2E);  // m = -inf: 0
+      m = cm;
+    }
+    const float nb = -m * L2E;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += ex2_approx(fmaf(z[i], L2E, nb));
+  }
+  float rm = m;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) rm = fmaxf(rm, __shfl_xor_sync(0xffffffffu, rm, o));
+  float rs = m > -INFINITY ? s * ex2_approx((m - rm) * L2E) : 0.0f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);
+  const float lse = rm + logf(rs);
+  // threshold: the lane maximum of rank k - 1
+  int rank = 0;
+#pragma unroll
+  for (int l = 0; l < 32; ++l) {
+    const float o = __shfl_sync(0xffffffffu, m, l);
+    rank += (o > m || (o == m && l < lane)) ? 1 : 0;
+  }
+  const uint32_t who = __ballot_sync(0xffffffffu, rank == k - 1);
+  const float thr = __shfl_sync(0xffffffffu, m, __ffs(who) - 1);
+
+  int n = 0;  // candidates of the row
+  for (int c0 = 0; c0 < pieces; c0 += 32) {
+    const int c = c0 + lane;
+    float z[8];
+    float cm = -INFINITY;
+    if (c < pieces) {
+      load(c, z);
+      cm = max3(z[0], z[1], z[2]);
+      cm = max3(cm, z[3], z[4]);
+      cm = max3(cm, z[5], z[6]);
+      cm = fmaxf(cm, z[7]);
+    }
+    if (__any_sync(0xffffffffu, c < pieces && cm >= thr)) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const bool hit = c < pieces && 8 * c + i < N && z[i] >= thr;
+        const uint32_t b = __ballot_sync(0xffffffffu, hit);
+        const int at = n + __popc(b & ((1u << lane) - 1u));
+        if (hit && at < TK_CAND) cand_s[w][at] = topk_key(z[i], 8 * c + i);
+        n += __popc(b);
+      }
+    }
+  }
+  __syncwarp();
+  unsigned long long mine[TK_CAND / 32];
+#pragma unroll
+  for (int j = 0; j < TK_CAND / 32; ++j) mine[j] = j * 32 + lane < n ? cand_s[w][j * 32 + lane] : 0ull;
+  unsigned long long last = ~0ull;
+  for (int j = 0; j < k; ++j) {
+    unsigned long long best = 0;
+    if (n <= TK_CAND) {
+#pragma unroll
+      for (int t = 0; t < TK_CAND / 32; ++t)
+        if (mine[t] < last && mine[t] > best) best = mine[t];
+    } else {
+      for (int c = lane; c < pieces; c += 32) {
+        float z[8];
+        load(c, z);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const unsigned long long e = topk_key(z[i], 8 * c + i);
+          if (8 * c + i < N && e < last && e > best) best = e;
+        }
+      }
+    }
+    best = warp_max_u64(best);
+    last = best;
+    if (lane == 0) {
+      const uint32_t u = static_cast<uint32_t>(best >> 32);
+      const float z = __uint_as_float((u & 0x80000000u) ? (u ^ 0x80000000u) : ~u);
+      ids[static_cast<int64_t>(row) * k + j] = best ? static_cast<int64_t>(0xffffffffu - static_cast<uint32_t>(best)) : -1;
+      logp[static_cast<int64_t>(row) * k + j] = best ? z - lse : -INFINITY;
+    }
+  }
+}
+
+}  // namespace
+}  // namespace vx
+
+extern "C" {
+
+// Rows per block: about 60 MB of bf16 logits, whole 128-row tiles.
+int64_t vx_ctc_topk_rows(int64_t N) {
+  if (N <= 0) return 0;
+  const int64_t tile_bytes = (N + 7) / 8 * 8 * 2 * 128;
+  const int64_t tiles = (60ll << 20) / tile_bytes;
+  return 128 * (tiles < 1 ? 1 : tiles);
+}
+
+int vx_ctc_topk(const vx_gemm_desc* desc, int k, void* logits, int64_t rows, float* logp, int64_t* ids, void* stream) {
+  using namespace vx;
+  if (!desc) return fail(-1, "desc must not be NULL");
+  if (desc->struct_size != static_cast<int32_t>(sizeof(vx_gemm_desc)))
+    return fail(-1, "vx_gemm_desc.struct_size=%d, expected %d", desc->struct_size, (int)sizeof(vx_gemm_desc));
+  const int64_t M = desc->M, N = desc->N, K = desc->K;
+  if (M < 0 || N <= 0 || N > 0x7fffffffll) return fail(-1, "bad shape");
+  if (k <= 0 || k > 16 || k > N) return fail(-1, "k must be in 1..16 and at most N");
+  if (desc->fmt == VX_FMT_FP8_1X128 || desc->fmt == VX_FMT_BLK16_A) return fail(-1, "vx_ctc_topk runs on ROWSCALE, MX32 and NV16");
+  if (M == 0) return 0;
+  if (!logits || !logp || !ids || !aligned16(logits)) return fail(-1, "logits (16-byte aligned), logp and ids must not be NULL");
+  if (rows <= 0 || (rows < M && rows % 128 != 0)) return fail(-1, "rows must cover M or be a multiple of 128");
+  const int64_t ld = (N + 7) / 8 * 8;
+  for (int64_t r0 = 0; r0 < M; r0 += rows) {
+    const int64_t m = M - r0 < rows ? M - r0 : rows;
+    vx_gemm_desc d = *desc;
+    d.M = m;
+    d.a_codes = static_cast<const uint8_t*>(desc->a_codes) + r0 * desc->lda;
+    d.a_scales = static_cast<const uint8_t*>(desc->a_scales) +
+                 (desc->fmt == VX_FMT_ROWSCALE ? r0 : r0 / 128 * vx_sf_kgroups(desc->fmt, K) * 512);
+    d.epilogue = desc->bias ? VX_EPI_BIAS : VX_EPI_NONE;
+    d.out_dtype = VX_BF16; d.out = logits; d.ldo = ld;
+    const int rc = vx_bsgemm(&d, stream);
+    if (rc) return rc;
+    VX_CUDA_OK(launch_dependent(topk_rows_kernel, dim3(static_cast<unsigned>((m + TK_WARPS - 1) / TK_WARPS)), dim3(TK_WARPS * 32), 0,
+                                static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(logits), ld, static_cast<int>(N),
+                                static_cast<int>(m), k, logp + r0 * k, ids + r0 * k));
+  }
+  return 0;
+}
+
+}  // extern "C"
