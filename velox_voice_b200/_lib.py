@@ -30,6 +30,8 @@ GEMM_STREAM_B = 2
 GEMM_WIDE_TILES = 4
 GEMM_NARROW_TILES = 8
 GEMM_OUT_HEADS = 16
+GEMM_POS_F32 = 64
+GEMM_CONST_B = 128
 
 EXPORTS = (
     "vx_abi_version",
@@ -61,6 +63,10 @@ EXPORTS = (
     "vx_bsgemm_residual_ln_supported",
     "vx_bsgemm_residual_ln",
     "vx_bsgemm_residual_ln2",
+    "vx_sf_from_natural_pair",
+    "vx_rowscale_linear",
+    "vx_ctc_topk_rows",
+    "vx_ctc_topk",
 )
 
 
@@ -157,6 +163,14 @@ def load(build_if_missing: bool = True) -> C.CDLL:
         lib.vx_amax.argtypes = [vp, i32, i64, i64, i64, vp, vp]
         lib.vx_sf_from_natural.restype = i32
         lib.vx_sf_from_natural.argtypes = [i32, vp, i64, i64, vp, vp]
+        lib.vx_sf_from_natural_pair.restype = i32
+        lib.vx_sf_from_natural_pair.argtypes = [i32, vp, i64, vp, i32, vp, i64, vp, i64, vp]
+        lib.vx_rowscale_linear.restype = i32
+        lib.vx_rowscale_linear.argtypes = [vp, i32, i64, i64, i64, vp, i64, vp, i64, vp, vp, vp, i64, vp]
+        lib.vx_ctc_topk_rows.restype = i64
+        lib.vx_ctc_topk_rows.argtypes = [i64]
+        lib.vx_ctc_topk.restype = i32
+        lib.vx_ctc_topk.argtypes = [C.POINTER(GemmDesc), i32, vp, i64, vp, vp, vp]
         lib.vx_bsgemm.restype = i32
         lib.vx_bsgemm.argtypes = [C.POINTER(GemmDesc), vp]
         lib.vx_blkscale_gemm_noalloc.restype = i32
@@ -199,6 +213,35 @@ def load(build_if_missing: bool = True) -> C.CDLL:
             raise RuntimeError("libvelox_b200.so: ABI version mismatch")
         _lib = lib
         return lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/vx_host.cpp): the extension module ``_vx_host`` on the loaded library."""
+    global _host
+    if _host is None:
+        lib = load()
+        with _lock:
+            if _host is None:
+                import importlib.util
+
+                from .ops import Quantized
+
+                path = _build.HOST_PATH
+                if not _build.host_is_current():
+                    try:
+                        _build.build_host()
+                    except Exception as e:  # no compiler on this machine: use the shipped module if any
+                        if not os.path.exists(path):
+                            raise RuntimeError(f"{path} is missing and cannot be built: {e}") from e
+                spec = importlib.util.spec_from_file_location("_vx_host", path)
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+                mod.init(lib._name, VeloxError, Quantized)
+                _host = mod
+    return _host
 
 
 class VeloxError(RuntimeError):

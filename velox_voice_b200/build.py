@@ -18,7 +18,11 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libvelox_b200.so")
 STAMP = os.path.join(LIB_DIR, "libvelox_b200.stamp")
-SOURCES = ("vx_api.cu", "vx_quant.cu", "vx_gemm.cu", "vx_noalloc.cu", "vx_pack.cu", "vx_mel.cu", "vx_attn.cu", "vx_gemm_ln.cu")
+SOURCES = ("vx_api.cu", "vx_quant.cu", "vx_gemm.cu", "vx_noalloc.cu", "vx_pack.cu", "vx_mel.cu", "vx_attn.cu", "vx_gemm_ln.cu", "vx_topk.cu")
+# native host path of the Python operators: a CPython extension against torch's headers (g++, no device code)
+HOST_SOURCE = "vx_host.cpp"
+HOST_PATH = os.path.join(LIB_DIR, "_vx_host.so")
+HOST_STAMP = os.path.join(LIB_DIR, "_vx_host.stamp")
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
@@ -106,8 +110,47 @@ def link(objects, out_path: str) -> str:
     return out_path
 
 
+def _host_digest() -> str:
+    import torch
+
+    with open(os.path.join(HERE, "..", "include", "velox_b200.h")) as f:
+        return _file_digest(HOST_SOURCE, f.read() + torch.__version__ + sys.version)
+
+
+def host_is_current() -> bool:
+    if not (os.path.exists(HOST_PATH) and os.path.exists(HOST_STAMP)):
+        return False
+    with open(HOST_STAMP) as f:
+        return f.read().strip() == _host_digest()
+
+
+def build_host(force: bool = False) -> str:
+    """Compile the host extension if its source, the C ABI, torch or Python changed."""
+    if not force and host_is_current():
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+
+    inc = os.path.join(os.path.dirname(torch.__file__), "include")
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc")), "include")
+    os.makedirs(LIB_DIR, exist_ok=True)
+    cmd = ["g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"), "-isystem", cuda,
+           "-isystem", sysconfig.get_paths()["include"], os.path.join(CSRC, HOST_SOURCE), "-o", HOST_PATH,
+           "-L" + lib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-ldl"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed on {HOST_SOURCE} ({res.returncode}):\n{res.stdout}\n{res.stderr}")
+    with open(HOST_STAMP, "w") as f:
+        f.write(_host_digest())
+    return HOST_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile the library if the sources changed; returns the path of the shared object."""
+    build_host(force)
     if not force and is_current():
         return LIB_PATH
     objects = compile_objects(force=force, verbose=verbose)

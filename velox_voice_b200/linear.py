@@ -17,6 +17,7 @@ import torch
 from torch import nn
 
 from . import ops
+from ._lib import GEMM_CONST_B
 from .ops import (
     EPI_BIAS,
     EPI_BIAS_GLU,
@@ -86,6 +87,10 @@ class PackedLinear:
             epi = EPI_BIAS
         else:
             epi = EPI_NONE
+        r = ops._host().bsgemm(a, self.q, epi, self.bias, residual, alpha, out_dtype, out,
+                               None if out_fmt is None else ops._fmt(out_fmt), out_amax, False, GEMM_CONST_B)
+        if r is not None:
+            return r
         return ops.bsgemm(a, self.q, epilogue=epi, bias=self.bias, residual=residual, alpha=alpha,
                           out_dtype=out_dtype, out=out, out_fmt=out_fmt, out_amax=out_amax)
 
@@ -101,6 +106,9 @@ class PackedLinear:
         """``x = alpha (a W^T + bias) + residual`` and ``ln_quantize(x, gamma, beta, eps)`` in one launch:
         ``(x, q)`` with the bits of the two separate calls.  With ``gamma2`` / ``beta2``: ``(LN(x), q)`` with
         ``q = ln_quantize(LN(x), gamma2, beta2)`` -- the end of a block (``ops.ln2_quantize``)."""
+        r = ops._host().residual_ln(a, self.q, self.bias, residual, gamma, beta, eps, alpha, out, gamma2, beta2, GEMM_CONST_B)
+        if r is not None:
+            return r
         return ops.bsgemm_residual_ln(a, self.q, bias=self.bias, residual=residual, gamma=gamma, beta=beta,
                                       eps=eps, alpha=alpha, out=out, gamma2=gamma2, beta2=beta2)
 
@@ -156,13 +164,16 @@ class DenseLinear(nn.Linear):
     def forward(self, x):
         precision = getattr(self, "precision", "fp32")
         if precision in ("nvfp4", "mxfp4"):
-            orig_shape = x.shape
-            x2 = x.reshape(-1, orig_shape[-1])
             if self._wq is None:
                 self._prequantize_weight(precision)
+            # quantize + one GEMM with the scales and the bias in its epilogue (fp32 out)
+            r = ops._host().rowscale_linear(x, self._wq, self._ws, self._parameters["bias"])
+            if r is not None:
+                return r
+            orig_shape = x.shape
+            x2 = x.reshape(-1, orig_shape[-1])
             if x2.dtype not in (torch.float32, torch.bfloat16):
                 x2 = x2.float()
-            # quantize + one GEMM with the scales and the bias in its epilogue (fp32 out)
             out = ops.rowscale_linear(x2, self._wq, self._ws, None if self.bias is None else self.bias.detach())
             return out.view(*orig_shape[:-1], self.out_features)
         return torch.nn.functional.linear(x, self.weight, self.bias)
@@ -186,6 +197,9 @@ class Nvfp4Linear(nn.Module):
             self.bias = None
 
     def forward(self, x):
+        r = ops._host().rowscale_linear(x, self.weight_q, self.weight_s, self.bias)
+        if r is not None:
+            return r
         orig_shape = x.shape
         x = x.reshape(-1, self.in_features)
         out = ops.rowscale_linear(x, self.weight_q, self.weight_s, self.bias)

@@ -53,6 +53,16 @@ _BLOCK = {FMT_BLK16_A: 16, FMT_BLK16_B: 16, FMT_NV16: 16, FMT_MX32: 32, FMT_FP8_
 
 
 _launches = 0
+_native = None  # the native host path (csrc/vx_host.cpp), loaded on first use
+
+
+def _host():
+    """The native host path: one C++ call per operator for ordinary arguments; its functions return None for anything
+    else, and the Python code below them then copies what has to be copied and words the errors."""
+    global _native
+    if _native is None:
+        _native = _lib.host()
+    return _native
 
 
 def _count(n: int = 1) -> None:
@@ -62,12 +72,14 @@ def _count(n: int = 1) -> None:
 
 def launch_count() -> int:
     """Kernels of this library launched since :func:`reset_launch_count` (host-side count)."""
-    return _launches
+    return _launches + (_native.launches() if _native is not None else 0)
 
 
 def reset_launch_count() -> None:
     global _launches
     _launches = 0
+    if _native is not None:
+        _native.reset_launches()
 
 
 def _fmt(fmt) -> int:
@@ -178,6 +190,9 @@ def quantize(
 ) -> Quantized:
     """Quantize + pack the rows of ``x`` [M, K] (f32 or bf16) in format ``fmt``."""
     fmt = _fmt(fmt)
+    q = (_native or _host()).quantize(x, fmt, natural, sf, amax_t)
+    if q is not None:
+        return q
     _require_cuda(x, "x")
     x = _rows2d(x, "x")
     M, K = x.shape
@@ -209,6 +224,10 @@ def ln_quantize(
 ):
     """LayerNorm(x) quantized in one pass.  Returns ``Quantized`` (and ``y`` if ``y_dtype``)."""
     fmt = _fmt(fmt)
+    if y_dtype is None:
+        q = (_native or _host()).ln_quantize(x, gamma, beta, eps, fmt, natural, sf, amax_t)
+        if q is not None:
+            return q
     _require_cuda(x, "x")
     x = _rows2d(x, "x")
     M, K = x.shape
@@ -371,6 +390,11 @@ def bsgemm(
     ``tiles`` overrides the FP4 tile shape the library would pick ("wide" 128 x 256, one
     accumulator; "narrow" 128 x 128, two accumulators); results do not depend on it.
     """
+    if not (direct_store or stream_b or tiles):
+        r = (_native or _host()).bsgemm(a, b, epilogue, bias, residual, alpha, out_dtype, out,
+                                        None if out_fmt is None else _fmt(out_fmt), out_amax, out_natural, 0)
+        if r is not None:
+            return r
     d, keep = _gemm_desc(a, b, bias)
     M, N, K = a.rows, b.rows, a.k
     dev = a.codes.device
@@ -440,6 +464,9 @@ def bsgemm_residual_ln(a: Quantized, b: Quantized, *, bias: Optional[torch.Tenso
     With ``gamma2`` / ``beta2`` (the end of a Conformer block): ``out`` receives ``y = LN(x; gamma, beta)``
     instead of x and ``q = ln_quantize(y, gamma2, beta2)`` -- the bits of the GEMM followed by
     ``ln2_quantize(x, gamma, beta, gamma2, beta2, eps, MX32, y=x)``.  Returns ``(y, q)``."""
+    r = (_native or _host()).residual_ln(a, b, bias, residual, gamma, beta, eps, alpha, out, gamma2, beta2, 0)
+    if r is not None:
+        return r
     d, keep = _gemm_desc(a, b, bias)
     M, N = a.rows, b.rows
     dev = a.codes.device
@@ -528,50 +555,32 @@ def bsgemm_argmax(a: Quantized, b: Quantized, bias: Optional[torch.Tensor] = Non
 
 
 def bsgemm_topk(a: Quantized, b: Quantized, bias: Optional[torch.Tensor] = None, k: int = 5, *, capacity: int = 64):
-    """``torch.topk(log_softmax(A . B^T + bias), k)`` of the bf16-rounded logits without writing the [M, N] matrix:
+    """``torch.topk(log_softmax(A . B^T + bias), k)`` of the bf16-rounded logits without a [M, N] matrix in HBM:
     the stream the reference's prefix beam search takes (``veloxvoice/stream/rescore.py:252-262``,
     ``cuda_ops.py:836-893``).  Returns ``(logp f32 [M, k], ids int64 [M, k])``, largest first, equal logits by
-    ascending column.  Two launches of the GEMM (arg-max + log-sum-exp partials, then the candidate pass against
-    the k-th largest 64-column-group maximum of each row) and two small kernels; rows whose candidate list
-    overflowed ``capacity`` (many equal bf16 logits) are redone from explicit logits."""
+    ascending column.  Per block of rows (about 60 MB of logits, which stay in L2) one launch of the GEMM and one
+    selection kernel (``vx_ctc_topk``); any number of equal logits is handled there, so ``capacity`` (entries per
+    row of the candidate list of an earlier route) is accepted and unused."""
     if a.fmt == FMT_FP8_1X128:
         raise ValueError("bsgemm_topk runs on the FP4 formats")
     if not 1 <= k <= 16:
         raise ValueError("k must be in 1..16")
+    r = (_native or _host()).topk(a, b, bias, k)
+    if r is not None:
+        return r
     d, keep = _gemm_desc(a, b, bias)
     M, N = a.rows, b.rows
-    dev = a.codes.device
     lib = _lib.load()
     nparts = int(lib.vx_ctc_lse_parts(N))
     if k > nparts:
         raise ValueError(f"k = {k} exceeds the number of 64-column groups ({nparts})")
-    keys = torch.empty((M,), dtype=torch.int64, device=dev)
-    parts = torch.empty((nparts, M, 2), dtype=torch.float32, device=dev)
-    d.epilogue = EPI_BIAS_ARGMAX
-    d.out_dtype, d.out, d.ldo = DT_F32, keys.data_ptr(), 1
-    d.lse_partials = parts.data_ptr()
-    _lib.check(lib.vx_bsgemm(C.byref(d), _stream()), "vx_bsgemm")
-    thr = torch.empty((M,), dtype=torch.float32, device=dev)
-    _lib.check(lib.vx_ctc_topk_threshold(parts.data_ptr(), N, M, k, thr.data_ptr(), _stream()), "vx_ctc_topk_threshold")
-    cand = torch.empty((M, capacity), dtype=torch.int64, device=dev)
-    cnt = torch.zeros((M,), dtype=torch.int32, device=dev)
-    over = torch.zeros((1,), dtype=torch.int32, device=dev)
-    d.topk_threshold, d.topk_candidates, d.topk_count, d.topk_capacity = thr.data_ptr(), cand.data_ptr(), cnt.data_ptr(), capacity
-    _lib.check(lib.vx_bsgemm(C.byref(d), _stream()), "vx_bsgemm")
-    ids = torch.empty((M, k), dtype=torch.int32, device=dev)
+    dev = a.codes.device
+    rows = min(int(lib.vx_ctc_topk_rows(N)), max(M, 1))
+    logits = torch.empty((rows, (N + 7) // 8 * 8), dtype=torch.bfloat16, device=dev)
     logp = torch.empty((M, k), dtype=torch.float32, device=dev)
-    _lib.check(lib.vx_ctc_topk_finish(cand.data_ptr(), cnt.data_ptr(), capacity, parts.data_ptr(), N, M, k, ids.data_ptr(),
-                                      logp.data_ptr(), over.data_ptr(), _stream()), "vx_ctc_topk_finish")
-    _count(4)
-    ids = ids.long()
-    if int(over.item()):
-        # rare: some rows hold more than `capacity` logits at or above their threshold (many equal bf16 values);
-        # those rows are redone from explicit logits
-        rows = (ids[:, 0] < 0).nonzero()[:, 0]
-        z = bsgemm(a, b, epilogue=EPI_BIAS if bias is not None else EPI_NONE, bias=bias, out_dtype=torch.bfloat16)
-        v, i = torch.topk(torch.log_softmax(z[rows].float(), dim=-1), k, dim=-1)
-        del z
-        logp[rows], ids[rows] = v, i
+    ids = torch.empty((M, k), dtype=torch.int64, device=dev)
+    _lib.check(lib.vx_ctc_topk(C.byref(d), k, logits.data_ptr(), rows, logp.data_ptr(), ids.data_ptr(), _stream()), "vx_ctc_topk")
+    _count(2 * -(-M // rows))
     del keep
     return logp, ids
 
@@ -611,6 +620,10 @@ def relpos_attention(q2: torch.Tensor, k2: torch.Tensor, v2: torch.Tensor, kv_le
     ``scaled_dot_product_attention(q2, k2, v2, scale=1.0)[..., :dk].transpose(0, 1).reshape(T, h * dk)``
     of ``veloxvoice/models/wenet/torch_conformer.py:514-519`` in one launch (``vx_relpos_attention``);
     keys at and beyond ``kv_len`` are masked (a padded span)."""
+    if out is None:
+        r = (_native or _host()).relpos_attention(q2, k2, v2, kv_len)
+        if r is not None:
+            return r
     for t, n in ((q2, "q2"), (k2, "k2"), (v2, "v2")):
         _require_cuda(t, n)
         if t.dtype != torch.bfloat16 or t.dim() != 3 or t.shape != q2.shape or t.device != q2.device:
@@ -637,6 +650,9 @@ def bsgemm_qkv_pack(a: Quantized, w_qkv: Quantized, bias: Optional[torch.Tensor]
     bf16 projection, without the [T, 3d] intermediate).  Returns bf16 [3, h, T, 2 dk]:
     ``packed[0]`` = q2, ``packed[1]`` = k2 (second half of every head row NOT written: it belongs
     to ``bsgemm_heads(pos, lp, out=packed[1], col_off=dk)``), ``packed[2]`` = v2."""
+    r = (_native or _host()).qkv_pack_gemm(a, w_qkv, bias, pos_u, pos_v, scale, packed)
+    if r is not None:
+        return r
     d, keep = _gemm_desc(a, w_qkv, bias)
     if a.fmt == FMT_ROWSCALE:
         raise ValueError("the fused fold pack runs in the block-scaled formats and FP8, not per-row scales")
@@ -671,6 +687,9 @@ def bsgemm_heads(a: Quantized, w: Quantized, bias: Optional[torch.Tensor], out: 
     """``A . W^T (+ bias)`` written head-major: ``out`` bf16 [h, M, width], result column n goes to
     ``out[n // dk, m, col_off + n % dk]`` with dk = N / h.  With ``out = packed[1]`` and
     ``col_off = dk`` this puts lp(pos_emb) where the attention fold pack wants it."""
+    r = (_native or _host()).heads_gemm(a, w, bias, out, col_off)
+    if r is not None:
+        return r
     d, keep = _gemm_desc(a, w, bias)
     _require_cuda(out, "out")
     if out.dim() != 3:
@@ -801,6 +820,9 @@ def dgx_mxfp4_blkscale_gemm(
 
     scale_a: ue8m0 u8 [K/16][M/2] (row pairs); scale_b: ue8m0 u8 [K/16][N].
     """
+    r = (_native or _host()).blkscale_gemm(pack_a, pack_b, scale_a, scale_b)
+    if r is not None:
+        return r
     _require_cuda(pack_a, "pack_a")
     pa, pb = _rows2d(pack_a, "pack_a"), _rows2d(pack_b, "pack_b")
     M, N, K = pa.shape[0], pb.shape[0], pa.shape[1] * 2
@@ -835,6 +857,9 @@ def rowscale_linear(x2d: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, bias:
     column scales and adds the bias.  The reference's ``DenseLinear.forward``
     (``veloxvoice/models/wenet/torch_conformer.py:251-266``) spends a pad copy, a cast, the
     quantizer, the GEMM, a slice and a bias add on the same result."""
+    r = (_native or _host()).rowscale_linear(x2d, wq, ws, bias)
+    if r is not None:
+        return r
     a = quantize(x2d, FMT_ROWSCALE, sf=False)
     b = _as_quantized_rowscale(wq, ws)
     if bias is None:
@@ -1015,6 +1040,9 @@ def power_mel_log_tf32(spec, mel, cmvn_mean=None, cmvn_istd=None):
     the tensor cores, fp32 accumulation), for any number of frames.  spec complex64 [T, F]
     (``torch.fft.rfft`` output), mel f32 [M, F], cmvn_mean / cmvn_istd f32 [M] or None -> f32 [T, M].
     Raises when the filterbank does not fit the kernel (``vx_power_mel_log_supported``)."""
+    r = (_native or _host()).power_mel_log(spec, mel, cmvn_mean, cmvn_istd)
+    if r is not None:
+        return r
     _require_cuda(spec, "spec")
     _require_cuda(mel, "mel")
     if spec.dim() != 2 or mel.dim() != 2 or spec.shape[1] != mel.shape[1]:
@@ -1052,6 +1080,10 @@ def power_mel_log(spec, mel, cmvn_mean, cmvn_istd):
     for a filterbank the kernel does not take, the fp32 formula the reference runs through cuBLAS
     (``cuda_ops.py:138-148``), so short inputs stay fp32-grade as its tests expect
     (``tests/kernels/test_power_mel_log.py:80-88,180-203``)."""
+    if isinstance(spec, torch.Tensor) and spec.dim() == 2 and spec.shape[0] >= 64:
+        r = (_native or _host()).power_mel_log(spec, mel, cmvn_mean, cmvn_istd)
+        if r is not None:
+            return r
     _require_cuda(spec, "spec")
     _require_cuda(mel, "mel")
     if spec.dim() == 2 and mel.dim() == 2 and spec.shape[0] >= 64 and _lib.load().vx_power_mel_log_supported(spec.shape[1], mel.shape[0]):

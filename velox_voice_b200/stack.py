@@ -13,7 +13,8 @@ convolution and its norm/activation are NOT linear layers and are outside this l
 stack passes the value projection straight to ``lo`` and the GLU output straight to ``pw2``,
 so it measures and validates every linear of the encoder with the real operand shapes.
 
-Kernel sequence per block (13 launches; the reference issues >= 4 per linear):
+Kernel sequence per block (13 launches, issued by the native host path ``csrc/vx_host.cpp``; the reference issues >= 4
+per linear):
 ``GEMM(bias, swish, FP4 out) -> GEMM(bias, 0.5 residual)`` for each FFN (the second one behind
 its ``ln_quant``), ``ln_quant -> GEMM(bias) [qkv] -> quant -> GEMM(bias, residual) [lo]``,
 ``GEMM [lp]``, ``ln_quant -> GEMM(bias, GLU) -> quant -> GEMM(bias, residual)``, and one
@@ -131,6 +132,7 @@ class ConformerLinearStack:
                 self.ln[b + n] = (weights[b + n + ".g"].to(dev).float(), weights[b + n + ".b"].to(dev).float())
         self.ln["after"] = (weights["after.g"].to(dev).float(), weights["after.b"].to(dev).float())
         pack("ctc", "ctc.w", "ctc.b")
+        self._plan = None
         # NV16 needs a per-tensor amax for every activation it quantizes: calibrated once
         self.amax: Dict[str, torch.Tensor] = {}
         if amax:
@@ -146,74 +148,45 @@ class ConformerLinearStack:
             raise RuntimeError(f"nv16 stack: no calibrated amax for {key!r} (run calibrate())")
         return t
 
-    def _lnq(self, key: str, x: torch.Tensor):
-        g, b = self.ln[key]
-        return ops.ln_quantize(x, g, b, self.cfg.eps, self.fmt, amax_t=self._amax(key, None))
-
-    def _q(self, key: str, x: torch.Tensor):
-        return ops.quantize(x, self.fmt, natural=self.fmt == FMT_FP8_1X128, amax_t=self._amax(key, x))
-
-    def _residual(self, name: str, a, x: torch.Tensor, alpha: float, next_ln: Optional[str],
-                  then_ln: Optional[str] = None):
-        """``x <- alpha * linear(a) + x`` and, when ``next_ln`` names the LayerNorm that reads x next, its
-        quantized output: one launch where the fused kernel covers the layer, else two.  With ``then_ln`` (the
-        end of a block): ``x <- LN_next_ln(x)`` is what is stored and the quantized output is that of
-        ``LN_then_ln`` of it."""
-        lin = self.p[name]
-        if next_ln is None:
-            return lin(a, residual=x, alpha=alpha, out=x), None
-        g, be = self.ln[next_ln]
-        g2, be2 = self.ln[then_ln] if then_ln is not None else (None, None)
-        if self.fuse_ln and x.shape[0] >= self.fuse_ln_min_frames and lin.residual_ln_supported():
-            return lin.residual_ln(a, residual=x, gamma=g, beta=be, eps=self.cfg.eps, alpha=alpha, out=x,
-                                   gamma2=g2, beta2=be2)
-        x = lin(a, residual=x, alpha=alpha, out=x)
-        if then_ln is None:
-            return x, self._lnq(next_ln, x)
-        # norm_final of this block + the LayerNorm that reads it next, one kernel
-        return x, ops.ln2_quantize(x, g, be, g2, be2, self.cfg.eps, self.fmt, y=x, amax_t=self._amax(then_ln, None))
-
-    def _ffn(self, b: str, ff: str, ln: str, x: torch.Tensor, q=None, next_ln: Optional[str] = None,
-             then_ln: Optional[str] = None):
-        if q is None:
-            q = self._lnq(b + ln, x)
-        if self.fuse_ffn:
-            h = self.p[b + ff + ".w1"](q, act="swish", out_fmt=self.fmt, out_amax=self._amax(b + ff + ".h", None))
-        else:
-            h = self._q(b + ff + ".h", self.p[b + ff + ".w1"](q, act="swish"))
-        return self._residual(b + ff + ".w2", h, x, 0.5, next_ln, then_ln)
+    def _host_plan(self):
+        """The pass as the native host path walks it: packed weights, LayerNorm parameters and (NV16) calibrated
+        maxima, per block in the order of ``vx_host.cpp``.  Built once; calibration drops it."""
+        if self._plan is None:
+            cfg = self.cfg
+            layers, norms, amax = [], [], []
+            for i in range(cfg.blocks):
+                b = f"b{i}."
+                for n in ("ffm.w1", "ffm.w2", "qkv", "lo", "lp", "pw1", "pw2", "ff.w1", "ff.w2"):
+                    layers.append((self.p[b + n].q, self.p[b + n].bias))
+                for n in ("ln_ffm", "ln_mha", "ln_conv", "ln_ff", "ln_final"):
+                    norms.append(self.ln[b + n])
+                if self.fmt == FMT_NV16:
+                    amax += [self._amax(b + n, None) for n in ("ln_ffm", "ffm.h", "ln_mha", "ctx", "ln_conv", "glu", "ln_ff", "ff.h")]
+            layers.append((self.p["ctc"].q, self.p["ctc"].bias))
+            norms.append(self.ln["after"])
+            if self.fmt == FMT_NV16:
+                amax += [self._amax("after", None), self.amax.get("pos")]
+            self._plan = ops._host().stack_plan(self.fmt, cfg.d_model, cfg.ffn, cfg.conv_pw // 2, cfg.vocab, cfg.eps, self.fuse_ffn,
+                                                cfg.blocks, tuple(layers), tuple(norms), tuple(amax))
+        return self._plan
 
     # ---- forward
     def forward(self, x: torch.Tensor, pos: Optional[torch.Tensor] = None, *, return_hidden: bool = False,
                 ids_only: bool = False, keys=None, ids=None, out_logits: Optional[torch.Tensor] = None):
         """x: bf16 [T, d_model] residual stream (overwritten in place); returns bf16 logits [T, vocab]
-        (written into ``out_logits`` when given: bf16 [T, vocab], unit column stride)."""
-        cfg = self.cfg
-        if x.dtype != torch.bfloat16 or x.dim() != 2 or x.shape[1] != cfg.d_model:
+        (written into ``out_logits`` when given: bf16 [T, vocab], unit column stride).
+
+        One call of the native host path issues every launch of the pass (``vx_host.cpp``,
+        ``stack_forward``); its intermediates share one workspace block."""
+        if x.dtype != torch.bfloat16 or x.dim() != 2 or x.shape[1] != self.cfg.d_model:
             raise ValueError("x must be bf16 [T, d_model]")
-        d = cfg.d_model
-        pos_q = self._q("pos", pos) if pos is not None else None
-        q_in = None  # first LayerNorm of the block, already applied by the previous block's last kernel
-        for i in range(cfg.blocks):
-            b = f"b{i}."
-            x, q = self._ffn(b, "ffm", "ln_ffm", x, q_in, next_ln=b + "ln_mha")
-            qkv = self.p[b + "qkv"](q)
-            if pos_q is not None:
-                self.p[b + "lp"](pos_q)  # feeds the attention scores only
-            ctx = self._q(b + "ctx", qkv[:, 2 * d:])
-            x, q = self._residual(b + "lo", ctx, x, 1.0, b + "ln_conv")
-            gl = self.p[b + "pw1"](q)
-            x, q = self._residual(b + "pw2", self._q(b + "glu", gl), x, 1.0, b + "ln_ff")
-            # norm_final of this block + the LayerNorm that reads it next (first of the next block, or
-            # after_norm) behind the second FFN: x <- LN_final(x), q_in <- quantize(LN_next(x))
-            nxt = f"b{i + 1}.ln_ffm" if i + 1 < cfg.blocks else "after"
-            x, q_in = self._ffn(b, "ff", "ln_ff", x, q, next_ln=b + "ln_final", then_ln=nxt)
-        if q_in is None:  # zero blocks
-            q_in = self._lnq("after", x)
-        if ids_only:
-            return self.p["ctc"].argmax(q_in, keys=keys, ids=ids)
-        logits = self.p["ctc"](q_in, out=out_logits)
-        return (logits, x) if return_hidden else logits
+        if pos is not None and self.fmt == FMT_NV16:
+            self._amax("pos", pos)  # must have been calibrated
+        if pos is not None and pos.stride(1) != 1:
+            pos = pos.contiguous()
+        fused = self.fuse_ln and x.shape[0] >= self.fuse_ln_min_frames
+        out = ops._host().stack_forward(self._host_plan(), x, pos, fused, 1 if ids_only else 0, keys, ids, out_logits)
+        return (out, x) if return_hidden and not ids_only else out
 
     def forward_ids(self, x: torch.Tensor, pos: Optional[torch.Tensor] = None, *, keys=None, ids=None):
         """Greedy CTC ids int32 [T] of ``forward(x, pos).argmax(1)`` without writing the logits."""
@@ -281,6 +254,7 @@ class ConformerLinearStack:
         for k, v in rec.items():
             # head-room so that unseen frames rarely exceed the calibrated range
             self.amax[k] = torch.tensor([v * 1.25], dtype=torch.float32, device=self.device)
+        self._plan = None
         return rec
 
 
