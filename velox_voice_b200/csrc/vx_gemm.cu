@@ -50,7 +50,8 @@ constexpr int TILE_BYTES = BM * STAGE_ROW_BYTES;  // 16 KB
 constexpr int MAX_STAGES = 8;          // ring slots (the arena size decides how many are used)
 constexpr int ARENA_BYTES = 156 * 1024;
 constexpr int RESIDENT_MAX_KSTAGES = 4;                  // B kept in shared memory up to 4 K stages
-constexpr int NUM_THREADS = 576;       // 2 + 16 warps (2 + 28 for the FFN up-projection, see epi_warps)
+constexpr int EPI_WARPS = 16;
+constexpr int NUM_THREADS = (2 + EPI_WARPS) * 32;
 // Registers are granted to a CTA in units of four warps: 18 warps count as 20, so the budget
 // is 65536 / 640 = 102 -> 96 registers per thread (112 does not launch).
 
@@ -62,7 +63,9 @@ constexpr int FP8_ACCS = 4;              // FP8 accumulators in tensor memory (1
 constexpr int FP8_SB_BYTES_PER_KB = 16 * 32 * 4;  // epilogue tables of B scales: 16 warps x 32 columns per K block
 
 // tensor-memory columns
-constexpr int TM_ACC0 = 0, TM_SFA = 256, TM_SFB = 320, TM_COLS = 512;  // SFA: 2 x 32, SFB: up to 128 columns
+// (accumulators in front; A's scale factors at 256, or at 384 behind three 128-column accumulators, B's 64 columns further on)
+constexpr int TM_ACC0 = 0, TM_COLS = 512;
+__host__ __device__ constexpr int tm_sfa_col(int accs) { return accs == 3 ? 384 : 256; }
 
 // FP4 kinds come in two tile shapes: 128 x 256 with one accumulator (fewest MMA instructions
 // and least operand traffic per output) and 128 x 128 with two accumulators (the epilogue of
@@ -76,30 +79,8 @@ __host__ __device__ constexpr bool kind_vec4(int kind) { return kind == KIND_FP4
 // MX32 and the per-row-scaled format: every scale a power of two (see swish4p)
 __host__ __device__ constexpr bool kind_pow2_scales(int kind) { return kind == KIND_FP4_VEC2 || kind == KIND_FP4_VEC2_N128; }
 
-// Epilogue warps of a kernel instance.  A CTA holds at most 32 warps and the epilogue needs whole
-// groups of four (one warp per 32-lane quadrant of tensor memory; the quadrant is also the warp's
-// scheduler), so 28 is the ceiling.
-//   16  every epilogue but one: warp (quadrant, column group) owns 32 rows x 64 columns of a wide
-//       tile (32 x 32 of a narrow one), the same part of every tile;
-//   28  Swish + FP4 output on the narrow tile (the FFN up-projection when the caller asks for
-//       narrow tiles; the wide tile is the default).  That epilogue is bound by
-//       the latency of its own arithmetic -- dependent multiply / ex2 / rcp chains, four warps
-//       per scheduler, all in the same phase because one barrier starts them -- so it runs on
-//       seven warps per scheduler which take the 32 x 32 chunks of the tile stream ROUND ROBIN
-//       (chunk n = 4 * tile + column group goes to warp n mod 7 of the quadrant): the warps of a
-//       scheduler then sit in different tiles and different phases, and the two accumulators of
-//       the narrow tile keep the MMAs two tiles ahead.
-// (The same round-robin hand-out on the WIDE tile was measured too: 178 vs 115 us -- its one
-// accumulator is released only when the last of its eight chunks has found a free warp.)
-#ifndef VX_RR_WIDE
-#define VX_RR_WIDE 0
-#endif
-__host__ __device__ constexpr bool epi_round_robin(int kind, int epi, int out) {
-  return epi == VX_EPI_BIAS_SWISH && out == 2 && (VX_RR_WIDE || kind_bn(kind) == 128);
-}
-__host__ __device__ constexpr int epi_warps(int kind, int epi, int out) { return epi_round_robin(kind, epi, out) ? 28 : 16; }
-__host__ __device__ constexpr int num_threads(int kind, int epi, int out) { return (2 + epi_warps(kind, epi, out)) * 32; }
-
+// Sixteen epilogue warps: warp (quadrant of tensor memory, column group) owns 32 rows x 64 columns of a wide tile (32 x 32 of a
+// narrow one), the same part of every tile.
 struct GemmParams {
   int64_t M, N, K;
   int m_tiles, n_tiles, k_stages;
@@ -122,6 +103,7 @@ struct GemmParams {
   int sfb_resident;       // 1: B streams, but its scale factors are copied to tensor memory once
                           //    (the CTA owns one n-block, as with b_resident)
   int num_slots;          // ring slots in use (a multiple of `group`)
+  int accs;               // accumulators of 128 columns in the ring (2 or 3; kernels that ring them, see UNITS)
   int group;              // K stages per full / empty barrier (2 when a whole K = 512 tile is one wait)
   int a_slot_bytes;       // bytes of one A tile + its scale-factor atoms in the arena
   int b_slot_bytes;       // same for one B tile (BN rows)
@@ -207,6 +189,14 @@ __device__ __forceinline__ float tanh_approx(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// The TANH form on h = z / 2 (already halved).
+__device__ __forceinline__ void swish4p_half(uint64_t& ha, uint64_t& hb) {
+  float h0, h1, h2, h3;
+  unpack_f32x2(ha, h0, h1);
+  unpack_f32x2(hb, h2, h3);
+  ha = fma_f32x2(ha, pack_f32x2(tanh_approx(h0), tanh_approx(h1)), ha);
+  hb = fma_f32x2(hb, pack_f32x2(tanh_approx(h2), tanh_approx(h3)), hb);
+}
 //
 // TANH = true: z sigmoid(z) = h + h tanh(h), h = z / 2, with tanh.approx -- one special-function
 // operation, one packed multiply and one packed fused multiply-add per pair: 2 instructions per value
@@ -221,12 +211,9 @@ template <bool TANH>
 __device__ __forceinline__ void swish4p(uint64_t& za, uint64_t& zb) {
   if constexpr (TANH) {
     const uint64_t half2 = pack_f32x2(0.5f, 0.5f);
-    const uint64_t ha = mul_f32x2(za, half2), hb = mul_f32x2(zb, half2);
-    float h0, h1, h2, h3;
-    unpack_f32x2(ha, h0, h1);
-    unpack_f32x2(hb, h2, h3);
-    za = fma_f32x2(ha, pack_f32x2(tanh_approx(h0), tanh_approx(h1)), ha);
-    zb = fma_f32x2(hb, pack_f32x2(tanh_approx(h2), tanh_approx(h3)), hb);
+    za = mul_f32x2(za, half2);
+    zb = mul_f32x2(zb, half2);
+    swish4p_half(za, zb);
     return;
   }
   const uint64_t nl2e = pack_f32x2(-1.4426950408889634f, -1.4426950408889634f);
@@ -278,12 +265,26 @@ __device__ __forceinline__ void swish_group8(const uint32_t (&r)[32], int g, con
       za = mul_f32x2(za, g2);
       zb = mul_f32x2(zb, g2);
     }
-    if constexpr (BIAS) {
-      const float4 b = *reinterpret_cast<const float4*>(bias_s + 4 * q4);
-      za = add_f32x2(za, pack_f32x2(b.x, b.y));
-      zb = add_f32x2(zb, pack_f32x2(b.z, b.w));
+    if constexpr (!NV16) {
+      // (acc + bias) / 2 = fma(acc, 1/2, bias / 2) bit for bit; the caller's table holds bias / 2
+      const uint64_t half2 = pack_f32x2(0.5f, 0.5f);
+      if constexpr (BIAS) {
+        const float4 b = *reinterpret_cast<const float4*>(bias_s + 4 * q4);
+        za = fma_f32x2(za, half2, pack_f32x2(b.x, b.y));
+        zb = fma_f32x2(zb, half2, pack_f32x2(b.z, b.w));
+      } else {
+        za = mul_f32x2(za, half2);
+        zb = mul_f32x2(zb, half2);
+      }
+      swish4p_half(za, zb);
+    } else {
+      if constexpr (BIAS) {
+        const float4 b = *reinterpret_cast<const float4*>(bias_s + 4 * q4);
+        za = add_f32x2(za, pack_f32x2(b.x, b.y));
+        zb = add_f32x2(zb, pack_f32x2(b.z, b.w));
+      }
+      swish4p<false>(za, zb);
     }
-    swish4p<!NV16>(za, zb);
     out[2 * i] = za;
     out[2 * i + 1] = zb;
   }
@@ -291,7 +292,7 @@ __device__ __forceinline__ void swish_group8(const uint32_t (&r)[32], int g, con
 // Block scale(s) of 32 finished values (16 packed pairs): the scale byte(s), little end first, and
 // the reciprocal(s) to normalise with (NV16: rcp0 for values 0..15, rcp1 for 16..31).
 template <bool NV16>
-__device__ __forceinline__ uint32_t chunk_scales_p(const uint64_t (&sv)[16], float g_out, float& rcp0, float& rcp1) {
+__device__ __forceinline__ uint32_t chunk_scales_p(const uint64_t (&sv)[16], const Nv16Tensor& nv, const float* nv_tab, float& rcp0, float& rcp1) {
   if constexpr (!NV16) {
     float a = 0.0f;
 #pragma unroll
@@ -317,7 +318,7 @@ __device__ __forceinline__ uint32_t chunk_scales_p(const uint64_t (&sv)[16], flo
       }
       uint32_t byte;
       float rcp;
-      nv16_block(a, g_out, byte, rcp);
+      nv.block(a, nv_tab, byte, rcp);
       if (hh == 0) rcp0 = rcp; else rcp1 = rcp;
       sb |= byte << (8 * hh);
     }
@@ -328,13 +329,12 @@ __device__ __forceinline__ uint32_t chunk_scales_p(const uint64_t (&sv)[16], flo
 template <bool NV16>
 __device__ __forceinline__ uint32_t encode_group8(const uint64_t (&sv)[16], int g, float rcp0, float rcp1) {
   const uint64_t v[4] = {sv[4 * g], sv[4 * g + 1], sv[4 * g + 2], sv[4 * g + 3]};
-  if constexpr (NV16) return e2m1_pack8p<false, false, true>(v, g < 2 ? rcp0 : rcp1);
-  else return e2m1_pack8p<true, false, true>(v, rcp0);
+  return e2m1_pack8p<false, true>(v, NV16 && g >= 2 ? rcp1 : rcp0);
 }
 
 template <bool NV16>
 __device__ __forceinline__ uint32_t swish_quant_chunk(const uint32_t (&r)[32], const float* bias_s, bool scale_acc,
-                                                      float g_ab, float g_out, uint32_t (&w)[4]) {
+                                                      float g_ab, const Nv16Tensor& nv, const float* nv_tab, uint32_t (&w)[4]) {
   uint64_t sv[16];
   const uint64_t g2 = pack_f32x2(g_ab, g_ab);
   // (the bias test once per chunk, not once per four values: the epilogue is bound by instruction issue)
@@ -356,7 +356,7 @@ __device__ __forceinline__ uint32_t swish_quant_chunk(const uint32_t (&r)[32], c
     }
   }
   float rcp0, rcp1;
-  const uint32_t sbytes = chunk_scales_p<NV16>(sv, g_out, rcp0, rcp1);
+  const uint32_t sbytes = chunk_scales_p<NV16>(sv, nv, nv_tab, rcp0, rcp1);
 #pragma unroll
   for (int g = 0; g < 4; ++g) w[g] = encode_group8<NV16>(sv, g, rcp0, rcp1);
   return sbytes;
@@ -498,7 +498,7 @@ __device__ __forceinline__ uint32_t store_chunk_fp4(const GemmParams& p, const i
     for (int q = 0; q < 4; ++q) {
       const float v[8] = {z[8 * q], z[8 * q + 1], z[8 * q + 2], z[8 * q + 3],
                           z[8 * q + 4], z[8 * q + 5], z[8 * q + 6], z[8 * q + 7]};
-      w[q] = e2m1_pack8<true, false>(v, rcp);
+      w[q] = e2m1_pack8<false>(v, rcp);
     }
     sbytes = byte;
   } else {
@@ -515,7 +515,7 @@ __device__ __forceinline__ uint32_t store_chunk_fp4(const GemmParams& p, const i
       for (int q = 0; q < 2; ++q) {
         const int b = 16 * h + 8 * q;
         const float v[8] = {z[b], z[b + 1], z[b + 2], z[b + 3], z[b + 4], z[b + 5], z[b + 6], z[b + 7]};
-        w[2 * h + q] = e2m1_pack8<false, false>(v, rcp);
+        w[2 * h + q] = e2m1_pack8<false>(v, rcp);
       }
       sbytes |= byte << (8 * h);
     }
@@ -550,7 +550,7 @@ unsigned long long* g_trace_buffer = nullptr;
 //   2  FP4 re-quantized in the operands' own block format (MX32 for the 32-block kinds, NV16
 //      for the 16-block kinds).
 template <int KIND, int EPI, int OUT>
-__global__ void __launch_bounds__(num_threads(KIND, EPI, OUT), 1)
+__global__ void __launch_bounds__(NUM_THREADS, 1)
 bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
               const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ CUtensorMap tmap_res,
               const GemmParams p) {
@@ -571,21 +571,20 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   constexpr int SFB_COLS = 4 * NRT;          // TMEM columns of one K atom of B scale factors
   constexpr int NCH = (WIDE && !GLU) ? 2 : 1;  // 32-column chunks per epilogue warp
   constexpr int GATE_OFF = BNT / 2;          // GLU: gate columns follow the value columns
-  // Chunk-sequential reads of the wide tile: the second 32-column chunk is read only after the
-  // first is finished.  That halves the live accumulator registers (the kernel is capped at 96
-  // per thread; with both chunks live the plain-bias epilogue spills, 75 vs 67 us for the fused
-  // QKV projection at T = 90000) and releases tensor memory a little later.  Swish epilogues
-  // are bound by their own arithmetic, so the later release costs them nothing; the residual
-  // epilogue is the one that loses by it (77 vs 79 us for the FFN down-projection) and keeps both
-  // chunks in flight.
-  constexpr bool SEQ = (EPI == VX_EPI_BIAS_SWISH || EPI == VX_EPI_BIAS || EPI == VX_EPI_NONE) && NCH == 2;
+  // Chunk-sequential reads of the wide tile: the second 32-column chunk of a warp is read only after the
+  // first is finished, which halves the live accumulator registers (the kernel is capped at 96
+  // per thread).  The two chunks lie in different HALVES of the tile (columns [0, 128) and [128, 256)), and the halves are
+  // accumulators of their own in a ring of three (two where the scale factors leave no room, then both at once): each
+  // is published and handed back by itself, so the MMAs of the next half run ahead of the epilogue by up to two, which takes
+  // up the skew between the warps of a scheduler.  With one barrier for all 256 columns the 1,700 cycles of a K = 512
+  // tile's MMAs and the epilogue took turns, and the slowest of sixteen warps held up the next tile.
+  // The residual epilogue (both chunks' residual blocks in flight) keeps the tile whole.
+  constexpr bool SEQ = (EPI == VX_EPI_BIAS_SWISH || EPI == VX_EPI_BIAS || EPI == VX_EPI_NONE || EPI == VX_EPI_BIAS_QKVPACK) && NCH == 2;
+  constexpr int CH_STRIDE = SEQ ? 128 : 32;  // columns between the chunks of a warp
+  constexpr bool UNITS = !FP8 && (SEQ || !WIDE);  // ring of 128-column accumulators: half tiles, or the narrow kernel's tiles
   // Swish + FP4 output (the FFN up-projection): its own register-lean path, see swish_quant_chunk.
   constexpr bool SWQ = EPI == VX_EPI_BIAS_SWISH && OUT == 2;
-  constexpr int EPW = epi_warps(KIND, EPI, OUT);   // epilogue warps
-  constexpr int BIAS_PER_WARP = 1024 / EPW;        // floats of sm.bias_s per epilogue warp
-  constexpr bool SWQ_RR = epi_round_robin(KIND, EPI, OUT);     // chunks of the tile stream dealt round robin
-  constexpr int NCH_SWQ = kind_bn(KIND) / 128;                 // 32-column chunks per warp on the Swish + FP4 path (16 warps)
-
+  static_assert(!SWQ || WIDE, "Swish + FP4 output runs on the wide tile");
   const int out_dtype = OUT == 1 ? static_cast<int>(VX_BF16) : (OUT == 2 ? static_cast<int>(VX_FP4) : p.out_dtype);
   const bool tma_store = OUT == 1 ? true : (OUT == 2 ? false : p.tma_store != 0);
   const bool tma_residual = OUT == 1 ? EPI == VX_EPI_BIAS_RESIDUAL : (OUT == 2 ? false : p.tma_residual != 0);
@@ -643,9 +642,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     }
     for (int a = 0; a < FP8_ACCS; ++a) {
       mbar_init(&sm.tmem_full[a], 1);
-      // one arrival per 32 x 32 part (16 per accumulator; a wide accumulator read chunk by chunk has 32),
-      // or one per warp where a warp reads its two chunks of the wide tile itself
-      mbar_init(&sm.tmem_empty[a], (SWQ_RR && WIDE) ? 32 : 16);
+      mbar_init(&sm.tmem_empty[a], EPI_WARPS);
     }
     mbar_init(&sm.b_full, 1);
     mbar_init(&sm.sfb_done, 1);
@@ -798,7 +795,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         sfa_col_j[j] = atom * 4;
         sfb_col_j[j] = atom * SFB_COLS;
       }
-      const uint32_t tm_sfa = tmem_base + TM_SFA, tm_sfb = tmem_base + TM_SFB;
+      const uint32_t tm_sfa = tmem_base + (UNITS ? tm_sfa_col(p.accs) : tm_sfa_col(2)), tm_sfb = tm_sfa + 64;
       if (!FP8 && sf_unit) {
         const uint64_t d = make_desc_sf(smem_u32(unit_sf));
         CP(tm_sfa, d);
@@ -876,23 +873,27 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
       } else {
         const int G = p.group, k_groups = p.k_stages / G, ngs = nslots / G;
         uint32_t sfsel = 0;  // which half of the scale-factor columns this group uses
+        const uint32_t accs = UNITS ? p.accs : 1;
+        const bool split = SEQ && accs == 3;  // half tiles one after the other (else both at the end of the tile)
+        const uint32_t sfb_alt = accs == 3 ? 32u : 64u;  // second buffer of streamed B scale factors
+        uint32_t us = 0, uph = 1;             // accumulator filled next, parity of the wait for its release
+        auto next_acc = [&] { if (++us == accs) { us = 0; uph ^= 1; } };
         for (int i = 0; i < my_tiles && ok; ++i) {
           for (int kg = 0; kg < k_groups; ++kg) {
-            const uint32_t acc = WIDE ? 0u : (group & 1);
             if (kg == 0) {
-              const uint32_t use = WIDE ? group : (group >> 1);
-              if (!mbar_wait_spin(&sm.tmem_empty[acc], (use & 1) ^ 1, p.status, 2)) { ok = false; break; }
+              if (!mbar_wait_spin(&sm.tmem_empty[us], uph, p.status, 2)) { ok = false; break; }
+              if (SEQ && !split && !mbar_wait_spin(&sm.tmem_empty[1], uph, p.status, 2)) { ok = false; break; }
               tc_fence_after();  // orders the epilogue's tcgen05.ld of this buffer before the MMAs
               TRACE(i, 0);
             }
             if (!mbar_wait_spin(&sm.full[s], ph, p.status, 3)) { ok = false; break; }
             TRACE(i, kg < 2 ? 1 + kg : 2);
-            const uint32_t d_tmem = tmem_base + TM_ACC0 + acc * 128;
+            const uint32_t d_tmem = tmem_base + TM_ACC0 + us * 128;
             const uint32_t a_lo0 = ring_lo + s * G * slot_lo;
             // (Issuing the next tile's scale-factor copies ahead of this wait was tried: the
             // tcgen05.commit that publishes the accumulator then fires ~1400 cycles later.)
             const uint32_t sfa_buf = tm_sfa + sfsel * 32;
-            const uint32_t sfb_buf = tm_sfb + (owns_nb ? 0u : sfsel * 64);
+            const uint32_t sfb_buf = tm_sfb + (owns_nb ? 0u : sfsel * sfb_alt);
             {
               if (with_sf) {
                 for (int u = 0; u < G; ++u) {
@@ -905,26 +906,46 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
               }
               if (kg == 0) TRACE(i, 3);
             }
-            for (int u = 0; u < G; ++u) {
-              const int ks = kg * G + u;
-              const uint32_t a_lo = a_lo0 + u * slot_lo;
-              const uint32_t b_lo = resident ? arena_lo + ks * bslot_lo : a_lo + aslot_lo;
-              {
+            // MMAs of this group: accumulator d, B rows / scale-factor columns offset by b_off / sfb_off, N field less n_less
+            auto issue = [&](uint32_t d, uint32_t b_off, uint32_t sfb_off, uint32_t n_less) {
+              for (int u = 0; u < G; ++u) {
+                const int ks = kg * G + u;
+                const uint32_t a_lo = a_lo0 + u * slot_lo;
+                const uint32_t b_lo = (resident ? arena_lo + ks * bslot_lo : a_lo + aslot_lo) + b_off;
                 const uint32_t sfa_t = with_sf ? sfa_buf + u * APS * 4 : tm_sfa;
-                const uint32_t sfb_t = with_sf ? sfb_buf + (owns_nb ? ks : u) * APS * SFB_COLS : tm_sfb;
+                const uint32_t sfb_t = (with_sf ? sfb_buf + (owns_nb ? ks : u) * APS * SFB_COLS : tm_sfb) + sfb_off;
   #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                  if (leader) mma_mxf4<VEC>(d_tmem, desc(a_lo + 2 * j, k128_hi), desc(b_lo + 2 * j, k128_hi), idesc_j[j],
+                  if (leader) mma_mxf4<VEC>(d, desc(a_lo + 2 * j, k128_hi), desc(b_lo + 2 * j, k128_hi), idesc_j[j] - n_less,
                                 sfa_t + sfa_col_j[j], sfb_t + sfb_col_j[j], (ks | j) != 0);
                 }
               }
+            };
+            if constexpr (SEQ) {
+              if (split) {
+                constexpr uint32_t N_LESS = static_cast<uint32_t>((BNT - 128) >> 3) << 17;  // N field of the descriptor: 256 -> 128
+                issue(d_tmem, 0, 0, N_LESS);
+                COMMIT(&sm.tmem_full[us]);
+                next_acc();
+                if (!mbar_wait_spin(&sm.tmem_empty[us], uph, p.status, 2)) { ok = false; break; }
+                tc_fence_after();
+                issue(tmem_base + TM_ACC0 + us * 128, (128 * STAGE_ROW_BYTES) >> 4, 4, N_LESS);
+              } else {
+                issue(d_tmem, 0, 0, 0);
+              }
+            } else {
+              issue(d_tmem, 0, 0, 0);
             }
             if (kg == 0) TRACE(i, 4);
             COMMIT(&sm.empty[s]);  // ring slots reusable once these MMAs have read them
             if (kg == 0) TRACE(i, 5);
             if (kg == k_groups - 1) {
-              COMMIT(&sm.tmem_full[acc]);
-              ++group;
+              COMMIT(&sm.tmem_full[us]);
+              next_acc();
+              if (SEQ && !split) {
+                COMMIT(&sm.tmem_full[us]);
+                next_acc();
+              }
               TRACE(i, 6);
             }
             sfsel ^= 1;
@@ -945,11 +966,20 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     constexpr int OUT_TILE_COLS = GLU ? BNT / 2 : BNT;
     const bool has_work = !(GLU && !WIDE) || cc < 2;  // 128-wide GLU: chunks 2, 3 are the gates of 0, 1
     const bool tr = tr_on && ew == 0 && lane == 0;
-    uint32_t group = 0;
+    uint32_t group = 0;  // FP8: rounds taken
+    const uint32_t accs = UNITS ? p.accs : 1;
+    uint32_t es = 0, eph = 0;  // accumulator read next, parity of the wait for it
+    auto next_acc = [&] { if (++es == accs) { es = 0; eph ^= 1; } };
     bool ok = true;
     float g_ab = 1.0f, g_out = 1.0f;
     if (p.a_amax && p.b_amax) g_ab = nv16_global(*p.a_amax) * nv16_global(*p.b_amax);
     if (p.out_amax) g_out = nv16_global(*p.out_amax);
+    Nv16Tensor nv;
+    float* const nv_tab = reinterpret_cast<float*>(sm.staging[ew & 15]);  // FP4 output does not stage: reciprocals by scale byte
+    if constexpr (SWQ && kind_vec4(KIND)) {
+      nv.init(g_out);
+      nv.fill(nv_tab, lane);
+    }
     const int kb_count = FP8 ? p.k_stages : 0;
     uint8_t* const stage0 = sm.staging[ew & 15];
     // TMA residual: the two halves of the staging buffer alternate per 32-column chunk.  The
@@ -962,7 +992,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     int bias_nb = -1;
     uint32_t best_key = 0;  // ARGMAX: best (value, column) of this thread's row in the current tile
     float lse_m = -INFINITY, lse_s = 0.0f;  // ARGMAX + log-sum-exp: running max / sum of 2^((z - max) log2 e) of the tile
-    float* const bias_w = sm.bias_s + ew * BIAS_PER_WARP;
+    float* const bias_w = sm.bias_s + ew * 64;
     const float* const bias_base = p.bias ? bias_w : nullptr;
     // FP8: per-warp tables of B scales at the end of the arena, [chunk][quadrant][kb][32];
     // a GLU warp also owns the table of its gate chunk (chunk cc + 2, whose warps are idle)
@@ -981,7 +1011,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     };
 
     int mb = mb0, nb = nb0;
-    const int col_base = (WIDE && EPW == 16) ? (GLU ? cc * 32 : cc * 64) : cc * 32;  // first accumulator column of this warp
+    const int col_base = WIDE && !GLU && !SEQ ? cc * 64 : cc * 32;  // first accumulator column of this warp
     bool res_inflight = false;
     if constexpr (EPI == VX_EPI_BIAS_RESIDUAL) {
       if (tma_residual && my_tiles > 0 && has_work) {
@@ -989,55 +1019,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         res_inflight = true;
       }
     }
-    if constexpr (SWQ_RR) {
-      // FFN up-projection, round robin: this quadrant's chunks n = CPT * tile + column group, this
-      // warp takes n = j, j + 7, j + 14, ...  Narrow tile: accumulator t & 1, published for the
-      // (t >> 1)-th time; wide tile: the one accumulator, published for the t-th time.  Every chunk
-      // is read by exactly one warp, which arrives once.
-      constexpr int CPT = BNT / 32;  // 32-column chunks per tile
-      const int j = ew >> 2;
-      const bool scale_acc = kind_vec4(KIND) && p.a_amax != nullptr;
-      int t_cur = 0;
-      for (int n = j; n < CPT * my_tiles && ok; n += EPW / 4) {
-        const int t = n / CPT, ccn = n % CPT;
-        while (t_cur < t) { next_tile(mb, nb); ++t_cur; }
-        const uint32_t acc = WIDE ? 0u : (t & 1);
-        if (tr) trace_rec(p, 2, t, 0);
-        if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[acc], (WIDE ? t : (t >> 1)) & 1, p.status, 4);
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) break;
-        tc_fence_after();
-        if (tr) trace_rec(p, 2, t, 1);
-        uint32_t r[32];
-        tc_ld_32x32b_x32(lane_addr + TM_ACC0 + acc * 128 + ccn * 32, r);
-        tc_wait_ld();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.tmem_empty[acc]);
-        if (tr) trace_rec(p, 2, t, 2);
-        const int64_t row = static_cast<int64_t>(mb) * BM + q * 32 + lane;
-        const bool row_ok = row < p.M;
-        const int64_t out_col0 = static_cast<int64_t>(nb) * BNT + ccn * 32;
-        if (out_col0 >= p.N) continue;  // N % 128 == 0: a chunk is whole or (wide tile, last column block) absent
-        uint32_t w[4];
-        const uint32_t sb = swish_quant_chunk<kind_vec4(KIND)>(r, p.bias ? p.bias + out_col0 : nullptr, scale_acc, g_ab, g_out, w);
-        if (row_ok)
-          *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + row * p.ldo + (out_col0 >> 1)) = make_uint4(w[0], w[1], w[2], w[3]);
-        // rows of the last tile beyond M get zero scale factors (the SF atoms cover whole 128-row tiles)
-        const uint32_t sbw = row_ok ? sb : 0u;
-        const int64_t sf_row = (row >> 7) * p.out_sf_kg * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
-        if constexpr (!kind_vec4(KIND)) {
-          p.out_sf[sf_row + (out_col0 >> 7) * 512 + ((out_col0 >> 5) & 3)] = static_cast<uint8_t>(sbw);
-          if (p.out_scales && row_ok) p.out_scales[row * (p.N >> 5) + (out_col0 >> 5)] = static_cast<uint8_t>(sbw);
-        } else {
-          *reinterpret_cast<uint16_t*>(p.out_sf + sf_row + (out_col0 >> 6) * 512 + ((out_col0 >> 5) & 1) * 2) = static_cast<uint16_t>(sbw);
-          if (p.out_scales && row_ok)
-            *reinterpret_cast<uint16_t*>(p.out_scales + row * (p.N >> 4) + (out_col0 >> 4)) = static_cast<uint16_t>(sbw);
-        }
-        if (tr) trace_rec(p, 2, t, 4);
-      }
-    }
-    for (int it = 0; it < (SWQ_RR ? 0 : my_tiles) && ok; ++it) {
+    for (int it = 0; it < my_tiles && ok; ++it) {
       const int64_t row = static_cast<int64_t>(mb) * BM + q * 32 + lane;
       const bool row_ok = row < p.M;
       const bool rows_ok = static_cast<int64_t>(mb) * BM + q * 32 < p.M;
@@ -1048,9 +1030,10 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         // (re)load this warp's bias values: lane i fetches the i-th column of each chunk
         __syncwarp();
         const int64_t c0 = static_cast<int64_t>(nb) * BNT + col_base + lane;
-        const int64_t c1 = GLU ? c0 + GATE_OFF : c0 + 32;
-        bias_w[lane] = c0 < p.N ? __ldg(p.bias + c0) : 0.0f;
-        if (BIAS_PER_WARP >= 64) bias_w[32 + lane] = c1 < p.N ? __ldg(p.bias + c1) : 0.0f;
+        const int64_t c1 = GLU ? c0 + GATE_OFF : c0 + CH_STRIDE;
+        constexpr float BIAS_SCALE = SWQ && !kind_vec4(KIND) ? 0.5f : 1.0f;  // see swish_group8
+        bias_w[lane] = BIAS_SCALE * (c0 < p.N ? __ldg(p.bias + c0) : 0.0f);
+        bias_w[32 + lane] = BIAS_SCALE * (c1 < p.N ? __ldg(p.bias + c1) : 0.0f);
         __syncwarp();
         bias_nb = nb;
       }
@@ -1059,31 +1042,28 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         // 32-column chunk at a time (the second chunk of a wide tile is read from tensor memory
         // only after the first is finished, so that one chunk's registers are live at a time;
         // the MMAs of the next tile then run under the arithmetic of the second chunk)
-        const uint32_t acc = WIDE ? 0u : (group & 1);
-        const uint32_t acc_addr = lane_addr + TM_ACC0 + acc * 128 + col_base;
+        const uint32_t acc_addr = lane_addr + TM_ACC0 + col_base;
         if (tr) trace_rec(p, 2, it, 0);
-        if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[acc], (WIDE ? group : (group >> 1)) & 1, p.status, 4);
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) break;
-        tc_fence_after();
-        if (tr) trace_rec(p, 2, it, 1);
-        ++group;
         const bool scale_acc = kind_vec4(KIND) && p.a_amax != nullptr;
 #pragma unroll
-        for (int h = 0; h < NCH_SWQ; ++h) {
+        for (int h = 0; h < 2; ++h) {  // halves of the tile
+          if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[es], eph, p.status, 4);
+          ok = __shfl_sync(0xffffffffu, ok, 0);
+          if (!ok) break;
+          tc_fence_after();
+          if (tr && h == 0) trace_rec(p, 2, it, 1);
           uint32_t r[32];
-          tc_ld_32x32b_x32(acc_addr + h * 32, r);
+          tc_ld_32x32b_x32(acc_addr + es * 128, r);
           tc_wait_ld();
-          if (h == NCH_SWQ - 1) {  // the whole accumulator is out of tensor memory
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.tmem_empty[acc]);
-          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.tmem_empty[es]);
+          next_acc();
           if (tr && h == 0) trace_rec(p, 2, it, 2);
-          const int64_t out_col0 = static_cast<int64_t>(nb) * BNT + col_base + h * 32;
+          const int64_t out_col0 = static_cast<int64_t>(nb) * BNT + col_base + h * CH_STRIDE;
           uint32_t w[4];
           const uint32_t sb = swish_quant_chunk<kind_vec4(KIND)>(r, bias_base ? bias_base + h * 32 : nullptr, scale_acc, g_ab,
-                                                                 g_out, w);
+                                                                 nv, nv_tab, w);
           if (out_col0 < p.N) {
             if (row_ok)
               *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + row * p.ldo + (out_col0 >> 1)) =
@@ -1101,8 +1081,9 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
                 *reinterpret_cast<uint16_t*>(p.out_scales + row * (p.N >> 4) + (out_col0 >> 4)) = static_cast<uint16_t>(sbw);
             }
           }
-          if (tr && h == 0) trace_rec(p, 2, it, 4);
+          if (tr) trace_rec(p, 2, it, h == 0 ? 4 : 6);
         }
+        if (!ok) break;
         mb = mb_next;
         nb = nb_next;
         continue;
@@ -1193,9 +1174,8 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
       } else {
         if (tr) trace_rec(p, 2, it, 0);
         // one polling lane per warp (512 polling threads would starve the MMA-issuing thread)
-        const uint32_t acc = WIDE ? 0u : (group & 1);
-        const uint32_t acc_addr = lane_addr + TM_ACC0 + acc * 128 + col_base;
-        if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[acc], (WIDE ? group : (group >> 1)) & 1, p.status, 4);
+        const uint32_t acc_addr = lane_addr + TM_ACC0 + es * 128 + col_base;
+        if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[es], eph, p.status, 4);
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
         tc_fence_after();
@@ -1204,7 +1184,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           uint32_t r[32];
 #pragma unroll
           for (int h = 0; h < (SEQ ? 1 : NCH); ++h) {
-            tc_ld_32x32b_x32(acc_addr + h * 32, r);
+            tc_ld_32x32b_x32(acc_addr + h * CH_STRIDE, r);
             tc_wait_ld();
 #pragma unroll
             for (int i = 0; i < 32; ++i) z[h][i] = __uint_as_float(r[i]);
@@ -1217,13 +1197,11 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           }
         }
         if (tr) trace_rec(p, 2, it, 2);
-        if constexpr (!SEQ) {
-          // the accumulator is in registers: hand tensor memory back to the MMA warp
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.tmem_empty[acc]);
-        }
-        ++group;
+        // the accumulator (SEQ: its first half) is in registers: hand tensor memory back to the MMA warp
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.tmem_empty[es]);
+        next_acc();
       }
 
       if (has_work) {
@@ -1231,20 +1209,25 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         for (int h = 0; h < NCH; ++h) {
           if constexpr (SEQ) {
             // second chunk: read it now (its registers were free for the first chunk's
-            // arithmetic), then hand tensor memory back
+            // arithmetic), then hand the second half of the tile back
             if (h == 1) {
+              if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[es], eph, p.status, 4);
+              ok = __shfl_sync(0xffffffffu, ok, 0);
+              if (!ok) break;
+              tc_fence_after();
               uint32_t r[32];
-              tc_ld_32x32b_x32(lane_addr + TM_ACC0 + col_base + 32, r);
+              tc_ld_32x32b_x32(lane_addr + TM_ACC0 + es * 128 + col_base, r);
               tc_wait_ld();
 #pragma unroll
               for (int i = 0; i < 32; ++i) z[1][i] = __uint_as_float(r[i]);
               tc_fence_before();
               __syncwarp();
-              if (lane == 0) mbar_arrive(&sm.tmem_empty[0]);
+              if (lane == 0) mbar_arrive(&sm.tmem_empty[es]);
+              next_acc();
             }
           }
-          const int64_t acc_col0 = static_cast<int64_t>(nb) * BNT + col_base + h * 32;       // accumulator / bias column
-          const int64_t out_col0 = static_cast<int64_t>(nb) * OUT_TILE_COLS + col_base + h * 32;  // output column
+          const int64_t acc_col0 = static_cast<int64_t>(nb) * BNT + col_base + h * CH_STRIDE;       // accumulator / bias column
+          const int64_t out_col0 = static_cast<int64_t>(nb) * OUT_TILE_COLS + col_base + h * CH_STRIDE;  // output column
           const bool box_ok = rows_ok && out_col0 < n_out;
           if constexpr (!FP8) {
             if (sf_unit) {
@@ -1902,7 +1885,12 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, 
       grid = groups * p.n_tiles;
     }
   }
-  VX_CUDA_OK(launch_dependent(bsgemm_kernel<KIND, EPI, OUT>, dim3(grid), dim3(num_threads(KIND, EPI, OUT)), kSmemBytes, st, ta, tb,
+  // A third 128-column accumulator where the scale factors leave 128 columns for it: A's take 64, B's resident ones at most 64;
+  // a wide tile is cut into halves only when its whole K arrives as one group.
+  const bool sfb_small = !with_sf || p.k_stages * SFB_STAGE_COLS <= 64;
+  if (BNT == 256) p.accs = p.b_resident && p.group == p.k_stages && sfb_small ? 3 : 2;
+  else p.accs = (!p.b_resident && !p.sfb_resident) || sfb_small ? 3 : 2;
+  VX_CUDA_OK(launch_dependent(bsgemm_kernel<KIND, EPI, OUT>, dim3(grid), dim3(NUM_THREADS), kSmemBytes, st, ta, tb,
                               to, tr, p));
   VX_CUDA_OK(cudaGetLastError());
   return 0;
@@ -1914,7 +1902,8 @@ int dispatch_out(int out, const CUtensorMap& ta, const CUtensorMap& tb, const CU
   constexpr bool fp4_out_ok = KIND != KIND_FP8 && (EPI == VX_EPI_NONE || EPI == VX_EPI_BIAS || EPI == VX_EPI_BIAS_SWISH);
   if constexpr (EPI != VX_EPI_BIAS_ARGMAX) {
     if (out == 1) return launch<KIND, EPI, 1>(ta, tb, to, tr, p, res, st);
-    if constexpr (fp4_out_ok) {
+    // (Swish + FP4 output has no narrow-tile instance, see vx_bsgemm)
+    if constexpr (fp4_out_ok && (EPI != VX_EPI_BIAS_SWISH || kind_bn(KIND) == 256)) {
       if (out == 2) return launch<KIND, EPI, 2>(ta, tb, to, tr, p, res, st);
     }
   }
@@ -2044,13 +2033,12 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
       };
       if (0.55 * static_cast<double>(rounds(ntn)) < 0.95 * static_cast<double>(rounds(ntw))) narrow = true;
     }
-    // Swish + FP4 output (the FFN up-projection) stays on the wide tile: the narrow tile's
-    // 28-warp round-robin epilogue is faster per value, but its N = 128 MMAs read A from shared
-    // memory twice as often and that chain then bounds the tile (measured 144 vs 134 us at
-    // T = 90000); VX_GEMM_NARROW_TILES selects it.
     if (d->flags & VX_GEMM_WIDE_TILES) narrow = false;
     if (argmax && d->lse_partials) narrow = false;  // the partials are laid out per 64-column group of the wide tile
-    if ((d->flags & VX_GEMM_NARROW_TILES) && epi != VX_EPI_BIAS_GLU) narrow = true;
+    // Swish + FP4 output in the operands' format (the FFN up-projection) exists for the wide tile only: on the narrow one its
+    // N = 128 MMAs read A from shared memory twice as often and that chain bounds the tile (144 vs 134 us at T = 90000).
+    const bool swish_fp4 = epi == VX_EPI_BIAS_SWISH && d->out_dtype == VX_FP4 && d->out_fmt == (vec2 ? VX_FMT_MX32 : VX_FMT_NV16) && fmt != VX_FMT_ROWSCALE;
+    if ((d->flags & VX_GEMM_NARROW_TILES) && epi != VX_EPI_BIAS_GLU && !swish_fp4) narrow = true;
     if (narrow) kind = vec2 ? KIND_FP4_VEC2_N128 : KIND_FP4_VEC4_N128;
   }
   const int BN = kind_bn(kind);

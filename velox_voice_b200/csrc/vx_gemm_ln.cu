@@ -533,7 +533,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         ue8m0_from_amax(fmaxf(max3(a[0], a[1], a[2]), a[3]), byte, rcp);
         uint32_t wd[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) wd[c] = e2m1_pack8p<true, false, true>(v[c], rcp);
+        for (int c = 0; c < 4; ++c) wd[c] = e2m1_pack8p<false, true>(v[c], rcp);
         // word of step c belongs to piece (c + g) & 3: rotate the four words back by g
         if (g & 1) { const uint32_t tt = wd[3]; wd[3] = wd[2]; wd[2] = wd[1]; wd[1] = wd[0]; wd[0] = tt; }
         if (g & 2) { uint32_t tt = wd[0]; wd[0] = wd[2]; wd[2] = tt; tt = wd[1]; wd[1] = wd[3]; wd[3] = tt; }

@@ -134,7 +134,7 @@ __device__ __forceinline__ void quant_chunk(const QuantParams& p, I row0, int c,
 
   if constexpr (FMT == VX_FMT_ROWSCALE) {
     if (active) {
-      *reinterpret_cast<uint32_t*>(p.codes + row0 * ldc + (k0 >> 1)) = e2m1_pack8p<true, CANON, NUDGE>(v[0], row_rcp);
+      *reinterpret_cast<uint32_t*>(p.codes + row0 * ldc + (k0 >> 1)) = e2m1_pack8p<CANON, NUDGE>(v[0], row_rcp);
     }
   } else if constexpr (FMT == VX_FMT_FP8_1X128) {
     float a = amax8p(v[0]);
@@ -164,8 +164,8 @@ __device__ __forceinline__ void quant_chunk(const QuantParams& p, I row0, int c,
     for (int r = 0; r < RP; ++r) {
       if (active) {
         uint32_t w;
-        if constexpr (FMT == VX_FMT_NV16) w = e2m1_pack8p<false, CANON, true>(v[r], rcp);
-        else w = e2m1_pack8p<true, CANON, NUDGE>(v[r], rcp);
+        if constexpr (FMT == VX_FMT_NV16) w = e2m1_pack8p<CANON, true>(v[r], rcp);
+        else w = e2m1_pack8p<CANON, NUDGE>(v[r], rcp);
         *reinterpret_cast<uint32_t*>(p.codes + (row0 + r) * ldc + (k0 >> 1)) = w;
       }
     }
@@ -637,8 +637,12 @@ __global__ void __launch_bounds__(256, LN ? VX_R2_MIN_BLOCKS_LN : VX_R2_MIN_BLOC
   // set-up done (LayerNorm parameters are constants of the model): from here on the kernel touches what
   // the previous kernel of the stream produced
   pdl_wait();
-  float g = 1.0f;
-  if constexpr (FMT == VX_FMT_NV16) g = nv16_global(*p.amax);
+  __shared__ float nv_s[FMT == VX_FMT_NV16 ? 8 : 1][128];  // per warp: reciprocals by scale byte
+  Nv16Tensor nv;
+  if constexpr (FMT == VX_FMT_NV16) {
+    nv.init(nv16_global(*p.amax));
+    nv.fill(nv_s[w], lane);
+  }
 
   auto issue = [&](int slot, int u) {
     if (lane == 0) {
@@ -796,7 +800,7 @@ __global__ void __launch_bounds__(256, LN ? VX_R2_MIN_BLOCKS_LN : VX_R2_MIN_BLOC
         float rcp;
         ue8m0_from_amax(fmaxf(max3(a[0], a[1], a[2]), a[3]), byte, rcp);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) wd[c] = e2m1_pack8p<true, CANON, NUDGE>(v[c], rcp);
+        for (int c = 0; c < 4; ++c) wd[c] = e2m1_pack8p<CANON, NUDGE>(v[c], rcp);
         if (valid) {
           if (p.sf) p.sf[sf_offset<int>(row, j >> 2, static_cast<int>(p.sf_kg)) + (j & 3)] = static_cast<uint8_t>(byte);
           if (p.scales) static_cast<uint8_t*>(p.scales)[row * 16 + j] = static_cast<uint8_t>(byte);
@@ -812,10 +816,10 @@ __global__ void __launch_bounds__(256, LN ? VX_R2_MIN_BLOCKS_LN : VX_R2_MIN_BLOC
         }
         uint32_t b_lo, b_hi;
         float r_lo, r_hi;
-        nv16_block(a_lo, g, b_lo, r_lo);
-        nv16_block(a_hi, g, b_hi, r_hi);
+        nv.block(a_lo, nv_s[w], b_lo, r_lo);
+        nv.block(a_hi, nv_s[w], b_hi, r_hi);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) wd[c] = e2m1_pack8p<false, CANON, true>(v[c], ((c + rot) & 2) == 0 ? r_lo : r_hi);
+        for (int c = 0; c < 4; ++c) wd[c] = e2m1_pack8p<CANON, true>(v[c], ((c + rot) & 2) == 0 ? r_lo : r_hi);
         if (valid) {
           if (p.sf)
             *reinterpret_cast<uint16_t*>(p.sf + sf_offset<int>(row, j >> 1, static_cast<int>(p.sf_kg)) + (j & 1) * 2) =

@@ -33,13 +33,15 @@ __device__ __forceinline__ void ue8m0_from_amax(float amax, uint32_t& byte, floa
 // 3.5} strictly exceeded, sign = (q < 0) -- is "round to nearest E2M1 value, ties toward zero,
 // capped at 4.0".  The hardware converter (cvt.rn.satfinite.e2m1x2.f32) rounds ties to even
 // and reaches 6.0.  It is made to follow the reference by two cheap corrections:
-//   * the converter never sees a tie: q is replaced by q' = q when its last mantissa bit is
-//     set, else by the next fp32 value toward zero, which has it set (all six thresholds have
-//     that bit clear).  q <= t gives q' < t and q > t gives q' > t for every threshold t, so
-//     round-to-nearest of q' is the reference's code.  q' = (q * (1 - 2^-24)) | 1: the product
-//     rounds to the fp32 neighbour toward zero for every normal q (subnormal q stay put; they
-//     encode as zero either way).  For a power-of-two rcp the factor is folded into rcp
-//     (rcp * (1 - 2^-24) is exact), saving the second multiplication;
+//   * q is pulled toward zero by 0.72 * 2^-24 of itself, q' = fma(q, -0.72 * 2^-24, q), one packed operation for two
+//     values.  In units of the last place that is 0.36 * m for a q with significand m in [1, 2), so rounding leaves q
+//     alone below m = 1.39 and moves it to the fp32 neighbour toward zero above.  At the thresholds:
+//       0.75, 1.75, 3.5  (m = 1.5, 1.75; the converter's tie goes UP, to the even code): q = t becomes t - 1 ulp, which
+//                        rounds down as the reference wants; q = t + 1 ulp becomes t, whose tie goes up as it should;
+//       0.25, 1.25, 2.5  (m = 1 or 1.25; the converter's tie goes DOWN): q = t + 1 ulp stays; q = t stays (1.25, 2.5) or
+//                        moves down (0.25: the fp32 grid is twice as fine below a power of two).
+//     q farther from a threshold never reaches it.  (Checked against the rule over every fp32 value within 2,000,000 ulps of
+//     each threshold.)  The form used before, q * (1 - 2^-24) | 1, took two logic operations per pair more;
 //   * code 7 (6.0, reached for |q| > 5) is turned into code 6 on the packed word.
 // q is formed as (v * rcp) + (+0) with two separate roundings: a product that is -0 or
 // underflows to -0 becomes +0, so the sign bit equals (q < 0) exactly (a fused multiply-add
@@ -70,6 +72,7 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   return r;
 }
 constexpr float kTowardZero = 0.99999994f;  // 1 - 2^-24
+constexpr float kPull = -0x1.70a3d8p-25f;   // -0.72 * 2^-24
 
 // max(a, b, c) in one instruction (three-input form of sm_100)
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -107,31 +110,29 @@ __device__ __forceinline__ uint32_t e2m1_cvt8(const float (&r)[8]) {
 // CANON_ZERO = false skips the "+ (+0)": a product that is (or underflows to) -0 then encodes as
 // nibble 8 (-0) where the reference writes 0 -- the same value.  The GEMM epilogue uses it (its
 // inputs are -0 only for an exactly -0 pre-activation); the quantizers keep the reference's bytes.
-template <bool POW2, bool CANON_ZERO = true>
+template <bool CANON_ZERO = true>
 __device__ __forceinline__ uint32_t e2m1_pack8(const float (&v)[8], float rcp) {
-  const float m = POW2 ? __fmul_rn(rcp, kTowardZero) : rcp;
   float r[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    float q = __fmul_rn(v[j], m);
+    float q = __fmul_rn(v[j], rcp);
     if (CANON_ZERO) q = __fadd_rn(q, 0.0f);  // -0 -> +0
-    if (!POW2) q = __fmul_rn(q, kTowardZero);
-    r[j] = __uint_as_float(__float_as_uint(q) | 1u);
+    r[j] = __fmaf_rn(q, kPull, q);
   }
   return e2m1_cvt8(r);
 }
 
 // The same encode on four packed pairs with packed fp32 arithmetic (two values per multiply /
 // add; every element sees exactly the operations of e2m1_pack8, so the bytes are the same).
-// NUDGE = false drops the "| 1": allowed when the values are bf16 numbers and rcp is a power of
+// NUDGE = false folds the pull into rcp: allowed when the values are bf16 numbers and rcp is a power of
 // two.  q = v * rcp then has at most 8 significant bits, so its fp32 neighbour toward zero --
 // which the folded factor (1 - 2^-24) produces -- lies on the same side of every threshold as q,
 // below it when q is a threshold, and is never a threshold itself.
-template <bool POW2, bool CANON_ZERO, bool NUDGE>
+template <bool CANON_ZERO, bool NUDGE>
 __device__ __forceinline__ uint32_t e2m1_pack8p(const uint64_t (&v)[4], float rcp) {
-  const float m = POW2 ? __fmul_rn(rcp, kTowardZero) : rcp;
+  const float m = NUDGE ? rcp : __fmul_rn(rcp, kTowardZero);
   const uint64_t m2 = pack_f32x2(m, m);
-  const uint64_t t2 = pack_f32x2(kTowardZero, kTowardZero);
+  const uint64_t k2 = pack_f32x2(kPull, kPull);
   float r[8];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -143,15 +144,8 @@ __device__ __forceinline__ uint32_t e2m1_pack8p(const uint64_t (&v)[4], float rc
       unpack_f32x2(q, a, b);
       q = pack_f32x2(__fadd_rn(a, 0.0f), __fadd_rn(b, 0.0f));
     }
-    if (!POW2) q = mul_f32x2(q, t2);
-    float lo, hi;
-    unpack_f32x2(q, lo, hi);
-    if (NUDGE) {
-      lo = __uint_as_float(__float_as_uint(lo) | 1u);
-      hi = __uint_as_float(__float_as_uint(hi) | 1u);
-    }
-    r[2 * j] = lo;
-    r[2 * j + 1] = hi;
+    if (NUDGE) q = fma_f32x2(q, k2, q);
+    unpack_f32x2(q, r[2 * j], r[2 * j + 1]);
   }
   return e2m1_cvt8(r);
 }
@@ -168,6 +162,42 @@ __device__ __forceinline__ void nv16_block(float a16, float g, uint32_t& byte, f
   const float d = __fmul_rn(g, e4m3_to_float(byte));
   rcp = d > 0.0f ? __frcp_rn(d) : 0.0f;
 }
+// The same bits for many blocks of one tensor: the quotient by the tensor's constant 6 g from the correctly rounded
+// reciprocal of 6 g and one remainder step (Markstein, IBM J. Res. Dev. 34(1), 1990: with r = RN(1/d) and q = RN(a r),
+// RN(q + r (a - q d)) is the correctly rounded a / d), and the reciprocal of g * scale -- there are 127 scales -- from a
+// table: 5 instructions per block instead of a division and a reciprocal.  Outside a range in which no intermediate
+// value is subnormal or overflows the plain form is used.
+struct Nv16Tensor {
+  float g, d6, r6;
+  __device__ __forceinline__ void init(float global) {
+    g = global;
+    d6 = __fmul_rn(6.0f, g);
+    r6 = d6 > 0x1p-80f && d6 < 0x1p80f ? __frcp_rn(d6) : 0.0f;
+  }
+  // entry `byte` of the reciprocal table (128 entries)
+  __device__ __forceinline__ float entry(uint32_t byte) const {
+    const float d = __fmul_rn(g, e4m3_to_float(byte));
+    return d > 0.0f ? __frcp_rn(d) : 0.0f;
+  }
+  // this warp's table (512 bytes of shared memory)
+  __device__ __forceinline__ void fill(float* tab, int lane) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tab[i * 32 + lane] = entry(i * 32 + lane);
+    __syncwarp();
+  }
+  __device__ __forceinline__ void block(float a16, const float* tab, uint32_t& byte, float& rcp) const {
+    float t;
+    if (r6 != 0.0f) {
+      // (a quotient below 2^-10 or above 448 encodes as zero or 448 whatever its last bits are)
+      const float q = __fmul_rn(a16, r6);
+      t = q > 1e6f ? q : __fmaf_rn(__fmaf_rn(-q, d6, a16), r6, q);
+    } else {
+      t = __fdiv_rn(a16, d6);
+    }
+    byte = __nv_cvt_float_to_fp8(t, __NV_SATFINITE, __NV_E4M3);
+    rcp = tab[byte & 0x7fu];
+  }
+};
 __device__ __forceinline__ float nv16_global(float amax_t) {
   return amax_t == 0.0f ? 1.0f : __fdiv_rn(amax_t, 2688.0f);
 }
