@@ -46,7 +46,8 @@ enum vx_epilogue {
   VX_EPI_NONE = 0,      /* out = acc (* scales)                      */
   VX_EPI_BIAS = 1,      /* out = acc + bias[n]                       */
   VX_EPI_BIAS_SWISH = 2,/* out = silu(acc + bias[n])                 */
-  VX_EPI_BIAS_GLU = 3,  /* out[:, j] = (acc_a + b_a) * sigmoid(acc_b + b_b), GLU-interleaved weights */
+  VX_EPI_BIAS_GLU = 3,  /* out[:, j] = (acc_a + b_a) * sigmoid(acc_b + b_b), GLU-interleaved weights; FP4 output (MX32 / NV16
+                           operands, the same format): what vx_quantize_pack makes of the bf16 result */
   VX_EPI_BIAS_RESIDUAL = 4, /* out = residual + alpha * (acc + bias[n]) */
   VX_EPI_BIAS_ARGMAX = 5, /* no [M, N] output: per row the first column holding the maximum of
                             bf16(acc + bias[n]); `out` = u64 keys [M], see vx_argmax_ids */
@@ -161,7 +162,7 @@ typedef struct vx_gemm_desc {
   void* topk_candidates;       /*   threshold is appended to that row's list: u64 [M][topk_capacity] =                      */
   int32_t* topk_count;         /*   (order-preserving logit bits << 32) | (0xFFFFFFFF - column); i32 [M], zeroed by the caller */
   int32_t topk_capacity;       /*   entries per row; appends beyond it are counted but not stored (see vx_ctc_topk_finish)  */
-  int32_t reserved0;
+  int32_t quant_col0;          /* VX_GEMM_QUANT_TAIL: first column that is also quantized */
 } vx_gemm_desc;
 
 /* VX_EPI_BIAS_GLU expects the rows of B (and the bias) interleaved per tile of vx_glu_tile(fmt)
@@ -181,6 +182,10 @@ int vx_glu_tile(int fmt);
 #define VX_GEMM_POS_F32 64     /* BIAS_QKVPACK: pos_u / pos_v are fp32, rounded to bf16 on use */
 #define VX_GEMM_CONST_B 128    /* B (codes, scales) is a constant that was packed by vx_quantize_pack from fp32, or with
                                   natural-layout scales: its loads may start under the tail of the previous launch */
+#define VX_GEMM_QUANT_TAIL 1024 /* bf16 output (NONE / BIAS, MX32 / NV16): the columns from quant_col0 on are also quantized in
+                                  out_fmt = fmt, the bits of vx_quantize_pack on them: out_scales = codes u8 [M, (N - quant_col0) / 2]
+                                  (dense), out_scales_sf = SF atoms.  The value third of a fused QKV projection that feeds the
+                                  next linear needs no quantizer launch then */
 
 int vx_bsgemm(const vx_gemm_desc* desc, void* stream);
 

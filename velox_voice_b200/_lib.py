@@ -32,6 +32,7 @@ GEMM_NARROW_TILES = 8
 GEMM_OUT_HEADS = 16
 GEMM_POS_F32 = 64
 GEMM_CONST_B = 128
+GEMM_QUANT_TAIL = 1024
 
 EXPORTS = (
     "vx_abi_version",
@@ -112,7 +113,7 @@ class GemmDesc(C.Structure):
         ("topk_candidates", C.c_void_p),
         ("topk_count", C.c_void_p),
         ("topk_capacity", C.c_int32),
-        ("reserved0", C.c_int32),
+        ("quant_col0", C.c_int32),
     ]
 
 

@@ -121,6 +121,9 @@ struct GemmParams {
   int out_fmt;
   uint8_t* out_sf;
   uint8_t* out_scales;
+  uint8_t* tail_codes;    // VX_GEMM_QUANT_TAIL: codes of the columns from quant_col0 on, dense rows
+  int quant_col0;
+  int tail_tiles, plain_groups;  // n-blocks of the tail (0: CTAs are dealt evenly) and CTAs per other n-block
   int64_t out_sf_kg;
   const float* out_amax;
   // head-major bf16 output (attention fold pack)
@@ -479,6 +482,39 @@ __device__ __forceinline__ void store_chunk_direct(const GemmParams& p, const fl
   }
 }
 
+// The bf16 values of a 32-column chunk quantized to E2M1 as the stand-alone quantizer does it on a bf16 tensor: codes and
+// scale bytes (1 or 2, little end first).
+__device__ __forceinline__ uint32_t quant_bf16_chunk(const int out_fmt, const float (&z)[32], float g_out, uint32_t (&w)[4]) {
+  uint64_t v[4][4];
+  float a[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t pk = pack_bf16x2(z[8 * q + 2 * i], z[8 * q + 2 * i + 1]);
+      v[q][i] = pack_f32x2(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u));
+    }
+    a[q] = amax8p(v[q]);
+  }
+  uint32_t byte;
+  float rcp;
+  if (out_fmt == VX_FMT_MX32) {
+    ue8m0_from_amax(fmaxf(max3(a[0], a[1], a[2]), a[3]), byte, rcp);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) w[q] = e2m1_pack8p<true, false>(v[q], rcp);
+    return byte;
+  }
+  uint32_t sbytes = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    nv16_block(fmaxf(a[2 * h], a[2 * h + 1]), g_out, byte, rcp);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) w[2 * h + q] = e2m1_pack8p<true, true>(v[2 * h + q], rcp);
+    sbytes |= byte << (8 * h);
+  }
+  return sbytes;
+}
+
 // Re-quantize one 32-column chunk of an output row to E2M1 (MX32: one UE8M0 scale; NV16: two
 // E4M3 scales) -- the same arithmetic as the stand-alone quantizer.  Returns the scale bytes
 // (1 or 2, little end first) for the caller to assemble into SF words.
@@ -548,7 +584,8 @@ unsigned long long* g_trace_buffer = nullptr;
 //   0  chosen at run time (fp32 / bf16 / FP4, TMA or direct stores, per-row-scaled format);
 //   1  bf16 through staged TMA stores, residual (if any) prefetched by TMA;
 //   2  FP4 re-quantized in the operands' own block format (MX32 for the 32-block kinds, NV16
-//      for the 16-block kinds).
+//      for the 16-block kinds);
+//   4  as 1, and the columns from quant_col0 on are also quantized (VX_GEMM_QUANT_TAIL).
 template <int KIND, int EPI, int OUT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -585,12 +622,12 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   // Swish + FP4 output (the FFN up-projection): its own register-lean path, see swish_quant_chunk.
   constexpr bool SWQ = EPI == VX_EPI_BIAS_SWISH && OUT == 2;
   static_assert(!SWQ || WIDE, "Swish + FP4 output runs on the wide tile");
-  const int out_dtype = OUT == 1 ? static_cast<int>(VX_BF16) : (OUT == 2 ? static_cast<int>(VX_FP4) : p.out_dtype);
-  const bool tma_store = OUT == 1 ? true : (OUT == 2 ? false : p.tma_store != 0);
-  const bool tma_residual = OUT == 1 ? EPI == VX_EPI_BIAS_RESIDUAL : (OUT == 2 ? false : p.tma_residual != 0);
-  const bool sf_unit = (OUT == 1 || OUT == 2) ? false : p.sf_unit != 0;
+  const int out_dtype = OUT == 1 || OUT == 4 ? static_cast<int>(VX_BF16) : (OUT == 2 ? static_cast<int>(VX_FP4) : p.out_dtype);
+  const bool tma_store = OUT == 1 || OUT == 4 ? true : (OUT == 2 ? false : p.tma_store != 0);
+  const bool tma_residual = OUT == 1 ? EPI == VX_EPI_BIAS_RESIDUAL : (OUT == 2 || OUT == 4 ? false : p.tma_residual != 0);
+  const bool sf_unit = (OUT == 1 || OUT == 2 || OUT == 4) ? false : p.sf_unit != 0;
   constexpr bool TOPK = EPI == VX_EPI_BIAS_ARGMAX && OUT == 3;  // OUT 3: the run-time route + the top-k candidate pass
-  const int out_fmt = OUT == 2 ? static_cast<int>(kind_vec4(KIND) ? VX_FMT_NV16 : VX_FMT_MX32) : p.out_fmt;
+  const int out_fmt = OUT == 2 || OUT == 4 ? static_cast<int>(kind_vec4(KIND) ? VX_FMT_NV16 : VX_FMT_MX32) : p.out_fmt;
   const bool tr_on = kPhaseTrace && p.trace != nullptr && blockIdx.x == 0;  // phase trace requested (CTA 0 only)
 
   const int warp = threadIdx.x >> 5;
@@ -609,17 +646,25 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   // tiles t0, t0 + grid, ... with n fastest.  No division inside the loops.
   const int total_tiles = p.m_tiles * p.n_tiles;
   int my_tiles, mb0, nb0;
+  int step_m = static_cast<int>(gridDim.x) / p.n_tiles;
   if (owns_nb) {
-    nb0 = blockIdx.x % p.n_tiles;
-    mb0 = blockIdx.x / p.n_tiles;
-    const int mstep = gridDim.x / p.n_tiles;
-    my_tiles = mb0 < p.m_tiles ? (p.m_tiles - mb0 + mstep - 1) / mstep : 0;
+    // (quantized tail: its n-blocks, the last ones, have more CTAs than the others, see launch())
+    int b = blockIdx.x, first = 0, count = p.n_tiles;
+    if (OUT == 4 && p.tail_tiles) {
+      const int plain = p.n_tiles - p.tail_tiles, plain_ctas = plain * p.plain_groups;
+      const bool in_tail = b >= plain_ctas;
+      if (in_tail) { b -= plain_ctas; first = plain; }
+      count = in_tail ? p.tail_tiles : plain;
+      step_m = in_tail ? (static_cast<int>(gridDim.x) - plain_ctas) / p.tail_tiles : p.plain_groups;
+    }
+    nb0 = first + b % count;
+    mb0 = b / count;
+    my_tiles = mb0 < p.m_tiles ? (p.m_tiles - mb0 + step_m - 1) / step_m : 0;
   } else {
     mb0 = blockIdx.x / p.n_tiles;
     nb0 = blockIdx.x - mb0 * p.n_tiles;
     my_tiles = static_cast<int>(blockIdx.x) < total_tiles ? (total_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
   }
-  const int step_m = static_cast<int>(gridDim.x) / p.n_tiles;
   const int step_n = owns_nb ? 0 : static_cast<int>(gridDim.x) % p.n_tiles;
   auto next_tile = [&](int& mb, int& nb) {
     mb += step_m;
@@ -1089,6 +1134,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         continue;
       }
       float z[NCH][32], gate[32];
+      float row_scale = 0.0f, col_scale[NCH] = {};
       if constexpr (FP8) {
         // B scales of this warp's columns, transposed into its private table [kb][32]
         // (lane <-> column while loading; every lane reads whole rows of it afterwards)
@@ -1173,6 +1219,15 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         if (!ok) break;
       } else {
         if (tr) trace_rec(p, 2, it, 0);
+        if (sf_unit) {
+          // per-row-scaled format: this row's scale and, lane by lane, those of the warp's columns, fetched while the MMAs run
+          row_scale = row_ok ? ue8m0_to_float(p.row_scale_u8[row]) : 0.0f;
+#pragma unroll
+          for (int h = 0; h < NCH; ++h) {
+            const int64_t ncol = static_cast<int64_t>(nb) * BNT + col_base + h * CH_STRIDE + lane;
+            col_scale[h] = ncol < p.N ? ue8m0_to_float(p.col_scale_u8[ncol]) : 0.0f;
+          }
+        }
         // one polling lane per warp (512 polling threads would starve the MMA-issuing thread)
         const uint32_t acc_addr = lane_addr + TM_ACC0 + es * 128 + col_base;
         if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[es], eph, p.status, 4);
@@ -1232,11 +1287,8 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           if constexpr (!FP8) {
             if (sf_unit) {
               // reference order: raw * row_scale * col_scale
-              const float row_scale = row_ok ? ue8m0_to_float(p.row_scale_u8[row]) : 0.0f;
-              const int64_t ncol = acc_col0 + lane;
-              const float csv = ncol < p.N ? ue8m0_to_float(p.col_scale_u8[ncol]) : 0.0f;
 #pragma unroll
-              for (int i = 0; i < 32; ++i) z[h][i] = z[h][i] * row_scale * __shfl_sync(0xffffffffu, csv, i);
+              for (int i = 0; i < 32; ++i) z[h][i] = z[h][i] * row_scale * __shfl_sync(0xffffffffu, col_scale[h], i);
             } else if (kind_vec4(KIND) && p.a_amax) {
 #pragma unroll
               for (int i = 0; i < 32; ++i) z[h][i] = __fmul_rn(z[h][i], g_ab);
@@ -1405,7 +1457,16 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
               }
             }
           } else if (out_dtype == VX_FP4) {
-            const uint32_t sb = store_chunk_fp4(p, out_fmt, z[h], row, out_col0, g_out, row_ok && out_col0 < n_out);
+            uint32_t sb;
+            if constexpr (GLU) {
+              // the operand of the next GEMM: what the quantizer makes of the bf16 GLU output
+              uint32_t w[4];
+              sb = quant_bf16_chunk(out_fmt, z[h], g_out, w);
+              if (row_ok && out_col0 < n_out)
+                *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + row * p.ldo + (out_col0 >> 1)) = make_uint4(w[0], w[1], w[2], w[3]);
+            } else {
+              sb = store_chunk_fp4(p, out_fmt, z[h], row, out_col0, g_out, row_ok && out_col0 < n_out);
+            }
             if (out_col0 < n_out) {
               // this chunk's scale byte(s) inside the row's SF word(s); rows of the last tile
               // beyond M get zero scale factors (the SF atoms cover whole 128-row tiles)
@@ -1423,6 +1484,19 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
               }
             }
           } else if (tma_store) {
+            if constexpr (OUT == 4) {
+              if (out_col0 >= p.quant_col0 && out_col0 < n_out) {
+                uint32_t w[4];
+                const uint32_t sb = quant_bf16_chunk(out_fmt, z[h], g_out, w);
+                const int tc = static_cast<int>(out_col0) - p.quant_col0;  // column inside the tail
+                if (row_ok)
+                  *reinterpret_cast<uint4*>(p.tail_codes + row * ((n_out - p.quant_col0) >> 1) + (tc >> 1)) = make_uint4(w[0], w[1], w[2], w[3]);
+                const uint32_t sbw = row_ok ? sb : 0u;  // (rows beyond M: zero scale factors)
+                uint8_t* const sf = p.out_sf + (row >> 7) * p.out_sf_kg * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
+                if constexpr (!kind_vec4(KIND)) sf[(tc >> 7) * 512 + ((tc >> 5) & 3)] = static_cast<uint8_t>(sbw);
+                else *reinterpret_cast<uint16_t*>(sf + (tc >> 6) * 512 + ((tc >> 5) & 1) * 2) = static_cast<uint16_t>(sbw);
+              }
+            }
             // stage 32 rows x 32 columns (swizzled like the tensor map), then one TMA store
             uint8_t* buf = stage0;
             if (res_smem) {
@@ -1491,7 +1565,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
       mb = mb_next;
       nb = nb_next;
     }
-    if (tma_store && lane == 0) tma_store_wait_all<0>();
+    if (tma_store && lane == 0) tma_store_wait_read<0>();  // (shared memory is read; the writes complete with the grid)
   }
 
   // ---- tear-down
@@ -1871,6 +1945,24 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, 
     int groups = sms / p.n_tiles;
     if (groups > p.m_tiles) groups = p.m_tiles;
     grid = groups * p.n_tiles;
+    p.tail_tiles = 0;
+    if (OUT == 4 && p.quant_col0 % BNT == 0 && p.quant_col0 > 0 && groups < p.m_tiles) {
+      // A tile of the tail takes about 1.6 times as long (90.6 us for 6 x 24 equal groups where the plain projection takes
+      // 57): the SMs are split so that both kinds finish together -- the split with the fewest weighted rounds.
+      const int tail = p.n_tiles - p.quant_col0 / BNT, plain = p.n_tiles - tail;
+      double best = 1e30;
+      for (int g = 1; plain * g + tail <= sms; ++g) {
+        int t = (sms - plain * g) / tail;
+        if (t > p.m_tiles) t = p.m_tiles;
+        const double r1 = (p.m_tiles + g - 1) / g, r2 = 1.6 * ((p.m_tiles + t - 1) / t), cost = r1 > r2 ? r1 : r2;
+        if (cost < best) {
+          best = cost;
+          p.tail_tiles = tail;
+          p.plain_groups = g;
+          grid = plain * g + tail * t;
+        }
+      }
+    }
   } else {
     const int slots = arena / (p.a_slot_bytes + p.b_slot_bytes);
     p.num_slots = slots > MAX_STAGES ? MAX_STAGES : slots;
@@ -1899,12 +1991,16 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, 
 template <int KIND, int EPI>
 int dispatch_out(int out, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to,
                  const CUtensorMap& tr, GemmParams& p, bool res, cudaStream_t st) {
-  constexpr bool fp4_out_ok = KIND != KIND_FP8 && (EPI == VX_EPI_NONE || EPI == VX_EPI_BIAS || EPI == VX_EPI_BIAS_SWISH);
+  constexpr bool fp4_out_ok = KIND != KIND_FP8 && (EPI == VX_EPI_NONE || EPI == VX_EPI_BIAS || EPI == VX_EPI_BIAS_SWISH ||
+                                                   (EPI == VX_EPI_BIAS_GLU && kind_bn(KIND) == 256));
   if constexpr (EPI != VX_EPI_BIAS_ARGMAX) {
     if (out == 1) return launch<KIND, EPI, 1>(ta, tb, to, tr, p, res, st);
     // (Swish + FP4 output has no narrow-tile instance, see vx_bsgemm)
     if constexpr (fp4_out_ok && (EPI != VX_EPI_BIAS_SWISH || kind_bn(KIND) == 256)) {
       if (out == 2) return launch<KIND, EPI, 2>(ta, tb, to, tr, p, res, st);
+    }
+    if constexpr (KIND != KIND_FP8 && (EPI == VX_EPI_NONE || EPI == VX_EPI_BIAS)) {
+      if (out == 4) return launch<KIND, EPI, 4>(ta, tb, to, tr, p, res, st);
     }
   }
   if constexpr (EPI == VX_EPI_BIAS_ARGMAX && KIND != KIND_FP8) {
@@ -1970,7 +2066,7 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
   const bool qkvpack = epi == VX_EPI_BIAS_QKVPACK;
   const bool out_heads = (d->flags & VX_GEMM_OUT_HEADS) != 0;
   constexpr int32_t kKnownFlags = VX_GEMM_DIRECT_STORE | VX_GEMM_STREAM_B | VX_GEMM_WIDE_TILES | VX_GEMM_NARROW_TILES |
-                                  VX_GEMM_OUT_HEADS | VX_GEMM_POS_F32 | VX_GEMM_CONST_B;
+                                  VX_GEMM_OUT_HEADS | VX_GEMM_POS_F32 | VX_GEMM_CONST_B | VX_GEMM_QUANT_TAIL;
   if (d->flags & ~kKnownFlags) return fail(-1, "unknown bits in flags (0x%x)", d->flags & ~kKnownFlags);
   if (qkvpack && fmt == VX_FMT_ROWSCALE)
     return fail(-1, "BIAS_QKVPACK is not available for the per-row-scaled format (use a block-scaled format or FP8)");
@@ -2094,26 +2190,46 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
     p.topk_cap = d->topk_capacity;
   } else if (d->out_dtype == VX_FP4) {
     if (d->out_fmt != VX_FMT_MX32 && d->out_fmt != VX_FMT_NV16) return fail(-1, "FP4 output: out_fmt must be MX32 or NV16");
-    if (epi == VX_EPI_BIAS_GLU || epi == VX_EPI_BIAS_RESIDUAL) return fail(-1, "FP4 output supports NONE / BIAS / BIAS_SWISH");
+    if (epi == VX_EPI_BIAS_RESIDUAL) return fail(-1, "FP4 output supports NONE / BIAS / BIAS_SWISH / BIAS_GLU");
+    if (epi == VX_EPI_BIAS_GLU && d->out_fmt != (fmt == VX_FMT_MX32 || fmt == VX_FMT_NV16 ? fmt : -1))
+      return fail(-1, "FP4 output behind GLU: MX32 or NV16 operands and the same output format");
     if (!d->out_scales_sf || !aligned16(d->out_scales_sf)) return fail(-1, "FP4 output needs out_scales_sf (16-byte aligned)");
     if (d->out_fmt == VX_FMT_NV16 && !d->out_amax) return fail(-1, "NV16 output needs out_amax");
-    if (N % 128 != 0) return fail(-1, "FP4 output needs N %% 128 == 0");
-    if (!aligned16(d->out) || d->ldo % 16 != 0 || d->ldo < N / 2) return fail(-1, "FP4 output rows must be 16-byte aligned");
+    if (n_out % 128 != 0) return fail(-1, "FP4 output needs a multiple of 128 output columns");
+    if (!aligned16(d->out) || d->ldo % 16 != 0 || d->ldo < n_out / 2) return fail(-1, "FP4 output rows must be 16-byte aligned");
     p.out_fmt = d->out_fmt;
     p.out_sf = static_cast<uint8_t*>(d->out_scales_sf);
     p.out_scales = static_cast<uint8_t*>(d->out_scales);
-    p.out_sf_kg = sf_kgroups(d->out_fmt, N);
+    p.out_sf_kg = sf_kgroups(d->out_fmt, n_out);
     p.out_amax = d->out_amax;
     if (p.out_scales && (reinterpret_cast<uintptr_t>(p.out_scales) & 3)) return fail(-1, "out_scales must be 4-byte aligned");
   } else {
     if (d->ldo < n_out) return fail(-1, "ldo=%lld < output columns %lld", (long long)d->ldo, (long long)n_out);
   }
+  const bool tail = (d->flags & VX_GEMM_QUANT_TAIL) != 0;
+  if (tail) {
+    const int64_t cols = N - d->quant_col0;
+    if ((fmt != VX_FMT_MX32 && fmt != VX_FMT_NV16) || d->out_fmt != fmt || d->out_dtype != VX_BF16 || (epi != VX_EPI_NONE && epi != VX_EPI_BIAS) ||
+        out_heads || (d->flags & VX_GEMM_DIRECT_STORE))
+      return fail(-1, "VX_GEMM_QUANT_TAIL: MX32 / NV16 operands, out_fmt the same, epilogue NONE / BIAS, bf16 output");
+    if (d->quant_col0 < 0 || d->quant_col0 % 128 != 0 || cols <= 0 || cols % 256 != 0)
+      return fail(-1, "VX_GEMM_QUANT_TAIL: quant_col0 a multiple of 128, a multiple of 256 columns behind it");
+    if (!d->out_scales || !aligned16(d->out_scales) || !d->out_scales_sf || !aligned16(d->out_scales_sf) || (fmt == VX_FMT_NV16 && !d->out_amax))
+      return fail(-1, "VX_GEMM_QUANT_TAIL needs out_scales (codes), out_scales_sf (both 16-byte aligned) and, for NV16, out_amax");
+    if (!aligned16(d->out) || (d->ldo * 2) % 16 != 0) return fail(-1, "VX_GEMM_QUANT_TAIL: 16-byte aligned output rows");
+    p.out_fmt = d->out_fmt;
+    p.out_sf = static_cast<uint8_t*>(d->out_scales_sf);
+    p.tail_codes = static_cast<uint8_t*>(d->out_scales);
+    p.quant_col0 = d->quant_col0;
+    p.out_sf_kg = sf_kgroups(d->out_fmt, cols);
+    p.out_amax = d->out_amax;
+  }
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (argmax) VX_CUDA_OK(cudaMemsetAsync(d->out, 0, static_cast<size_t>(M) * 8, st));
-  if (!argmax && d->out_dtype == VX_FP4 && p.out_sf_kg * (d->out_fmt == VX_FMT_MX32 ? 128 : 64) != N) {
+  if (!argmax && d->out_dtype == VX_FP4 && p.out_sf_kg * (d->out_fmt == VX_FMT_MX32 ? 128 : 64) != n_out) {
     // k-groups beyond N must read as zero (rows of the last tile beyond M: written as zero by the epilogue)
-    VX_CUDA_OK(cudaMemsetAsync(p.out_sf, 0, static_cast<size_t>(vx_sf_bytes(d->out_fmt, M, N)), st));
+    VX_CUDA_OK(cudaMemsetAsync(p.out_sf, 0, static_cast<size_t>(vx_sf_bytes(d->out_fmt, M, n_out)), st));
   }
 
   CUtensorMap ta, tb, to;
@@ -2153,7 +2269,7 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
   int out_route = 0;
   if (!p.sf_unit) {
     if (d->out_dtype == VX_BF16 && p.tma_store && (epi != VX_EPI_BIAS_RESIDUAL || p.tma_residual) && !argmax)
-      out_route = 1;
+      out_route = tail ? 4 : 1;
     else if (d->out_dtype == VX_FP4 && !argmax && d->out_fmt == (vec2 ? VX_FMT_MX32 : VX_FMT_NV16))
       out_route = 2;
   }

@@ -549,7 +549,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         *reinterpret_cast<uint16_t*>(p.sf_out + off) = static_cast<uint16_t>(row_ok ? sf2 : 0u);
       }
     }
-    if (lane == 0) tma_store_wait_all<0>();
+    if (lane == 0) tma_store_wait_read<0>();  // (shared memory is read; the writes complete with the grid)
   }
 
   // ---- tear-down

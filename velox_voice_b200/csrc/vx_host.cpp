@@ -597,6 +597,7 @@ struct Plan {
   bool fuse_ffn;
   int blocks;
   std::vector<Lin> lin;          // [block][L_COUNT], then the CTC head
+  Lin lp_all{};                  // the positional projections of all blocks as one weight (codes nullptr: none)
   std::vector<Norm> norm;        // [block][N_COUNT], then after_norm
   std::vector<const float*> am;  // [block][A_COUNT], then after_norm, then the positions (NV16)
   PyObject* owners = nullptr;
@@ -660,18 +661,28 @@ struct Pass {
     d.out_dtype = VX_BF16; d.out = out; d.ldo = ldo;
     run(d);
   }
-  // Swish with the result re-quantized in the epilogue
-  void gemm_swish_quant(const Act& a, const Lin& w, const Act& h) {
-    vx_gemm_desc d = desc(a, w, VX_EPI_BIAS_SWISH);
+  // Swish or GLU with the result quantized in the epilogue
+  void gemm_quant(const Act& a, const Lin& w, int epi, const Act& h) {
+    vx_gemm_desc d = desc(a, w, epi);
     d.out_dtype = VX_FP4; d.out = h.codes; d.ldo = code_ld(h.K);
     d.out_fmt = p.fmt; d.out_scales_sf = h.scales; d.out_amax = h.amax;
     run(d);
   }
+  // bf16 result whose columns from `col0` on are also quantized in the epilogue
+  void gemm_tail_quant(const Act& a, const Lin& w, void* out, int64_t ldo, int64_t col0, const Act& t) {
+    vx_gemm_desc d = desc(a, w, VX_EPI_BIAS);
+    d.out_dtype = VX_BF16; d.out = out; d.ldo = ldo;
+    d.flags |= VX_GEMM_QUANT_TAIL;
+    d.out_fmt = p.fmt; d.out_scales = t.codes; d.out_scales_sf = t.scales; d.out_amax = t.amax; d.quant_col0 = static_cast<int>(col0);
+    run(d);
+  }
   // x <- alpha w(a) + x, then the LayerNorm(s) that read x next and the quantizer: `n2` set = x <- LN_n(x) is stored and
   // LN_n2 of it quantized (the end of a block)
-  void residual(const Act& a, const Lin& w, void* x, int64_t ldx, float alpha, const Norm& n, const Norm* n2, const Act& q, bool fused) {
+  // (`from`: the residual is read there, x otherwise)
+  void residual(const Act& a, const Lin& w, void* x, int64_t ldx, float alpha, const Norm& n, const Norm* n2, const Act& q, bool fused,
+                const void* from = nullptr, int64_t ldf = 0) {
     vx_gemm_desc d = desc(a, w, VX_EPI_BIAS_RESIDUAL);
-    d.residual = x; d.residual_dtype = VX_BF16; d.ldr = ldx; d.alpha = alpha;
+    d.residual = from ? from : x; d.residual_dtype = VX_BF16; d.ldr = from ? ldf : ldx; d.alpha = alpha;
     d.out_dtype = VX_BF16; d.out = x; d.ldo = ldx;
     if (fused && g.vx_bsgemm_residual_ln_supported(p.fmt, w.N, w.K)) {
       if (n2)
@@ -694,11 +705,16 @@ void plan_free(PyObject* cap) {
   delete p;
 }
 
-// stack_plan(fmt, d, ffn, glu, vocab, eps, fuse_ffn, blocks, layers, norms, amax) -> capsule
+// Frames up to which the positional projections of all blocks run as one launch: they depend on the positions only, and
+// a pass this short is bound by its launches (twelve of 5 us against one of 10 us at 375 frames).  Beyond it their
+// outputs would take blocks * d_model columns of workspace for nothing.
+constexpr int64_t LP_BATCH_MAX = 4096;
+
+// stack_plan(fmt, d, ffn, glu, vocab, eps, fuse_ffn, blocks, layers, norms, amax, lp_all | None) -> capsule
 //   layers: sequence of (Quantized, bias | None); norms: sequence of (gamma, beta); amax: sequence of tensors, or empty
 PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   VX_BEGIN
-  VX_ARGS(11)
+  VX_ARGS(12)
   auto plan = std::make_unique<Plan>();
   plan->fmt = static_cast<int>(as_long(a[0]));
   plan->d = as_long(a[1]); plan->ffn = as_long(a[2]); plan->glu = as_long(a[3]); plan->vocab = as_long(a[4]);
@@ -733,19 +749,25 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PyObject* o = PyTuple_GET_ITEM(a[10], i);
     plan->am.push_back(o == Py_None ? nullptr : f32(o));
   }
+  if (a[11] != Py_None) {
+    Operand w;
+    if (!read_operand(a[11], w) || w.rows != plan->blocks * plan->d) bad("stack_plan: bad batched positional projection");
+    plan->lp_all = {w.codes->data_ptr(), w.codes->stride(0), w.scales, w.amax, nullptr, w.rows, w.k};
+  }
   PyObject* cap = PyCapsule_New(plan.get(), "velox_stack_plan", plan_free);
   if (!cap) return nullptr;
-  plan->owners = PyTuple_Pack(3, a[8], a[9], a[10]);
+  plan->owners = PyTuple_Pack(4, a[8], a[9], a[10], a[11]);
   plan.release();
   return cap;
   VX_END
 }
 
-// stack_forward(plan, x, pos | None, fused_ln, head, keys | None, ids | None, logits | None) -> logits / ids
-//   x bf16 [T, d] (overwritten); head 0: bf16 logits [T, vocab], 1: greedy ids i32 [T]
+// stack_forward(plan, x, pos | None, fused_ln, head, keys | None, ids | None, logits | None, source | None) -> logits / ids
+//   x bf16 [T, d] (overwritten; with `source`, bf16 [T, d], the features are read there and x only receives the residual
+//   stream); head 0: bf16 logits [T, vocab], 1: greedy ids i32 [T]
 PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   VX_BEGIN
-  VX_ARGS(8)
+  VX_ARGS(9)
   const Plan* plan = static_cast<const Plan*>(PyCapsule_GetPointer(a[0], "velox_stack_plan"));
   if (!plan) return nullptr;
   const Plan& p = *plan;
@@ -759,6 +781,16 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const at::Device dev = xt.device();
   const int64_t M = xt.size(0), ldx = xt.stride(0), d = p.d;
   void* const x = xt.data_ptr();
+  const void* src = nullptr;
+  int64_t ld_src = 0;
+  if (a[8] != Py_None) {
+    if (!is_cuda_tensor(a[8])) bad("source must be a CUDA tensor");
+    const at::Tensor& t = THPVariable_Unpack(a[8]);
+    if (t.scalar_type() != at::kBFloat16 || !rows2d(t) || t.sizes() != xt.sizes() || t.device() != xt.device())
+      bad("source must be bf16 of x's shape on x's device with unit column stride");
+    src = t.data_ptr();
+    ld_src = t.stride(0);
+  }
   Pass s{p, M, stream()};
   const bool with_pos = a[2] != Py_None;
   if (with_pos && !is_cuda_tensor(a[2])) bad("pos must be a CUDA tensor");
@@ -771,7 +803,8 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (big < M * p.glu * 2) big = M * p.glu * 2;
   big = (big + 255) / 256 * 256;
   const int64_t bp = sp.act_bytes(d);
-  const int64_t total = ba + bc + big + bp + sp.M * d * 2;
+  const bool lp_batched = with_pos && p.lp_all.codes && sp.M <= LP_BATCH_MAX;
+  const int64_t total = ba + bc + big + bp + sp.M * d * 2 * (lp_batched ? p.blocks : 1);
   const at::Tensor ws = empty({total}, at::kByte, dev);
   uint8_t* const base = static_cast<uint8_t*>(ws.data_ptr());
   uint8_t* const w_act = base;
@@ -789,34 +822,46 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     sp.quantize(pt.data_ptr(), dtype_code(pt), pt.stride(0), pos_q);
   }
   const bool fused = a[3] == Py_True;
-  auto ffn = [&](const Act& q, const Lin& w1, const Lin& w2, const float* am_h, const Norm& n, const Norm* n2, const Act& q_next) {
+  if (lp_batched) sp.gemm(pos_q, p.lp_all, VX_EPI_NONE, w_lp, p.blocks * d);
+  // the quantizers of the value third and of the GLU output run in the epilogues that produce them
+  const bool in_epilogue = p.fmt != VX_FMT_FP8_1X128 && d % 256 == 0 && p.glu % 256 == 0;
+  auto ffn = [&](const Act& q, const Lin& w1, const Lin& w2, const float* am_h, const Norm& n, const Norm* n2, const Act& q_next,
+                 const void* from = nullptr) {
     const Act h = s.act(w_big, p.ffn, am_h);
     if (p.fuse_ffn) {
-      s.gemm_swish_quant(q, w1, h);
+      s.gemm_quant(q, w1, VX_EPI_BIAS_SWISH, h);
     } else {
       void* const hb = w_big + s.act_bytes(p.ffn);
       s.gemm(q, w1, VX_EPI_BIAS_SWISH, hb, p.ffn);
       s.quantize(hb, VX_BF16, p.ffn, h);
     }
-    s.residual(h, w2, x, ldx, 0.5f, n, n2, q_next, fused);
+    s.residual(h, w2, x, ldx, 0.5f, n, n2, q_next, fused, from, ld_src);
   };
   Act q = s.act(w_act, d, p.amax(p.blocks > 0 ? A_FFM : 0));
-  s.ln_quantize(x, ldx, p.norm[p.blocks > 0 ? N_FFM : 0], q);
+  s.ln_quantize(src ? src : x, src ? ld_src : ldx, p.norm[p.blocks > 0 ? N_FFM : 0], q);
   for (int i = 0; i < p.blocks; ++i) {
     const Lin* L = &p.lin[i * L_COUNT];
     const Norm* n = &p.norm[i * N_COUNT];
     const float* const* am = p.am.empty() ? nullptr : &p.am[i * A_COUNT];
     auto mx = [&](int k) { return am ? am[k] : nullptr; };
     Act q_mha = s.act(w_act, d, mx(A_MHA)), q_conv = s.act(w_act, d, mx(A_CONV)), q_ff = s.act(w_act, d, mx(A_FF));
-    ffn(q, L[L_FFM1], L[L_FFM2], mx(A_FFM_H), n[N_MHA], nullptr, q_mha);
-    s.gemm(q_mha, L[L_QKV], VX_EPI_BIAS, w_big, 3 * d);
-    if (with_pos) sp.gemm(pos_q, L[L_LP], VX_EPI_BIAS, w_lp, d);  // feeds the attention scores only
+    ffn(q, L[L_FFM1], L[L_FFM2], mx(A_FFM_H), n[N_MHA], nullptr, q_mha, i == 0 ? src : nullptr);
     const Act ctx = s.act(w_ctx, d, mx(A_CTX));
-    s.quantize(w_big + 2 * d * 2, VX_BF16, 3 * d, ctx);
+    if (in_epilogue) {
+      s.gemm_tail_quant(q_mha, L[L_QKV], w_big, 3 * d, 2 * d, ctx);
+    } else {
+      s.gemm(q_mha, L[L_QKV], VX_EPI_BIAS, w_big, 3 * d);
+      s.quantize(w_big + 2 * d * 2, VX_BF16, 3 * d, ctx);
+    }
+    if (with_pos && !lp_batched) sp.gemm(pos_q, L[L_LP], VX_EPI_BIAS, w_lp, d);  // feeds the attention scores only
     s.residual(ctx, L[L_LO], x, ldx, 1.0f, n[N_CONV], nullptr, q_conv, fused);
-    s.gemm(q_conv, L[L_PW1], VX_EPI_BIAS_GLU, w_big, p.glu);
     const Act gl = s.act(w_ctx, p.glu, mx(A_GLU));
-    s.quantize(w_big, VX_BF16, p.glu, gl);
+    if (in_epilogue) {
+      s.gemm_quant(q_conv, L[L_PW1], VX_EPI_BIAS_GLU, gl);
+    } else {
+      s.gemm(q_conv, L[L_PW1], VX_EPI_BIAS_GLU, w_big, p.glu);
+      s.quantize(w_big, VX_BF16, p.glu, gl);
+    }
     s.residual(gl, L[L_PW2], x, ldx, 1.0f, n[N_FF], nullptr, q_ff, fused);
     // norm_final of this block and the LayerNorm that reads it next: the first of the next block, or after_norm
     const bool last = i + 1 == p.blocks;

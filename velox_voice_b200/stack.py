@@ -13,13 +13,13 @@ convolution and its norm/activation are NOT linear layers and are outside this l
 stack passes the value projection straight to ``lo`` and the GLU output straight to ``pw2``,
 so it measures and validates every linear of the encoder with the real operand shapes.
 
-Kernel sequence per block (13 launches, issued by the native host path ``csrc/vx_host.cpp``; the reference issues >= 4
-per linear):
-``GEMM(bias, swish, FP4 out) -> GEMM(bias, 0.5 residual)`` for each FFN (the second one behind
-its ``ln_quant``), ``ln_quant -> GEMM(bias) [qkv] -> quant -> GEMM(bias, residual) [lo]``,
-``GEMM [lp]``, ``ln_quant -> GEMM(bias, GLU) -> quant -> GEMM(bias, residual)``, and one
-``ln2_quant`` kernel that applies norm_final, stores the residual stream and hands the next
-block's first FFN (or the CTC head, through after_norm) its quantized input.  The greedy head
+Kernel sequence per block (13 launches, 9 where the residual GEMMs also run the LayerNorm + quantizer behind
+them; issued by the native host path ``csrc/vx_host.cpp``; the reference issues >= 4 per linear):
+``GEMM(bias, swish, FP4 out) -> GEMM(bias, 0.5 residual)`` for each FFN (the second one behind its ``ln_quant``),
+``ln_quant -> GEMM(bias, value third also quantized) [qkv] -> GEMM(bias, residual) [lo]``, ``GEMM [lp]`` (one launch
+for all blocks on short inputs), ``ln_quant -> GEMM(bias, GLU, FP4 out) -> GEMM(bias, residual)``, and one ``ln2_quant``
+kernel that applies norm_final, stores the residual stream and hands the next block's first FFN (or the CTC head,
+through after_norm) its quantized input (FP8: 15, the value third and the GLU output have quantizer launches).  The greedy head
 (:meth:`ConformerLinearStack.forward_ids`) takes the per-frame argmax inside the CTC GEMM's
 epilogue, so the [T, vocab] logits are never written.
 
@@ -42,6 +42,13 @@ from .linear import PackedLinear, glu_tile
 from .ops import FMT_FP8_1X128, FMT_MX32, FMT_NV16
 
 
+# Frames from which the residual GEMMs run the LayerNorm + quantizer behind them (two-CTA clusters, a row block each).  Up
+# to 37 row blocks the separate residual GEMM takes a single round over 148 SMs (four column blocks each) and is faster
+# (12 blocks, 3,750 frames: 955 vs 996 us); beyond, its second round costs more than the clusters' work (5,000 frames:
+# 1,228 vs 1,155 us; 9,472: 1,550 vs 1,392; 40,000: 4,267 vs 4,102).
+FUSE_LN_FRAMES = 37 * 128 + 1
+
+
 @dataclass
 class StackConfig:
     d_model: int = 512
@@ -54,9 +61,7 @@ class StackConfig:
     eps: float = 1e-5
     fuse_ffn: bool = True  # keep the FFN intermediate in FP4 (re-quantized in the up-GEMM epilogue)
     fuse_ln: bool = True   # MX32, d_model 512: the residual GEMMs also run the LayerNorm + quantizer behind them
-    # ... from this many frames on: the fused kernel walks 128-row blocks with 74 two-CTA clusters at ~5 us a
-    # block, which pays once every cluster has a few blocks (per step: 8.64 vs 9.13 ms at 90,000 frames, 2.82
-    # vs 2.89 ms at 22,500) and no longer does on a short shard (11,250 frames, 88 blocks: 1.81 vs 1.80 ms)
+    # ... at the latest from this many frames on (a smaller value moves the line down; see FUSE_LN_FRAMES)
     fuse_ln_min_frames: int = 16384
 
     def flops_per_frame(self) -> int:
@@ -108,7 +113,7 @@ class ConformerLinearStack:
         # VELOX_B200_FUSE_LN_MIN_FRAMES overrides their frame threshold, for A/B timing)
         self.fuse_ln = (bool(cfg.fuse_ln) and os.environ.get("VELOX_B200_FUSE_LN", "1") != "0"
                         and ops.residual_ln_supported(self.fmt, cfg.d_model, cfg.d_model))
-        self.fuse_ln_min_frames = int(os.environ.get("VELOX_B200_FUSE_LN_MIN_FRAMES", cfg.fuse_ln_min_frames))
+        self.fuse_ln_min_frames = int(os.environ.get("VELOX_B200_FUSE_LN_MIN_FRAMES", min(cfg.fuse_ln_min_frames, FUSE_LN_FRAMES)))
         dev = self.device
         self.p: Dict[str, PackedLinear] = {}
         self.ln: Dict[str, Tuple[torch.Tensor, torch.Tensor]] = {}
@@ -167,14 +172,27 @@ class ConformerLinearStack:
             if self.fmt == FMT_NV16:
                 amax += [self._amax("after", None), self.amax.get("pos")]
             self._plan = ops._host().stack_plan(self.fmt, cfg.d_model, cfg.ffn, cfg.conv_pw // 2, cfg.vocab, cfg.eps, self.fuse_ffn,
-                                                cfg.blocks, tuple(layers), tuple(norms), tuple(amax))
+                                                cfg.blocks, tuple(layers), tuple(norms), tuple(amax), self._lp_all())
         return self._plan
+
+    def _lp_all(self):
+        """The positional projections of all blocks as one weight [blocks * d_model, d_model] (short passes run them in
+        one launch), or None where their packed rows cannot simply be stacked."""
+        cfg = self.cfg
+        if cfg.blocks == 0 or cfg.d_model % 128 != 0 or self.fmt == FMT_NV16:  # (NV16: a tensor scale per weight)
+            return None
+        qs = [self.p[f"b{i}.lp"].q for i in range(cfg.blocks)]
+        cat = lambda ts: None if ts[0] is None else torch.cat(ts)
+        return ops.Quantized(self.fmt, cfg.blocks * cfg.d_model, cfg.d_model, cat([q.codes for q in qs]), cat([q.scales for q in qs]),
+                             cat([q.sf for q in qs]), None)
 
     # ---- forward
     def forward(self, x: torch.Tensor, pos: Optional[torch.Tensor] = None, *, return_hidden: bool = False,
-                ids_only: bool = False, keys=None, ids=None, out_logits: Optional[torch.Tensor] = None):
+                ids_only: bool = False, keys=None, ids=None, out_logits: Optional[torch.Tensor] = None,
+                source: Optional[torch.Tensor] = None):
         """x: bf16 [T, d_model] residual stream (overwritten in place); returns bf16 logits [T, vocab]
-        (written into ``out_logits`` when given: bf16 [T, vocab], unit column stride).
+        (written into ``out_logits`` when given: bf16 [T, vocab], unit column stride).  With ``source``
+        (bf16 of x's shape) the features are read from there and x only receives the residual stream.
 
         One call of the native host path issues every launch of the pass (``vx_host.cpp``,
         ``stack_forward``); its intermediates share one workspace block."""
@@ -185,7 +203,8 @@ class ConformerLinearStack:
         if pos is not None and pos.stride(1) != 1:
             pos = pos.contiguous()
         fused = self.fuse_ln and x.shape[0] >= self.fuse_ln_min_frames
-        out = ops._host().stack_forward(self._host_plan(), x, pos, fused, 1 if ids_only else 0, keys, ids, out_logits)
+        out = ops._host().stack_forward(self._host_plan(), x, pos, fused, 1 if ids_only else 0, keys, ids, out_logits,
+                                         source)
         return (out, x) if return_hidden and not ids_only else out
 
     def forward_ids(self, x: torch.Tensor, pos: Optional[torch.Tensor] = None, *, keys=None, ids=None):
@@ -290,8 +309,7 @@ class CompiledStack:
         torch.cuda.synchronize(dev)
 
     def _body(self):
-        self._x.copy_(self.x_in)
-        self.ids = self.stack.forward_ids(self._x, self.pos, keys=self._keys, ids=self._ids)
+        self.ids = self.stack.forward(self._x, self.pos, ids_only=True, keys=self._keys, ids=self._ids, source=self.x_in)
 
     def run(self):
         self.graph.replay()
