@@ -193,7 +193,9 @@ int vx_bsgemm(const vx_gemm_desc* desc, void* stream);
  * vx_quantize_pack(ROWSCALE) of the activation rows and vx_bsgemm (NONE / BIAS, fp32 out).  Replaces
  * DenseLinear.forward (veloxvoice/models/wenet/torch_conformer.py:251-266: pad copy, cast, quantizer, GEMM, slice, bias add).
  *   w_codes u8 [N, K/2] (row stride ldw bytes), w_scales u8 [N]: the packed weight, a constant as for VX_GEMM_CONST_B;
- *   scratch at least M * (K/2 + 1) bytes, 16-byte aligned: the quantized activation. */
+ *   scratch at least vx_rowscale_linear_scratch(M, N, K) bytes, 16-byte aligned: the quantized activation (0 bytes and
+ *   NULL where few rows run in one launch). */
+int64_t vx_rowscale_linear_scratch(int64_t M, int64_t N, int64_t K);
 int vx_rowscale_linear(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const void* w_codes, int64_t ldw,
                        const void* w_scales, int64_t N, const float* bias, void* scratch, float* out, int64_t ldo, void* stream);
 

@@ -66,6 +66,7 @@ EXPORTS = (
     "vx_bsgemm_residual_ln2",
     "vx_sf_from_natural_pair",
     "vx_rowscale_linear",
+    "vx_rowscale_linear_scratch",
     "vx_ctc_topk_rows",
     "vx_ctc_topk",
 )
@@ -166,6 +167,8 @@ def load(build_if_missing: bool = True) -> C.CDLL:
         lib.vx_sf_from_natural.argtypes = [i32, vp, i64, i64, vp, vp]
         lib.vx_sf_from_natural_pair.restype = i32
         lib.vx_sf_from_natural_pair.argtypes = [i32, vp, i64, vp, i32, vp, i64, vp, i64, vp]
+        lib.vx_rowscale_linear_scratch.restype = i64
+        lib.vx_rowscale_linear_scratch.argtypes = [i64, i64, i64]
         lib.vx_rowscale_linear.restype = i32
         lib.vx_rowscale_linear.argtypes = [vp, i32, i64, i64, i64, vp, i64, vp, i64, vp, vp, vp, i64, vp]
         lib.vx_ctc_topk_rows.restype = i64

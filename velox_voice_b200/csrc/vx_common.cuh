@@ -73,6 +73,9 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Per-row quantization of an activation: vx_quantize_pack(ROWSCALE) that lets the next launch start under its tail.
+int quantize_rowscale_activation(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, void* codes, void* scales, void* stream);
+
 #define VX_CUDA_OK(expr)                                                        \
   do {                                                                          \
     cudaError_t _e = (expr);                                                    \

@@ -29,7 +29,7 @@ namespace {
 #define VX_FUNCS(X)                                                                                                 \
   X(vx_last_error) X(vx_quantize_pack) X(vx_ln_quantize_pack) X(vx_ln2_quantize_pack) X(vx_amax) X(vx_bsgemm)        \
   X(vx_bsgemm_residual_ln_supported) X(vx_bsgemm_residual_ln) X(vx_bsgemm_residual_ln2) X(vx_argmax_ids) X(vx_relpos_attention)   \
-  X(vx_power_mel_log) X(vx_power_mel_log_supported) X(vx_sf_from_natural_pair) X(vx_rowscale_linear) X(vx_ctc_topk_rows) X(vx_ctc_topk)
+  X(vx_power_mel_log) X(vx_power_mel_log_supported) X(vx_sf_from_natural_pair) X(vx_rowscale_linear) X(vx_rowscale_linear_scratch) X(vx_ctc_topk_rows) X(vx_ctc_topk)
 struct Api {
 #define X(f) decltype(&::f) f = nullptr;
   VX_FUNCS(X)
@@ -373,8 +373,8 @@ PyObject* py_residual_ln(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   VX_END
 }
 
-// rowscale_linear(x [..., K], wq [N, K/2], ws [N], bias | None) -> f32 [..., N] | None: the reference's per-row lane, both
-// launches of a layer.
+// rowscale_linear(x [..., K], wq [N, K/2], ws [N], bias | None) -> f32 [..., N] | None: the reference's per-row lane, one
+// or two launches.
 PyObject* py_rowscale_linear(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   VX_BEGIN
   VX_ARGS(4)
@@ -391,14 +391,16 @@ PyObject* py_rowscale_linear(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   bool ok = true;
   const float* bias = vector_arg(p[3], N, dev, ok);
   if (!ok) Py_RETURN_NONE;
-  const at::Tensor scratch = empty({M * (K / 2 + 1)}, at::kByte, dev);
+  const int64_t need = g.vx_rowscale_linear_scratch(M, N, K);
+  at::Tensor scratch;
+  if (need) scratch = empty({need}, at::kByte, dev);
   c10::SmallVector<int64_t, 8> shape(x.sizes().begin(), x.sizes().end());
   shape.back() = N;
   const at::Tensor out = empty(shape, at::kFloat, dev);
-  check(g.vx_rowscale_linear(x.data_ptr(), dt, M, K, K, wq.data_ptr(), wq.stride(0), ws.data_ptr(), N, bias, scratch.data_ptr(),
+  check(g.vx_rowscale_linear(x.data_ptr(), dt, M, K, K, wq.data_ptr(), wq.stride(0), ws.data_ptr(), N, bias, ptr(scratch),
                              static_cast<float*>(out.data_ptr()), N, stream()),
         "vx_rowscale_linear");
-  count(2);
+  count(need ? 2 : 1);
   return wrap(out);
   VX_END
 }

@@ -229,4 +229,39 @@ __device__ __forceinline__ float ue8m0_to_float(uint32_t byte) {
   return __uint_as_float(byte ? (byte << 23) : 0x00400000u);
 }
 
+// Eight consecutive elements as loaded (not yet converted): lets a kernel issue the loads of
+// rows it will work on later before it works on the current one.  Converted, the eight values
+// are four packed fp32 pairs (element 2 i in the low half of pair i): the arithmetic below uses
+// the packed fp32x2 instructions of sm_100, which round each half exactly like the scalar ones.
+template <typename T> struct Raw8;
+template <> struct Raw8<__nv_bfloat16> {
+  uint4 u;
+  // plain (coherent) loads: the LayerNorm kernels may store y over x while other rows are still read
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { u = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void zero() { u = make_uint4(0, 0, 0, 0); }
+  __device__ __forceinline__ void get(uint64_t (&v)[4]) const {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = pack_f32x2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+  }
+};
+template <> struct Raw8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void load(const float* p) {
+    a = *reinterpret_cast<const float4*>(p);
+    b = *(reinterpret_cast<const float4*>(p) + 1);
+  }
+  __device__ __forceinline__ void zero() { a = b = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ __forceinline__ void get(uint64_t (&v)[4]) const {
+    v[0] = pack_f32x2(a.x, a.y); v[1] = pack_f32x2(a.z, a.w);
+    v[2] = pack_f32x2(b.x, b.y); v[3] = pack_f32x2(b.z, b.w);
+  }
+};
+
+__device__ __forceinline__ float warp_max(float a) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
+  return a;
+}
+
 }  // namespace vx
