@@ -9,20 +9,24 @@
 // CUDA kernel for the chunked case is veloxvoice/kernels/csrc/velox_chunk_rel_pos_attn.cu:23-114).  The zero
 // half of v2 is never read and the result lands token-major, ready for the output projection's quantizer.
 //
-// One CTA = 128 queries of one head, all on the 5th-generation tensor cores (tcgen05.mma kind::f16, bf16
-// operands, fp32 accumulators in tensor memory):
-//   warp 0      TMA producer: Q once, then K (and V) tiles of 128 keys through a three-stage ring;
-//   warp 1      MMA issuer: S = Q K^T (128 x 128 x 128) into one of two S accumulators, O += P V
-//               (128 x 64 x 128; V is read in its natural [key][dv] layout as an MN-major operand);
-//   warps 2..9  softmax, one query row per thread straight out of tensor memory; two warps share a row
-//               (64 of a tile's 128 keys each) and exchange their maxima / sums through shared memory once.
+// One CTA = 128 queries of one head, TWO CTAs PER SM (half the shared and tensor memory each), all on the 5th-generation
+// tensor cores (tcgen05.mma kind::f16, bf16 operands, fp32 accumulators in tensor memory):
+//   warps 0..3  softmax, one query row per thread straight out of tensor memory, 64 keys per step;
+//   warp 4      TMA producer: K and V tiles of 64 keys through a four-stage ring;
+//   warp 5      MMA issuer: S = Q K^T (128 x 64 x 128) into one of two S buffers, O += P V (128 x 64 x 64; V is read in its
+//               natural [key][dv] layout as an MN-major operand).
+// Q and P are A operands in TENSOR MEMORY: Q is put there once by the softmax warps, P (bf16) replaces the S it was made
+// from, so the MMAs read only K and V from shared memory and no proxy fence stands between the softmax and P V.
+// Tensor memory (256 columns): S0 | S1 (64 each; P in the lower half) | O (64) | Q (64).
 // One pass over the keys with a lazily updated reference maximum: p = 2^((s - m_ref) log2 e) is formed
 // against the reference m_ref the row has used so far, which only moves when a tile's maximum exceeds it by
 // more than 2^8 (so p never exceeds 256 and nothing overflows in bf16 or fp32).  When it moves -- typically in
-// the first tiles of a row only -- the row sum and the row's part of the O accumulator in tensor memory are
-// multiplied by 2^((m_old - m_new) log2 e) (tcgen05.ld / tcgen05.st of 32 columns per warp) before the next
-// P V product is released.  P is written as bf16 into the swizzled K-major tile the P V product reads; O is
-// divided by the row sum once at the end.
+// the first tiles of a row only -- the row sum and the row's O accumulator are multiplied by 2^((m_old - m_new) log2 e)
+// (tcgen05.ld / tcgen05.st) before the next P V product is released.  O is divided by the row sum once at the end.
+// What bounds it: the special-function unit (64 exponentials per row and step, 16 lanes per cycle and SM: 512 cycles per CTA and
+// step against 384 of MMAs), as long as the two CTAs of an SM fill each other's hand-over latencies.  The form with one
+// CTA of eight softmax warps per SM, P through shared memory and a maximum exchange between two warps per row took 3,200
+// cycles per 128 x 128 tile: 99 us for 3,750 frames and 8 heads -> MEASURED
 // Every mbarrier wait is bounded.
 
 #include <cuda.h>
@@ -34,40 +38,39 @@
 
 #include "vx_common.cuh"
 #include "vx_ptx.cuh"
+#include "vx_quant_math.cuh"
 #include "vx_tmap.cuh"
 
 namespace vx {
 namespace {
 
 constexpr int AT_BM = 128;   // queries per CTA = TMEM lanes
-constexpr int AT_BN = 128;   // keys per tile
+constexpr int AT_BN = 64;    // keys per tile
 constexpr int AT_D = 128;    // folded head dimension (2 dk)
 constexpr int AT_DV = 64;    // value dimension (dk)
-constexpr int AT_PANEL = AT_BM * 128;            // one 64-column bf16 panel of 128 rows: 16 KB
-constexpr int AT_Q_BYTES = 2 * AT_PANEL;          // 32 KB
-constexpr int AT_K_BYTES = 2 * AT_PANEL;          // 32 KB
-constexpr int AT_V_BYTES = AT_BN * AT_DV * 2;     // 16 KB
-constexpr int AT_STAGE = AT_K_BYTES + AT_V_BYTES; // 48 KB
-constexpr int AT_P_BYTES = 2 * AT_PANEL;          // 32 KB
-constexpr int AT_NS = 3;                          // K / V stages in flight
-constexpr int AT_SMEM = AT_Q_BYTES + AT_NS * AT_STAGE + AT_P_BYTES + 1024;
-constexpr int AT_SOFTMAX_WARPS = 8;  // two per 32-row quadrant of tensor memory: 64 of a tile's 128 keys each
-constexpr int AT_THREADS = (2 + AT_SOFTMAX_WARPS) * 32;
-constexpr uint32_t AT_TM_S = 0, AT_TM_O = 256;    // S0 | S1 (128 columns each) | O (64 columns)
+constexpr int AT_K_PANEL = AT_BN * 128;           // one 64-column bf16 panel of a K tile: 8 KB
+constexpr int AT_K_BYTES = 2 * AT_K_PANEL;
+constexpr int AT_V_BYTES = AT_BN * AT_DV * 2;     // 8 KB
+constexpr int AT_STAGE = AT_K_BYTES + AT_V_BYTES; // 24 KB
+constexpr int AT_NS = 4;                          // K / V stages in flight
+constexpr int AT_SMEM = AT_NS * AT_STAGE + 1024;
+constexpr int AT_SOFTMAX_WARPS = 4;
+constexpr int AT_THREADS = (AT_SOFTMAX_WARPS + 2) * 32;
+constexpr uint32_t AT_TM_S = 0, AT_TM_O = 128, AT_TM_Q = 192, AT_TM_COLS = 256;
 
 struct AttnParams {
   int64_t T;        // queries and keys per head
   int64_t kv_len;   // keys j >= kv_len are masked
   int heads;
+  const __nv_bfloat16* q;
   __nv_bfloat16* out;
   int64_t ldo;
   int* status;
 };
 
 struct AttnBarriers {
-  uint64_t q_full, kv_full[AT_NS], kv_empty[AT_NS], s_full[2], s_empty[2], p_full, p_empty, o_full;
+  uint64_t q_full, kv_full[AT_NS], kv_empty[AT_NS], s_full[2], p_full[2], pv_done;
   uint32_t tmem_base;
-  float xch[2][2][AT_BM];  // [tile parity][half][row]: tile maxima (finally row sums) of the two warps that share a row
 };
 
 // bf16 x bf16 -> fp32, A K-major; B K-major or MN-major (b_mn)
@@ -75,11 +78,12 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int M, int N, bool b_mn) 
   return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | (static_cast<uint32_t>(N >> 3) << 17) |
          (static_cast<uint32_t>(M >> 4) << 24);
 }
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// A from tensor memory (lane = row, two consecutive K elements per 32-bit column), B from shared memory
+__device__ __forceinline__ void mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // shared-memory descriptor with the 128-byte swizzle and explicit leading / stride byte offsets
@@ -114,43 +118,35 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-__global__ void __launch_bounds__(AT_THREADS, 1)
-relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                   const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
+__global__ void __launch_bounds__(AT_THREADS, 2)
+relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* const base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* const q_s = base;
-  uint8_t* const st_s = base + AT_Q_BYTES;        // AT_NS stages of [K | V]
-  uint8_t* const p_s = st_s + AT_NS * AT_STAGE;
+  uint8_t* const st_s = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   __shared__ AttnBarriers bar;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.y;
   const int64_t q0 = static_cast<int64_t>(blockIdx.x) * AT_BM;
-  const int nkb = static_cast<int>((p.kv_len + AT_BN - 1) / AT_BN);
-  const int iters = nkb;
+  const int steps = static_cast<int>((p.kv_len + AT_BN - 1) / AT_BN);
   const int row_base = static_cast<int>(head * p.T);  // this head's token 0 in the [heads * T, 128] views
 
   if (threadIdx.x == 0) {
-    mbar_init(&bar.q_full, 1);
+    mbar_init(&bar.q_full, AT_SOFTMAX_WARPS);
     for (int s = 0; s < AT_NS; ++s) {
       mbar_init(&bar.kv_full[s], 1);
       mbar_init(&bar.kv_empty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bar.s_full[s], 1);
-      mbar_init(&bar.s_empty[s], AT_SOFTMAX_WARPS);
+      mbar_init(&bar.p_full[s], AT_SOFTMAX_WARPS);
     }
-    mbar_init(&bar.p_full, AT_SOFTMAX_WARPS);
-    mbar_init(&bar.p_empty, 1);
-    mbar_init(&bar.o_full, 1);
+    mbar_init(&bar.pv_done, 1);
     mbar_fence_init();
-    prefetch_tmap(&tm_q);
     prefetch_tmap(&tm_k);
     prefetch_tmap(&tm_v);
   }
-  if (warp == 1) {
-    tmem_alloc(&bar.tmem_base, 512);
+  if (warp == AT_SOFTMAX_WARPS + 1) {
+    tmem_alloc(&bar.tmem_base, AT_TM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -159,207 +155,201 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   const uint32_t tmem_base = bar.tmem_base;
   pdl_wait();  // set-up done: from here on the kernel touches what the previous kernel of the stream produced
 
-  if (warp == 0) {
+  if (warp == AT_SOFTMAX_WARPS) {
     // =========================== TMA producer ===========================
     if (lane == 0) {
-      mbar_expect_tx(&bar.q_full, AT_Q_BYTES);
-      tma_load_2d(q_s, &tm_q, 0, row_base + static_cast<int>(q0), &bar.q_full);
-      tma_load_2d(q_s + AT_PANEL, &tm_q, 64, row_base + static_cast<int>(q0), &bar.q_full);
-      for (int it = 0; it < iters; ++it) {
-        const int s = it % AT_NS, j = it;
-        if (!mbar_wait(&bar.kv_empty[s], ((it / AT_NS) & 1) ^ 1, p.status, 20)) break;
+      for (int j = 0; j < steps; ++j) {
+        const int s = j % AT_NS;
+        if (!mbar_wait(&bar.kv_empty[s], ((j / AT_NS) & 1) ^ 1, p.status, 20)) break;
         uint8_t* const dst = st_s + s * AT_STAGE;
-        mbar_expect_tx(&bar.kv_full[s], AT_K_BYTES + AT_V_BYTES);
+        mbar_expect_tx(&bar.kv_full[s], AT_STAGE);
         tma_load_2d(dst, &tm_k, 0, row_base + j * AT_BN, &bar.kv_full[s]);
-        tma_load_2d(dst + AT_PANEL, &tm_k, 64, row_base + j * AT_BN, &bar.kv_full[s]);
+        tma_load_2d(dst + AT_K_PANEL, &tm_k, 64, row_base + j * AT_BN, &bar.kv_full[s]);
         tma_load_2d(dst + AT_K_BYTES, &tm_v, 0, row_base + j * AT_BN, &bar.kv_full[s]);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == AT_SOFTMAX_WARPS + 1) {
     // =========================== MMA issuer ===========================
     const bool leader = elect_one();
     const uint32_t idesc_s = make_idesc_bf16(AT_BM, AT_BN, false);
     const uint32_t idesc_o = make_idesc_bf16(AT_BM, AT_DV, true);
-    const uint32_t q_u32 = smem_u32(q_s), st_u32 = smem_u32(st_s), p_u32 = smem_u32(p_s);
+    const uint32_t st_u32 = smem_u32(st_s);
     bool ok = mbar_wait_spin(&bar.q_full, 0, p.status, 21);
-    // S(it) = Q K_j^T into accumulator it & 1
-    auto issue_s = [&](int it) {
-      const int s = it & 1, ks = it % AT_NS;  // S accumulator, K / V stage
-      if (!mbar_wait_spin(&bar.kv_full[ks], (it / AT_NS) & 1, p.status, 22)) return false;
-      if (!mbar_wait_spin(&bar.s_empty[s], ((it >> 1) & 1) ^ 1, p.status, 23)) return false;
+    // S(j) = Q K_j^T into buffer j & 1 (the P V product of step j - 2, which read P there, has completed)
+    auto issue_s = [&](int j) {
+      if (!mbar_wait_spin(&bar.kv_full[j % AT_NS], (j / AT_NS) & 1, p.status, 22)) return false;
       tc_fence_after();
       if (leader) {
-        const uint32_t k_u32 = st_u32 + ks * AT_STAGE;
+        const uint32_t k_u32 = st_u32 + (j % AT_NS) * AT_STAGE;
 #pragma unroll
-        for (int i = 0; i < AT_D / 16; ++i) {
-          const uint32_t off = (i >> 2) * AT_PANEL + (i & 3) * 32;
-          mma_bf16(tmem_base + AT_TM_S + s * 128, make_desc_k128(q_u32 + off), make_desc_k128(k_u32 + off), idesc_s, i != 0);
-        }
-        tc_commit(&bar.s_full[s]);
+        for (int i = 0; i < AT_D / 16; ++i)
+          mma_bf16_ta(tmem_base + AT_TM_S + (j & 1) * AT_BN, tmem_base + AT_TM_Q + i * 8,
+                      make_desc_k128(k_u32 + (i >> 2) * AT_K_PANEL + (i & 3) * 32), idesc_s, i != 0);
+        if (j & 1) tc_commit(&bar.s_full[1]);
+        else tc_commit(&bar.s_full[0]);
       }
       __syncwarp();
       return true;
     };
-    if (ok && iters > 0) ok = issue_s(0);
-    for (int it = 0; it < iters && ok; ++it) {
-      if (it + 1 < iters) ok = issue_s(it + 1);
-      if (!ok) break;
-      {
-        const int n = it;
-        if (!mbar_wait_spin(&bar.p_full, n & 1, p.status, 24)) { ok = false; break; }
-        tc_fence_after();
-        if (leader) {
-          const uint32_t v_u32 = st_u32 + (it % AT_NS) * AT_STAGE + AT_K_BYTES;
+    if (ok) ok = issue_s(0);
+    if (ok && steps > 1) ok = issue_s(1);
+    for (int j = 0; j < steps && ok; ++j) {
+      if (!mbar_wait_spin(&bar.p_full[j & 1], (j >> 1) & 1, p.status, 24)) { ok = false; break; }
+      tc_fence_after();
+      if (leader) {
+        const uint32_t v_u32 = st_u32 + (j % AT_NS) * AT_STAGE + AT_K_BYTES;
+        // V tile as TMA wrote it: one 128-byte row of 64 dv values per key, 8-key swizzle atoms 1 KB apart
+        // (the stride offset of the MN-major operand); 64 dv values are one group along N, so the leading
+        // offset is not used.  A K = 16 step is two atoms.
 #pragma unroll
-          for (int i = 0; i < AT_BN / 16; ++i) {
-            const uint32_t aoff = (i >> 2) * AT_PANEL + (i & 3) * 32;
-            // V tile as TMA wrote it: one 128-byte row of 64 dv values per key, 8-key swizzle atoms 1 KB apart
-            // (the stride offset of the MN-major operand); 64 dv values are one group along N, so the leading
-            // offset is not used.  A K = 16 step is two atoms.
-            mma_bf16(tmem_base + AT_TM_O, make_desc_k128(p_u32 + aoff), make_desc_sw128(v_u32 + i * 16 * 128, 0, 1024),
-                     idesc_o, (n | i) != 0);
-          }
-          tc_commit(&bar.p_empty);
-          tc_commit(&bar.kv_empty[it % AT_NS]);
-          if (it == iters - 1) tc_commit(&bar.o_full);
-        }
-        __syncwarp();
+        for (int i = 0; i < AT_BN / 16; ++i)
+          mma_bf16_ta(tmem_base + AT_TM_O, tmem_base + AT_TM_S + (j & 1) * AT_BN + i * 8, make_desc_sw128(v_u32 + i * 16 * 128, 0, 1024),
+                      idesc_o, (j | i) != 0);
+        tc_commit(&bar.pv_done);
+        tc_commit(&bar.kv_empty[j % AT_NS]);
+      }
+      __syncwarp();
+      if (j + 2 < steps) {
+        if (!mbar_wait_spin(&bar.pv_done, j & 1, p.status, 23)) { ok = false; break; }
+        ok = issue_s(j + 2);
       }
     }
   } else {
-    // =========================== softmax: warps 2..9 ===========================
-    // warp -> (quadrant q of tensor memory = rows 32 q .. 32 q + 31, half of the tile's keys / of O's columns)
-    const int q = warp & 3, half = (warp - 2) >> 2;
-    const int row = q * 32 + lane;
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    // =========================== softmax: warps 0..3, thread = query row ===========================
+    const int row = warp * 32 + lane;
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+    const int64_t tq = q0 + row;
     constexpr float L2E = 1.4426950408889634f;
     const float NEG_INF = __int_as_float(0xff800000);
-    float m_ref = NEG_INF;  // reference maximum of the row, in units of log2 (s * log2 e)
-    float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    auto softmax_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(AT_SOFTMAX_WARPS * 32) : "memory"); };
-    bool ok = true;
-    int syncs = 0;  // named barriers this thread has executed (every softmax thread executes nkb + 1 of them)
-    for (int it = 0; it < iters && ok; ++it) {
-      const int b = it & 1;
-      if (lane == 0) ok = mbar_wait(&bar.s_full[b], (it >> 1) & 1, p.status, 25);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      tc_fence_after();
-      const int n_valid = static_cast<int>(p.kv_len - static_cast<int64_t>(it) * AT_BN);  // >= 128: the whole tile
-      // this warp's 64 keys of the tile, scaled to log2 units
-      float t[2][32];
+    {
+      // this row's Q: 128 bf16 -> 64 columns
+      const uint4* src = reinterpret_cast<const uint4*>(p.q + (static_cast<int64_t>(row_base) + (tq < p.T ? tq : 0)) * AT_D);
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
+      for (int h = 0; h < 2; ++h) {
         uint32_t r[32];
-        tc_ld_32x32b_x32(lane_addr + AT_TM_S + b * 128 + (half * 2 + cc) * 32, r);
-        tc_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 32; ++i) t[cc][i] = __uint_as_float(r[i]) * L2E;
+        for (int i = 0; i < 8; ++i) {
+          const uint4 u = src[h * 8 + i];
+          r[4 * i] = u.x; r[4 * i + 1] = u.y; r[4 * i + 2] = u.z; r[4 * i + 3] = u.w;
+        }
+        tc_st_32x32b_x32(lane_addr + AT_TM_Q + h * 32, r);
       }
+      tc_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bar.s_empty[b]);  // S is in registers: the accumulator may be overwritten
-      if (n_valid < AT_BN) {
-        // the last tile of a span whose length is not a multiple of 128: keys beyond kv_len count as -inf
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if ((half * 2 + cc) * 32 + i >= n_valid) t[cc][i] = NEG_INF;
-      }
-      float m4[4] = {NEG_INF, NEG_INF, NEG_INF, NEG_INF};
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-        for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], t[cc][i]);
-      const float mine = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-      bar.xch[it & 1][half][row] = mine;
-      softmax_sync();
-      ++syncs;
-      const float m_tile = fmaxf(mine, bar.xch[it & 1][half ^ 1][row]);
-      // The reference of a row moves when the tile's maximum exceeds it by more than 8 (both warps of a row
-      // decide alike: same lanes, same values).  Then the row sum and this warp's 32 columns of O are scaled by
-      // 2^(m_ref - m_tile).  The tensor-memory accesses are warp-wide, so the warp goes through them when any of
-      // its rows moves; the other rows scale by one.  Before the first P V product there is nothing to scale.
-      const bool moves = m_tile > m_ref + 8.0f;
-      const bool any_moves = __any_sync(0xffffffffu, moves);
-      const float alpha = moves ? ex2f(m_ref - m_tile) : 1.0f;  // 0 for m_ref = -inf
-      if (moves) m_ref = m_tile;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) l4[i] *= alpha;
-      // the exponentials (the special-function unit is the busiest pipe here) run while the tensor core is still
-      // on the previous tile's P V product
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          t[cc][i] = ex2f(t[cc][i] - m_ref);
-          l4[i & 3] += t[cc][i];
-        }
-      // P V of the previous tile complete: the P tile may be overwritten and O may be corrected
-      if (lane == 0) ok = mbar_wait(&bar.p_empty, (it & 1) ^ 1, p.status, 26);
+      if (lane == 0) mbar_arrive(&bar.q_full);
+    }
+    float m_ref = NEG_INF;  // reference maximum of the row, in units of log2 (s * log2 e)
+    uint64_t l2[2] = {0ull, 0ull};  // row sum, four partial sums as packed pairs
+    bool ok = true;
+    for (int j = 0; j < steps; ++j) {
+      const int b = j & 1;
+      if (lane == 0) ok = mbar_wait_spin(&bar.s_full[b], (j >> 1) & 1, p.status, 25);
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
-      if (any_moves && it > 0) {
-        tc_fence_after();
-        uint32_t o[32];
-        tc_ld_32x32b_x32(lane_addr + AT_TM_O + half * 32, o);
-        tc_wait_ld();
+      tc_fence_after();
+      uint32_t s[2][32];
+      tc_ld_32x32b_x32(lane_addr + AT_TM_S + b * AT_BN, s[0]);
+      tc_ld_32x32b_x32(lane_addr + AT_TM_S + b * AT_BN + 32, s[1]);
+      tc_wait_ld();
+      const int n_valid = static_cast<int>(p.kv_len - static_cast<int64_t>(j) * AT_BN);  // >= 64: the whole tile
+      if (n_valid < AT_BN) {
+        // the last tile of a span whose length is not a multiple of 64: keys beyond kv_len count as -inf
 #pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-        tc_st_32x32b_x32(lane_addr + AT_TM_O + half * 32, o);
-        tc_wait_st();
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i >= n_valid) s[c][i] = 0xff800000u;
       }
+      float m4[4];
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c = half * 2 + cc;
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t* v = &s[q >> 1][(q & 1) * 16];
+        float m = fmaxf(__uint_as_float(v[0]), __uint_as_float(v[1]));
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const float* e = &t[cc][g * 8];
-          const int c8 = c * 4 + g;  // 16-byte chunk of the row: 8 keys
-          uint8_t* dst = p_s + (c8 >> 3) * AT_PANEL + row * 128 + (((c8 & 7) ^ (row & 7)) << 4);
-          *reinterpret_cast<uint4*>(dst) = make_uint4(bf16x2(e[0], e[1]), bf16x2(e[2], e[3]), bf16x2(e[4], e[5]), bf16x2(e[6], e[7]));
+        for (int i = 2; i < 16; i += 2) m = max3(m, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+        m4[q] = m;
+      }
+      const float m_tile = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * L2E;
+      // The reference of a row moves when the tile's maximum exceeds it by more than 8.  Then the row sum and the row's O are
+      // scaled by 2^(m_ref - m_tile).  The tensor-memory accesses are warp-wide, so the warp goes through them when any of
+      // its rows moves; the other rows scale by one.  Before the first P V product there is nothing to scale.
+      const bool moves = m_tile > m_ref + 8.0f;
+      if (__any_sync(0xffffffffu, moves)) {
+        const float alpha = moves ? ex2f(m_ref - m_tile) : 1.0f;  // 0 for m_ref = -inf
+        if (moves) m_ref = m_tile;
+        const uint64_t a2 = pack_f32x2(alpha, alpha);
+        l2[0] = mul_f32x2(l2[0], a2);
+        l2[1] = mul_f32x2(l2[1], a2);
+        if (j > 0) {
+          if (lane == 0) ok = mbar_wait_spin(&bar.pv_done, (j - 1) & 1, p.status, 26);  // P V of the previous step complete
+          ok = __shfl_sync(0xffffffffu, ok, 0);
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t o[32];
+            tc_ld_32x32b_x32(lane_addr + AT_TM_O + h * 32, o);
+            tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tc_st_32x32b_x32(lane_addr + AT_TM_O + h * 32, o);
+          }
         }
       }
-      tc_fence_before();         // O corrections before the P V product that the arrival below releases
-      fence_proxy_async_smem();  // P written by the generic proxy -> visible to the tensor core
+      const uint64_t k2 = pack_f32x2(L2E, L2E), n2 = pack_f32x2(-m_ref, -m_ref);
+      uint32_t pk[32];
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          float x0, x1;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), k2, n2), x0, x1);
+          x0 = ex2f(x0);
+          x1 = ex2f(x1);
+          l2[(i >> 1) & 1] = add_f32x2(l2[(i >> 1) & 1], pack_f32x2(x0, x1));
+          pk[c * 16 + (i >> 1)] = bf16x2(x0, x1);
+        }
+      tc_st_32x32b_x32(lane_addr + AT_TM_S + b * AT_BN, pk);  // P over the S it came from
+      tc_wait_st();
+      tc_fence_before();  // P and the O correction before the P V product that the arrival releases
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bar.p_full);
+      if (lane == 0) mbar_arrive(&bar.p_full[b]);
     }
-    // O / l -> bf16 -> out[t, head * dk + :]; this warp stores 32 of the 64 value columns
+    // O / l -> bf16 -> out[t, head * dk + :]
     if (ok) {
-      if (lane == 0) ok = mbar_wait(&bar.o_full, 0, p.status, 27);
+      if (lane == 0) ok = mbar_wait_spin(&bar.pv_done, (steps - 1) & 1, p.status, 27);
       ok = __shfl_sync(0xffffffffu, ok, 0);
     }
-    // Every softmax thread executes the same number of named barriers whatever happened above: a warp whose
-    // bounded wait ran out makes up for the ones it skipped, so that the others cannot be left waiting for it.
-    while (syncs < iters) { softmax_sync(); ++syncs; }
-    const float lmine = (l4[0] + l4[1]) + (l4[2] + l4[3]);
-    bar.xch[iters & 1][half][row] = lmine;
-    softmax_sync();
-    const float inv = 1.0f / (lmine + bar.xch[iters & 1][half ^ 1][row]);
     if (ok) {
       tc_fence_after();
-      const int64_t tq = q0 + row;
-      uint32_t r[32];
-      tc_ld_32x32b_x32(lane_addr + AT_TM_O + half * 32, r);
-      tc_wait_ld();
-      if (tq < p.T) {
-        uint4* dst = reinterpret_cast<uint4*>(p.out + tq * p.ldo + head * AT_DV + half * 32);
+      float a0, a1, b0, b1;
+      unpack_f32x2(l2[0], a0, a1);
+      unpack_f32x2(l2[1], b0, b1);
+      const float inv = 1.0f / ((a0 + a1) + (b0 + b1));
+      __nv_bfloat16* const dst = p.out + tq * p.ldo + head * AT_DV;
 #pragma unroll
-        for (int g = 0; g < 4; ++g)
-          dst[g] = make_uint4(bf16x2(__uint_as_float(r[8 * g]) * inv, __uint_as_float(r[8 * g + 1]) * inv),
-                              bf16x2(__uint_as_float(r[8 * g + 2]) * inv, __uint_as_float(r[8 * g + 3]) * inv),
-                              bf16x2(__uint_as_float(r[8 * g + 4]) * inv, __uint_as_float(r[8 * g + 5]) * inv),
-                              bf16x2(__uint_as_float(r[8 * g + 6]) * inv, __uint_as_float(r[8 * g + 7]) * inv));
+      for (int h = 0; h < 2; ++h) {
+        uint32_t r[32];
+        tc_ld_32x32b_x32(lane_addr + AT_TM_O + h * 32, r);
+        tc_wait_ld();
+        if (tq < p.T) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g)
+            reinterpret_cast<uint4*>(dst)[h * 4 + g] =
+                make_uint4(bf16x2(__uint_as_float(r[8 * g]) * inv, __uint_as_float(r[8 * g + 1]) * inv),
+                           bf16x2(__uint_as_float(r[8 * g + 2]) * inv, __uint_as_float(r[8 * g + 3]) * inv),
+                           bf16x2(__uint_as_float(r[8 * g + 4]) * inv, __uint_as_float(r[8 * g + 5]) * inv),
+                           bf16x2(__uint_as_float(r[8 * g + 6]) * inv, __uint_as_float(r[8 * g + 7]) * inv));
+        }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == AT_SOFTMAX_WARPS + 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, AT_TM_COLS);
   }
 }
 
@@ -377,16 +367,15 @@ extern "C" int vx_relpos_attention(const void* q2, const void* k2, const void* v
   if (static_cast<int64_t>(heads) * T + AT_BM >= (1ll << 31)) return fail(-1, "heads * T must stay below 2^31");
   if (!aligned16(q2) || !aligned16(k2) || !aligned16(v2) || !aligned16(out) || ldo < static_cast<int64_t>(heads) * AT_DV || (ldo * 2) % 16 != 0)
     return fail(-1, "operands must be 16-byte aligned, out rows at least heads * head_dim wide");
-  CUtensorMap tq, tk, tv;
+  CUtensorMap tk, tv;
   const int64_t rows = static_cast<int64_t>(heads) * T;
-  int rc = make_tmap_2d(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, q2, rows, AT_D, AT_D * 2, 64, AT_BM);
-  if (rc) return rc;
-  rc = make_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, k2, rows, AT_D, AT_D * 2, 64, AT_BN);
+  int rc = make_tmap_2d(&tk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, k2, rows, AT_D, AT_D * 2, 64, AT_BN);
   if (rc) return rc;
   rc = make_tmap_2d(&tv, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, v2, rows, AT_D, AT_D * 2, 64, AT_BN);
   if (rc) return rc;
   AttnParams p{};
   p.T = T; p.kv_len = kv_len; p.heads = heads;
+  p.q = static_cast<const __nv_bfloat16*>(q2);
   p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo;
   p.status = device_status_ptr();
   int dev = 0;
@@ -398,6 +387,6 @@ extern "C" int vx_relpos_attention(const void* q2, const void* k2, const void* v
     if (dev_cached) attr_done.fetch_or(1ull << dev, std::memory_order_release);
   }
   const dim3 grid(static_cast<unsigned>((T + AT_BM - 1) / AT_BM), static_cast<unsigned>(heads));
-  VX_CUDA_OK(launch_dependent(relpos_attn_kernel, grid, dim3(AT_THREADS), AT_SMEM, static_cast<cudaStream_t>(stream), tq, tk, tv, p));
+  VX_CUDA_OK(launch_dependent(relpos_attn_kernel, grid, dim3(AT_THREADS), AT_SMEM, static_cast<cudaStream_t>(stream), tk, tv, p));
   return 0;
 }
