@@ -621,6 +621,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   constexpr bool UNITS = !FP8 && (SEQ || !WIDE);  // ring of 128-column accumulators: half tiles, or the narrow kernel's tiles
   // Swish + FP4 output (the FFN up-projection): its own register-lean path, see swish_quant_chunk.
   constexpr bool SWQ = EPI == VX_EPI_BIAS_SWISH && OUT == 2;
+  constexpr bool WAIT_CALL = !SWQ;  // its epilogue holds a whole half tile across the wait: 28.9 us inline, 30.8 called (27,000 x 768 x 3072)
   static_assert(!SWQ || WIDE, "Swish + FP4 output runs on the wide tile");
   const int out_dtype = OUT == 1 || OUT == 4 ? static_cast<int>(VX_BF16) : (OUT == 2 ? static_cast<int>(VX_FP4) : p.out_dtype);
   const bool tma_store = OUT == 1 || OUT == 4 ? true : (OUT == 2 ? false : p.tma_store != 0);
@@ -781,9 +782,9 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         const uint8_t* sfa_row = p.sfa + (static_cast<int64_t>(mb) * p.sf_kg) * 512;
         const uint32_t slot_tx = TILE_BYTES + sf_atom_bytes + (resident ? 0u : b_tx(nb));
         for (int kg = 0; kg < k_groups; ++kg) {
-          if (!mbar_wait(&sm.empty[s], ph ^ 1, p.status, 1)) { ok = false; break; }
+          if (!mbar_wait<WAIT_CALL>(&sm.empty[s], ph ^ 1, p.status, 1)) { ok = false; break; }
           if (sfb_pending && s == static_cast<uint32_t>(nslots - 1)) {
-            if (!mbar_wait(&sm.sfb_done, 0, p.status, 7)) { ok = false; break; }
+            if (!mbar_wait<WAIT_CALL>(&sm.sfb_done, 0, p.status, 7)) { ok = false; break; }
             sfb_pending = false;
           }
           if (tr_on) trace_rec(p, 0, i, kg < 4 ? kg : 3);
@@ -856,12 +857,12 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
             CP(col0 + a * SFB_COLS + rt * 4, desc(b_lo + b_sf_lo + (rt * APS + a) * 32, sf_hi));
       };
       if (resident) {
-        if (!mbar_wait(&sm.b_full, 0, p.status, 5)) ok = false;
+        if (!mbar_wait<WAIT_CALL>(&sm.b_full, 0, p.status, 5)) ok = false;
         tc_fence_after();
         if (ok && with_sf)  // B's scale factors stay in tensor memory for the whole kernel
           for (int ks = 0; ks < p.k_stages; ++ks) cp_sfb(arena_lo + ks * bslot_lo, tm_sfb + ks * APS * SFB_COLS);
       } else if (sfb_res) {
-        if (!mbar_wait(&sm.b_full, 0, p.status, 5)) ok = false;
+        if (!mbar_wait<WAIT_CALL>(&sm.b_full, 0, p.status, 5)) ok = false;
         tc_fence_after();
         if (ok) {
           const uint32_t st_lo = (arena_u32 + (nslots - 1) * slot_bytes + a_slot) >> 4;
@@ -890,12 +891,12 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
               if ((u & 1) == 0) {
                 const int pr = u >> 1;
                 const uint32_t use = pr ? use1 : use0;
-                if (!mbar_wait_spin(&sm.tmem_empty[pr], (use & 1) ^ 1, p.status, 2)) { ok = false; break; }
+                if (!mbar_wait_spin<WAIT_CALL>(&sm.tmem_empty[pr], (use & 1) ^ 1, p.status, 2)) { ok = false; break; }
                 if (pr) ++use1; else ++use0;
                 tc_fence_after();  // orders the epilogue's tcgen05.ld of these buffers before the MMAs
               }
               if (in_group == 0) {
-                if (!mbar_wait_spin(&sm.full[s], ph, p.status, 3)) { ok = false; break; }
+                if (!mbar_wait_spin<WAIT_CALL>(&sm.full[s], ph, p.status, 3)) { ok = false; break; }
                 tc_fence_after();
               }
               if (kb0 == 0) TRACE(i, 2 * u);
@@ -926,12 +927,12 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         for (int i = 0; i < my_tiles && ok; ++i) {
           for (int kg = 0; kg < k_groups; ++kg) {
             if (kg == 0) {
-              if (!mbar_wait_spin(&sm.tmem_empty[us], uph, p.status, 2)) { ok = false; break; }
-              if (SEQ && !split && !mbar_wait_spin(&sm.tmem_empty[1], uph, p.status, 2)) { ok = false; break; }
+              if (!mbar_wait_spin<WAIT_CALL>(&sm.tmem_empty[us], uph, p.status, 2)) { ok = false; break; }
+              if (SEQ && !split && !mbar_wait_spin<WAIT_CALL>(&sm.tmem_empty[1], uph, p.status, 2)) { ok = false; break; }
               tc_fence_after();  // orders the epilogue's tcgen05.ld of this buffer before the MMAs
               TRACE(i, 0);
             }
-            if (!mbar_wait_spin(&sm.full[s], ph, p.status, 3)) { ok = false; break; }
+            if (!mbar_wait_spin<WAIT_CALL>(&sm.full[s], ph, p.status, 3)) { ok = false; break; }
             TRACE(i, kg < 2 ? 1 + kg : 2);
             const uint32_t d_tmem = tmem_base + TM_ACC0 + us * 128;
             const uint32_t a_lo0 = ring_lo + s * G * slot_lo;
@@ -972,7 +973,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
                 issue(d_tmem, 0, 0, N_LESS);
                 COMMIT(&sm.tmem_full[us]);
                 next_acc();
-                if (!mbar_wait_spin(&sm.tmem_empty[us], uph, p.status, 2)) { ok = false; break; }
+                if (!mbar_wait_spin<WAIT_CALL>(&sm.tmem_empty[us], uph, p.status, 2)) { ok = false; break; }
                 tc_fence_after();
                 issue(tmem_base + TM_ACC0 + us * 128, (128 * STAGE_ROW_BYTES) >> 4, 4, N_LESS);
               } else {
@@ -1092,8 +1093,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         const bool scale_acc = kind_vec4(KIND) && p.a_amax != nullptr;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {  // halves of the tile
-          if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[es], eph, p.status, 4);
-          ok = __shfl_sync(0xffffffffu, ok, 0);
+          ok = __all_sync(0xffffffffu, mbar_wait_spin<WAIT_CALL>(&sm.tmem_full[es], eph, p.status, 4));
           if (!ok) break;
           tc_fence_after();
           if (tr && h == 0) trace_rec(p, 2, it, 1);
@@ -1161,8 +1161,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         for (int kb0 = 0; kb0 < kb_count && ok; kb0 += FP8_ACCS) {
           // one round: up to four K blocks, block u in accumulator u, published together
           const int nkb = kb_count - kb0 < FP8_ACCS ? kb_count - kb0 : FP8_ACCS;
-          if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[0], group & 1, p.status, 4);
-          ok = __shfl_sync(0xffffffffu, ok, 0);
+          ok = __all_sync(0xffffffffu, mbar_wait_spin<WAIT_CALL>(&sm.tmem_full[0], group & 1, p.status, 4));
           if (!ok) break;
           ++group;
           tc_fence_after();
@@ -1230,8 +1229,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         }
         // one polling lane per warp (512 polling threads would starve the MMA-issuing thread)
         const uint32_t acc_addr = lane_addr + TM_ACC0 + es * 128 + col_base;
-        if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[es], eph, p.status, 4);
-        ok = __shfl_sync(0xffffffffu, ok, 0);
+        ok = __all_sync(0xffffffffu, mbar_wait_spin<WAIT_CALL>(&sm.tmem_full[es], eph, p.status, 4));
         if (!ok) break;
         tc_fence_after();
         if (tr) trace_rec(p, 2, it, 1);
@@ -1266,8 +1264,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
             // second chunk: read it now (its registers were free for the first chunk's
             // arithmetic), then hand the second half of the tile back
             if (h == 1) {
-              if (lane == 0) ok = mbar_wait_spin(&sm.tmem_full[es], eph, p.status, 4);
-              ok = __shfl_sync(0xffffffffu, ok, 0);
+              ok = __all_sync(0xffffffffu, mbar_wait_spin<WAIT_CALL>(&sm.tmem_full[es], eph, p.status, 4));
               if (!ok) break;
               tc_fence_after();
               uint32_t r[32];
@@ -1311,7 +1308,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
                 if (h + 1 < NCH) res_issue(res_chunk + 1, mb, out_col0 + 32);
                 else res_issue(res_chunk + 1, mb_next, static_cast<int64_t>(nb_next) * OUT_TILE_COLS + col_base);
               }
-              if (!mbar_wait(&sm.res_full[res_chunk & 1][ew], (res_chunk >> 1) & 1, p.status, 6)) { ok = false; break; }
+              if (!mbar_wait<WAIT_CALL>(&sm.res_full[res_chunk & 1][ew], (res_chunk >> 1) & 1, p.status, 6)) { ok = false; break; }
               res_smem = res_half;
             }
           }

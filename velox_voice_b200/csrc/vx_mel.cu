@@ -167,15 +167,13 @@ __global__ void __launch_bounds__(MEL_THREADS, 1) power_mel_log_kernel(const Mel
     fetch(0, ca);
     for (int64_t n = 0; n < items && ok; n += 2) {
       fetch(n + 1, cb);
-      if (lane == 0) ok = mbar_wait(&bar.empty[s], ph ^ 1, p.status, 11, abortp);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
+      ok = __all_sync(0xffffffffu, mbar_wait<true>(&bar.empty[s], ph ^ 1, p.status, 11, abortp));
       if (!ok) break;
       publish(s, ca);
       if (++s == static_cast<uint32_t>(p.ring)) { s = 0; ph ^= 1; }
       if (n + 1 >= items) break;
       fetch(n + 2, ca);
-      if (lane == 0) ok = mbar_wait(&bar.empty[s], ph ^ 1, p.status, 11, abortp);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
+      ok = __all_sync(0xffffffffu, mbar_wait<true>(&bar.empty[s], ph ^ 1, p.status, 11, abortp));
       if (!ok) break;
       publish(s, cb);
       if (++s == static_cast<uint32_t>(p.ring)) { s = 0; ph ^= 1; }
@@ -217,8 +215,7 @@ __global__ void __launch_bounds__(MEL_THREADS, 1) power_mel_log_kernel(const Mel
     bool ok = true;
     for (int i = 0; i < my_tiles && ok; ++i) {
       const uint32_t a = i & 1;
-      if (lane == 0) ok = mbar_wait(&bar.acc_full[a], (i >> 1) & 1, p.status, 14, abortp);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
+      ok = __all_sync(0xffffffffu, mbar_wait<true>(&bar.acc_full[a], (i >> 1) & 1, p.status, 14, abortp));
       if (!ok) break;
       tc_fence_after();
       const int64_t row = (static_cast<int64_t>(blockIdx.x) + static_cast<int64_t>(i) * gridDim.x) * MEL_BM + warp * 32 + lane;
@@ -379,7 +376,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
         const int64_t t0 = tile_frame(i);
         const int nc = chunks_of(t0);
         for (int c = 0; c < nc; ++c) {
-          if (!mbar_wait(&bar.raw_empty[s], ph ^ 1, p.status, 11, abortp)) { ok = false; break; }
+          if (!mbar_wait<true>(&bar.raw_empty[s], ph ^ 1, p.status, 11, abortp)) { ok = false; break; }
           const int64_t row = t0 + c * MT_ROWS;
           const int64_t rows = p.T - row < MT_ROWS ? p.T - row : MT_ROWS;
           // (an odd number of rows, the end of the input only, may leave 8 bytes: the transform warp fetches them itself)
@@ -403,12 +400,10 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
     for (int i = 0; i < my_tiles && ok; ++i) {
       const int64_t t0 = tile_frame(i);
       const int b = i & 1, nc = chunks_of(t0);
-      if (lane == 0) ok = mbar_wait(&bar.b_empty[b], ((i >> 1) & 1) ^ 1, p.status, 12, abortp);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
+      ok = __all_sync(0xffffffffu, mbar_wait<true>(&bar.b_empty[b], ((i >> 1) & 1) ^ 1, p.status, 12, abortp));
       if (!ok) break;
       for (int r = w; r < MT_N && r / MT_ROWS < nc; r += MT_XF) {
-        if (lane == 0) ok = mbar_wait(&bar.raw_full[s], ph, p.status, 13, abortp);
-        ok = __shfl_sync(0xffffffffu, ok, 0);
+        ok = __all_sync(0xffffffffu, mbar_wait<true>(&bar.raw_full[s], ph, p.status, 13, abortp));
         if (!ok) break;
         const int64_t row = t0 + r;
         if (row < p.T) {
@@ -484,8 +479,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
     bool ok = true;
     for (int i = 0; i < my_tiles && ok; ++i) {
       const int b = i & 1;
-      if (lane == 0) ok = mbar_wait(&bar.acc_full[b], (i >> 1) & 1, p.status, 16, abortp);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
+      ok = __all_sync(0xffffffffu, mbar_wait<true>(&bar.acc_full[b], (i >> 1) & 1, p.status, 16, abortp));
       if (!ok) break;
       tc_fence_after();
       uint32_t r[MT_N];

@@ -59,58 +59,75 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// One poll without the hint.
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Wall-clock limit of one wait.  Whole kernels here run for well under 100 ms.
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 
 // status word layout: 0 = ok; else (code << 24) | (site << 16) | (blockIdx.x & 0xffff)
-// Slow path of a wait (kept inline: an out-of-line call was measured slower in most kernels): polls against the
-// wall clock (%globaltimer, slow to read) and gives up after `limit_ns`.  `abort` (optional) is a
-// flag in shared memory that the first role of a CTA to give up raises: the other roles of that
-// CTA then leave their own waits at once instead of running out their own limits one after another.
-__device__ __forceinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, int* status, int site,
-                                               volatile int* abort = nullptr, uint64_t limit_ns = kWaitLimitNs) {
-  const uint64_t t0 = globaltimer_ns();
+// The loop of a wait.  Polls, and every EVERY polls looks at the wall clock (%globaltimer, slow to read); gives up
+// `limit_ns` after its first look.  `abort` (optional) is a flag in shared memory that the first role of a CTA to give up
+// raises: the other roles of that CTA then leave their own waits instead of running out their own limits one after another.
+template <bool PARK, uint32_t EVERY>
+__device__ __forceinline__ bool mbar_wait_loop(uint64_t* bar, uint32_t parity, int* status, int site, volatile int* abort,
+                                               uint64_t limit_ns) {
+  uint64_t t0 = 0;
   uint32_t spins = 0;
+#pragma unroll 1
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((++spins & 0x3f) == 0) {
+    if (PARK ? mbar_try_wait(bar, parity) : mbar_poll(bar, parity)) return true;
+    if ((++spins & (EVERY - 1)) == 0) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
       if (abort && *abort) return false;
-      if (globaltimer_ns() - t0 > limit_ns) {
-        if (status) atomicCAS(status, 0, (1 << 24) | ((site & 0xff) << 16) | (blockIdx.x & 0xffff));
-        if (abort) *abort = 1;
-        return false;
-      }
+      if (now - t0 > limit_ns) break;
     }
   }
+  if (status) atomicCAS(status, 0, (1 << 24) | ((site & 0xff) << 16) | (blockIdx.x & 0xffff));
+  if (abort) *abort = 1;
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, int* status, int site,
+                                               volatile int* abort = nullptr, uint64_t limit_ns = kWaitLimitNs) {
+  return mbar_wait_loop<true, 64>(bar, parity, status, site, abort, limit_ns);
+}
+template <bool PARK>
+static __device__ __noinline__ bool mbar_wait_call(uint64_t* bar, uint32_t parity, int* status, int site, volatile int* abort) {
+  return mbar_wait_loop<PARK, PARK ? 64 : 16384>(bar, parity, status, site, abort, kWaitLimitNs);
 }
 
-// Parked wait: each poll may suspend the thread for up to 20 us, so a wait that succeeds
-// within 64 polls never reads the clock.
+// The waits look once before they enter the loop: the exit of a loop costs a warp about 80 cycles (its lanes may leave at
+// different turns); a wait that finds its phase complete takes 55 cycles instead of 135.  The lanes of a warp wait together:
+// a wait by lane 0 and a shuffle of the outcome take 270.  CALL keeps the loop out of line: less code to fetch, which tells
+// where a kernel runs for microseconds, but registers to save where many are live.
+// Parked wait: each poll may suspend the thread for up to 20 us.
+template <bool CALL = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int site,
                                           volatile int* abort = nullptr) {
-#pragma unroll 1
-  for (uint32_t spins = 0; spins < 64; ++spins)
-    if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_slow(bar, parity, status, site, abort);
+  if (__builtin_expect(mbar_poll(bar, parity), 1)) return true;
+  if (CALL) return mbar_wait_call<true>(bar, parity, status, site, abort);
+  return mbar_wait_loop<true, 64>(bar, parity, status, site, abort, kWaitLimitNs);
 }
 
 // Same contract, plain polling without the suspend hint: for the MMA-issuing warp and the
-// epilogue's polling lane, whose reaction time is on the critical path of every tile.
+// epilogue warps, whose reaction time is on the critical path of every tile.
+template <bool CALL = false>
 __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, int* status, int site,
                                                volatile int* abort = nullptr) {
-#pragma unroll 1
-  for (uint32_t spins = 0; spins < 100000; ++spins) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return mbar_wait_slow(bar, parity, status, site, abort);
+  if (__builtin_expect(mbar_poll(bar, parity), 1)) return true;
+  if (CALL) return mbar_wait_call<false>(bar, parity, status, site, abort);
+  return mbar_wait_loop<false, 16384>(bar, parity, status, site, abort, kWaitLimitNs);
 }
 
 // ------------------------------------------------------------------ proxies / fences

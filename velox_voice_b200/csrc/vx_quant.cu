@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(256, VX_QUANT_MIN_BLOCKS) quant_kernel(const Q
     uint32_t par = 0;
 #pragma unroll 1
     for (I u = u_first; u < nunits; u += warps) {
-      if (!mbar_wait(&full_w[slot], par, p.status, 8)) break;
+      if (!mbar_wait<true>(&full_w[slot], par, p.status, 8)) break;
       uint64_t v[2][1][4];
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(256, lnq_min_blocks(CH)) ln_quant_kernel(const
     uint32_t par = 0;
 #pragma unroll 1
     for (I u = u_first; u < nunits; u += warps) {
-      if (!mbar_wait(&full_w[slot], par, p.status, 8)) break;
+      if (!mbar_wait<true>(&full_w[slot], par, p.status, 8)) break;
       uint64_t v[CH][RP][4];
 #pragma unroll
       for (int c = 0; c < CH; ++c) {
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(256, LN ? VX_R2_MIN_BLOCKS_LN : VX_R2_MIN_BLOC
   uint32_t par = 0;
 #pragma unroll 1
   for (int u = u_first; u < nunits; u += warps) {
-    if (!mbar_wait(&full_w[slot], par, p.status, 8)) break;
+    if (!mbar_wait<true>(&full_w[slot], par, p.status, 8)) break;
     const int row = 2 * u + h;
     const bool valid = row < M;
     uint64_t v[4][4];
