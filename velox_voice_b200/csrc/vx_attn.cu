@@ -12,21 +12,25 @@
 // One CTA = 128 queries of one head, TWO CTAs PER SM (half the shared and tensor memory each), all on the 5th-generation
 // tensor cores (tcgen05.mma kind::f16, bf16 operands, fp32 accumulators in tensor memory):
 //   warps 0..3  softmax, one query row per thread straight out of tensor memory, 64 keys per step;
-//   warp 4      TMA producer: K and V tiles of 64 keys through a four-stage ring;
-//   warp 5      MMA issuer: S = Q K^T (128 x 64 x 128) into one of two S buffers, O += P V (128 x 64 x 64; V is read in its
-//               natural [key][dv] layout as an MN-major operand).
-// Q and P are A operands in TENSOR MEMORY: Q is put there once by the softmax warps, P (bf16) replaces the S it was made
-// from, so the MMAs read only K and V from shared memory and no proxy fence stands between the softmax and P V.
-// Tensor memory (256 columns): S0 | S1 (64 each; P in the lower half) | O (64) | Q (64).
+//   warp 4      TMA producer: K and V tiles of 64 keys through two four-stage rings;
+//   warp 5      MMA issuer: S = Q K^T (128 x 64 x 128), O += P V (128 x 64 x 64; V is read in its natural [key][dv] layout
+//               as an MN-major operand).
+// Q and P are A operands in TENSOR MEMORY: Q is put there once by the softmax warps, P (bf16) each step, so the MMAs read
+// only K and V from shared memory (with Q there too they were bound by it) and no proxy fence stands between the softmax
+// and P V.  P has columns of its own, so that S of step j + 1 is issued as soon as the softmax of step j has READ its S, and
+// is there when the softmax gets to it.
+// Tensor memory (256 columns): S (64) | P0 | P1 (32 each) | O (64) | Q (64).
 // One pass over the keys with a lazily updated reference maximum: p = 2^((s - m_ref) log2 e) is formed
 // against the reference m_ref the row has used so far, which only moves when a tile's maximum exceeds it by
 // more than 2^8 (so p never exceeds 256 and nothing overflows in bf16 or fp32).  When it moves -- typically in
 // the first tiles of a row only -- the row sum and the row's O accumulator are multiplied by 2^((m_old - m_new) log2 e)
 // (tcgen05.ld / tcgen05.st) before the next P V product is released.  O is divided by the row sum once at the end.
-// What bounds it: the special-function unit (64 exponentials per row and step, 16 lanes per cycle and SM: 512 cycles per CTA and
-// step against 384 of MMAs), as long as the two CTAs of an SM fill each other's hand-over latencies.  The form with one
-// CTA of eight softmax warps per SM, P through shared memory and a maximum exchange between two warps per row took 3,200
-// cycles per 128 x 128 tile: 99 us for 3,750 frames and 8 heads -> MEASURED
+// What bounds it: the two softmax warps of an SM partition and the special-function unit that they share (64 exponentials per
+// row and step, 16 lanes per cycle and SM: 512 cycles per CTA and step; the MMAs take 400).  3,750 frames and 8 heads: 99 us
+// with one CTA per SM, P through shared memory and a maximum exchange between two warps per row (3,200 cycles per 128 x 128
+// tile); 62 us with two CTAs and P over S, where the round trip of a buffer -- P V, then the S behind it -- made the softmax
+// wait 340 cycles a step; 58 us like this.  Neither eight softmax warps per CTA in two independent groups (73 us) nor a
+// quarter of the exponentials as polynomials on the fp32 pipe (64 us) helped.
 // Every mbarrier wait is bounded.
 
 #include <cuda.h>
@@ -51,12 +55,11 @@ constexpr int AT_DV = 64;    // value dimension (dk)
 constexpr int AT_K_PANEL = AT_BN * 128;           // one 64-column bf16 panel of a K tile: 8 KB
 constexpr int AT_K_BYTES = 2 * AT_K_PANEL;
 constexpr int AT_V_BYTES = AT_BN * AT_DV * 2;     // 8 KB
-constexpr int AT_STAGE = AT_K_BYTES + AT_V_BYTES; // 24 KB
-constexpr int AT_NS = 4;                          // K / V stages in flight
-constexpr int AT_SMEM = AT_NS * AT_STAGE + 1024;
+constexpr int AT_NS = 4;                          // K and V tiles in flight
+constexpr int AT_SMEM = AT_NS * (AT_K_BYTES + AT_V_BYTES) + 1024;
 constexpr int AT_SOFTMAX_WARPS = 4;
 constexpr int AT_THREADS = (AT_SOFTMAX_WARPS + 2) * 32;
-constexpr uint32_t AT_TM_S = 0, AT_TM_O = 128, AT_TM_Q = 192, AT_TM_COLS = 256;
+constexpr uint32_t AT_TM_S = 0, AT_TM_P = 64, AT_TM_O = 128, AT_TM_Q = 192, AT_TM_COLS = 256;
 
 struct AttnParams {
   int64_t T;        // queries and keys per head
@@ -69,7 +72,7 @@ struct AttnParams {
 };
 
 struct AttnBarriers {
-  uint64_t q_full, kv_full[AT_NS], kv_empty[AT_NS], s_full[2], p_full[2], pv_done;
+  uint64_t q_full, k_full[AT_NS], k_empty[AT_NS], v_full[AT_NS], v_empty[AT_NS], s_full, s_empty, p_full[2], pv_done[2], o_full;
   uint32_t tmem_base;
 };
 
@@ -85,16 +88,6 @@ __device__ __forceinline__ void mma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, ui
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
-}
-// shared-memory descriptor with the 128-byte swizzle and explicit leading / stride byte offsets
-__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4);
-  d |= static_cast<uint64_t>((lbo >> 4) & 0x3fff) << 16;
-  d |= static_cast<uint64_t>((sbo >> 4) & 0x3fff) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
 }
 __device__ __forceinline__ void tc_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile(
@@ -122,7 +115,8 @@ __global__ void __launch_bounds__(AT_THREADS, 2)
 relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* const st_s = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* const k_s = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* const v_s = k_s + AT_NS * AT_K_BYTES;
   __shared__ AttnBarriers bar;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.y;
@@ -132,15 +126,19 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
   if (threadIdx.x == 0) {
     mbar_init(&bar.q_full, AT_SOFTMAX_WARPS);
+    mbar_init(&bar.s_full, 1);
+    mbar_init(&bar.s_empty, AT_SOFTMAX_WARPS);
+    mbar_init(&bar.o_full, 1);
     for (int s = 0; s < AT_NS; ++s) {
-      mbar_init(&bar.kv_full[s], 1);
-      mbar_init(&bar.kv_empty[s], 1);
+      mbar_init(&bar.k_full[s], 1);
+      mbar_init(&bar.k_empty[s], 1);
+      mbar_init(&bar.v_full[s], 1);
+      mbar_init(&bar.v_empty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
-      mbar_init(&bar.s_full[s], 1);
       mbar_init(&bar.p_full[s], AT_SOFTMAX_WARPS);
+      mbar_init(&bar.pv_done[s], 1);
     }
-    mbar_init(&bar.pv_done, 1);
     mbar_fence_init();
     prefetch_tmap(&tm_k);
     prefetch_tmap(&tm_v);
@@ -158,61 +156,75 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   if (warp == AT_SOFTMAX_WARPS) {
     // =========================== TMA producer ===========================
     if (lane == 0) {
-      for (int j = 0; j < steps; ++j) {
+      auto load_k = [&](int j) {
         const int s = j % AT_NS;
-        if (!mbar_wait(&bar.kv_empty[s], ((j / AT_NS) & 1) ^ 1, p.status, 20)) break;
-        uint8_t* const dst = st_s + s * AT_STAGE;
-        mbar_expect_tx(&bar.kv_full[s], AT_STAGE);
-        tma_load_2d(dst, &tm_k, 0, row_base + j * AT_BN, &bar.kv_full[s]);
-        tma_load_2d(dst + AT_K_PANEL, &tm_k, 64, row_base + j * AT_BN, &bar.kv_full[s]);
-        tma_load_2d(dst + AT_K_BYTES, &tm_v, 0, row_base + j * AT_BN, &bar.kv_full[s]);
+        if (!mbar_wait(&bar.k_empty[s], ((j / AT_NS) & 1) ^ 1, p.status, 20)) return false;
+        uint8_t* const dst = k_s + s * AT_K_BYTES;
+        mbar_expect_tx(&bar.k_full[s], AT_K_BYTES);
+        tma_load_2d(dst, &tm_k, 0, row_base + j * AT_BN, &bar.k_full[s]);
+        tma_load_2d(dst + AT_K_PANEL, &tm_k, 64, row_base + j * AT_BN, &bar.k_full[s]);
+        return true;
+      };
+      bool ok = load_k(0);
+      for (int j = 0; j < steps && ok; ++j) {  // K runs one tile ahead of V
+        if (j + 1 < steps && !load_k(j + 1)) break;
+        const int s = j % AT_NS;
+        if (!mbar_wait(&bar.v_empty[s], ((j / AT_NS) & 1) ^ 1, p.status, 29)) break;
+        mbar_expect_tx(&bar.v_full[s], AT_V_BYTES);
+        tma_load_2d(v_s + s * AT_V_BYTES, &tm_v, 0, row_base + j * AT_BN, &bar.v_full[s]);
       }
     }
   } else if (warp == AT_SOFTMAX_WARPS + 1) {
     // =========================== MMA issuer ===========================
+    // (warp-uniform control flow; descriptors are one 32-bit add each: low word = shared address >> 4, constant high word)
     const bool leader = elect_one();
     const uint32_t idesc_s = make_idesc_bf16(AT_BM, AT_BN, false);
     const uint32_t idesc_o = make_idesc_bf16(AT_BM, AT_DV, true);
-    const uint32_t st_u32 = smem_u32(st_s);
+    const uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+    auto desc = [&](uint32_t lo) { return (static_cast<uint64_t>(desc_hi) << 32) | lo; };
+    const uint32_t k_lo = smem_u32(k_s) >> 4, v_lo = smem_u32(v_s) >> 4;
     bool ok = mbar_wait_spin(&bar.q_full, 0, p.status, 21);
-    // S(j) = Q K_j^T into buffer j & 1 (the P V product of step j - 2, which read P there, has completed)
-    auto issue_s = [&](int j) {
-      if (!mbar_wait_spin(&bar.kv_full[j % AT_NS], (j / AT_NS) & 1, p.status, 22)) return false;
+    uint32_t ks = 0, kph = 0, vs = 0, vph = 0;  // ring positions
+    auto issue_s = [&]() {  // S of the next tile
+      if (!mbar_wait_spin(&bar.k_full[ks], kph, p.status, 22)) return false;
       tc_fence_after();
-      if (leader) {
-        const uint32_t k_u32 = st_u32 + (j % AT_NS) * AT_STAGE;
+      const uint32_t kt = k_lo + ks * (AT_K_BYTES >> 4);
 #pragma unroll
-        for (int i = 0; i < AT_D / 16; ++i)
-          mma_bf16_ta(tmem_base + AT_TM_S + (j & 1) * AT_BN, tmem_base + AT_TM_Q + i * 8,
-                      make_desc_k128(k_u32 + (i >> 2) * AT_K_PANEL + (i & 3) * 32), idesc_s, i != 0);
-        if (j & 1) tc_commit(&bar.s_full[1]);
-        else tc_commit(&bar.s_full[0]);
+      for (int i = 0; i < AT_D / 16; ++i)
+        if (leader)
+          mma_bf16_ta(tmem_base + AT_TM_S, tmem_base + AT_TM_Q + i * 8, desc(kt + (i >> 2) * (AT_K_PANEL >> 4) + (i & 3) * 2), idesc_s, i != 0);
+      if (leader) {
+        tc_commit(&bar.s_full);
+        tc_commit(&bar.k_empty[ks]);
       }
-      __syncwarp();
+      if (++ks == AT_NS) { ks = 0; kph ^= 1; }
       return true;
     };
-    if (ok) ok = issue_s(0);
-    if (ok && steps > 1) ok = issue_s(1);
+    if (ok) ok = issue_s();
     for (int j = 0; j < steps && ok; ++j) {
-      if (!mbar_wait_spin(&bar.p_full[j & 1], (j >> 1) & 1, p.status, 24)) { ok = false; break; }
+      const uint32_t b = j & 1, par = (j >> 1) & 1;
+      if (j + 1 < steps) {
+        // the softmax of this step has read its S
+        if (!mbar_wait_spin(&bar.s_empty, j & 1, p.status, 23)) { ok = false; break; }
+        tc_fence_after();
+        ok = issue_s();
+        if (!ok) break;
+      }
+      if (!mbar_wait_spin(&bar.v_full[vs], vph, p.status, 30) || !mbar_wait_spin(&bar.p_full[b], par, p.status, 24)) { ok = false; break; }
       tc_fence_after();
-      if (leader) {
-        const uint32_t v_u32 = st_u32 + (j % AT_NS) * AT_STAGE + AT_K_BYTES;
-        // V tile as TMA wrote it: one 128-byte row of 64 dv values per key, 8-key swizzle atoms 1 KB apart
-        // (the stride offset of the MN-major operand); 64 dv values are one group along N, so the leading
-        // offset is not used.  A K = 16 step is two atoms.
+      // V tile as TMA wrote it: one 128-byte row of 64 dv values per key, 8-key swizzle atoms 1 KB apart
+      // (the stride offset of the MN-major operand); 64 dv values are one group along N, so the leading
+      // offset is not used.  A K = 16 step is two atoms.
+      const uint32_t vt = v_lo + vs * (AT_V_BYTES >> 4), pt = tmem_base + AT_TM_P + b * (AT_BN / 2);
 #pragma unroll
-        for (int i = 0; i < AT_BN / 16; ++i)
-          mma_bf16_ta(tmem_base + AT_TM_O, tmem_base + AT_TM_S + (j & 1) * AT_BN + i * 8, make_desc_sw128(v_u32 + i * 16 * 128, 0, 1024),
-                      idesc_o, (j | i) != 0);
-        tc_commit(&bar.pv_done);
-        tc_commit(&bar.kv_empty[j % AT_NS]);
+      for (int i = 0; i < AT_BN / 16; ++i)
+        if (leader) mma_bf16_ta(tmem_base + AT_TM_O, pt + i * 8, desc(vt + i * ((16 * 128) >> 4)), idesc_o, (j | i) != 0);
+      if (leader) {
+        tc_commit(&bar.pv_done[b]);
+        tc_commit(&bar.v_empty[vs]);
+        if (j == steps - 1) tc_commit(&bar.o_full);
       }
-      __syncwarp();
-      if (j + 2 < steps) {
-        if (!mbar_wait_spin(&bar.pv_done, j & 1, p.status, 23)) { ok = false; break; }
-        ok = issue_s(j + 2);
-      }
+      if (++vs == AT_NS) { vs = 0; vph ^= 1; }
     }
   } else {
     // =========================== softmax: warps 0..3, thread = query row ===========================
@@ -244,14 +256,16 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     bool ok = true;
     for (int j = 0; j < steps; ++j) {
       const int b = j & 1;
-      if (lane == 0) ok = mbar_wait_spin(&bar.s_full[b], (j >> 1) & 1, p.status, 25);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
+      ok = __all_sync(0xffffffffu, mbar_wait_spin(&bar.s_full, j & 1, p.status, 25));
       if (!ok) break;
       tc_fence_after();
       uint32_t s[2][32];
-      tc_ld_32x32b_x32(lane_addr + AT_TM_S + b * AT_BN, s[0]);
-      tc_ld_32x32b_x32(lane_addr + AT_TM_S + b * AT_BN + 32, s[1]);
+      tc_ld_32x32b_x32(lane_addr + AT_TM_S, s[0]);
+      tc_ld_32x32b_x32(lane_addr + AT_TM_S + 32, s[1]);
       tc_wait_ld();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar.s_empty);  // S is in registers: that of the next step may be written
       const int n_valid = static_cast<int>(p.kv_len - static_cast<int64_t>(j) * AT_BN);  // >= 64: the whole tile
       if (n_valid < AT_BN) {
         // the last tile of a span whose length is not a multiple of 64: keys beyond kv_len count as -inf
@@ -282,8 +296,7 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         l2[0] = mul_f32x2(l2[0], a2);
         l2[1] = mul_f32x2(l2[1], a2);
         if (j > 0) {
-          if (lane == 0) ok = mbar_wait_spin(&bar.pv_done, (j - 1) & 1, p.status, 26);  // P V of the previous step complete
-          ok = __shfl_sync(0xffffffffu, ok, 0);
+          ok = __all_sync(0xffffffffu, mbar_wait_spin(&bar.pv_done[b ^ 1], ((j - 1) >> 1) & 1, p.status, 26));  // P V of the previous step complete
           if (!ok) break;
           tc_fence_after();
 #pragma unroll
@@ -310,7 +323,12 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           l2[(i >> 1) & 1] = add_f32x2(l2[(i >> 1) & 1], pack_f32x2(x0, x1));
           pk[c * 16 + (i >> 1)] = bf16x2(x0, x1);
         }
-      tc_st_32x32b_x32(lane_addr + AT_TM_S + b * AT_BN, pk);  // P over the S it came from
+      if (j >= 2) {  // P V of step j - 2 has read this buffer
+        ok = __all_sync(0xffffffffu, mbar_wait_spin(&bar.pv_done[b], ((j >> 1) & 1) ^ 1, p.status, 28));
+        if (!ok) break;
+        tc_fence_after();
+      }
+      tc_st_32x32b_x32(lane_addr + AT_TM_P + b * (AT_BN / 2), pk);
       tc_wait_st();
       tc_fence_before();  // P and the O correction before the P V product that the arrival releases
       __syncwarp();
@@ -318,8 +336,7 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
     // O / l -> bf16 -> out[t, head * dk + :]
     if (ok) {
-      if (lane == 0) ok = mbar_wait_spin(&bar.pv_done, (steps - 1) & 1, p.status, 27);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
+      ok = __all_sync(0xffffffffu, mbar_wait_spin(&bar.o_full, 0, p.status, 27));
     }
     if (ok) {
       tc_fence_after();
