@@ -369,6 +369,16 @@ __device__ __forceinline__ uint32_t swish_quant_chunk(const uint32_t (&r)[32], c
 // Epilogue of one 32-column chunk held in registers by one thread (one output row).
 //   z[i]  accumulator value of logical column `ncol0 + i` (after scales)
 //   For GLU the caller passes value and gate chunks and `ncol0` in OUTPUT columns.
+// z += 32 bias values cached in shared memory by this warp (all lanes read the same words)
+__device__ __forceinline__ void add_bias32(float (&z)[32], const float* bias_s) {
+#pragma unroll
+  for (int i = 0; i < 32; i += 4) {
+    const float4 b = *reinterpret_cast<const float4*>(bias_s + i);
+    // (explicit roundings: every schedule of a kernel must produce the same bits)
+    z[i] = __fadd_rn(z[i], b.x); z[i + 1] = __fadd_rn(z[i + 1], b.y);
+    z[i + 2] = __fadd_rn(z[i + 2], b.z); z[i + 3] = __fadd_rn(z[i + 3], b.w);
+  }
+}
 template <int EPI, bool RES_TMA, bool TANH = false>
 struct ChunkOut {
   // Applies bias / activation / residual in place.  `bias_s` / `gate_s`: 32 bias values of the
@@ -379,22 +389,8 @@ struct ChunkOut {
                                                int lane) {
     if constexpr (EPI != VX_EPI_NONE) {
       if (bias_s) {
-        // bias values cached in shared memory by this warp (all lanes read the same words)
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const float4 b = *reinterpret_cast<const float4*>(bias_s + i);
-          // (explicit roundings: every schedule of a kernel must produce the same bits)
-          z[i] = __fadd_rn(z[i], b.x); z[i + 1] = __fadd_rn(z[i + 1], b.y);
-          z[i + 2] = __fadd_rn(z[i + 2], b.z); z[i + 3] = __fadd_rn(z[i + 3], b.w);
-        }
-        if constexpr (EPI == VX_EPI_BIAS_GLU) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            const float4 b = *reinterpret_cast<const float4*>(gate_s + i);
-            gate[i] = __fadd_rn(gate[i], b.x); gate[i + 1] = __fadd_rn(gate[i + 1], b.y);
-            gate[i + 2] = __fadd_rn(gate[i + 2], b.z); gate[i + 3] = __fadd_rn(gate[i + 3], b.w);
-          }
-        }
+        add_bias32(z, bias_s);
+        if constexpr (EPI == VX_EPI_BIAS_GLU) add_bias32(gate, gate_s);
       }
     }
     if constexpr (EPI == VX_EPI_BIAS_SWISH) {
@@ -1040,12 +1036,10 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     float lse_m = -INFINITY, lse_s = 0.0f;  // ARGMAX + log-sum-exp: running max / sum of 2^((z - max) log2 e) of the tile
     float* const bias_w = sm.bias_s + ew * 64;
     const float* const bias_base = p.bias ? bias_w : nullptr;
-    // FP8: per-warp tables of B scales at the end of the arena, [chunk][quadrant][kb][32];
-    // a GLU warp also owns the table of its gate chunk (chunk cc + 2, whose warps are idle)
+    // FP8: per-warp tables of B scales at the end of the arena, [chunk][quadrant][kb][32]
     int sb_nb = -1;
     float* const sb_all = reinterpret_cast<float*>(sm.arena + ARENA_BYTES - kb_count * FP8_SB_BYTES_PER_KB);
     float* const sb_tab = sb_all + ((cc * 4 + q) * kb_count) * 32;
-    float* const sb_gate = sb_all + ((((cc + 2) & 3) * 4 + q) * kb_count) * 32;
 
     // residual block of (mb, tile column c0) -> staging half `c & 1` (TMA, 32 rows x 32 bf16)
     auto res_issue = [&](uint32_t c, int mb_, int64_t out_col) {
@@ -1054,6 +1048,27 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         tma_load_2d(stage0 + (c & 1) * (STAGING_BYTES / 2), &tmap_res, static_cast<int>(out_col), mb_ * BM + q * 32,
                     &sm.res_full[c & 1][ew]);
       }
+    };
+
+    // FP8: the row scales of one round (four K blocks), fetched a round ahead: loaded block by block they were waited for
+    // between the blocks (QKV projection, 90,000 x 512 x 1536: call 192 us, 183 like this).
+    static_assert(FP8_ACCS == 4, "load_sa fetches one round");
+    float4 sa4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const bool sa_vec = FP8 && (kb_count & 3) == 0 && (reinterpret_cast<uintptr_t>(p.fa) & 15) == 0;
+    auto load_sa = [&](int64_t r, int kb) {
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (r < p.M) {
+        const float* const src = p.fa + r * kb_count + kb;
+        if (sa_vec) {
+          v = *reinterpret_cast<const float4*>(src);
+        } else {
+          v.x = src[0];
+          if (kb + 1 < kb_count) v.y = src[1];
+          if (kb + 2 < kb_count) v.z = src[2];
+          if (kb + 3 < kb_count) v.w = src[3];
+        }
+      }
+      return v;
     };
 
     int mb = mb0, nb = nb0;
@@ -1143,24 +1158,19 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           const int64_t ncol = static_cast<int64_t>(nb) * BNT + col_base + lane;
           const float* src = p.fb + ncol * kb_count;
           for (int kb = 0; kb < kb_count; ++kb) sb_tab[kb * 32 + lane] = ncol < p.N ? src[kb] : 0.0f;
-          if constexpr (GLU) {
-            if (has_work) {
-              const int64_t gcol = ncol + GATE_OFF;
-              const float* gsrc = p.fb + gcol * kb_count;
-              for (int kb = 0; kb < kb_count; ++kb) sb_gate[kb * 32 + lane] = gcol < p.N ? gsrc[kb] : 0.0f;
-            }
-          }
           __syncwarp();
           sb_nb = nb;
         }
         // promote each 128-wide K block: z += tmem * (sa[row, kb] * sb[col, kb])
 #pragma unroll
-        for (int i = 0; i < 32; ++i) { z[0][i] = 0.0f; gate[i] = 0.0f; }
-        const float* sa_row = p.fa + row * kb_count;
-        float sa_next = row_ok ? *sa_row : 0.0f;
+        for (int i = 0; i < 32; ++i) z[0][i] = 0.0f;
+        if (it == 0) sa4 = load_sa(row, 0);
         for (int kb0 = 0; kb0 < kb_count && ok; kb0 += FP8_ACCS) {
           // one round: up to four K blocks, block u in accumulator u, published together
           const int nkb = kb_count - kb0 < FP8_ACCS ? kb_count - kb0 : FP8_ACCS;
+          float4 sa_next4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (kb0 + FP8_ACCS < kb_count) sa_next4 = load_sa(row, kb0 + FP8_ACCS);
+          else sa_next4 = load_sa(it + 1 < my_tiles ? static_cast<int64_t>(mb_next) * BM + q * 32 + lane : p.M, 0);
           ok = __all_sync(0xffffffffu, mbar_wait_spin<WAIT_CALL>(&sm.tmem_full[0], group & 1, p.status, 4));
           if (!ok) break;
           ++group;
@@ -1169,8 +1179,8 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
 #pragma unroll 1
           for (int u = 0; u < nkb; ++u) {
             const int kb = kb0 + u;
-            const float sa = sa_next;
-            if (kb + 1 < kb_count && row_ok) sa_next = sa_row[kb + 1];
+            const float sa = sa4.x;
+            sa4 = make_float4(sa4.y, sa4.z, sa4.w, 0.0f);
             const uint64_t sa2 = pack_f32x2(sa, sa);
             // acc[i] += r[i] * (sa * table[i]).  The scale products are a packed fp32x2
             // multiply (both operands come as pairs: sb from shared memory, sa duplicated); the
@@ -1194,28 +1204,42 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
             };
             const uint32_t acc_addr = lane_addr + TM_ACC0 + u * 128 + col_base;
             uint32_t r[32];
-            if constexpr (GLU) {
-              if (has_work) {  // gate first, so that one register block serves both loads
-                tc_ld_32x32b_x32(acc_addr + GATE_OFF, r);
-                tc_wait_ld();
-                promote(gate, r, sb_gate + kb * 32);
-              }
-            }
-            if (has_work) {
-              tc_ld_32x32b_x32(acc_addr, r);
-              tc_wait_ld();
-            }
+            tc_ld_32x32b_x32(acc_addr, r);
+            tc_wait_ld();
             if ((u & 1) || u == nkb - 1) {
               // both accumulators of the pair are in registers: hand the pair back
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive(&sm.tmem_empty[u >> 1]);
             }
-            if (has_work) promote(z[0], r, sb_tab + kb * 32);
+            promote(z[0], r, sb_tab + kb * 32);
             if (tr && kb0 == 0) trace_rec(p, 2, it, 1 + u);
           }
+          sa4 = sa_next4;
         }
         if (!ok) break;
+        if constexpr (GLU) {
+          // The warps of the gate columns (chunks 2, 3) pass sigmoid(gate) to those of the value columns through their own
+          // staging buffer, [column][lane].  Barriers of the residual blocks, which GLU does not have: [0] passed, [1] taken.
+          // (The value warps promoting both chunks, 8 of 16 warps idle, spilled 600 bytes: 60,000 x 512 x 1024: call 294 us, 109 like this.)
+          const int vw = ew & 7;  // value warp of the pair
+          float* const pass = reinterpret_cast<float*>(sm.staging[vw + 8]) + lane;
+          if (!has_work) {
+            if (bias_base) add_bias32(z[0], bias_base);
+            if (it > 0 && !mbar_wait<WAIT_CALL>(&sm.res_full[1][vw], (it - 1) & 1, p.status, 10)) { ok = false; break; }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) pass[i * 32] = sigmoid_f(z[0][i]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.res_full[0][vw]);
+          } else {
+            if (bias_base) add_bias32(z[0], bias_base);
+            if (!mbar_wait<WAIT_CALL>(&sm.res_full[0][vw], it & 1, p.status, 10)) { ok = false; break; }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) z[0][i] *= pass[i * 32];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.res_full[1][vw]);
+          }
+        }
       } else {
         if (tr) trace_rec(p, 2, it, 0);
         if (sf_unit) {
@@ -1313,7 +1337,8 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
             }
           }
           if (tr && h == 0 && !FP8) trace_rec(p, 2, it, 3);
-          ChunkOut<EPI, OUT == 1, kind_pow2_scales(KIND)>::apply(p, z[h], gate, row, bias_base ? bias_base + h * 32 : nullptr, bias_base + 32, out_col0,
+          if constexpr (!(FP8 && GLU))
+            ChunkOut<EPI, OUT == 1, kind_pow2_scales(KIND)>::apply(p, z[h], gate, row, bias_base ? bias_base + h * 32 : nullptr, bias_base + 32, out_col0,
                                row_ok, res_smem, lane);
           if (tr && h == 0 && !FP8) trace_rec(p, 2, it, 4);
 
