@@ -1031,7 +1031,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     uint32_t res_chunk = 0;  // chunks consumed so far
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const bool dbuf = out_dtype == VX_BF16 && !tma_residual;  // bf16 boxes alternate the two halves
-    uint32_t store_count = 0;
+    uint32_t store_count = 0;  // boxes handed to the TMA by this warp
     int bias_nb = -1;
     uint32_t best_key = 0;  // ARGMAX: best (value, column) of this thread's row in the current tile
     float lse_m = -INFINITY, lse_s = 0.0f;  // ARGMAX + log-sum-exp: running max / sum of 2^((z - max) log2 e) of the tile
@@ -1531,7 +1531,10 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
             } else {
               if (lane == 0) tma_store_wait_read<0>();
             }
-            ++store_count;
+            // (Only boxes that leave count: the wait above is for the second-last STORE.  Counting chunks beyond the last column, the
+            // halves of a warp whose second chunk does not exist -- columns 192..255 of a tile that ends before them -- were one
+            // and the same, rewritten while the previous tile's store could still be reading it.)
+            if (box_ok) ++store_count;
             __syncwarp();
             if (out_dtype == VX_BF16) {
               // 64-byte rows, 64-byte swizzle: 16-byte slot index ^= (row >> 1) & 3
