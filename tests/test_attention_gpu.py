@@ -81,3 +81,30 @@ def test_attention_argument_errors(ops):
         ops.relpos_attention(q2[..., :64].contiguous(), k2[..., :64].contiguous(), v2[..., :64].contiguous())
     with pytest.raises(ValueError):
         ops.relpos_attention(q2.float(), k2.float(), v2.float())
+
+
+@pytest.mark.parametrize("top", [3, 70, 127])
+@pytest.mark.parametrize("T", [128, 300])
+def test_largest_probability_of_the_first_keys_is_exact(T, top):
+    """Rows whose weight is all but on one key: P is rounded to bf16 relative to the row's reference maximum, so where that is the
+    largest score itself the probability is exactly 1 and the result is v to its own rounding (8 significant bits: 2^-8).
+    The reference is the maximum of the first 128 keys: `top` in either half of them, a score 1..5 below it in the other half."""
+    from velox_voice_b200 import ops
+
+    torch.manual_seed(top)
+    h, dk = 8, 64
+    q = torch.zeros(h, T, 128)
+    k = torch.zeros(h, T, 128)
+    q[..., 0] = 1.0 + torch.rand(h, T)
+    k[..., 0] = -30.0
+    k[:, top, 0] = 4.0
+    k[:, (top + 64) % 128, 0] = 0.5
+    v = torch.zeros(h, T, 128)
+    v[..., :dk] = torch.randn(h, T, dk)
+    q, k, v = (t.cuda().bfloat16() for t in (q, k, v))
+    out = ops.relpos_attention(q, k, v).double().view(T, h, dk).transpose(0, 1)
+    w = torch.softmax(q.double() @ k.double().transpose(1, 2), -1)
+    ref = w @ v[..., :dk].double()
+    # the other key (weight at most e^-3.5 of the first) is rounded too: 2^-8 of its share
+    share = torch.exp(torch.tensor(-3.5)).item() * v[..., :dk].abs().amax().double()
+    assert ((out - ref).abs() <= 2.0 ** -8 * (ref.abs() + 2 * share)).all()

@@ -21,15 +21,16 @@
 // is there when the softmax gets to it.
 // Tensor memory (256 columns): S (64) | P0 | P1 (32 each) | O (64) | Q (64).
 // One pass over the keys with a lazily updated reference maximum: p = 2^((s - m_ref) log2 e) is formed
-// against the reference m_ref the row has used so far, which only moves when a tile's maximum exceeds it by
-// more than 2^8 (so p never exceeds 256 and nothing overflows in bf16 or fp32).  When it moves -- typically in
-// the first tiles of a row only -- the row sum and the row's O accumulator are multiplied by 2^((m_old - m_new) log2 e)
+// against the reference m_ref the row has used so far, at first the maximum of its first 128 keys, which only moves when a
+// step's maximum exceeds it by more than 2^8 (so p never exceeds 256 and nothing overflows in bf16 or fp32).  When it moves -- in
+// few rows and steps -- the row sum and the row's O accumulator are multiplied by 2^((m_old - m_new) log2 e)
 // (tcgen05.ld / tcgen05.st) before the next P V product is released.  O is divided by the row sum once at the end.
 // What bounds it: the two softmax warps of an SM partition and the special-function unit that they share (64 exponentials per
 // row and step, 16 lanes per cycle and SM: 512 cycles per CTA and step; the MMAs take 400).  3,750 frames and 8 heads: 99 us
 // with one CTA per SM, P through shared memory and a maximum exchange between two warps per row (3,200 cycles per 128 x 128
 // tile); 62 us with two CTAs and P over S, where the round trip of a buffer -- P V, then the S behind it -- made the softmax
-// wait 340 cycles a step; 58 us like this.  Neither eight softmax warps per CTA in two independent groups (73 us) nor a
+// wait 340 cycles a step; 58 us with the maximum of the first 64 keys as reference, 60 us like this.  (The shared maximum in every
+// pair of steps: 70 us, the softmax then waits for the second S.)  Neither eight softmax warps per CTA in two independent groups (73 us) nor a
 // quarter of the exponentials as polynomials on the fp32 pipe (64 us) helped.
 // Every mbarrier wait is bounded.
 
@@ -252,29 +253,29 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       if (lane == 0) mbar_arrive(&bar.q_full);
     }
     float m_ref = NEG_INF;  // reference maximum of the row, in units of log2 (s * log2 e)
-    uint64_t l2[2] = {0ull, 0ull};  // row sum, four partial sums as packed pairs
+    uint64_t la[2] = {0ull, 0ull}, lb[2] = {0ull, 0ull};  // row sums of the even and the odd steps, four partial sums each as packed pairs
     bool ok = true;
-    for (int j = 0; j < steps; ++j) {
-      const int b = j & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait_spin(&bar.s_full, j & 1, p.status, 25));
-      if (!ok) break;
+    // S of step j into registers; keys beyond kv_len (the last step of a span whose length is not a multiple of 64) count as -inf
+    auto read_s = [&](int j, uint32_t (&s)[2][32]) {
+      if (!__all_sync(0xffffffffu, mbar_wait_spin(&bar.s_full, j & 1, p.status, 25))) return false;
       tc_fence_after();
-      uint32_t s[2][32];
       tc_ld_32x32b_x32(lane_addr + AT_TM_S, s[0]);
       tc_ld_32x32b_x32(lane_addr + AT_TM_S + 32, s[1]);
       tc_wait_ld();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.s_empty);  // S is in registers: that of the next step may be written
-      const int n_valid = static_cast<int>(p.kv_len - static_cast<int64_t>(j) * AT_BN);  // >= 64: the whole tile
+      const int n_valid = static_cast<int>(p.kv_len - static_cast<int64_t>(j) * AT_BN);  // >= 64: the whole step
       if (n_valid < AT_BN) {
-        // the last tile of a span whose length is not a multiple of 64: keys beyond kv_len count as -inf
 #pragma unroll
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             if (c * 32 + i >= n_valid) s[c][i] = 0xff800000u;
       }
+      return true;
+    };
+    auto max_s = [&](const uint32_t (&s)[2][32]) {
       float m4[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -284,32 +285,10 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         for (int i = 2; i < 16; i += 2) m = max3(m, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
         m4[q] = m;
       }
-      const float m_tile = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * L2E;
-      // The reference of a row moves when the tile's maximum exceeds it by more than 8.  Then the row sum and the row's O are
-      // scaled by 2^(m_ref - m_tile).  The tensor-memory accesses are warp-wide, so the warp goes through them when any of
-      // its rows moves; the other rows scale by one.  Before the first P V product there is nothing to scale.
-      const bool moves = m_tile > m_ref + 8.0f;
-      if (__any_sync(0xffffffffu, moves)) {
-        const float alpha = moves ? ex2f(m_ref - m_tile) : 1.0f;  // 0 for m_ref = -inf
-        if (moves) m_ref = m_tile;
-        const uint64_t a2 = pack_f32x2(alpha, alpha);
-        l2[0] = mul_f32x2(l2[0], a2);
-        l2[1] = mul_f32x2(l2[1], a2);
-        if (j > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait_spin(&bar.pv_done[b ^ 1], ((j - 1) >> 1) & 1, p.status, 26));  // P V of the previous step complete
-          if (!ok) break;
-          tc_fence_after();
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t o[32];
-            tc_ld_32x32b_x32(lane_addr + AT_TM_O + h * 32, o);
-            tc_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tc_st_32x32b_x32(lane_addr + AT_TM_O + h * 32, o);
-          }
-        }
-      }
+      return fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+    };
+    // P of step j against the row's reference, its sum into l, P V released
+    auto put_p = [&](int j, const uint32_t (&s)[2][32], uint64_t (&l)[2]) {
       const uint64_t k2 = pack_f32x2(L2E, L2E), n2 = pack_f32x2(-m_ref, -m_ref);
       uint32_t pk[32];
 #pragma unroll
@@ -320,19 +299,75 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), k2, n2), x0, x1);
           x0 = ex2f(x0);
           x1 = ex2f(x1);
-          l2[(i >> 1) & 1] = add_f32x2(l2[(i >> 1) & 1], pack_f32x2(x0, x1));
+          l[(i >> 1) & 1] = add_f32x2(l[(i >> 1) & 1], pack_f32x2(x0, x1));
           pk[c * 16 + (i >> 1)] = bf16x2(x0, x1);
         }
       if (j >= 2) {  // P V of step j - 2 has read this buffer
-        ok = __all_sync(0xffffffffu, mbar_wait_spin(&bar.pv_done[b], ((j >> 1) & 1) ^ 1, p.status, 28));
-        if (!ok) break;
+        if (!__all_sync(0xffffffffu, mbar_wait_spin(&bar.pv_done[j & 1], ((j >> 1) & 1) ^ 1, p.status, 28))) return false;
         tc_fence_after();
       }
-      tc_st_32x32b_x32(lane_addr + AT_TM_P + b * (AT_BN / 2), pk);
+      tc_st_32x32b_x32(lane_addr + AT_TM_P + (j & 1) * (AT_BN / 2), pk);
       tc_wait_st();
       tc_fence_before();  // P and the O correction before the P V product that the arrival releases
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bar.p_full[b]);
+      if (lane == 0) mbar_arrive(&bar.p_full[j & 1]);
+      return true;
+    };
+    int j = 0;
+    {
+      // The first two steps share their maximum: most rows never move their reference again, and with the first 64 keys alone
+      // a row whose largest probability lies among the next 64 would have it rounded instead of exactly 1 (relative error
+      // against fp64 for 128 keys, scores of standard deviation 3: 2.04e-3, 1.75e-3 like this).
+      uint32_t s0[2][32], s1[2][32];
+      ok = read_s(0, s0);
+      if (ok) {
+        float m = max_s(s0);
+        if (steps > 1) ok = read_s(1, s1);
+        if (steps > 1 && ok) m = fmaxf(m, max_s(s1));
+        m_ref = __fmul_rn(m, L2E);
+        if (ok) ok = put_p(0, s0, la);
+        if (ok && steps > 1) ok = put_p(1, s1, lb);
+      }
+      j = steps > 1 ? 2 : 1;
+    }
+    for (; ok && j < steps; ++j) {
+      uint32_t s[2][32];
+      ok = read_s(j, s);
+      if (!ok) break;
+      const float m_step = __fmul_rn(max_s(s), L2E);
+      // The reference of a row moves when the step's maximum exceeds it by more than 8.  Then the row sum and the row's O are
+      // scaled by 2^(m_ref - m_step).  The tensor-memory accesses are warp-wide, so the warp goes through them when any of
+      // its rows moves; the other rows scale by one.
+      const bool moves = m_step > m_ref + 8.0f;
+      if (__any_sync(0xffffffffu, moves)) {
+        const float alpha = moves ? ex2f(m_ref - m_step) : 1.0f;  // 0 for m_ref = -inf
+        if (moves) m_ref = m_step;
+        const uint64_t a2 = pack_f32x2(alpha, alpha);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          la[i] = mul_f32x2(la[i], a2);
+          lb[i] = mul_f32x2(lb[i], a2);
+        }
+        ok = __all_sync(0xffffffffu, mbar_wait_spin(&bar.pv_done[(j & 1) ^ 1], ((j - 1) >> 1) & 1, p.status, 26));  // P V of the previous step complete
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t o[32];
+          tc_ld_32x32b_x32(lane_addr + AT_TM_O + h * 32, o);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tc_st_32x32b_x32(lane_addr + AT_TM_O + h * 32, o);
+        }
+      }
+      ok = put_p(j, s, la);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {  // the other sum is next
+        const uint64_t t = la[i];
+        la[i] = lb[i];
+        lb[i] = t;
+      }
     }
     // O / l -> bf16 -> out[t, head * dk + :]
     if (ok) {
@@ -340,10 +375,13 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
     if (ok) {
       tc_fence_after();
-      float a0, a1, b0, b1;
-      unpack_f32x2(l2[0], a0, a1);
-      unpack_f32x2(l2[1], b0, b1);
-      const float inv = 1.0f / ((a0 + a1) + (b0 + b1));
+      auto sum4 = [](const uint64_t (&l)[2]) {
+        float a0, a1, b0, b1;
+        unpack_f32x2(l[0], a0, a1);
+        unpack_f32x2(l[1], b0, b1);
+        return (a0 + a1) + (b0 + b1);
+      };
+      const float inv = 1.0f / (sum4(la) + sum4(lb));
       __nv_bfloat16* const dst = p.out + tq * p.ldo + head * AT_DV;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
