@@ -1,0 +1,42 @@
+"""Rules of the device code that no single run can show: read from the sources."""
+
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "velox_voice_b200", "csrc")
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+@pytest.mark.parametrize("name,kernel", [("vx_gemm_ln.cu", "bsgemm_residual_ln_kernel("), ("vx_gemm.cu", "bsgemm_kernel("),
+                                         ("vx_attn.cu", "relpos_attn_kernel("), ("vx_mel.cu", "power_mel_log_dense_kernel("),
+                                         ("vx_mel.cu", "power_mel_log_kernel(")])
+def test_waits_before_warp_wide_tensor_memory_accesses_end_in_a_vote(name, kernel):
+    """tcgen05.ld, .st and .wait are warp-wide.  A poll of an mbarrier can answer lane by lane, so the lanes of a warp can leave
+    a waiting loop on different turns: before such an access they have to be brought together (a vote or __syncwarp).  Held
+    for every wait by all lanes from which such an access can be reached without one."""
+    text = source(name)
+    text = text[text.index(kernel):]
+    end = re.search(r"\n}\n", text)
+    text = text[:end.end()]
+    aligned = re.compile(r"\btc_(ld|st|wait)\w*\(")
+    wait = re.compile(r"\bmbar_wait\w*(<\w+>)?\(")
+    gather = re.compile(r"__all_sync|__syncwarp|__shfl\w*_sync|__any_sync|__syncthreads|__ballot_sync")
+    role = re.compile(r"\n  } else\b")  # the next role of a warp-specialised kernel: other warps
+    event = re.compile("|".join(f"(?:{r.pattern})" for r in (aligned, wait, gather, role)))
+    open_wait = None
+    for m in event.finditer(text):
+        t = m.group(0)
+        if wait.fullmatch(t):
+            line = text[text.rfind("\n", 0, m.start()):m.start()]
+            if "__all_sync" not in line:
+                open_wait = text[m.start():m.start() + 60]
+        elif gather.fullmatch(t) or role.fullmatch(t):
+            open_wait = None
+        else:
+            assert open_wait is None, f"{name}: {t} can be reached by a part of a warp behind {open_wait!r}"

@@ -336,9 +336,13 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     for (int i = 0; i < my_tiles && ok; ++i, mb += nclusters) {
       const int64_t row = static_cast<int64_t>(mb) * LN_BM + row_in;
       const bool row_ok = row < p.M;
-      if (!mbar_wait(&sm.tmem_full, i & 1, p.status, 24)) { ok = false; break; }
+      // (Every wait of these warps ends in a vote: a poll can answer lane by lane, so lanes can leave a waiting loop on different
+      // turns, and nothing else would bring them together again before the warp-wide tcgen05.ld / st below.)
+      ok = __all_sync(0xffffffffu, mbar_wait(&sm.tmem_full, i & 1, p.status, 24));
+      if (!ok) break;
       tc_fence_after();
-      if (!mbar_wait(&sm.res_full[ew], i & 1, p.status, 27)) { ok = false; break; }
+      ok = __all_sync(0xffffffffu, mbar_wait(&sm.res_full[ew], i & 1, p.status, 27));
+      if (!ok) break;
       // ---- pass 1: x = bf16(alpha (acc + bias) + residual), block statistics
       float SQ[4];
 #pragma unroll
@@ -409,7 +413,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       // the staging block is free, and reduces the 16 block sums of the row: (rstd, -mean rstd) as packed pairs
       auto finish_stats = [&](uint32_t b, uint32_t parity, bool staging_free, uint64_t& R2, uint64_t& N2) -> bool {
         // (plain polling: at this point every epilogue warp of the quadrant waits, nobody is robbed of issue slots)
-        const bool landed = mbar_wait_spin(&sm.xch[b][q], parity, p.status, 25);
+        const bool landed = __all_sync(0xffffffffu, mbar_wait_spin(&sm.xch[b][q], parity, p.status, 25));
         tc_wait_st_all();  // the bf16 copy is in tensor memory before the next pass reads it back
         if (!landed) return false;
         if (g == 0 && lane == 0) mbar_expect_tx(&sm.xch[b][q], LN_XCH_BYTES);  // armed for the next use
