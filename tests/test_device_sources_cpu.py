@@ -40,3 +40,14 @@ def test_waits_before_warp_wide_tensor_memory_accesses_end_in_a_vote(name, kerne
             open_wait = None
         else:
             assert open_wait is None, f"{name}: {t} can be reached by a part of a warp behind {open_wait!r}"
+
+
+@pytest.mark.parametrize("name", ["vx_gemm_ln.cu", "vx_gemm.cu"])
+def test_stores_are_complete_before_a_kernel_ends(name):
+    """Writes of a bulk store are ordered by waiting for its group, not by the end of the thread that issued it; the `.read`
+    form says only that shared memory may be reused.  The last wait before the tear-down is the full one."""
+    text = source(name)
+    waits = [m.group(1) for m in re.finditer(r"tma_store_wait_(read|all)<0>\(\)", text)]
+    assert text.count("tma_store_commit()") >= 1 and waits[-1] == "all"
+    last = text.rindex("tma_store_wait_all<0>()")
+    assert text.rindex("tma_store_commit()") < last < text.index("tmem_dealloc(tmem_base", last)

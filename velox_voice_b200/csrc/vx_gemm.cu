@@ -1591,7 +1591,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
       mb = mb_next;
       nb = nb_next;
     }
-    if (tma_store && lane == 0) tma_store_wait_read<0>();  // (shared memory is read; the writes complete with the grid)
+    if (tma_store && lane == 0) tma_store_wait_all<0>();  // the writes, not only the reads of shared memory: the next launch may be waiting for this grid to end
   }
 
   // ---- tear-down

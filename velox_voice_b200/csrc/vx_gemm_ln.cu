@@ -553,7 +553,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         *reinterpret_cast<uint16_t*>(p.sf_out + off) = static_cast<uint16_t>(row_ok ? sf2 : 0u);
       }
     }
-    if (lane == 0) tma_store_wait_read<0>();  // (shared memory is read; the writes complete with the grid)
+    if (lane == 0) tma_store_wait_all<0>();  // the writes, not only the reads of shared memory: the next launch may be waiting for this grid to end
   }
 
   // ---- tear-down
