@@ -51,3 +51,13 @@ def test_stores_are_complete_before_a_kernel_ends(name):
     assert text.count("tma_store_commit()") >= 1 and waits[-1] == "all"
     last = text.rindex("tma_store_wait_all<0>()")
     assert text.rindex("tma_store_commit()") < last < text.index("tmem_dealloc(tmem_base", last)
+
+
+def test_the_gemm_triggers_the_next_launch_only_behind_its_own_wait():
+    """One thread that triggers counts for its CTA.  The producer's lane reads weights ahead of its wait, so the trigger must
+    not be reachable for it, nor for any thread, without the wait in front."""
+    text = source("vx_gemm.cu")
+    text = text[text.index("bsgemm_kernel("):]
+    text = text[:re.search(r"\n}\n", text).end()]
+    assert text.count("pdl_launch_dependents()") == 1
+    assert re.search(r"if \(warp != 0 \|\| my_tiles == 0\) {\s*pdl_wait\(\);\s*pdl_launch_dependents\(\);\s*}", text)

@@ -718,12 +718,15 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   const uint32_t tmem_base = sm.tmem_base;
   const int n_sf_tiles = static_cast<int>((p.N + 127) >> 7);  // 128-row SF tiles of B that exist
   // Set-up is done.  Everything below may touch what the previous kernel of the stream produced (A,
-  // residual, output buffers), so every thread waits for it here -- except the producer thread, which
+  // residual, output buffers), so every warp waits for it here -- except the producer's, whose one active lane
   // first starts the loads of its resident weights (constants of the model) and then waits.
-  const bool producer_thread = warp == 0 && lane == 0 && my_tiles > 0;
-  if (!producer_thread) pdl_wait();
-  // The trigger stands behind the wait: launches further ahead only queue up (12 blocks, 375 frames: 891 us with it at the start, 842).
-  pdl_launch_dependents();  // the next kernel of the stream may be scheduled as SMs free up (it waits for this one)
+  // The next launch is triggered behind the wait, by the warps that have waited: earlier, launches further ahead only queue up
+  // (12 blocks, 375 frames: 891 us with the trigger at the start, 842 like this), and nothing could be said about what is
+  // complete when the next kernel starts.
+  if (warp != 0 || my_tiles == 0) {
+    pdl_wait();
+    pdl_launch_dependents();  // the next kernel of the stream may be scheduled as SMs free up (it waits for this one)
+  }
 
   if (warp == 0) {
     // =========================== TMA producer ===========================
