@@ -61,3 +61,11 @@ def test_the_gemm_triggers_the_next_launch_only_behind_its_own_wait():
     text = text[:re.search(r"\n}\n", text).end()]
     assert text.count("pdl_launch_dependents()") == 1
     assert re.search(r"if \(warp != 0 \|\| my_tiles == 0\) {\s*pdl_wait\(\);\s*pdl_launch_dependents\(\);\s*}", text)
+
+
+def test_the_wait_for_the_other_ctas_sums_acquires_at_cluster_scope():
+    """st.async of the peer completes the exchange barrier with a release at cluster scope; a wait that acquires at the default
+    scope, the CTA, does not pair with it."""
+    text = source("vx_gemm_ln.cu")
+    assert re.findall(r"mbar_wait\w*\(&sm\.xch", text) == ["mbar_wait_spin_cluster(&sm.xch"]
+    assert "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64" in source("vx_ptx.cuh")

@@ -412,8 +412,9 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       // waits for the sums of exchange b, arms its barrier for the next use, fetches the next residual block when
       // the staging block is free, and reduces the 16 block sums of the row: (rstd, -mean rstd) as packed pairs
       auto finish_stats = [&](uint32_t b, uint32_t parity, bool staging_free, uint64_t& R2, uint64_t& N2) -> bool {
-        // (plain polling: at this point every epilogue warp of the quadrant waits, nobody is robbed of issue slots)
-        const bool landed = __all_sync(0xffffffffu, mbar_wait_spin(&sm.xch[b][q], parity, p.status, 25));
+        // (plain polling: at this point every epilogue warp of the quadrant waits, nobody is robbed of issue slots; half of the
+        // sums come from the other CTA)
+        const bool landed = __all_sync(0xffffffffu, mbar_wait_spin_cluster(&sm.xch[b][q], parity, p.status, 25));
         tc_wait_st_all();  // the bf16 copy is in tensor memory before the next pass reads it back
         if (!landed) return false;
         if (g == 0 && lane == 0) mbar_expect_tx(&sm.xch[b][q], LN_XCH_BYTES);  // armed for the next use

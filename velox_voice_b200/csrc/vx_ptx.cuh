@@ -72,6 +72,19 @@ __device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same, acquiring at cluster scope: for a barrier that another CTA of the cluster completes.
+__device__ __forceinline__ bool mbar_poll_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Wall-clock limit of one wait.  Whole kernels here run for well under 100 ms.
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
 
@@ -128,6 +141,13 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, i
   if (__builtin_expect(mbar_poll(bar, parity), 1)) return true;
   if (CALL) return mbar_wait_call<false>(bar, parity, status, site, abort);
   return mbar_wait_loop<false, 16384>(bar, parity, status, site, abort, kWaitLimitNs);
+}
+
+// Plain polling at cluster scope: what other CTAs of the cluster wrote ahead of the completion is visible behind it.
+__device__ __forceinline__ bool mbar_wait_spin_cluster(uint64_t* bar, uint32_t parity, int* status, int site) {
+  if (__builtin_expect(mbar_poll_cluster(bar, parity), 1)) return true;
+  // (the loop polls at CTA scope; the poll that ends the wait is the acquiring one)
+  return mbar_wait_loop<false, 16384>(bar, parity, status, site, nullptr, kWaitLimitNs) && mbar_poll_cluster(bar, parity);
 }
 
 // ------------------------------------------------------------------ proxies / fences
