@@ -169,6 +169,11 @@ long as_long(PyObject* o) {
   if (v == -1 && PyErr_Occurred()) throw PyFail{};
   return v;
 }
+bool as_bool(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw PyFail{};
+  return v != 0;
+}
 double as_double(PyObject* o) {
   const double v = PyFloat_AsDouble(o);
   if (v == -1.0 && PyErr_Occurred()) throw PyFail{};
@@ -203,7 +208,7 @@ PyObject* py_quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const at::Tensor& x = THPVariable_Unpack(a[0]);
   const int dt = dtype_code(x), fmt = static_cast<int>(as_long(a[1]));
   if (dt < 0 || !rows2d(x)) Py_RETURN_NONE;
-  const bool natural = a[2] == Py_True || fmt == VX_FMT_ROWSCALE || fmt == VX_FMT_FP8_1X128;
+  const bool natural = as_bool(a[2]) || fmt == VX_FMT_ROWSCALE || fmt == VX_FMT_FP8_1X128;
   const int64_t M = x.size(0), K = x.size(1);
   const float* am = nullptr;
   PyObject* amax = a[4];
@@ -221,7 +226,7 @@ PyObject* py_quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   } else if (amax != Py_None) {
     Py_RETURN_NONE;
   }
-  const Outputs o = alloc_outputs(fmt, M, K, x.device(), natural, a[3] == Py_True);
+  const Outputs o = alloc_outputs(fmt, M, K, x.device(), natural, as_bool(a[3]));
   const int rc = g.vx_quantize_pack(x.data_ptr(), dt, M, K, x.stride(0), fmt, ptr(o.codes), o.codes.stride(0), ptr(o.scales), ptr(o.sf),
                                     am, stream());
   if (rc) Py_XDECREF(made);
@@ -253,8 +258,8 @@ PyObject* py_ln_quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   } else if (a[7] != Py_None) {
     Py_RETURN_NONE;
   }
-  const bool natural = a[5] == Py_True || fmt == VX_FMT_ROWSCALE || fmt == VX_FMT_FP8_1X128;
-  const Outputs o = alloc_outputs(fmt, M, K, x.device(), natural, a[6] == Py_True);
+  const bool natural = as_bool(a[5]) || fmt == VX_FMT_ROWSCALE || fmt == VX_FMT_FP8_1X128;
+  const Outputs o = alloc_outputs(fmt, M, K, x.device(), natural, as_bool(a[6]));
   check(g.vx_ln_quantize_pack(x.data_ptr(), dt, M, K, x.stride(0), gamma, beta, static_cast<float>(as_double(a[3])), fmt, ptr(o.codes),
                               o.codes.stride(0), ptr(o.scales), ptr(o.sf), am, nullptr, 0, K, stream()),
         "vx_ln_quantize_pack");
@@ -301,7 +306,7 @@ PyObject* py_bsgemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
     } else if (ofmt != VX_FMT_MX32 || p[9] != Py_None) {
       Py_RETURN_NONE;
     }
-    const Outputs o = alloc_outputs(ofmt, d.M, n_out, dev, p[10] == Py_True, true);
+    const Outputs o = alloc_outputs(ofmt, d.M, n_out, dev, as_bool(p[10]), true);
     d.out_dtype = VX_FP4; d.out = ptr(o.codes); d.ldo = o.codes.stride(0);
     d.out_fmt = ofmt; d.out_scales_sf = ptr(o.sf); d.out_scales = ptr(o.scales);
     check(g.vx_bsgemm(&d, stream()), "vx_bsgemm");
@@ -721,7 +726,7 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   plan->fmt = static_cast<int>(as_long(a[0]));
   plan->d = as_long(a[1]); plan->ffn = as_long(a[2]); plan->glu = as_long(a[3]); plan->vocab = as_long(a[4]);
   plan->eps = static_cast<float>(as_double(a[5]));
-  plan->fuse_ffn = a[6] == Py_True;
+  plan->fuse_ffn = as_bool(a[6]);
   plan->blocks = static_cast<int>(as_long(a[7]));
   auto bad = [](const char* what) { PyErr_SetString(PyExc_ValueError, what); throw PyFail{}; };
   for (int i = 8; i < 11; ++i)
@@ -823,7 +828,7 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     pos_q = sp.act(w_pos, d, p.amax(p.blocks * A_COUNT + 1));
     sp.quantize(pt.data_ptr(), dtype_code(pt), pt.stride(0), pos_q);
   }
-  const bool fused = a[3] == Py_True;
+  const bool fused = as_bool(a[3]);
   if (lp_batched) sp.gemm(pos_q, p.lp_all, VX_EPI_NONE, w_lp, p.blocks * d);
   // the quantizers of the value third and of the GLU output run in the epilogues that produce them
   const bool in_epilogue = p.fmt != VX_FMT_FP8_1X128 && d % 256 == 0 && p.glu % 256 == 0;
