@@ -144,3 +144,29 @@ def test_remaining_operators_agree_on_both_routes(ops, monkeypatch):
     for kv in (None, 0, 65, T, T + 1):
         assert same(*both_routes(ops, monkeypatch, lambda: ops.relpos_attention(*qkv, kv)))
     assert same(*both_routes(ops, monkeypatch, lambda: ops.relpos_attention(qkv[0], qkv[1].transpose(0, 1).contiguous().transpose(0, 1), qkv[2])))
+
+
+def test_dense_linear_bias_need_not_be_a_parameter():
+    """Pruning and parametrization turn `bias` into a plain attribute or a property of the module."""
+    from torch.nn.utils import parametrize
+
+    from velox_voice_b200.linear import DenseLinear
+
+    torch.manual_seed(5)
+    w, b = torch.randn(256, 128), torch.randn(256)
+    x = torch.randn(20, 128, device="cuda")
+
+    def make():
+        lin = DenseLinear(w, b).cuda().requires_grad_(False)
+        lin.precision = "mxfp4"
+        return lin
+
+    want = make()(x)
+    lin = make()
+    bias = lin.bias.detach()
+    del lin.bias
+    lin.bias = bias
+    assert torch.equal(lin(x), want)
+    lin = make()
+    parametrize.register_parametrization(lin, "bias", torch.nn.Identity())
+    assert torch.equal(lin(x), want)

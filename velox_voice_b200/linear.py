@@ -167,7 +167,7 @@ class DenseLinear(nn.Linear):
             if self._wq is None:
                 self._prequantize_weight(precision)
             # quantize + one GEMM with the scales and the bias in its epilogue (fp32 out)
-            r = ops._host().rowscale_linear(x, self._wq, self._ws, self._parameters["bias"])
+            r = ops._host().rowscale_linear(x, self._wq, self._ws, self.bias)
             if r is not None:
                 return r
             orig_shape = x.shape
