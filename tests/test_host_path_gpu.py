@@ -170,3 +170,10 @@ def test_dense_linear_bias_need_not_be_a_parameter():
     lin = make()
     parametrize.register_parametrization(lin, "bias", torch.nn.Identity())
     assert torch.equal(lin(x), want)
+
+
+def test_rowscale_linear_takes_matrices_only(ops):
+    wq, ws = ops.per_row_col_quantize(torch.randn(64, 128, device="cuda"))
+    for shape in ((128,), (2, 3, 128)):
+        with pytest.raises(ValueError):
+            ops.rowscale_linear(torch.randn(*shape, device="cuda"), wq, ws)

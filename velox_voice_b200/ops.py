@@ -852,12 +852,12 @@ def nvfp4_linear(x, wq, ws, P=4, C=8, w_bf16=None):
 
 
 def rowscale_linear(x2d: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor, bias: Optional[torch.Tensor] = None):
-    """``x2d [M, K] @ W^T (+ bias)`` on the reference's per-row-scaled FP4 lane, fp32 out, in two
-    launches: quantize the activation rows, then one GEMM whose epilogue applies the row and
-    column scales and adds the bias.  The reference's ``DenseLinear.forward``
+    """``x2d [M, K] @ W^T (+ bias)`` on the reference's per-row-scaled FP4 lane, fp32 out: one
+    launch for few rows, else two -- quantize the activation rows, then one GEMM whose epilogue applies the
+    row and column scales and adds the bias.  The reference's ``DenseLinear.forward``
     (``veloxvoice/models/wenet/torch_conformer.py:251-266``) spends a pad copy, a cast, the
     quantizer, the GEMM, a slice and a bias add on the same result."""
-    r = (_native or _host()).rowscale_linear(x2d, wq, ws, bias)
+    r = (_native or _host()).rowscale_linear(x2d, wq, ws, bias) if x2d.dim() == 2 else None
     if r is not None:
         return r
     a = quantize(x2d, FMT_ROWSCALE, sf=False)
