@@ -177,3 +177,18 @@ def test_rowscale_linear_takes_matrices_only(ops):
     for shape in ((128,), (2, 3, 128)):
         with pytest.raises(ValueError):
             ops.rowscale_linear(torch.randn(*shape, device="cuda"), wq, ws)
+
+
+def test_fold_pack_takes_unaligned_fp32_biases(ops):
+    """fp32 positional biases at any address: a slice of a parameter that does not start on 16 bytes."""
+    torch.manual_seed(4)
+    h, dk, M = 8, 64, 70
+    a = ops.quantize(torch.randn(M, 512, device="cuda"), "mx32")
+    w = ops.quantize(0.05 * torch.randn(3 * h * dk, 512, device="cuda"), "mx32")
+    u, v = torch.randn(h, dk, device="cuda"), torch.randn(h, dk, device="cuda")
+    buf = torch.empty(2 * h * dk + 3, device="cuda")
+    uo, vo = buf[1:1 + h * dk].view(h, dk).copy_(u), buf[3 + h * dk:].view(h, dk).copy_(v)
+    for uu, vv in ((uo, v), (u, vo)):
+        got = ops.bsgemm_qkv_pack(a, w, None, uu, vv, 0.125)
+        want = ops.bsgemm_qkv_pack(a, w, None, u, v, 0.125)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1][..., :dk], want[1][..., :dk]) and torch.equal(got[2], want[2])

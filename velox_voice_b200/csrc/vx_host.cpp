@@ -517,6 +517,8 @@ PyObject* py_qkv_pack_gemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   if (!ok || u.dim() != 2 || u.sizes() != v.sizes() || v.scalar_type() != pt || (pt != at::kFloat && pt != at::kBFloat16) ||
       !u.is_contiguous() || !v.is_contiguous() || u.device() != dev || v.device() != dev)
     Py_RETURN_NONE;
+  // (the kernel reads 16 bytes at a time; the general route's cast to bf16 copies fp32 biases of any address)
+  if (((reinterpret_cast<uintptr_t>(u.data_ptr()) | reinterpret_cast<uintptr_t>(v.data_ptr())) & 15) != 0) Py_RETURN_NONE;
   const int64_t h = u.size(0), dk = u.size(1);
   if (d.N != 3 * h * dk) Py_RETURN_NONE;
   at::Tensor packed;
