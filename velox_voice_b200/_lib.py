@@ -237,9 +237,8 @@ def host():
                 if not _build.host_is_current():
                     try:
                         _build.build_host()
-                    except Exception as e:  # no compiler on this machine: use the shipped module if any
-                        if not os.path.exists(path):
-                            raise RuntimeError(f"{path} is missing and cannot be built: {e}") from e
+                    except Exception as e:  # (one for another torch, Python or C ABI is not loaded: its calls would go through a wrong layout)
+                        raise RuntimeError(f"{path} does not belong to this torch, Python and C ABI and cannot be rebuilt: {e}") from e
                 spec = importlib.util.spec_from_file_location("_vx_host", path)
                 mod = importlib.util.module_from_spec(spec)
                 spec.loader.exec_module(mod)
