@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(TK_WARPS * 32) topk_rows_kernel(const __nv_bfl
         if (8 * c + i >= N) z[i] = -INFINITY;
     }
   };
-  float m = -INFINITY, s = 0.0f;
+  float m = -INFINITY, s = 0.0f, nb = 0.0f;  // nb = -m log2 e; 0 while only masked columns came: they add 2^-inf = 0
 #pragma unroll 4
   for (int c = lane; c < pieces; c += 32) {
     float z[8];
@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(TK_WARPS * 32) topk_rows_kernel(const __nv_bfl
     if (cm > m) {
       s *= ex2_approx((m - cm) * L2E);  // m = -inf: 0
       m = cm;
+      nb = -m * L2E;
     }
-    const float nb = -m * L2E;
 #pragma unroll
     for (int i = 0; i < 8; ++i) s += ex2_approx(fmaf(z[i], L2E, nb));
   }
