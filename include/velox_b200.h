@@ -286,8 +286,8 @@ int vx_ctc_topk_finish(const void* candidates, const int32_t* count, int capacit
 
 /* The same top-k through bf16 logits that exist for a block of rows at a time: per block one launch of the head into
  * `logits` (scratch, bf16 [rows][N rounded up to 8], `rows` = a multiple of 128 or >= M) and one kernel that reads it back
- * while it is in L2 (vx_ctc_topk_rows(N): rows per block for that).  desc: operands, scales and bias of the head (fmt
- * ROWSCALE, MX32 or NV16); its output side is ignored.  Writes logp f32 [M, k] = logit - logsumexp and ids i64 [M, k],
+ * while it is in L2 (vx_ctc_topk_rows(N): rows per block for that).  desc: operands, scales and bias of the head (an
+ * FP4 format); its output side is ignored.  Writes logp f32 [M, k] = logit - logsumexp and ids i64 [M, k],
  * largest first, equal logits by ascending column, for any number of equal logits.  k <= 16. */
 int64_t vx_ctc_topk_rows(int64_t N);
 int vx_ctc_topk(const vx_gemm_desc* desc, int k, void* logits, int64_t rows, float* logp, int64_t* ids, void* stream);

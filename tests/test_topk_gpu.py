@@ -40,3 +40,11 @@ def test_masked_columns(ops, N, masked):
     mask = {"first_piece": col < 8, "lane": (col % 256) < 8, "all_but_16": (col % (N // 16)) != 3, "tail": col >= 256}[masked]
     bias[mask] = float("-inf")
     _check(ops, a, b, bias, 4)
+
+
+def test_per_16_format(ops):
+    torch.manual_seed(6)
+    M, N, K = 130, 5538, 512
+    a = ops.quantize(torch.randn(M, K, device="cuda"), "blk16_a")
+    b = ops.quantize(0.05 * torch.randn(N, K, device="cuda"), "blk16_b")
+    _check(ops, a, b, torch.randn(N, device="cuda"), 5)

@@ -182,7 +182,7 @@ int vx_ctc_topk(const vx_gemm_desc* desc, int k, void* logits, int64_t rows, flo
   const int64_t M = desc->M, N = desc->N, K = desc->K;
   if (M < 0 || N <= 0 || N > 0x7fffffffll) return fail(-1, "bad shape");
   if (k <= 0 || k > 16 || k > N) return fail(-1, "k must be in 1..16 and at most N");
-  if (desc->fmt == VX_FMT_FP8_1X128 || desc->fmt == VX_FMT_BLK16_A) return fail(-1, "vx_ctc_topk runs on ROWSCALE, MX32 and NV16");
+  if (desc->fmt == VX_FMT_FP8_1X128) return fail(-1, "vx_ctc_topk runs on the FP4 formats");
   if (M == 0) return 0;
   if (!logits || !logp || !ids || !aligned16(logits)) return fail(-1, "logits (16-byte aligned), logp and ids must not be NULL");
   if (rows <= 0 || (rows < M && rows % 128 != 0)) return fail(-1, "rows must cover M or be a multiple of 128");
