@@ -48,3 +48,42 @@ def test_per_16_format(ops):
     a = ops.quantize(torch.randn(M, K, device="cuda"), "blk16_a")
     b = ops.quantize(0.05 * torch.randn(N, K, device="cuda"), "blk16_b")
     _check(ops, a, b, torch.randn(N, device="cuda"), 5)
+
+
+@pytest.mark.parametrize("M,k,capacity", [(130, 5, 64), (1, 1, 4), (257, 16, 256), (40, 5, 6)])
+def test_entry_points_without_logits(ops, M, k, capacity):
+    """vx_bsgemm with lse_partials, vx_ctc_topk_threshold, the candidate pass and vx_ctc_topk_finish: the top-k without a
+    logits buffer.  A row whose candidates do not fit its list is reported (ids -1) and counted in `overflow`."""
+    from velox_voice_b200 import _lib
+
+    torch.manual_seed(M)
+    N, K = 5538, 512
+    a = ops.quantize(torch.randn(M, K, device="cuda"), "mx32", natural=False)
+    b = ops.quantize(0.05 * torch.randn(N, K, device="cuda"), "mx32")
+    bias = torch.randn(N, device="cuda")
+    lib = _lib.load()
+    st = torch.cuda.current_stream().cuda_stream
+    parts = torch.empty(int(lib.vx_ctc_lse_parts(N)), M, 2, device="cuda")
+    keys = torch.empty(M, dtype=torch.int64, device="cuda")
+    thr, logp = torch.empty(M, device="cuda"), torch.empty(M, k, device="cuda")
+    cand = torch.empty(M, capacity, dtype=torch.int64, device="cuda")
+    cnt, over = torch.zeros(M, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ids = torch.empty(M, k, dtype=torch.int32, device="cuda")
+    d, keep = ops._gemm_desc(a, b, bias)
+    d.epilogue, d.out_dtype, d.out, d.ldo, d.lse_partials = ops.EPI_BIAS_ARGMAX, _lib.DT_F32, keys.data_ptr(), 1, parts.data_ptr()
+    _lib.check(lib.vx_bsgemm(C.byref(d), st), "vx_bsgemm")
+    _lib.check(lib.vx_ctc_topk_threshold(parts.data_ptr(), N, M, k, thr.data_ptr(), st), "vx_ctc_topk_threshold")
+    d.topk_threshold, d.topk_candidates, d.topk_count, d.topk_capacity = thr.data_ptr(), cand.data_ptr(), cnt.data_ptr(), capacity
+    _lib.check(lib.vx_bsgemm(C.byref(d), st), "vx_bsgemm")
+    _lib.check(lib.vx_ctc_topk_finish(cand.data_ptr(), cnt.data_ptr(), capacity, parts.data_ptr(), N, M, k, ids.data_ptr(),
+                                      logp.data_ptr(), over.data_ptr(), st), "vx_ctc_topk_finish")
+    z = ops.bsgemm(a, b, epilogue=ops.EPI_BIAS, bias=bias, out_dtype=torch.bfloat16)
+    n = (z.float() >= thr[:, None]).sum(1)
+    assert torch.equal(n.int(), cnt) and int(over) == int((n > capacity).any())
+    full = n > capacity
+    assert (ids[full] == -1).all()
+    want_logp, want_ids = ops.bsgemm_topk(a, b, bias, k)
+    assert torch.equal(ids[~full].long(), want_ids[~full])
+    # two summation orders of the fp32 log-sum-exp of one row (see _check)
+    assert torch.allclose(logp[~full], want_logp[~full], rtol=0, atol=4e-5)
+    del keep
