@@ -1,0 +1,103 @@
+"""The stack's native pass against the same layer sequence issued operator by operator, and what a program may change
+between passes."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def by_operators(stack, x, pos=None):
+    """The pass as separate public calls: bf16 logits and the final residual stream."""
+    from velox_voice_b200 import ops
+
+    cfg, fmt, d = stack.cfg, stack.fmt, stack.cfg.d_model
+    am = lambda k: stack.amax.get(k)
+    nat = fmt == ops.FMT_FP8_1X128
+    lnq = lambda k, t: ops.ln_quantize(t, *stack.ln[k], cfg.eps, fmt, amax_t=am(k))
+    q = lambda k, t: ops.quantize(t, fmt, natural=nat, amax_t=am(k))
+    if pos is not None:
+        q("pos", pos)
+    a = None
+    for i in range(cfg.blocks):
+        b = f"b{i}."
+        for ff, ln in (("ffm", "ln_ffm"), ("ff", "ln_ff")):
+            if a is None or ff == "ff":
+                a = lnq(b + ln, x)
+            if stack.fuse_ffn:
+                h = stack.p[b + ff + ".w1"](a, act="swish", out_fmt=fmt, out_amax=am(b + ff + ".h"))
+            else:
+                h = q(b + ff + ".h", stack.p[b + ff + ".w1"](a, act="swish"))
+            x = stack.p[b + ff + ".w2"](h, residual=x, alpha=0.5)
+            if ff == "ffm":
+                qkv = stack.p[b + "qkv"](lnq(b + "ln_mha", x))
+                x = stack.p[b + "lo"](q(b + "ctx", qkv[:, 2 * d:]), residual=x)
+                x = stack.p[b + "pw2"](q(b + "glu", stack.p[b + "pw1"](lnq(b + "ln_conv", x))), residual=x)
+        nxt = f"b{i + 1}.ln_ffm" if i + 1 < cfg.blocks else "after"
+        y = torch.empty_like(x)
+        a = ops.ln2_quantize(x, *stack.ln[b + "ln_final"], *stack.ln[nxt], cfg.eps, fmt, y=y, amax_t=am(nxt))
+        x = y
+    if a is None:
+        a = lnq("after", x)
+    return stack.p["ctc"](a), x
+
+
+def build(fmt="mx32", seed=0, **kw):
+    from velox_voice_b200.stack import ConformerLinearStack, StackConfig, make_weights
+
+    cfg = StackConfig(fmt=fmt, **kw)
+    w = make_weights(cfg, seed=seed)
+    g = torch.Generator().manual_seed(seed)
+    for k in w:
+        if w[k].dim() == 1:
+            w[k] = w[k] + 0.05 * torch.randn(w[k].shape, generator=g)
+    stack = ConformerLinearStack(cfg, w)
+    if fmt == "nv16":
+        x = torch.randn(256, cfg.d_model, generator=g).cuda().bfloat16()
+        stack.calibrate(x, x)
+    return stack
+
+
+@pytest.mark.parametrize("fmt,kw", [("mx32", {}), ("nv16", {}), ("fp8_1x128", {}), ("mx32", dict(fuse_ffn=False)), ("nv16", dict(fuse_ffn=False)),
+                                    ("mx32", dict(d_model=256, heads=4, ffn=1024, conv_pw=512, vocab=101)),
+                                    ("mx32", dict(d_model=384, heads=6, ffn=1536, conv_pw=768, vocab=1000)),
+                                    ("nv16", dict(d_model=768, heads=12, ffn=3072, conv_pw=1536, vocab=1000)),
+                                    ("mx32", dict(blocks=0))])
+def test_native_pass_has_the_bytes_of_the_operators(fmt, kw):
+    kw = {"blocks": 2, **kw}
+    stack = build(fmt, **kw)
+    d = stack.cfg.d_model
+    torch.manual_seed(7)
+    for T in (1, 130, 777, 5000):
+        x = torch.randn(T, d, device="cuda").bfloat16()
+        pos = torch.randn(T, d, device="cuda")
+        want, hidden = by_operators(stack, x.clone())
+        wide = torch.zeros(T, d + 64, device="cuda", dtype=torch.bfloat16)
+        wide[:, 32:32 + d] = x
+        for xx, pp in ((x.clone(), None), (x.clone(), pos.bfloat16()), (x.clone(), pos), (x.clone(), pos.T.contiguous().T),
+                       (wide[:, 32:32 + d], None)):
+            got, h = stack.forward(xx, pp, return_hidden=True)
+            assert torch.equal(got, want) and torch.equal(h, hidden), T
+        buf, src = torch.empty_like(x), x.clone()
+        assert torch.equal(stack.forward(buf, pos, source=src), want) and torch.equal(src, x)
+        assert torch.equal(stack.forward_ids(x.clone(), pos).long(), want.float().argmax(1))
+
+
+@pytest.mark.parametrize("fmt", ["mx32", "fp8_1x128"])
+def test_no_frames(fmt):
+    stack = build(fmt, blocks=2)
+    x = torch.empty(0, 512, device="cuda", dtype=torch.bfloat16)
+    assert stack.forward(x, x.clone()).shape == (0, stack.cfg.vocab) and stack.forward_ids(x).shape == (0,)
+
+
+def test_frames_of_the_fused_launches_are_the_callers_to_choose():
+    from velox_voice_b200 import ops
+
+    x = torch.randn(5000, 512, device="cuda").bfloat16()
+    count = {}
+    for least in (None, 1, 5000, 5001, 1 << 30):
+        stack = build(blocks=1, **({} if least is None else {"fuse_ln_min_frames": least}))
+        ops.reset_launch_count()
+        stack.forward_ids(x.clone())
+        count[least] = ops.launch_count()
+    assert count[1] == count[5000] == count[None] < count[5001] == count[1 << 30]

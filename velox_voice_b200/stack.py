@@ -42,11 +42,12 @@ from .linear import PackedLinear, glu_tile
 from .ops import FMT_FP8_1X128, FMT_MX32, FMT_NV16
 
 
-# Frames from which the residual GEMMs run the LayerNorm + quantizer behind them (two-CTA clusters, a row block each).  Up
-# to 37 row blocks the separate residual GEMM takes a single round over 148 SMs (four column blocks each) and is faster
-# (12 blocks, 3,750 frames: 955 vs 996 us); beyond, its second round costs more than the clusters' work (5,000 frames:
-# 1,228 vs 1,155 us; 9,472: 1,550 vs 1,392; 40,000: 4,267 vs 4,102).
-FUSE_LN_FRAMES = 37 * 128 + 1
+def fuse_ln_frames(sms: int, d_model: int) -> int:
+    """Frames from which the residual GEMMs run the LayerNorm + quantizer behind them (two-CTA clusters, a row block each) unless
+    the caller chooses.  As long as the separate residual GEMM takes a single round -- a tile of 128 x 128 per SM, 37 row blocks
+    of four tiles on 148 SMs -- it is faster (12 blocks, 3,750 frames: 955 vs 996 us); beyond, its second round costs more than
+    the clusters' work (5,000 frames: 1,228 vs 1,155 us; 9,472: 1,550 vs 1,392; 40,000: 4,267 vs 4,102)."""
+    return sms // max(d_model // 128, 1) * 128 + 1
 
 
 @dataclass
@@ -61,8 +62,8 @@ class StackConfig:
     eps: float = 1e-5
     fuse_ffn: bool = True  # keep the FFN intermediate in FP4 (re-quantized in the up-GEMM epilogue)
     fuse_ln: bool = True   # MX32, d_model 512: the residual GEMMs also run the LayerNorm + quantizer behind them
-    # ... at the latest from this many frames on (a smaller value moves the line down; see FUSE_LN_FRAMES)
-    fuse_ln_min_frames: int = 16384
+    # ... from this many frames on (None: where they are faster, see fuse_ln_frames)
+    fuse_ln_min_frames: Optional[int] = None
 
     def flops_per_frame(self) -> int:
         """Algorithmic FLOPs of the linears per encoder frame (2 * N * K each)."""
@@ -113,8 +114,11 @@ class ConformerLinearStack:
         # VELOX_B200_FUSE_LN_MIN_FRAMES overrides their frame threshold, for A/B timing)
         self.fuse_ln = (bool(cfg.fuse_ln) and os.environ.get("VELOX_B200_FUSE_LN", "1") != "0"
                         and ops.residual_ln_supported(self.fmt, cfg.d_model, cfg.d_model))
-        self.fuse_ln_min_frames = int(os.environ.get("VELOX_B200_FUSE_LN_MIN_FRAMES", min(cfg.fuse_ln_min_frames, FUSE_LN_FRAMES)))
         dev = self.device
+        least = os.environ.get("VELOX_B200_FUSE_LN_MIN_FRAMES", cfg.fuse_ln_min_frames)
+        if least is None:
+            least = fuse_ln_frames(torch.cuda.get_device_properties(dev).multi_processor_count, cfg.d_model)
+        self.fuse_ln_min_frames = int(least)
         self.p: Dict[str, PackedLinear] = {}
         self.ln: Dict[str, Tuple[torch.Tensor, torch.Tensor]] = {}
 
