@@ -192,3 +192,44 @@ def test_fold_pack_takes_unaligned_fp32_biases(ops):
         got = ops.bsgemm_qkv_pack(a, w, None, uu, vv, 0.125)
         want = ops.bsgemm_qkv_pack(a, w, None, u, v, 0.125)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1][..., :dk], want[1][..., :dk]) and torch.equal(got[2], want[2])
+
+
+def test_host_calls_release_the_interpreter():
+    """A forward pass that blocks in its launches (the stream's queue is full) lets other Python threads run."""
+    import threading
+    import time
+
+    from velox_voice_b200.stack import ConformerLinearStack, StackConfig, make_weights
+
+    cfg = StackConfig(blocks=2)
+    stack = ConformerLinearStack(cfg, make_weights(cfg))
+    x, pos = torch.randn(128, 512, device="cuda").bfloat16(), torch.randn(128, 512, device="cuda").bfloat16()
+    stack.forward_ids(x.clone(), pos)
+    torch.cuda.synchronize()
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.002)
+
+    t = threading.Thread(target=tick)
+    t.start()
+    try:
+        torch.cuda._sleep(1_500_000_000)  # about 0.8 s of an occupied stream
+        t0 = time.perf_counter()
+        while time.perf_counter() - t0 < 0.25:  # fill the queue until a call blocks
+            t1 = time.perf_counter()
+            for _ in range(20):
+                stack.forward_ids(x, pos)
+            if time.perf_counter() - t1 > 0.2:
+                break
+    finally:
+        end = time.perf_counter()
+        stop.set()
+        t.join()
+    torch.cuda.synchronize()
+    seen = [v for v in ticks if t0 <= v <= end]
+    assert end - t0 > 0.2, "the queue never filled"
+    gaps = [b - a for a, b in zip([t0] + seen, seen + [end])]
+    assert max(gaps) < 0.1, f"no other thread ran for {max(gaps):.3f} s of {end - t0:.3f} s"

@@ -43,14 +43,24 @@ std::atomic<int64_t> g_launches{0};
 
 void count(int64_t n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-struct PyFail {};  // a Python error is set
+struct PyFail {};                           // a Python error is set
+struct CallFail { int rc; const char* what; };  // a C-ABI call failed on this thread
 
 void check(int rc, const char* what) {
-  if (rc == 0) return;
-  if (rc < 0) PyErr_Format(g_error, "%s: argument error: %s", what, g.vx_last_error());
-  else PyErr_Format(g_error, "%s: CUDA error %d: %s", what, rc, g.vx_last_error());
-  throw PyFail{};
+  if (rc != 0) throw CallFail{rc, what};
 }
+void set_error(const CallFail& f) {
+  if (f.rc < 0) PyErr_Format(g_error, "%s: argument error: %s", f.what, g.vx_last_error());
+  else PyErr_Format(g_error, "%s: CUDA error %d: %s", f.what, f.rc, g.vx_last_error());
+}
+
+// Allocations and launches run without the interpreter lock: a launch blocks while the stream's queue is full, and an
+// allocation may wait for the device.  No Python object is touched in its scope; tensors that come out of Python objects
+// other threads may change (the fields of a Quantized, a plan's layers) are held by value.
+struct NoGil {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
 
 // ---------------------------------------------------------------- small helpers
 at::Tensor empty(at::IntArrayRef size, at::ScalarType dt, const at::Device& dev) {
@@ -75,6 +85,7 @@ bool vector_ok(const at::Tensor& t, int64_t n, const at::Device& dev) {
   return t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() >= n && t.device() == dev;
 }
 // optional fp32 vector argument: its pointer, or sets `ok` to false when the general route has to look at it
+const float* f32_ptr(const at::Tensor& t) { return t.defined() ? static_cast<const float*>(t.data_ptr()) : nullptr; }
 const float* vector_arg(PyObject* o, int64_t n, const at::Device& dev, bool& ok) {
   if (o == Py_None) return nullptr;
   if (!is_cuda_tensor(o)) { ok = false; return nullptr; }
@@ -119,9 +130,7 @@ PyObject* make_quantized(int fmt, int64_t M, int64_t K, const Outputs& o, PyObje
 struct Operand {
   int fmt = -1;
   int64_t rows = 0, k = 0;
-  const at::Tensor* codes = nullptr;
-  const void* scales = nullptr;
-  const float* amax = nullptr;
+  at::Tensor codes, scales, amax;
 };
 // false: not an ordinary operand (the general route decides what it is)
 bool read_operand(PyObject* o, Operand& r) {
@@ -129,7 +138,7 @@ bool read_operand(PyObject* o, Operand& r) {
   auto get = [&](PyObject* name) {
     PyObject* v = PyObject_GetAttr(o, name);
     if (!v) throw PyFail{};
-    Py_DECREF(v);  // the instance keeps it alive for the duration of the call
+    Py_DECREF(v);  // (the instance keeps it alive until the tensor in it has been taken)
     return v;
   };
   r.fmt = static_cast<int>(PyLong_AsLong(get(s_fmt)));
@@ -139,28 +148,28 @@ bool read_operand(PyObject* o, Operand& r) {
   PyObject* c = get(s_codes);
   PyObject* s = get(has_sf(r.fmt) ? s_sf : s_scales);
   if (!is_cuda_tensor(c) || !is_cuda_tensor(s)) return false;
-  r.codes = &THPVariable_Unpack(c);
-  r.scales = THPVariable_Unpack(s).data_ptr();
-  if (r.codes->dim() != 2) return false;
+  r.codes = THPVariable_Unpack(c);
+  r.scales = THPVariable_Unpack(s);
+  if (r.codes.dim() != 2) return false;
   if (r.fmt == VX_FMT_NV16) {
     PyObject* a = get(s_amax);
     if (!is_cuda_tensor(a)) return false;
-    r.amax = static_cast<const float*>(THPVariable_Unpack(a).data_ptr());
+    r.amax = THPVariable_Unpack(a);
   }
   return true;
 }
 bool operands(PyObject* pa, PyObject* pb, Operand& a, Operand& b, vx_gemm_desc& d) {
   if (!read_operand(pa, a) || !read_operand(pb, b)) return false;
   if (a.fmt == VX_FMT_BLK16_A ? b.fmt != VX_FMT_BLK16_B : a.fmt != b.fmt) return false;
-  if (a.k != b.k || a.codes->device() != b.codes->device()) return false;
+  if (a.k != b.k || a.codes.device() != b.codes.device()) return false;
   d = vx_gemm_desc{};
   d.struct_size = sizeof(vx_gemm_desc);
   d.fmt = a.fmt;
   d.M = a.rows; d.N = b.rows; d.K = a.k;
-  d.a_codes = a.codes->data_ptr(); d.lda = a.codes->stride(0);
-  d.b_codes = b.codes->data_ptr(); d.ldb = b.codes->stride(0);
-  d.a_scales = a.scales; d.b_scales = b.scales;
-  d.a_amax = a.amax; d.b_amax = b.amax;
+  d.a_codes = a.codes.data_ptr(); d.lda = a.codes.stride(0);
+  d.b_codes = b.codes.data_ptr(); d.ldb = b.codes.stride(0);
+  d.a_scales = a.scales.data_ptr(); d.b_scales = b.scales.data_ptr();
+  d.a_amax = f32_ptr(a.amax); d.b_amax = f32_ptr(b.amax);
   return true;
 }
 
@@ -184,7 +193,12 @@ double as_double(PyObject* o) {
   HANDLE_TH_ERRORS                                                  \
   try {
 #define VX_END                                                      \
-  } catch (const PyFail&) { return nullptr; }                       \
+  } catch (const PyFail&) {                                         \
+    return nullptr;                                                 \
+  } catch (const CallFail& f) {                                     \
+    set_error(f);                                                   \
+    return nullptr;                                                 \
+  }                                                                 \
   END_HANDLE_TH_ERRORS
 #define VX_ARGS(n)                                                                   \
   if (nargs != (n)) {                                                                \
@@ -210,29 +224,23 @@ PyObject* py_quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (dt < 0 || !rows2d(x)) Py_RETURN_NONE;
   const bool natural = as_bool(a[2]) || fmt == VX_FMT_ROWSCALE || fmt == VX_FMT_FP8_1X128;
   const int64_t M = x.size(0), K = x.size(1);
-  const float* am = nullptr;
-  PyObject* amax = a[4];
-  PyObject* made = nullptr;
-  if (fmt == VX_FMT_NV16) {
-    if (amax == Py_None) {
-      const at::Tensor t = tensor_amax(x, dt);
-      am = static_cast<const float*>(t.data_ptr());
-      amax = made = wrap(t);
-    } else if (is_cuda_tensor(amax)) {
-      am = static_cast<const float*>(THPVariable_Unpack(amax).data_ptr());
-    } else {
-      Py_RETURN_NONE;
-    }
-  } else if (amax != Py_None) {
-    Py_RETURN_NONE;
+  const bool sf = as_bool(a[3]), measure = fmt == VX_FMT_NV16 && a[4] == Py_None;
+  at::Tensor amax;
+  if (fmt == VX_FMT_NV16 ? !measure && !is_cuda_tensor(a[4]) : a[4] != Py_None) Py_RETURN_NONE;
+  if (fmt == VX_FMT_NV16 && !measure) amax = THPVariable_Unpack(a[4]);
+  Outputs o;
+  {
+    NoGil nogil;
+    if (measure) amax = tensor_amax(x, dt);
+    o = alloc_outputs(fmt, M, K, x.device(), natural, sf);
+    check(g.vx_quantize_pack(x.data_ptr(), dt, M, K, x.stride(0), fmt, ptr(o.codes), o.codes.stride(0), ptr(o.scales), ptr(o.sf),
+                             f32_ptr(amax), stream()),
+          "vx_quantize_pack");
+    count();
   }
-  const Outputs o = alloc_outputs(fmt, M, K, x.device(), natural, as_bool(a[3]));
-  const int rc = g.vx_quantize_pack(x.data_ptr(), dt, M, K, x.stride(0), fmt, ptr(o.codes), o.codes.stride(0), ptr(o.scales), ptr(o.sf),
-                                    am, stream());
-  if (rc) Py_XDECREF(made);
-  check(rc, "vx_quantize_pack");
-  count();
-  PyObject* r = make_quantized(fmt, M, K, o, amax);
+  if (!measure) return make_quantized(fmt, M, K, o, a[4]);
+  PyObject* made = wrap(amax);
+  PyObject* r = make_quantized(fmt, M, K, o, made);
   Py_XDECREF(made);
   return r;
   VX_END
@@ -259,11 +267,17 @@ PyObject* py_ln_quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     Py_RETURN_NONE;
   }
   const bool natural = as_bool(a[5]) || fmt == VX_FMT_ROWSCALE || fmt == VX_FMT_FP8_1X128;
-  const Outputs o = alloc_outputs(fmt, M, K, x.device(), natural, as_bool(a[6]));
-  check(g.vx_ln_quantize_pack(x.data_ptr(), dt, M, K, x.stride(0), gamma, beta, static_cast<float>(as_double(a[3])), fmt, ptr(o.codes),
-                              o.codes.stride(0), ptr(o.scales), ptr(o.sf), am, nullptr, 0, K, stream()),
-        "vx_ln_quantize_pack");
-  count();
+  const bool sf = as_bool(a[6]);
+  const float eps = static_cast<float>(as_double(a[3]));
+  Outputs o;
+  {
+    NoGil nogil;
+    o = alloc_outputs(fmt, M, K, x.device(), natural, sf);
+    check(g.vx_ln_quantize_pack(x.data_ptr(), dt, M, K, x.stride(0), gamma, beta, eps, fmt, ptr(o.codes), o.codes.stride(0), ptr(o.scales),
+                                ptr(o.sf), am, nullptr, 0, K, stream()),
+          "vx_ln_quantize_pack");
+    count();
+  }
   return make_quantized(fmt, M, K, o, a[7]);
   VX_END
 }
@@ -276,6 +290,11 @@ at::Tensor new_out(int64_t M, int64_t n, at::ScalarType dt, const at::Device& de
   return empty({M, n}, dt, dev);
 }
 
+void launch(const vx_gemm_desc& d) {
+  check(g.vx_bsgemm(&d, stream()), "vx_bsgemm");
+  count();
+}
+
 // bsgemm(a, b, epilogue, bias, residual, alpha, out_dtype, out, out_fmt, out_amax, out_natural, flags)
 //   -> Tensor | Quantized | None
 PyObject* py_bsgemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
@@ -284,7 +303,7 @@ PyObject* py_bsgemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   Operand a, b;
   vx_gemm_desc d;
   if (!operands(p[0], p[1], a, b, d)) Py_RETURN_NONE;
-  const at::Device dev = a.codes->device();
+  const at::Device dev = a.codes.device();
   bool ok = true;
   d.bias = vector_arg(p[3], d.N, dev, ok);
   if (!ok) Py_RETURN_NONE;
@@ -306,11 +325,15 @@ PyObject* py_bsgemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
     } else if (ofmt != VX_FMT_MX32 || p[9] != Py_None) {
       Py_RETURN_NONE;
     }
-    const Outputs o = alloc_outputs(ofmt, d.M, n_out, dev, as_bool(p[10]), true);
-    d.out_dtype = VX_FP4; d.out = ptr(o.codes); d.ldo = o.codes.stride(0);
-    d.out_fmt = ofmt; d.out_scales_sf = ptr(o.sf); d.out_scales = ptr(o.scales);
-    check(g.vx_bsgemm(&d, stream()), "vx_bsgemm");
-    count();
+    const bool natural = as_bool(p[10]);
+    Outputs o;
+    {
+      NoGil nogil;
+      o = alloc_outputs(ofmt, d.M, n_out, dev, natural, true);
+      d.out_dtype = VX_FP4; d.out = ptr(o.codes); d.ldo = o.codes.stride(0);
+      d.out_fmt = ofmt; d.out_scales_sf = ptr(o.sf); d.out_scales = ptr(o.scales);
+      launch(d);
+    }
     return make_quantized(ofmt, d.M, n_out, o, p[9]);
   }
   if (p[7] != Py_None) {
@@ -318,17 +341,22 @@ PyObject* py_bsgemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
     const at::Tensor& o = THPVariable_Unpack(p[7]);
     if (!rows2d(o) || o.size(0) != d.M || o.size(1) != n_out || o.device() != dev || dtype_code(o) < 0) Py_RETURN_NONE;
     d.out_dtype = dtype_code(o); d.out = o.data_ptr(); d.ldo = o.stride(0);
-    check(g.vx_bsgemm(&d, stream()), "vx_bsgemm");
-    count();
+    {
+      NoGil nogil;
+      launch(d);
+    }
     return Py_NewRef(p[7]);
   }
   if (!THPDtype_Check(p[6])) Py_RETURN_NONE;
   const at::ScalarType odt = reinterpret_cast<THPDtype*>(p[6])->scalar_type;
   if (odt != at::kFloat && odt != at::kBFloat16) Py_RETURN_NONE;
-  const at::Tensor o = new_out(d.M, n_out, odt, dev);
-  d.out_dtype = odt == at::kFloat ? VX_F32 : VX_BF16; d.out = o.data_ptr(); d.ldo = o.stride(0);
-  check(g.vx_bsgemm(&d, stream()), "vx_bsgemm");
-  count();
+  at::Tensor o;
+  {
+    NoGil nogil;
+    o = new_out(d.M, n_out, odt, dev);
+    d.out_dtype = odt == at::kFloat ? VX_F32 : VX_BF16; d.out = o.data_ptr(); d.ldo = o.stride(0);
+    launch(d);
+  }
   return wrap(o);
   VX_END
 }
@@ -340,7 +368,7 @@ PyObject* py_residual_ln(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   Operand a, b;
   vx_gemm_desc d;
   if (!operands(p[0], p[1], a, b, d)) Py_RETURN_NONE;
-  const at::Device dev = a.codes->device();
+  const at::Device dev = a.codes.device();
   bool ok = true;
   d.bias = vector_arg(p[2], d.N, dev, ok);
   const float* gamma = vector_arg(p[4], d.N, dev, ok);
@@ -351,7 +379,10 @@ PyObject* py_residual_ln(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   const at::Tensor& r = THPVariable_Unpack(p[3]);
   if (!rows2d(r) || r.size(0) != d.M || r.size(1) != d.N || r.device() != dev || dtype_code(r) < 0) Py_RETURN_NONE;
   at::Tensor out;
-  if (p[8] == Py_None) out = empty({d.M, d.N}, at::kBFloat16, dev);
+  if (p[8] == Py_None) {
+    NoGil nogil;
+    out = empty({d.M, d.N}, at::kBFloat16, dev);
+  }
   else if (is_cuda_tensor(p[8])) out = THPVariable_Unpack(p[8]);
   else Py_RETURN_NONE;
   if (!rows2d(out) || out.size(0) != d.M || out.size(1) != d.N || out.device() != dev || dtype_code(out) < 0) Py_RETURN_NONE;
@@ -361,13 +392,17 @@ PyObject* py_residual_ln(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   d.out_dtype = dtype_code(out); d.out = out.data_ptr(); d.ldo = out.stride(0);
   d.flags = static_cast<int>(as_long(p[11]));
   const float eps = static_cast<float>(as_double(p[6]));
-  const Outputs o = alloc_outputs(VX_FMT_MX32, d.M, d.N, dev, false, true);
-  if (!gamma2)
-    check(g.vx_bsgemm_residual_ln(&d, gamma, beta, eps, ptr(o.codes), o.codes.stride(0), ptr(o.sf), stream()), "vx_bsgemm_residual_ln");
-  else
-    check(g.vx_bsgemm_residual_ln2(&d, gamma, beta, gamma2, beta2, eps, ptr(o.codes), o.codes.stride(0), ptr(o.sf), stream()),
-          "vx_bsgemm_residual_ln2");
-  count();
+  Outputs o;
+  {
+    NoGil nogil;
+    o = alloc_outputs(VX_FMT_MX32, d.M, d.N, dev, false, true);
+    if (!gamma2)
+      check(g.vx_bsgemm_residual_ln(&d, gamma, beta, eps, ptr(o.codes), o.codes.stride(0), ptr(o.sf), stream()), "vx_bsgemm_residual_ln");
+    else
+      check(g.vx_bsgemm_residual_ln2(&d, gamma, beta, gamma2, beta2, eps, ptr(o.codes), o.codes.stride(0), ptr(o.sf), stream()),
+            "vx_bsgemm_residual_ln2");
+    count();
+  }
   PyObject* q = make_quantized(VX_FMT_MX32, d.M, d.N, o, Py_None);
   if (!q) return nullptr;
   PyObject* pair = PyTuple_New(2);
@@ -396,16 +431,20 @@ PyObject* py_rowscale_linear(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   bool ok = true;
   const float* bias = vector_arg(p[3], N, dev, ok);
   if (!ok) Py_RETURN_NONE;
-  const int64_t need = g.vx_rowscale_linear_scratch(M, N, K);
-  at::Tensor scratch;
-  if (need) scratch = empty({need}, at::kByte, dev);
-  c10::SmallVector<int64_t, 8> shape(x.sizes().begin(), x.sizes().end());
-  shape.back() = N;
-  const at::Tensor out = empty(shape, at::kFloat, dev);
-  check(g.vx_rowscale_linear(x.data_ptr(), dt, M, K, K, wq.data_ptr(), wq.stride(0), ws.data_ptr(), N, bias, ptr(scratch),
-                             static_cast<float*>(out.data_ptr()), N, stream()),
-        "vx_rowscale_linear");
-  count(need ? 2 : 1);
+  at::Tensor out;
+  {
+    NoGil nogil;
+    const int64_t need = g.vx_rowscale_linear_scratch(M, N, K);
+    at::Tensor scratch;
+    if (need) scratch = empty({need}, at::kByte, dev);
+    c10::SmallVector<int64_t, 8> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = N;
+    out = empty(shape, at::kFloat, dev);
+    check(g.vx_rowscale_linear(x.data_ptr(), dt, M, K, K, wq.data_ptr(), wq.stride(0), ws.data_ptr(), N, bias, ptr(scratch),
+                               static_cast<float*>(out.data_ptr()), N, stream()),
+          "vx_rowscale_linear");
+    count(need ? 2 : 1);
+  }
   return wrap(out);
   VX_END
 }
@@ -426,24 +465,27 @@ PyObject* py_blkscale_gemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   for (const at::Tensor* s : {&sa, &sb})
     if (s->scalar_type() != at::kByte || !s->is_contiguous() || s->device() != dev) Py_RETURN_NONE;
   if (sa.numel() < K / 16 * (M / 2) || sb.numel() < K / 16 * N) Py_RETURN_NONE;
-  const int64_t na = sf_bytes(VX_FMT_BLK16_A, M, K), nb = sf_bytes(VX_FMT_BLK16_B, N, K);
-  const at::Tensor scratch = empty({na + nb}, at::kByte, dev);
-  uint8_t* const sf = static_cast<uint8_t*>(scratch.data_ptr());
-  const at::Tensor out = empty({M, N}, at::kFloat, dev);
-  void* const st = stream();
-  check(g.vx_sf_from_natural_pair(VX_FMT_BLK16_A, sa.data_ptr(), M, sf, VX_FMT_BLK16_B, sb.data_ptr(), N, sf + na, K, st),
-        "vx_sf_from_natural_pair");
-  vx_gemm_desc d{};
-  d.struct_size = sizeof(d);
-  d.fmt = VX_FMT_BLK16_A;
-  d.M = M; d.N = N; d.K = K;
-  d.a_codes = pa.data_ptr(); d.lda = pa.stride(0);
-  d.b_codes = pb.data_ptr(); d.ldb = pb.stride(0);
-  d.a_scales = sf; d.b_scales = sf + na;
-  d.epilogue = VX_EPI_NONE;
-  d.out_dtype = VX_F32; d.out = out.data_ptr(); d.ldo = N;
-  check(g.vx_bsgemm(&d, st), "vx_bsgemm");
-  count(2);
+  at::Tensor out;
+  {
+    NoGil nogil;
+    const int64_t na = sf_bytes(VX_FMT_BLK16_A, M, K), nb = sf_bytes(VX_FMT_BLK16_B, N, K);
+    const at::Tensor scratch = empty({na + nb}, at::kByte, dev);
+    uint8_t* const sf = static_cast<uint8_t*>(scratch.data_ptr());
+    out = empty({M, N}, at::kFloat, dev);
+    check(g.vx_sf_from_natural_pair(VX_FMT_BLK16_A, sa.data_ptr(), M, sf, VX_FMT_BLK16_B, sb.data_ptr(), N, sf + na, K, stream()),
+          "vx_sf_from_natural_pair");
+    count();
+    vx_gemm_desc d{};
+    d.struct_size = sizeof(d);
+    d.fmt = VX_FMT_BLK16_A;
+    d.M = M; d.N = N; d.K = K;
+    d.a_codes = pa.data_ptr(); d.lda = pa.stride(0);
+    d.b_codes = pb.data_ptr(); d.ldb = pb.stride(0);
+    d.a_scales = sf; d.b_scales = sf + na;
+    d.epilogue = VX_EPI_NONE;
+    d.out_dtype = VX_F32; d.out = out.data_ptr(); d.ldo = N;
+    launch(d);
+  }
   return wrap(out);
   VX_END
 }
@@ -457,18 +499,23 @@ PyObject* py_topk(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   Operand a, b;
   vx_gemm_desc d;
   if (!operands(p[0], p[1], a, b, d) || a.fmt == VX_FMT_FP8_1X128) Py_RETURN_NONE;
-  const at::Device dev = a.codes->device();
+  const at::Device dev = a.codes.device();
   bool ok = true;
   d.bias = vector_arg(p[2], d.N, dev, ok);
   const long k = as_long(p[3]);
   if (!ok || k < 1 || k > 16 || (d.N + 255) / 256 * 4 < k || d.M == 0) Py_RETURN_NONE;
-  const at::Tensor logp = empty({d.M, k}, at::kFloat, dev), ids = empty({d.M, k}, at::kLong, dev);
-  const int64_t rows = g.vx_ctc_topk_rows(d.N), block = rows < d.M ? rows : d.M;
-  const at::Tensor scratch = at::Tensor(empty({block, (d.N + 7) / 8 * 8}, at::kBFloat16, dev));
-  check(g.vx_ctc_topk(&d, static_cast<int>(k), scratch.data_ptr(), block, static_cast<float*>(logp.data_ptr()),
-                      static_cast<int64_t*>(ids.data_ptr()), stream()),
-        "vx_ctc_topk");
-  count(2 * ((d.M + block - 1) / block));
+  at::Tensor logp, ids;
+  {
+    NoGil nogil;
+    logp = empty({d.M, k}, at::kFloat, dev);
+    ids = empty({d.M, k}, at::kLong, dev);
+    const int64_t rows = g.vx_ctc_topk_rows(d.N), block = rows < d.M ? rows : d.M;
+    const at::Tensor scratch = empty({block, (d.N + 7) / 8 * 8}, at::kBFloat16, dev);
+    check(g.vx_ctc_topk(&d, static_cast<int>(k), scratch.data_ptr(), block, static_cast<float*>(logp.data_ptr()),
+                        static_cast<int64_t*>(ids.data_ptr()), stream()),
+          "vx_ctc_topk");
+    count(2 * ((d.M + block - 1) / block));
+  }
   PyObject* pair = PyTuple_New(2);
   if (!pair) return nullptr;
   PyTuple_SET_ITEM(pair, 0, wrap(logp));
@@ -493,11 +540,16 @@ PyObject* py_relpos_attention(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   if (k->sizes() != q->sizes() || v->sizes() != q->sizes() || q->size(2) != 128 || k->device() != q->device() || v->device() != q->device())
     Py_RETURN_NONE;
   const int64_t h = q->size(0), T = q->size(1);
-  const at::Tensor out = empty({T, h * 64}, at::kBFloat16, q->device());
-  check(g.vx_relpos_attention(q->data_ptr(), k->data_ptr(), v->data_ptr(), T, static_cast<int>(h), 64,
-                              p[3] == Py_None ? 0 : as_long(p[3]), out.data_ptr(), h * 64, stream()),
-        "vx_relpos_attention");
-  count();
+  const int64_t kv_len = p[3] == Py_None ? 0 : as_long(p[3]);
+  at::Tensor out;
+  {
+    NoGil nogil;
+    out = empty({T, h * 64}, at::kBFloat16, q->device());
+    check(g.vx_relpos_attention(q->data_ptr(), k->data_ptr(), v->data_ptr(), T, static_cast<int>(h), 64, kv_len, out.data_ptr(), h * 64,
+                                stream()),
+          "vx_relpos_attention");
+    count();
+  }
   return wrap(out);
   VX_END
 }
@@ -509,7 +561,7 @@ PyObject* py_qkv_pack_gemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   Operand a, b;
   vx_gemm_desc d;
   if (!operands(p[0], p[1], a, b, d) || a.fmt == VX_FMT_ROWSCALE || !is_cuda_tensor(p[3]) || !is_cuda_tensor(p[4])) Py_RETURN_NONE;
-  const at::Device dev = a.codes->device();
+  const at::Device dev = a.codes.device();
   bool ok = true;
   d.bias = vector_arg(p[2], d.N, dev, ok);
   const at::Tensor &u = THPVariable_Unpack(p[3]), &v = THPVariable_Unpack(p[4]);
@@ -522,7 +574,10 @@ PyObject* py_qkv_pack_gemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   const int64_t h = u.size(0), dk = u.size(1);
   if (d.N != 3 * h * dk) Py_RETURN_NONE;
   at::Tensor packed;
-  if (p[6] == Py_None) packed = empty({3, h, d.M, 2 * dk}, at::kBFloat16, dev);
+  if (p[6] == Py_None) {
+    NoGil nogil;
+    packed = empty({3, h, d.M, 2 * dk}, at::kBFloat16, dev);
+  }
   else if (is_cuda_tensor(p[6])) packed = THPVariable_Unpack(p[6]);
   else Py_RETURN_NONE;
   if (packed.scalar_type() != at::kBFloat16 || !packed.is_contiguous() || packed.device() != dev ||
@@ -533,8 +588,10 @@ PyObject* py_qkv_pack_gemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   d.heads = static_cast<int>(h); d.head_dim = static_cast<int>(dk);
   d.pos_u = u.data_ptr(); d.pos_v = v.data_ptr(); d.qk_scale = static_cast<float>(as_double(p[5]));
   d.flags = pt == at::kFloat ? VX_GEMM_POS_F32 : 0;
-  check(g.vx_bsgemm(&d, stream()), "vx_bsgemm");
-  count();
+  {
+    NoGil nogil;
+    launch(d);
+  }
   return p[6] == Py_None ? wrap(packed) : Py_NewRef(p[6]);
   VX_END
 }
@@ -547,7 +604,7 @@ PyObject* py_heads_gemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   vx_gemm_desc d;
   const at::Tensor* out;
   if (!operands(p[0], p[1], a, b, d) || !bf16_cube(p[3], &out)) Py_RETURN_NONE;
-  const at::Device dev = a.codes->device();
+  const at::Device dev = a.codes.device();
   bool ok = true;
   d.bias = vector_arg(p[2], d.N, dev, ok);
   const int64_t h = out->size(0);
@@ -556,8 +613,10 @@ PyObject* py_heads_gemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   d.out_dtype = VX_BF16; d.out = out->data_ptr(); d.ldo = out->size(2);
   d.heads = static_cast<int>(h); d.head_dim = static_cast<int>(d.N / h); d.head_col_off = static_cast<int>(as_long(p[4]));
   d.flags = VX_GEMM_OUT_HEADS;
-  check(g.vx_bsgemm(&d, stream()), "vx_bsgemm");
-  count();
+  {
+    NoGil nogil;
+    launch(d);
+  }
   return Py_NewRef(p[3]);
   VX_END
 }
@@ -578,19 +637,23 @@ PyObject* py_power_mel_log(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   const float* mean = vector_arg(p[2], M, dev, ok);
   const float* istd = vector_arg(p[3], M, dev, ok);
   if (!ok || (mean == nullptr) != (istd == nullptr) || !g.vx_power_mel_log_supported(F, M)) Py_RETURN_NONE;
-  const at::Tensor out = empty({T, M}, at::kFloat, dev);
-  check(g.vx_power_mel_log(spec.data_ptr(), T, F, F, static_cast<const float*>(mel.data_ptr()), M, mel.stride(0), mean, istd,
-                           static_cast<float*>(out.data_ptr()), M, stream()),
-        "vx_power_mel_log");
-  count();
+  at::Tensor out;
+  {
+    NoGil nogil;
+    out = empty({T, M}, at::kFloat, dev);
+    check(g.vx_power_mel_log(spec.data_ptr(), T, F, F, static_cast<const float*>(mel.data_ptr()), M, mel.stride(0), mean, istd,
+                             static_cast<float*>(out.data_ptr()), M, stream()),
+          "vx_power_mel_log");
+    count();
+  }
   return wrap(out);
   VX_END
 }
 
 // ---------------------------------------------------------------- the encoder's linear stack
 // A plan holds what one forward pass needs besides its frames: the packed weights, LayerNorm parameters and calibrated
-// maxima as plain pointers (and references to the Python objects that own them).  forward() walks the layer sequence that
-// stack.py documents and issues every launch of the pass; its intermediate tensors live in one workspace block.
+// maxima as plain pointers, and the tensors they point into.  forward() walks the layer sequence that stack.py documents and
+// issues every launch of the pass; its intermediate tensors live in one workspace block.
 struct Lin {
   const void* codes; int64_t ld; const void* scales; const float* amax; const float* bias; int64_t N, K;
 };
@@ -609,7 +672,11 @@ struct Plan {
   Lin lp_all{};                  // the positional projections of all blocks as one weight (codes nullptr: none)
   std::vector<Norm> norm;        // [block][N_COUNT], then after_norm
   std::vector<const float*> am;  // [block][A_COUNT], then after_norm, then the positions (NV16)
-  PyObject* owners = nullptr;
+  std::vector<at::Tensor> keep;  // everything the pointers above point into
+  Lin layer(const Operand& w, const float* bias) {
+    for (const at::Tensor& t : {w.codes, w.scales, w.amax}) keep.push_back(t);
+    return {w.codes.data_ptr(), w.codes.stride(0), w.scales.data_ptr(), f32_ptr(w.amax), bias, w.rows, w.k};
+  }
   const float* amax(size_t i) const { return am.empty() ? nullptr : am[i]; }
 };
 
@@ -709,8 +776,6 @@ struct Pass {
 
 void plan_free(PyObject* cap) {
   Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(cap, "velox_stack_plan"));
-  if (!p) return;
-  Py_XDECREF(p->owners);
   delete p;
 }
 
@@ -737,6 +802,7 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (!is_cuda_tensor(o)) bad("stack_plan: CUDA tensors expected");
     const at::Tensor& t = THPVariable_Unpack(o);
     if (t.scalar_type() != at::kFloat || !t.is_contiguous()) bad("stack_plan: contiguous float32 vectors expected");
+    plan->keep.push_back(t);
     return static_cast<const float*>(t.data_ptr());
   };
   if (PyTuple_GET_SIZE(a[8]) != plan->blocks * L_COUNT + 1 || PyTuple_GET_SIZE(a[9]) != plan->blocks * N_COUNT + 1 ||
@@ -747,7 +813,7 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     Operand w;
     if (!PyTuple_Check(pr) || PyTuple_GET_SIZE(pr) != 2 || !read_operand(PyTuple_GET_ITEM(pr, 0), w)) bad("stack_plan: bad layer");
     PyObject* b = PyTuple_GET_ITEM(pr, 1);
-    plan->lin.push_back({w.codes->data_ptr(), w.codes->stride(0), w.scales, w.amax, b == Py_None ? nullptr : f32(b), w.rows, w.k});
+    plan->lin.push_back(plan->layer(w, b == Py_None ? nullptr : f32(b)));
   }
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[9]); ++i) {
     PyObject* pr = PyTuple_GET_ITEM(a[9], i);
@@ -761,49 +827,25 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (a[11] != Py_None) {
     Operand w;
     if (!read_operand(a[11], w) || w.rows != plan->blocks * plan->d) bad("stack_plan: bad batched positional projection");
-    plan->lp_all = {w.codes->data_ptr(), w.codes->stride(0), w.scales, w.amax, nullptr, w.rows, w.k};
+    plan->lp_all = plan->layer(w, nullptr);
   }
   PyObject* cap = PyCapsule_New(plan.get(), "velox_stack_plan", plan_free);
   if (!cap) return nullptr;
-  plan->owners = PyTuple_Pack(4, a[8], a[9], a[10], a[11]);
   plan.release();
   return cap;
   VX_END
 }
 
-// stack_forward(plan, x, pos | None, fused_ln, head, keys | None, ids | None, logits | None, source | None) -> logits / ids
-//   x bf16 [T, d] (overwritten; with `source`, bf16 [T, d], the features are read there and x only receives the residual
-//   stream); head 0: bf16 logits [T, vocab], 1: greedy ids i32 [T]
-PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
-  VX_BEGIN
-  VX_ARGS(9)
-  const Plan* plan = static_cast<const Plan*>(PyCapsule_GetPointer(a[0], "velox_stack_plan"));
-  if (!plan) return nullptr;
-  const Plan& p = *plan;
-  auto bad = [](const char* what) { PyErr_SetString(PyExc_ValueError, what); throw PyFail{}; };
-  if (!is_cuda_tensor(a[1])) {
-    PyErr_SetString(PyExc_RuntimeError, "x must be a CUDA tensor: this library has no CPU path");
-    return nullptr;
-  }
-  const at::Tensor& xt = THPVariable_Unpack(a[1]);
-  if (xt.scalar_type() != at::kBFloat16 || !rows2d(xt) || xt.size(1) != p.d) bad("x must be bf16 [T, d_model] with unit column stride");
+// Every launch of one pass.  `src` (row stride ld_src): the features, where they are not in x; `pt`: the positions, or not
+// defined; of the outputs those that the caller did not bring are made.
+void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld_src, const at::Tensor& pt, bool fused, bool greedy,
+                at::Tensor& keys, at::Tensor& ids, at::Tensor& logits) {
   const at::Device dev = xt.device();
   const int64_t M = xt.size(0), ldx = xt.stride(0), d = p.d;
   void* const x = xt.data_ptr();
-  const void* src = nullptr;
-  int64_t ld_src = 0;
-  if (a[8] != Py_None) {
-    if (!is_cuda_tensor(a[8])) bad("source must be a CUDA tensor");
-    const at::Tensor& t = THPVariable_Unpack(a[8]);
-    if (t.scalar_type() != at::kBFloat16 || !rows2d(t) || t.sizes() != xt.sizes() || t.device() != xt.device())
-      bad("source must be bf16 of x's shape on x's device with unit column stride");
-    src = t.data_ptr();
-    ld_src = t.stride(0);
-  }
+  const bool with_pos = pt.defined();
   Pass s{p, M, stream()};
-  const bool with_pos = a[2] != Py_None;
-  if (with_pos && !is_cuda_tensor(a[2])) bad("pos must be a CUDA tensor");
-  Pass sp{p, with_pos ? THPVariable_Unpack(a[2]).size(0) : 0, s.st};  // the positions' own rows
+  Pass sp{p, with_pos ? pt.size(0) : 0, s.st};  // the positions' own rows
 
   // workspace: [activations | positions | context / GLU activations | FFN intermediate or q|k|v or GLU output | lp output]
   const int64_t ba = s.act_bytes(d), bc = s.act_bytes(d > p.glu ? d : p.glu);
@@ -824,13 +866,9 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 
   Act pos_q{};
   if (with_pos) {
-    const at::Tensor& pt = THPVariable_Unpack(a[2]);
-    if (!rows2d(pt) || pt.size(1) != d || pt.device() != dev || dtype_code(pt) < 0)
-      bad("pos must be a float32 or bf16 [frames, d_model] tensor on x's device with unit column stride");
     pos_q = sp.act(w_pos, d, p.amax(p.blocks * A_COUNT + 1));
     sp.quantize(pt.data_ptr(), dtype_code(pt), pt.stride(0), pos_q);
   }
-  const bool fused = as_bool(a[3]);
   if (lp_batched) sp.gemm(pos_q, p.lp_all, VX_EPI_NONE, w_lp, p.blocks * d);
   // the quantizers of the value third and of the GLU output run in the epilogues that produce them
   const bool in_epilogue = p.fmt != VX_FMT_FP8_1X128 && d % 256 == 0 && p.glu % 256 == 0;
@@ -878,37 +916,79 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     ffn(q_ff, L[L_FF1], L[L_FF2], mx(A_FF_H), n[N_FINAL], last ? &p.norm[p.blocks * N_COUNT] : n + N_COUNT + N_FFM, q);
   }
   const Lin& head = p.lin[p.blocks * L_COUNT];
-  PyObject* result = nullptr;
-  if (as_long(a[4])) {
-    at::Tensor keys, ids;
-    auto out_vec = [&](PyObject* o, at::ScalarType dt, const char* what) {
-      if (o == Py_None) return empty({M}, dt, dev);
-      if (!is_cuda_tensor(o)) bad(what);
-      const at::Tensor& t = THPVariable_Unpack(o);
-      if (t.scalar_type() != dt || !t.is_contiguous() || t.numel() < M || t.device() != dev) bad(what);
-      return t;
-    };
-    keys = out_vec(a[5], at::kLong, "keys must be a contiguous int64 tensor with at least T entries");
-    ids = out_vec(a[6], at::kInt, "ids must be a contiguous int32 tensor with at least T entries");
-    vx_gemm_desc e = s.desc(q, head, VX_EPI_BIAS_ARGMAX);
+  vx_gemm_desc e = s.desc(q, head, greedy ? VX_EPI_BIAS_ARGMAX : VX_EPI_BIAS);
+  if (greedy) {
+    if (!keys.defined()) keys = empty({M}, at::kLong, dev);
+    if (!ids.defined()) ids = empty({M}, at::kInt, dev);
     e.out_dtype = VX_F32; e.out = keys.data_ptr(); e.ldo = 1;
     s.run(e);
     check(g.vx_argmax_ids(keys.data_ptr(), M, static_cast<int32_t*>(ids.data_ptr()), nullptr, s.st), "vx_argmax_ids");
     ++s.launches;
-    result = a[6] == Py_None ? wrap(ids) : Py_NewRef(a[6]);
   } else {
-    at::Tensor out;
-    if (a[7] == Py_None) out = new_out(M, p.vocab, at::kBFloat16, dev);
-    else if (is_cuda_tensor(a[7])) out = THPVariable_Unpack(a[7]);
-    if (!out.defined() || !rows2d(out) || out.size(0) != M || out.size(1) != p.vocab || out.device() != dev || dtype_code(out) < 0)
-      bad("out_logits must be a [T, vocab] CUDA tensor with unit column stride");
-    vx_gemm_desc e = s.desc(q, head, VX_EPI_BIAS);
-    e.out_dtype = dtype_code(out); e.out = out.data_ptr(); e.ldo = out.stride(0);
+    if (!logits.defined()) logits = new_out(M, p.vocab, at::kBFloat16, dev);
+    e.out_dtype = dtype_code(logits); e.out = logits.data_ptr(); e.ldo = logits.stride(0);
     s.run(e);
-    result = a[7] == Py_None ? wrap(out) : Py_NewRef(a[7]);
   }
   count(s.launches + sp.launches);
-  return result;
+}
+
+// stack_forward(plan, x, pos | None, fused_ln, head, keys | None, ids | None, logits | None, source | None) -> logits / ids
+//   x bf16 [T, d] (overwritten; with `source`, bf16 [T, d], the features are read there and x only receives the residual
+//   stream); head 0: bf16 logits [T, vocab], 1: greedy ids i32 [T]
+PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  VX_BEGIN
+  VX_ARGS(9)
+  const Plan* plan = static_cast<const Plan*>(PyCapsule_GetPointer(a[0], "velox_stack_plan"));
+  if (!plan) return nullptr;
+  const Plan& p = *plan;
+  auto bad = [](const char* what) { PyErr_SetString(PyExc_ValueError, what); throw PyFail{}; };
+  if (!is_cuda_tensor(a[1])) {
+    PyErr_SetString(PyExc_RuntimeError, "x must be a CUDA tensor: this library has no CPU path");
+    return nullptr;
+  }
+  const at::Tensor& xt = THPVariable_Unpack(a[1]);
+  if (xt.scalar_type() != at::kBFloat16 || !rows2d(xt) || xt.size(1) != p.d) bad("x must be bf16 [T, d_model] with unit column stride");
+  const at::Device dev = xt.device();
+  const int64_t M = xt.size(0), d = p.d;
+  const void* src = nullptr;
+  int64_t ld_src = 0;
+  if (a[8] != Py_None) {
+    if (!is_cuda_tensor(a[8])) bad("source must be a CUDA tensor");
+    const at::Tensor& t = THPVariable_Unpack(a[8]);
+    if (t.scalar_type() != at::kBFloat16 || !rows2d(t) || t.sizes() != xt.sizes() || t.device() != xt.device())
+      bad("source must be bf16 of x's shape on x's device with unit column stride");
+    src = t.data_ptr();
+    ld_src = t.stride(0);
+  }
+  const bool with_pos = a[2] != Py_None;
+  if (with_pos && !is_cuda_tensor(a[2])) bad("pos must be a CUDA tensor");
+  at::Tensor pt, keys, ids, logits;
+  if (with_pos) {
+    pt = THPVariable_Unpack(a[2]);
+    if (!rows2d(pt) || pt.size(1) != d || pt.device() != dev || dtype_code(pt) < 0)
+      bad("pos must be a float32 or bf16 [frames, d_model] tensor on x's device with unit column stride");
+  }
+  const bool fused = as_bool(a[3]), greedy = as_long(a[4]) != 0;
+  auto out_vec = [&](PyObject* o, at::ScalarType dt, const char* what, at::Tensor& t) {
+    if (o == Py_None) return;
+    if (!is_cuda_tensor(o)) bad(what);
+    t = THPVariable_Unpack(o);
+    if (t.scalar_type() != dt || !t.is_contiguous() || t.numel() < M || t.device() != dev) bad(what);
+  };
+  if (greedy) {
+    out_vec(a[5], at::kLong, "keys must be a contiguous int64 tensor with at least T entries", keys);
+    out_vec(a[6], at::kInt, "ids must be a contiguous int32 tensor with at least T entries", ids);
+  } else if (a[7] != Py_None) {
+    if (is_cuda_tensor(a[7])) logits = THPVariable_Unpack(a[7]);
+    if (!logits.defined() || !rows2d(logits) || logits.size(0) != M || logits.size(1) != p.vocab || logits.device() != dev || dtype_code(logits) < 0)
+      bad("out_logits must be a [T, vocab] CUDA tensor with unit column stride");
+  }
+  {
+    NoGil nogil;
+    stack_pass(p, xt, src, ld_src, pt, fused, greedy, keys, ids, logits);
+  }
+  PyObject* given = a[greedy ? 6 : 7];
+  return given == Py_None ? wrap(greedy ? ids : logits) : Py_NewRef(given);
   VX_END
 }
 
