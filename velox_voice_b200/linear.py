@@ -167,7 +167,10 @@ class DenseLinear(nn.Linear):
             if self._wq is None:
                 self._prequantize_weight(precision)
             # quantize + one GEMM with the scales and the bias in its epilogue (fp32 out)
-            r = ops._host().rowscale_linear(x, self._wq, self._ws, self.bias)
+            b = self._parameters.get("bias")
+            if b is None:  # no bias, or pruning / a parametrization made it an attribute of its own
+                b = self.bias
+            r = ops._host().rowscale_linear(x, self._wq, self._ws, b)
             if r is not None:
                 return r
             orig_shape = x.shape
