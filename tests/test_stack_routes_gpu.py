@@ -101,3 +101,54 @@ def test_frames_of_the_fused_launches_are_the_callers_to_choose():
         stack.forward_ids(x.clone())
         count[least] = ops.launch_count()
     assert count[1] == count[5000] == count[None] < count[5001] == count[1 << 30]
+
+
+def test_what_a_program_replaces_takes_effect():
+    """Layers, their weights and biases, LayerNorm parameters and calibrated maxima may be replaced between passes."""
+    torch.manual_seed(8)
+    x = torch.randn(200, 512, device="cuda").bfloat16()
+    other = build(seed=1, blocks=2)
+    stack = build(blocks=2)
+
+    def check():
+        want, _ = by_operators(stack, x.clone())
+        assert torch.equal(stack.forward(x.clone()), want)
+        return want
+
+    seen = [check()]
+    stack.p["b1.pw2"] = other.p["b1.pw2"]
+    seen.append(check())
+    stack.p["b0.qkv"].q = other.p["b0.qkv"].q
+    seen.append(check())
+    stack.p["ctc"].bias = other.p["ctc"].bias + 1.0
+    seen.append(check())
+    stack.ln["b0.ln_conv"] = (1.5 * stack.ln["b0.ln_conv"][0], stack.ln["b0.ln_conv"][1])
+    seen.append(check())
+    stack.ln["b1.ln_ff"] = tuple(t.bfloat16() for t in stack.ln["b1.ln_ff"])
+    seen.append(check())
+    stack.cfg.eps = 1e-2
+    seen.append(check())
+    stack.fuse_ffn = False
+    check()
+    assert all(not torch.equal(a, b) for a, b in zip(seen, seen[1:]))
+    stack = build("nv16", blocks=2)
+    first = check()
+    stack.amax["b0.ln_mha"] = 1.3 * stack.amax["b0.ln_mha"]
+    assert not torch.equal(check(), first)
+
+
+def test_widths_come_from_the_weights():
+    """The configuration's ffn, conv_pw and vocab describe a model; a pass runs the layers as they are.  What does not fit the
+    layer before it is refused."""
+    from velox_voice_b200.stack import ConformerLinearStack, StackConfig, make_weights
+
+    torch.manual_seed(9)
+    small = StackConfig(blocks=2, ffn=1024, conv_pw=512, vocab=999)
+    w = make_weights(small, seed=4)
+    stack = ConformerLinearStack(StackConfig(blocks=2), w)
+    x = torch.randn(140, 512, device="cuda").bfloat16()
+    want, _ = by_operators(stack, x.clone())
+    assert want.shape[1] == 999 and torch.equal(stack.forward(x.clone()), want)
+    stack.p["b0.ff.w1"] = build(blocks=1).p["b0.ff.w1"]  # 2,048 outputs in front of 1,024 inputs
+    with pytest.raises(ValueError):
+        stack.forward(x.clone())

@@ -18,6 +18,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <atomic>
 #include <string>
 #include <vector>
@@ -38,7 +39,7 @@ struct Api {
 
 PyObject* g_error = nullptr;      // VeloxError
 PyObject* g_quantized = nullptr;  // class Quantized
-PyObject *s_fmt, *s_rows, *s_k, *s_codes, *s_scales, *s_sf, *s_amax;
+PyObject *s_fmt, *s_rows, *s_k, *s_codes, *s_scales, *s_sf, *s_amax, *s_q, *s_bias;
 std::atomic<int64_t> g_launches{0};
 
 void count(int64_t n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
@@ -664,7 +665,7 @@ enum { A_FFM, A_FFM_H, A_MHA, A_CTX, A_CONV, A_GLU, A_FF, A_FF_H, A_COUNT };
 
 struct Plan {
   int fmt;
-  int64_t d, ffn, glu, vocab;
+  int64_t d, ffn = 0, glu = 0, vocab = 0;  // the widest FFN intermediate and GLU output of the blocks
   float eps;
   bool fuse_ffn;
   int blocks;
@@ -673,6 +674,7 @@ struct Plan {
   std::vector<Norm> norm;        // [block][N_COUNT], then after_norm
   std::vector<const float*> am;  // [block][A_COUNT], then after_norm, then the positions (NV16)
   std::vector<at::Tensor> keep;  // everything the pointers above point into
+  PyObject* made_of = nullptr;   // the Python objects the plan was made of, see py_stack_plan_current
   Lin layer(const Operand& w, const float* bias) {
     for (const at::Tensor& t : {w.codes, w.scales, w.amax}) keep.push_back(t);
     return {w.codes.data_ptr(), w.codes.stride(0), w.scales.data_ptr(), f32_ptr(w.amax), bias, w.rows, w.k};
@@ -776,6 +778,8 @@ struct Pass {
 
 void plan_free(PyObject* cap) {
   Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(cap, "velox_stack_plan"));
+  if (!p) return;
+  Py_XDECREF(p->made_of);
   delete p;
 }
 
@@ -784,55 +788,98 @@ void plan_free(PyObject* cap) {
 // outputs would take blocks * d_model columns of workspace for nothing.
 constexpr int64_t LP_BATCH_MAX = 4096;
 
-// stack_plan(fmt, d, ffn, glu, vocab, eps, fuse_ffn, blocks, layers, norms, amax, lp_all | None) -> capsule
-//   layers: sequence of (Quantized, bias | None); norms: sequence of (gamma, beta); amax: sequence of tensors, or empty
+// stack_plan(fmt, d, eps, fuse_ffn, blocks, layers, norms, amax, lp_all | None, made_of) -> capsule
+//   layers: sequence of (Quantized, bias | None); norms: sequence of (gamma, beta); amax: sequence of tensors, or empty;
+//   made_of: ((name, layer, Quantized, bias)...), ((name, (gamma, beta))...), ((name, maximum)...)
 PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   VX_BEGIN
-  VX_ARGS(12)
+  VX_ARGS(10)
   auto plan = std::make_unique<Plan>();
   plan->fmt = static_cast<int>(as_long(a[0]));
-  plan->d = as_long(a[1]); plan->ffn = as_long(a[2]); plan->glu = as_long(a[3]); plan->vocab = as_long(a[4]);
-  plan->eps = static_cast<float>(as_double(a[5]));
-  plan->fuse_ffn = as_bool(a[6]);
-  plan->blocks = static_cast<int>(as_long(a[7]));
+  plan->d = as_long(a[1]);
+  plan->eps = static_cast<float>(as_double(a[2]));
+  plan->fuse_ffn = as_bool(a[3]);
+  plan->blocks = static_cast<int>(as_long(a[4]));
   auto bad = [](const char* what) { PyErr_SetString(PyExc_ValueError, what); throw PyFail{}; };
-  for (int i = 8; i < 11; ++i)
+  for (int i = 5; i < 8; ++i)
     if (!PyTuple_Check(a[i])) bad("stack_plan: tuples expected");
-  auto f32 = [&](PyObject* o) -> const float* {
+  auto f32 = [&](PyObject* o, int64_t n) -> const float* {
     if (!is_cuda_tensor(o)) bad("stack_plan: CUDA tensors expected");
     const at::Tensor& t = THPVariable_Unpack(o);
-    if (t.scalar_type() != at::kFloat || !t.is_contiguous()) bad("stack_plan: contiguous float32 vectors expected");
+    if (t.scalar_type() != at::kFloat || !t.is_contiguous() || t.numel() < n) bad("stack_plan: contiguous float32 vectors of the layers' widths expected");
     plan->keep.push_back(t);
     return static_cast<const float*>(t.data_ptr());
   };
-  if (PyTuple_GET_SIZE(a[8]) != plan->blocks * L_COUNT + 1 || PyTuple_GET_SIZE(a[9]) != plan->blocks * N_COUNT + 1 ||
-      (PyTuple_GET_SIZE(a[10]) != 0 && PyTuple_GET_SIZE(a[10]) != plan->blocks * A_COUNT + 2))
+  if (PyTuple_GET_SIZE(a[5]) != plan->blocks * L_COUNT + 1 || PyTuple_GET_SIZE(a[6]) != plan->blocks * N_COUNT + 1 ||
+      (PyTuple_GET_SIZE(a[7]) != 0 && PyTuple_GET_SIZE(a[7]) != plan->blocks * A_COUNT + 2))
     bad("stack_plan: wrong number of layers, norms or maxima");
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[8]); ++i) {
-    PyObject* pr = PyTuple_GET_ITEM(a[8], i);
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[5]); ++i) {
+    PyObject* pr = PyTuple_GET_ITEM(a[5], i);
     Operand w;
     if (!PyTuple_Check(pr) || PyTuple_GET_SIZE(pr) != 2 || !read_operand(PyTuple_GET_ITEM(pr, 0), w)) bad("stack_plan: bad layer");
+    // the widths come from the layers; what follows one another has to fit
+    const int64_t d = plan->d;
+    const bool head = i == plan->blocks * L_COUNT;
+    const int l = head ? L_COUNT : static_cast<int>(i % L_COUNT);
+    const bool wide = l == L_FFM1 || l == L_FF1 || l == L_PW1 || head;  // its number of outputs is free
+    const int64_t before = l == L_FFM2 || l == L_FF2 ? plan->lin.back().N : (l == L_PW2 ? plan->lin.back().N / 2 : d);
+    if (w.fmt != plan->fmt || w.k != before || (!wide && w.rows != (l == L_QKV ? 3 * d : d)))
+      bad("a layer of the stack does not fit the format, d_model or the layer before it");
+    if (l == L_FFM1 || l == L_FF1) plan->ffn = std::max(plan->ffn, w.rows);
+    if (l == L_PW1) plan->glu = std::max(plan->glu, w.rows / 2);
+    if (head) plan->vocab = w.rows;
     PyObject* b = PyTuple_GET_ITEM(pr, 1);
-    plan->lin.push_back(plan->layer(w, b == Py_None ? nullptr : f32(b)));
+    plan->lin.push_back(plan->layer(w, b == Py_None ? nullptr : f32(b, w.rows)));
   }
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[9]); ++i) {
-    PyObject* pr = PyTuple_GET_ITEM(a[9], i);
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[6]); ++i) {
+    PyObject* pr = PyTuple_GET_ITEM(a[6], i);
     if (!PyTuple_Check(pr) || PyTuple_GET_SIZE(pr) != 2) bad("stack_plan: bad norm");
-    plan->norm.push_back({f32(PyTuple_GET_ITEM(pr, 0)), f32(PyTuple_GET_ITEM(pr, 1))});
+    plan->norm.push_back({f32(PyTuple_GET_ITEM(pr, 0), plan->d), f32(PyTuple_GET_ITEM(pr, 1), plan->d)});
   }
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[10]); ++i) {
-    PyObject* o = PyTuple_GET_ITEM(a[10], i);
-    plan->am.push_back(o == Py_None ? nullptr : f32(o));
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[7]); ++i) {
+    PyObject* o = PyTuple_GET_ITEM(a[7], i);
+    plan->am.push_back(o == Py_None ? nullptr : f32(o, 1));
   }
-  if (a[11] != Py_None) {
+  if (a[8] != Py_None) {
     Operand w;
-    if (!read_operand(a[11], w) || w.rows != plan->blocks * plan->d) bad("stack_plan: bad batched positional projection");
+    if (!read_operand(a[8], w) || w.rows != plan->blocks * plan->d) bad("stack_plan: bad batched positional projection");
     plan->lp_all = plan->layer(w, nullptr);
   }
   PyObject* cap = PyCapsule_New(plan.get(), "velox_stack_plan", plan_free);
   if (!cap) return nullptr;
+  plan->made_of = Py_NewRef(a[9]);
   plan.release();
   return cap;
+  VX_END
+}
+
+// stack_plan_current(plan, layers by name, norms by name, maxima by name, eps, fuse_ffn, blocks) -> bool: whether the stack still holds the
+// objects the plan was made of.  A program may replace a layer, its weight or bias, a LayerNorm's parameters or a maximum
+// between passes; about 10 us of a host call that is ahead of the GPU by more.
+PyObject* py_stack_plan_current(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  VX_BEGIN
+  VX_ARGS(7)
+  const Plan* plan = static_cast<const Plan*>(PyCapsule_GetPointer(a[0], "velox_stack_plan"));
+  if (!plan) return nullptr;
+  if (static_cast<float>(as_double(a[4])) != plan->eps || as_bool(a[5]) != plan->fuse_ffn || as_long(a[6]) != plan->blocks) Py_RETURN_FALSE;
+  for (int part = 0; part < 3; ++part) {
+    PyObject* entries = PyTuple_GET_ITEM(plan->made_of, part);
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(entries); ++i) {
+      PyObject* e = PyTuple_GET_ITEM(entries, i);
+      PyObject* now = PyDict_GetItemWithError(a[1 + part], PyTuple_GET_ITEM(e, 0));
+      if (!now && PyErr_Occurred()) throw PyFail{};
+      if ((now ? now : Py_None) != PyTuple_GET_ITEM(e, 1)) Py_RETURN_FALSE;
+      if (part > 0) continue;
+      PyObject* const names[2] = {s_q, s_bias};
+      for (int k = 0; k < 2; ++k) {
+        PyObject* v = PyObject_GetAttr(now, names[k]);
+        if (!v) throw PyFail{};
+        Py_DECREF(v);
+        if (v != PyTuple_GET_ITEM(e, 2 + k)) Py_RETURN_FALSE;
+      }
+    }
+  }
+  Py_RETURN_TRUE;
   VX_END
 }
 
@@ -871,16 +918,16 @@ void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld
   }
   if (lp_batched) sp.gemm(pos_q, p.lp_all, VX_EPI_NONE, w_lp, p.blocks * d);
   // the quantizers of the value third and of the GLU output run in the epilogues that produce them
-  const bool in_epilogue = p.fmt != VX_FMT_FP8_1X128 && d % 256 == 0 && p.glu % 256 == 0;
+  const bool fp4 = p.fmt != VX_FMT_FP8_1X128;
   auto ffn = [&](const Act& q, const Lin& w1, const Lin& w2, const float* am_h, const Norm& n, const Norm* n2, const Act& q_next,
                  const void* from = nullptr) {
-    const Act h = s.act(w_big, p.ffn, am_h);
+    const Act h = s.act(w_big, w1.N, am_h);
     if (p.fuse_ffn) {
       s.gemm_quant(q, w1, VX_EPI_BIAS_SWISH, h);
     } else {
-      void* const hb = w_big + s.act_bytes(p.ffn);
-      s.gemm(q, w1, VX_EPI_BIAS_SWISH, hb, p.ffn);
-      s.quantize(hb, VX_BF16, p.ffn, h);
+      void* const hb = w_big + s.act_bytes(w1.N);
+      s.gemm(q, w1, VX_EPI_BIAS_SWISH, hb, w1.N);
+      s.quantize(hb, VX_BF16, w1.N, h);
     }
     s.residual(h, w2, x, ldx, 0.5f, n, n2, q_next, fused, from, ld_src);
   };
@@ -894,7 +941,7 @@ void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld
     Act q_mha = s.act(w_act, d, mx(A_MHA)), q_conv = s.act(w_act, d, mx(A_CONV)), q_ff = s.act(w_act, d, mx(A_FF));
     ffn(q, L[L_FFM1], L[L_FFM2], mx(A_FFM_H), n[N_MHA], nullptr, q_mha, i == 0 ? src : nullptr);
     const Act ctx = s.act(w_ctx, d, mx(A_CTX));
-    if (in_epilogue) {
+    if (fp4 && d % 256 == 0) {
       s.gemm_tail_quant(q_mha, L[L_QKV], w_big, 3 * d, 2 * d, ctx);
     } else {
       s.gemm(q_mha, L[L_QKV], VX_EPI_BIAS, w_big, 3 * d);
@@ -902,12 +949,13 @@ void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld
     }
     if (with_pos && !lp_batched) sp.gemm(pos_q, L[L_LP], VX_EPI_BIAS, w_lp, d);  // feeds the attention scores only
     s.residual(ctx, L[L_LO], x, ldx, 1.0f, n[N_CONV], nullptr, q_conv, fused);
-    const Act gl = s.act(w_ctx, p.glu, mx(A_GLU));
-    if (in_epilogue) {
+    const int64_t glu = L[L_PW1].N / 2;
+    const Act gl = s.act(w_ctx, glu, mx(A_GLU));
+    if (fp4 && glu % 256 == 0) {
       s.gemm_quant(q_conv, L[L_PW1], VX_EPI_BIAS_GLU, gl);
     } else {
-      s.gemm(q_conv, L[L_PW1], VX_EPI_BIAS_GLU, w_big, p.glu);
-      s.quantize(w_big, VX_BF16, p.glu, gl);
+      s.gemm(q_conv, L[L_PW1], VX_EPI_BIAS_GLU, w_big, glu);
+      s.quantize(w_big, VX_BF16, glu, gl);
     }
     s.residual(gl, L[L_PW2], x, ldx, 1.0f, n[N_FF], nullptr, q_ff, fused);
     // norm_final of this block and the LayerNorm that reads it next: the first of the next block, or after_norm
@@ -1037,6 +1085,7 @@ PyMethodDef kMethods[] = {
     VX_METHOD("heads_gemm", py_heads_gemm),
     VX_METHOD("power_mel_log", py_power_mel_log),
     VX_METHOD("stack_plan", py_stack_plan),
+    VX_METHOD("stack_plan_current", py_stack_plan_current),
     VX_METHOD("stack_forward", py_stack_forward),
     {"launches", py_launches, METH_NOARGS, nullptr},
     {"reset_launches", py_reset, METH_NOARGS, nullptr},
@@ -1053,5 +1102,7 @@ PyMODINIT_FUNC PyInit__vx_host() {
   s_scales = PyUnicode_InternFromString("scales");
   s_sf = PyUnicode_InternFromString("sf");
   s_amax = PyUnicode_InternFromString("amax");
+  s_q = PyUnicode_InternFromString("q");
+  s_bias = PyUnicode_InternFromString("bias");
   return PyModule_Create(&kModule);
 }

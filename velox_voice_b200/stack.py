@@ -159,24 +159,27 @@ class ConformerLinearStack:
 
     def _host_plan(self):
         """The pass as the native host path walks it: packed weights, LayerNorm parameters and (NV16) calibrated
-        maxima, per block in the order of ``vx_host.cpp``.  Built once; calibration drops it."""
-        if self._plan is None:
+        maxima, per block in the order of ``vx_host.cpp``.  Made anew when the stack no longer holds what it was made of."""
+        host = ops._host()
+        if self._plan is None or not host.stack_plan_current(self._plan, self.p, self.ln, self.amax, self.cfg.eps,
+                                                                     self.fuse_ffn, self.cfg.blocks):
             cfg = self.cfg
             layers, norms, amax = [], [], []
             for i in range(cfg.blocks):
                 b = f"b{i}."
-                for n in ("ffm.w1", "ffm.w2", "qkv", "lo", "lp", "pw1", "pw2", "ff.w1", "ff.w2"):
-                    layers.append((self.p[b + n].q, self.p[b + n].bias))
-                for n in ("ln_ffm", "ln_mha", "ln_conv", "ln_ff", "ln_final"):
-                    norms.append(self.ln[b + n])
-                if self.fmt == FMT_NV16:
-                    amax += [self._amax(b + n, None) for n in ("ln_ffm", "ffm.h", "ln_mha", "ctx", "ln_conv", "glu", "ln_ff", "ff.h")]
-            layers.append((self.p["ctc"].q, self.p["ctc"].bias))
-            norms.append(self.ln["after"])
-            if self.fmt == FMT_NV16:
-                amax += [self._amax("after", None), self.amax.get("pos")]
-            self._plan = ops._host().stack_plan(self.fmt, cfg.d_model, cfg.ffn, cfg.conv_pw // 2, cfg.vocab, cfg.eps, self.fuse_ffn,
-                                                cfg.blocks, tuple(layers), tuple(norms), tuple(amax), self._lp_all())
+                layers += [b + n for n in ("ffm.w1", "ffm.w2", "qkv", "lo", "lp", "pw1", "pw2", "ff.w1", "ff.w2")]
+                norms += [b + n for n in ("ln_ffm", "ln_mha", "ln_conv", "ln_ff", "ln_final")]
+                amax += [b + n for n in ("ln_ffm", "ffm.h", "ln_mha", "ctx", "ln_conv", "glu", "ln_ff", "ff.h")]
+            layers.append("ctc")
+            norms.append("after")
+            amax = amax + ["after"] if self.fmt == FMT_NV16 else []
+            layers = tuple((n, self.p[n], self.p[n].q, self.p[n].bias) for n in layers)
+            norms = tuple((n, self.ln[n]) for n in norms)
+            amax = tuple((n, self._amax(n, None)) for n in amax) + ((("pos", self.amax.get("pos")),) if amax else ())
+            self._plan = host.stack_plan(self.fmt, cfg.d_model, cfg.eps, self.fuse_ffn, cfg.blocks,
+                                         tuple((q, bias) for _, _, q, bias in layers),
+                                         tuple((g.float().contiguous(), b.float().contiguous()) for _, (g, b) in norms),
+                                         tuple(t for _, t in amax), self._lp_all(), (layers, norms, amax))
         return self._plan
 
     def _lp_all(self):
