@@ -152,3 +152,52 @@ def test_widths_come_from_the_weights():
     stack.p["b0.ff.w1"] = build(blocks=1).p["b0.ff.w1"]  # 2,048 outputs in front of 1,024 inputs
     with pytest.raises(ValueError):
         stack.forward(x.clone())
+
+
+@pytest.mark.parametrize("fmt", ["mx32", "nv16", "fp8_1x128"])
+def test_a_plan_points_into_the_layers(fmt):
+    """Making the plan of a pass runs nothing on the device and makes no copies: it happens in the first pass, whose stream
+    or graph capture later passes need not have waited for."""
+    stack = build(fmt, blocks=3)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_stats()["allocation.all.allocated"]
+    stack._host_plan()
+    assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+    whole = stack._lp_all()
+    assert (whole is None) == (fmt == "nv16")
+    if whole is None:
+        return
+    for i in range(3):
+        q = stack.p[f"b{i}.lp"].q
+        for name in ("codes", "scales", "sf"):
+            part, t = getattr(q, name), getattr(whole, name)
+            assert (part is None) == (t is None)
+            assert t is None or part.data_ptr() == t[i * t.shape[0] // 3].data_ptr()
+    stack.p["b1.lp"].q.codes = stack.p["b1.lp"].q.codes.clone()
+    assert stack._lp_all() is None
+
+
+def test_first_pass_on_another_stream_and_in_a_capture():
+    torch.manual_seed(10)
+    x, pos = (torch.randn(300, 512, device="cuda").bfloat16() for _ in range(2))
+    want, _ = by_operators(build(blocks=2), x.clone())
+    stack = build(blocks=2)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = []
+    for s in streams:
+        with torch.cuda.stream(s):
+            got.append(stack.forward(x.clone(), pos))
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, want) for g in got)
+    stack = build(blocks=2)
+    stack.forward(x.clone())  # (one-time module loading is not to be captured; the plan is)
+    stack._plan = None
+    buf, graph = x.clone(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        out = stack.forward(buf, pos)
+    assert torch.equal(stack.forward(x.clone(), pos), want)  # before any replay
+    buf.copy_(x)
+    graph.replay()
+    assert torch.equal(out, want)

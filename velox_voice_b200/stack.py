@@ -141,6 +141,7 @@ class ConformerLinearStack:
                 self.ln[b + n] = (weights[b + n + ".g"].to(dev).float(), weights[b + n + ".b"].to(dev).float())
         self.ln["after"] = (weights["after.g"].to(dev).float(), weights["after.b"].to(dev).float())
         pack("ctc", "ctc.w", "ctc.b")
+        self._stack_positions()
         self._plan = None
         # NV16 needs a per-tensor amax for every activation it quantizes: calibrated once
         self.amax: Dict[str, torch.Tensor] = {}
@@ -182,16 +183,42 @@ class ConformerLinearStack:
                                          tuple(t for _, t in amax), self._lp_all(), (layers, norms, amax))
         return self._plan
 
-    def _lp_all(self):
-        """The positional projections of all blocks as one weight [blocks * d_model, d_model] (short passes run them in
-        one launch), or None where their packed rows cannot simply be stacked."""
+    def _stack_positions(self):
+        """Lays the packed positional projections of all blocks behind one another, as one weight [blocks * d_model, d_model]
+        (short passes run them in one launch); the layers keep views of it.  Done here and not with the plan: a plan is made
+        in whichever pass comes first, on its stream or inside its graph capture, and a launch that reads constant weights
+        ahead of the work before it must find them written."""
         cfg = self.cfg
+        self._positions: Optional[ops.Quantized] = None
         if cfg.blocks == 0 or cfg.d_model % 128 != 0 or self.fmt == FMT_NV16:  # (NV16: a tensor scale per weight)
-            return None
+            return
         qs = [self.p[f"b{i}.lp"].q for i in range(cfg.blocks)]
-        cat = lambda ts: None if ts[0] is None else torch.cat(ts)
-        return ops.Quantized(self.fmt, cfg.blocks * cfg.d_model, cfg.d_model, cat([q.codes for q in qs]), cat([q.scales for q in qs]),
-                             cat([q.sf for q in qs]), None)
+        self._positions = ops.Quantized(self.fmt, cfg.blocks * cfg.d_model, cfg.d_model, None, None, None, None)
+        for field in ("codes", "scales", "sf"):
+            parts = [getattr(q, field) for q in qs]
+            if parts[0] is not None:
+                whole = torch.cat(parts)
+                setattr(self._positions, field, whole)
+                for q, part in zip(qs, whole.chunk(cfg.blocks)):
+                    setattr(q, field, part)
+
+    def _lp_all(self):
+        """The stacked positional projections as long as every block's layer is its part of them, else None."""
+        whole, n = self._positions, self.cfg.blocks
+        if whole is None or whole.rows != n * self.cfg.d_model:
+            return None
+        for i in range(n):
+            layer = self.p[f"b{i}.lp"]
+            if layer.bias is not None:
+                return None
+            for field in ("codes", "scales", "sf"):
+                t, part = getattr(whole, field), getattr(layer.q, field)
+                if t is None and part is None:
+                    continue
+                if t is None or part is None or part.shape != (t.shape[0] // n, *t.shape[1:]) or \
+                        part.data_ptr() != t.data_ptr() + i * part.numel() * part.element_size():
+                    return None
+        return whole
 
     # ---- forward
     def forward(self, x: torch.Tensor, pos: Optional[torch.Tensor] = None, *, return_hidden: bool = False,
