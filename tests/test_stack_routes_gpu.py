@@ -137,6 +137,39 @@ def test_what_a_program_replaces_takes_effect():
     assert not torch.equal(check(), first)
 
 
+def test_new_tensors_and_storage_of_a_layer_take_effect():
+    """The fields of a layer's packed weight may be assigned, and a tensor may be given other storage: the pointers of the plan
+    would lead to the former one."""
+    torch.manual_seed(11)
+    x = torch.randn(200, 512, device="cuda").bfloat16()
+    for fmt in ("mx32", "nv16", "fp8_1x128"):
+        stack, other = build(fmt, blocks=2), build(fmt, seed=1, blocks=2)
+        scales = "scales" if fmt == "fp8_1x128" else "sf"
+
+        def changed(before):
+            want, _ = by_operators(stack, x.clone())
+            assert torch.equal(stack.forward(x.clone()), want) and not torch.equal(want, before)
+            return want
+
+        last = stack.forward(x.clone())
+        a, b = stack.p["b0.lo"].q, other.p["b0.lo"].q
+        a.codes = b.codes
+        last = changed(last)
+        setattr(a, scales, getattr(b, scales).roll(1, 0).contiguous())
+        last = changed(last)
+        stack.p["b1.pw1"].q.codes.data = other.p["b1.pw1"].q.codes.clone()
+        last = changed(last)
+        stack.p["b1.qkv"].bias.data = stack.p["b1.qkv"].bias + 1.0
+        last = changed(last)
+        stack.ln["after"][0].data = 2.0 * stack.ln["after"][0]
+        last = changed(last)
+        if fmt == "nv16":
+            a.amax = 2.0 * a.amax
+            last = changed(last)
+            a.amax.data = 2.0 * a.amax
+            changed(last)
+
+
 def test_widths_come_from_the_weights():
     """The configuration's ffn, conv_pw and vocab describe a model; a pass runs the layers as they are.  What does not fit the
     layer before it is refused."""

@@ -673,10 +673,22 @@ struct Plan {
   Lin lp_all{};                  // the positional projections of all blocks as one weight (codes nullptr: none)
   std::vector<Norm> norm;        // [block][N_COUNT], then after_norm
   std::vector<const float*> am;  // [block][A_COUNT], then after_norm, then the positions (NV16)
-  std::vector<at::Tensor> keep;  // everything the pointers above point into
+  // everything the pointers above point into, as it was when they were taken
+  struct Kept { at::Tensor t; const void* ptr; int64_t numel, ld; };
+  std::vector<Kept> kept;
   PyObject* made_of = nullptr;   // the Python objects the plan was made of, see py_stack_plan_current
+  static int64_t row_stride(const at::Tensor& t) { return t.dim() > 0 ? t.stride(0) : 0; }
+  void keep(const at::Tensor& t) {
+    if (t.defined()) kept.push_back({t, t.data_ptr(), t.numel(), row_stride(t)});
+  }
+  // a tensor may have been given other storage (`t.data = ...`), and its former one freed
+  bool in_place() const {
+    for (const Kept& k : kept)
+      if (k.t.data_ptr() != k.ptr || k.t.numel() != k.numel || row_stride(k.t) != k.ld) return false;
+    return true;
+  }
   Lin layer(const Operand& w, const float* bias) {
-    for (const at::Tensor& t : {w.codes, w.scales, w.amax}) keep.push_back(t);
+    for (const at::Tensor& t : {w.codes, w.scales, w.amax}) keep(t);
     return {w.codes.data_ptr(), w.codes.stride(0), w.scales.data_ptr(), f32_ptr(w.amax), bias, w.rows, w.k};
   }
   const float* amax(size_t i) const { return am.empty() ? nullptr : am[i]; }
@@ -790,7 +802,8 @@ constexpr int64_t LP_BATCH_MAX = 4096;
 
 // stack_plan(fmt, d, eps, fuse_ffn, blocks, layers, norms, amax, lp_all | None, made_of) -> capsule
 //   layers: sequence of (Quantized, bias | None); norms: sequence of (gamma, beta); amax: sequence of tensors, or empty;
-//   made_of: ((name, layer, Quantized, bias)...), ((name, (gamma, beta))...), ((name, maximum)...)
+//   made_of: ((name, layer, Quantized, bias, codes, scales of the GEMM, tensor maximum)...), ((name, (gamma, beta))...),
+//   ((name, maximum)...)
 PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   VX_BEGIN
   VX_ARGS(10)
@@ -807,7 +820,7 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (!is_cuda_tensor(o)) bad("stack_plan: CUDA tensors expected");
     const at::Tensor& t = THPVariable_Unpack(o);
     if (t.scalar_type() != at::kFloat || !t.is_contiguous() || t.numel() < n) bad("stack_plan: contiguous float32 vectors of the layers' widths expected");
-    plan->keep.push_back(t);
+    plan->keep(t);
     return static_cast<const float*>(t.data_ptr());
   };
   if (PyTuple_GET_SIZE(a[5]) != plan->blocks * L_COUNT + 1 || PyTuple_GET_SIZE(a[6]) != plan->blocks * N_COUNT + 1 ||
@@ -854,14 +867,24 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 }
 
 // stack_plan_current(plan, layers by name, norms by name, maxima by name, eps, fuse_ffn, blocks) -> bool: whether the stack still holds the
-// objects the plan was made of.  A program may replace a layer, its weight or bias, a LayerNorm's parameters or a maximum
-// between passes; about 10 us of a host call that is ahead of the GPU by more.
+// objects the plan was made of, with the storage they had.  A program may replace a layer, its weight or bias, a LayerNorm's parameters or a
+// maximum between passes; about 10 us of a host call that is ahead of the GPU by more.
 PyObject* py_stack_plan_current(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   VX_BEGIN
   VX_ARGS(7)
   const Plan* plan = static_cast<const Plan*>(PyCapsule_GetPointer(a[0], "velox_stack_plan"));
   if (!plan) return nullptr;
-  if (static_cast<float>(as_double(a[4])) != plan->eps || as_bool(a[5]) != plan->fuse_ffn || as_long(a[6]) != plan->blocks) Py_RETURN_FALSE;
+  if (static_cast<float>(as_double(a[4])) != plan->eps || as_bool(a[5]) != plan->fuse_ffn || as_long(a[6]) != plan->blocks ||
+      !plan->in_place())
+    Py_RETURN_FALSE;
+  PyObject* const in_layer[2] = {s_q, s_bias};
+  PyObject* const in_q[3] = {s_codes, has_sf(plan->fmt) ? s_sf : s_scales, s_amax};
+  auto same = [](PyObject* o, PyObject* name, PyObject* was) {
+    PyObject* v = PyObject_GetAttr(o, name);
+    if (!v) throw PyFail{};
+    Py_DECREF(v);
+    return v == was;
+  };
   for (int part = 0; part < 3; ++part) {
     PyObject* entries = PyTuple_GET_ITEM(plan->made_of, part);
     for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(entries); ++i) {
@@ -870,13 +893,10 @@ PyObject* py_stack_plan_current(PyObject*, PyObject* const* a, Py_ssize_t nargs)
       if (!now && PyErr_Occurred()) throw PyFail{};
       if ((now ? now : Py_None) != PyTuple_GET_ITEM(e, 1)) Py_RETURN_FALSE;
       if (part > 0) continue;
-      PyObject* const names[2] = {s_q, s_bias};
-      for (int k = 0; k < 2; ++k) {
-        PyObject* v = PyObject_GetAttr(now, names[k]);
-        if (!v) throw PyFail{};
-        Py_DECREF(v);
-        if (v != PyTuple_GET_ITEM(e, 2 + k)) Py_RETURN_FALSE;
-      }
+      for (int k = 0; k < 2; ++k)
+        if (!same(now, in_layer[k], PyTuple_GET_ITEM(e, 2 + k))) Py_RETURN_FALSE;
+      for (int k = 0; k < 3; ++k)
+        if (!same(PyTuple_GET_ITEM(e, 2), in_q[k], PyTuple_GET_ITEM(e, 4 + k))) Py_RETURN_FALSE;
     }
   }
   Py_RETURN_TRUE;

@@ -174,11 +174,11 @@ class ConformerLinearStack:
             layers.append("ctc")
             norms.append("after")
             amax = amax + ["after"] if self.fmt == FMT_NV16 else []
-            layers = tuple((n, self.p[n], self.p[n].q, self.p[n].bias) for n in layers)
+            layers = tuple((n, l, l.q, l.bias, l.q.codes, l.q.gemm_scales(), l.q.amax) for n, l in ((n, self.p[n]) for n in layers))
             norms = tuple((n, self.ln[n]) for n in norms)
             amax = tuple((n, self._amax(n, None)) for n in amax) + ((("pos", self.amax.get("pos")),) if amax else ())
             self._plan = host.stack_plan(self.fmt, cfg.d_model, cfg.eps, self.fuse_ffn, cfg.blocks,
-                                         tuple((q, bias) for _, _, q, bias in layers),
+                                         tuple(l[2:4] for l in layers),
                                          tuple((g.float().contiguous(), b.float().contiguous()) for _, (g, b) in norms),
                                          tuple(t for _, t in amax), self._lp_all(), (layers, norms, amax))
         return self._plan
