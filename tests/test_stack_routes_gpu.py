@@ -126,6 +126,12 @@ def test_what_a_program_replaces_takes_effect():
     seen.append(check())
     stack.ln["b1.ln_ff"] = tuple(t.bfloat16() for t in stack.ln["b1.ln_ff"])
     seen.append(check())
+    stack.ln["b1.ln_ff"][0].mul_(2.0)  # in place, where the kernels read a converted copy
+    seen.append(check())
+    stack.ln["b1.ln_ff"] = (torch.rand(1024, device="cuda")[::2], stack.ln["b1.ln_ff"][1])
+    seen.append(check())
+    stack.ln["b1.ln_ff"][0].add_(0.5)
+    seen.append(check())
     stack.cfg.eps = 1e-2
     seen.append(check())
     stack.fuse_ffn = False
@@ -196,7 +202,7 @@ def test_a_plan_points_into_the_layers(fmt):
     before = torch.cuda.memory_stats()["allocation.all.allocated"]
     stack._host_plan()
     assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
-    whole = stack._lp_all()
+    whole = stack._positions
     assert (whole is None) == (fmt == "nv16")
     if whole is None:
         return
@@ -206,8 +212,18 @@ def test_a_plan_points_into_the_layers(fmt):
             part, t = getattr(q, name), getattr(whole, name)
             assert (part is None) == (t is None)
             assert t is None or part.data_ptr() == t[i * t.shape[0] // 3].data_ptr()
+    x = torch.zeros(8, 512, device="cuda", dtype=torch.bfloat16)
+
+    def launches():
+        ops.reset_launch_count()
+        stack.forward_ids(x.clone(), x)
+        return ops.launch_count()
+
+    from velox_voice_b200 import ops
+
+    together = launches()
     stack.p["b1.lp"].q.codes = stack.p["b1.lp"].q.codes.clone()
-    assert stack._lp_all() is None
+    assert launches() == together + 2  # a launch per block
 
 
 def test_first_pass_on_another_stream_and_in_a_capture():

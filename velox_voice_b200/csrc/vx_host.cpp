@@ -676,7 +676,21 @@ struct Plan {
   // everything the pointers above point into, as it was when they were taken
   struct Kept { at::Tensor t; const void* ptr; int64_t numel, ld; };
   std::vector<Kept> kept;
-  PyObject* made_of = nullptr;   // the Python objects the plan was made of, see py_stack_plan_current
+  bool converted = false;        // a LayerNorm parameter was converted for this pass: the plan serves no other
+  // the Python objects the plan was made of, see py_stack_plan_current
+  struct Layer { PyObject *name, *layer, *q, *bias, *codes, *scales, *amax; };
+  struct Named { PyObject *name, *object; };
+  std::vector<Layer> layers;
+  std::vector<Named> norms, maxima;
+  std::vector<PyObject*> refs;
+  PyObject* own(PyObject* o) {  // (takes over a reference)
+    if (!o) throw PyFail{};
+    refs.push_back(o);
+    return o;
+  }
+  ~Plan() {
+    for (PyObject* o : refs) Py_DECREF(o);
+  }
   static int64_t row_stride(const at::Tensor& t) { return t.dim() > 0 ? t.stride(0) : 0; }
   void keep(const at::Tensor& t) {
     if (t.defined()) kept.push_back({t, t.data_ptr(), t.numel(), row_stride(t)});
@@ -789,10 +803,7 @@ struct Pass {
 };
 
 void plan_free(PyObject* cap) {
-  Plan* p = static_cast<Plan*>(PyCapsule_GetPointer(cap, "velox_stack_plan"));
-  if (!p) return;
-  Py_XDECREF(p->made_of);
-  delete p;
+  delete static_cast<Plan*>(PyCapsule_GetPointer(cap, "velox_stack_plan"));
 }
 
 // Frames up to which the positional projections of all blocks run as one launch: they depend on the positions only, and
@@ -800,13 +811,12 @@ void plan_free(PyObject* cap) {
 // outputs would take blocks * d_model columns of workspace for nothing.
 constexpr int64_t LP_BATCH_MAX = 4096;
 
-// stack_plan(fmt, d, eps, fuse_ffn, blocks, layers, norms, amax, lp_all | None, made_of) -> capsule
-//   layers: sequence of (Quantized, bias | None); norms: sequence of (gamma, beta); amax: sequence of tensors, or empty;
-//   made_of: ((name, layer, Quantized, bias, codes, scales of the GEMM, tensor maximum)...), ((name, (gamma, beta))...),
-//   ((name, maximum)...)
+// stack_plan(fmt, d, eps, fuse_ffn, blocks, layers, norms, maxima, positions | None) -> capsule
+//   layers: ((name, PackedLinear)...); norms: ((name, (gamma, beta))...); maxima: ((name, tensor | None)...), or empty;
+//   positions: the Quantized whose parts the positional projections of the blocks are
 PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   VX_BEGIN
-  VX_ARGS(10)
+  VX_ARGS(9)
   auto plan = std::make_unique<Plan>();
   plan->fmt = static_cast<int>(as_long(a[0]));
   plan->d = as_long(a[1]);
@@ -814,22 +824,54 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   plan->fuse_ffn = as_bool(a[3]);
   plan->blocks = static_cast<int>(as_long(a[4]));
   auto bad = [](const char* what) { PyErr_SetString(PyExc_ValueError, what); throw PyFail{}; };
-  for (int i = 5; i < 8; ++i)
+  const char* const vectors = "the stack's biases, LayerNorm parameters and maxima have to be CUDA vectors of the layers' widths";
+  for (int i = 5; i < 8; ++i) {
     if (!PyTuple_Check(a[i])) bad("stack_plan: tuples expected");
-  auto f32 = [&](PyObject* o, int64_t n) -> const float* {
-    if (!is_cuda_tensor(o)) bad("stack_plan: CUDA tensors expected");
-    const at::Tensor& t = THPVariable_Unpack(o);
-    if (t.scalar_type() != at::kFloat || !t.is_contiguous() || t.numel() < n) bad("stack_plan: contiguous float32 vectors of the layers' widths expected");
-    plan->keep(t);
-    return static_cast<const float*>(t.data_ptr());
-  };
+    for (Py_ssize_t j = 0; j < PyTuple_GET_SIZE(a[i]); ++j)
+      if (!PyTuple_Check(PyTuple_GET_ITEM(a[i], j)) || PyTuple_GET_SIZE(PyTuple_GET_ITEM(a[i], j)) != 2) bad("stack_plan: pairs expected");
+  }
   if (PyTuple_GET_SIZE(a[5]) != plan->blocks * L_COUNT + 1 || PyTuple_GET_SIZE(a[6]) != plan->blocks * N_COUNT + 1 ||
       (PyTuple_GET_SIZE(a[7]) != 0 && PyTuple_GET_SIZE(a[7]) != plan->blocks * A_COUNT + 2))
     bad("stack_plan: wrong number of layers, norms or maxima");
+  auto f32 = [&](PyObject* o, int64_t n) -> const float* {
+    if (!is_cuda_tensor(o)) bad(vectors);
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (t.scalar_type() != at::kFloat || !t.is_contiguous() || t.numel() < n) bad(vectors);
+    plan->keep(t);
+    return static_cast<const float*>(t.data_ptr());
+  };
+  // a LayerNorm's parameters may be of another type or strided; their copies are not kept, they would not follow the originals
+  auto norm_vector = [&](PyObject* o) -> const float* {
+    if (!is_cuda_tensor(o)) bad(vectors);
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (t.scalar_type() == at::kFloat && t.is_contiguous()) return f32(o, plan->d);
+    if (t.numel() < plan->d) bad(vectors);
+    plan->converted = true;
+    at::Tensor c;
+    {
+      NoGil nogil;
+      c = t.detach().to(at::kFloat).contiguous();
+    }
+    plan->keep(c);
+    return static_cast<const float*>(c.data_ptr());
+  };
+  const bool sf = has_sf(plan->fmt);
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[5]); ++i) {
-    PyObject* pr = PyTuple_GET_ITEM(a[5], i);
+    Plan::Layer y;
+    y.name = plan->own(Py_NewRef(PyTuple_GET_ITEM(PyTuple_GET_ITEM(a[5], i), 0)));
+    y.layer = plan->own(Py_NewRef(PyTuple_GET_ITEM(PyTuple_GET_ITEM(a[5], i), 1)));
+    y.q = plan->own(PyObject_GetAttr(y.layer, s_q));
+    y.bias = plan->own(PyObject_GetAttr(y.layer, s_bias));
+    if (reinterpret_cast<PyObject*>(Py_TYPE(y.q)) != g_quantized) bad("stack_plan: bad layer");
+    y.codes = plan->own(PyObject_GetAttr(y.q, s_codes));
+    y.scales = plan->own(PyObject_GetAttr(y.q, sf ? s_sf : s_scales));
+    if (sf && y.scales == Py_None) {  // made from the natural layout, and kept by the Quantized
+      plan->own(PyObject_CallMethod(y.q, "gemm_scales", nullptr));
+      y.scales = plan->own(PyObject_GetAttr(y.q, s_sf));
+    }
+    y.amax = plan->own(PyObject_GetAttr(y.q, s_amax));
     Operand w;
-    if (!PyTuple_Check(pr) || PyTuple_GET_SIZE(pr) != 2 || !read_operand(PyTuple_GET_ITEM(pr, 0), w)) bad("stack_plan: bad layer");
+    if (!read_operand(y.q, w)) bad("stack_plan: bad layer");
     // the widths come from the layers; what follows one another has to fit
     const int64_t d = plan->d;
     const bool head = i == plan->blocks * L_COUNT;
@@ -841,26 +883,36 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (l == L_FFM1 || l == L_FF1) plan->ffn = std::max(plan->ffn, w.rows);
     if (l == L_PW1) plan->glu = std::max(plan->glu, w.rows / 2);
     if (head) plan->vocab = w.rows;
-    PyObject* b = PyTuple_GET_ITEM(pr, 1);
-    plan->lin.push_back(plan->layer(w, b == Py_None ? nullptr : f32(b, w.rows)));
+    plan->lin.push_back(plan->layer(w, y.bias == Py_None ? nullptr : f32(y.bias, w.rows)));
+    plan->layers.push_back(y);
   }
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[6]); ++i) {
-    PyObject* pr = PyTuple_GET_ITEM(a[6], i);
-    if (!PyTuple_Check(pr) || PyTuple_GET_SIZE(pr) != 2) bad("stack_plan: bad norm");
-    plan->norm.push_back({f32(PyTuple_GET_ITEM(pr, 0), plan->d), f32(PyTuple_GET_ITEM(pr, 1), plan->d)});
+    PyObject* const e = PyTuple_GET_ITEM(a[6], i);
+    PyObject* const pr = PyTuple_GET_ITEM(e, 1);
+    if (!PyTuple_Check(pr) || PyTuple_GET_SIZE(pr) != 2) bad("stack_plan: a LayerNorm is a pair (gamma, beta)");
+    plan->norms.push_back({plan->own(Py_NewRef(PyTuple_GET_ITEM(e, 0))), plan->own(Py_NewRef(pr))});
+    const float* const gamma = norm_vector(PyTuple_GET_ITEM(pr, 0));
+    plan->norm.push_back({gamma, norm_vector(PyTuple_GET_ITEM(pr, 1))});
   }
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[7]); ++i) {
-    PyObject* o = PyTuple_GET_ITEM(a[7], i);
+    PyObject* const e = PyTuple_GET_ITEM(a[7], i);
+    PyObject* const o = PyTuple_GET_ITEM(e, 1);
+    plan->maxima.push_back({plan->own(Py_NewRef(PyTuple_GET_ITEM(e, 0))), plan->own(Py_NewRef(o))});
     plan->am.push_back(o == Py_None ? nullptr : f32(o, 1));
   }
-  if (a[8] != Py_None) {
+  if (a[8] != Py_None) {  // used as long as every block's projection is its part of it
     Operand w;
-    if (!read_operand(a[8], w) || w.rows != plan->blocks * plan->d) bad("stack_plan: bad batched positional projection");
-    plan->lp_all = plan->layer(w, nullptr);
+    bool parts = read_operand(a[8], w) && w.fmt == plan->fmt && w.k == plan->d && plan->blocks > 0 && w.rows == plan->blocks * plan->d;
+    for (int i = 0; parts && i < plan->blocks; ++i) {
+      const Lin& L = plan->lin[i * L_COUNT + L_LP];
+      const int64_t scale_bytes = static_cast<int64_t>(w.scales.nbytes()) / plan->blocks;
+      parts = !L.bias && L.ld == w.codes.stride(0) && L.codes == static_cast<uint8_t*>(w.codes.data_ptr()) + i * plan->d * L.ld &&
+              L.scales == static_cast<uint8_t*>(w.scales.data_ptr()) + i * scale_bytes;
+    }
+    if (parts) plan->lp_all = plan->layer(w, nullptr);
   }
   PyObject* cap = PyCapsule_New(plan.get(), "velox_stack_plan", plan_free);
   if (!cap) return nullptr;
-  plan->made_of = Py_NewRef(a[9]);
   plan.release();
   return cap;
   VX_END
@@ -875,30 +927,28 @@ PyObject* py_stack_plan_current(PyObject*, PyObject* const* a, Py_ssize_t nargs)
   const Plan* plan = static_cast<const Plan*>(PyCapsule_GetPointer(a[0], "velox_stack_plan"));
   if (!plan) return nullptr;
   if (static_cast<float>(as_double(a[4])) != plan->eps || as_bool(a[5]) != plan->fuse_ffn || as_long(a[6]) != plan->blocks ||
-      !plan->in_place())
+      plan->converted || !plan->in_place())
     Py_RETURN_FALSE;
-  PyObject* const in_layer[2] = {s_q, s_bias};
-  PyObject* const in_q[3] = {s_codes, has_sf(plan->fmt) ? s_sf : s_scales, s_amax};
+  auto held = [](PyObject* dict, PyObject* name) {
+    PyObject* now = PyDict_GetItemWithError(dict, name);
+    if (!now && PyErr_Occurred()) throw PyFail{};
+    return now ? now : Py_None;
+  };
   auto same = [](PyObject* o, PyObject* name, PyObject* was) {
     PyObject* v = PyObject_GetAttr(o, name);
     if (!v) throw PyFail{};
     Py_DECREF(v);
     return v == was;
   };
-  for (int part = 0; part < 3; ++part) {
-    PyObject* entries = PyTuple_GET_ITEM(plan->made_of, part);
-    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(entries); ++i) {
-      PyObject* e = PyTuple_GET_ITEM(entries, i);
-      PyObject* now = PyDict_GetItemWithError(a[1 + part], PyTuple_GET_ITEM(e, 0));
-      if (!now && PyErr_Occurred()) throw PyFail{};
-      if ((now ? now : Py_None) != PyTuple_GET_ITEM(e, 1)) Py_RETURN_FALSE;
-      if (part > 0) continue;
-      for (int k = 0; k < 2; ++k)
-        if (!same(now, in_layer[k], PyTuple_GET_ITEM(e, 2 + k))) Py_RETURN_FALSE;
-      for (int k = 0; k < 3; ++k)
-        if (!same(PyTuple_GET_ITEM(e, 2), in_q[k], PyTuple_GET_ITEM(e, 4 + k))) Py_RETURN_FALSE;
-    }
-  }
+  PyObject* const s_gemm_scales = has_sf(plan->fmt) ? s_sf : s_scales;
+  for (const Plan::Layer& y : plan->layers)
+    if (held(a[1], y.name) != y.layer || !same(y.layer, s_q, y.q) || !same(y.layer, s_bias, y.bias) || !same(y.q, s_codes, y.codes) ||
+        !same(y.q, s_gemm_scales, y.scales) || !same(y.q, s_amax, y.amax))
+      Py_RETURN_FALSE;
+  for (const Plan::Named& n : plan->norms)
+    if (held(a[2], n.name) != n.object) Py_RETURN_FALSE;
+  for (const Plan::Named& n : plan->maxima)
+    if (held(a[3], n.name) != n.object) Py_RETURN_FALSE;
   Py_RETURN_TRUE;
   VX_END
 }

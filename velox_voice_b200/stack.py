@@ -174,18 +174,15 @@ class ConformerLinearStack:
             layers.append("ctc")
             norms.append("after")
             amax = amax + ["after"] if self.fmt == FMT_NV16 else []
-            layers = tuple((n, l, l.q, l.bias, l.q.codes, l.q.gemm_scales(), l.q.amax) for n, l in ((n, self.p[n]) for n in layers))
+            layers = tuple((n, self.p[n]) for n in layers)
             norms = tuple((n, self.ln[n]) for n in norms)
             amax = tuple((n, self._amax(n, None)) for n in amax) + ((("pos", self.amax.get("pos")),) if amax else ())
-            self._plan = host.stack_plan(self.fmt, cfg.d_model, cfg.eps, self.fuse_ffn, cfg.blocks,
-                                         tuple(l[2:4] for l in layers),
-                                         tuple((g.float().contiguous(), b.float().contiguous()) for _, (g, b) in norms),
-                                         tuple(t for _, t in amax), self._lp_all(), (layers, norms, amax))
+            self._plan = host.stack_plan(self.fmt, cfg.d_model, cfg.eps, self.fuse_ffn, cfg.blocks, layers, norms, amax, self._positions)
         return self._plan
 
     def _stack_positions(self):
         """Lays the packed positional projections of all blocks behind one another, as one weight [blocks * d_model, d_model]
-        (short passes run them in one launch); the layers keep views of it.  Done here and not with the plan: a plan is made
+        (short passes run them in one launch, as long as every block's layer is its part of it); the layers keep views of it.  Done here and not with the plan: a plan is made
         in whichever pass comes first, on its stream or inside its graph capture, and a launch that reads constant weights
         ahead of the work before it must find them written."""
         cfg = self.cfg
@@ -201,24 +198,6 @@ class ConformerLinearStack:
                 setattr(self._positions, field, whole)
                 for q, part in zip(qs, whole.chunk(cfg.blocks)):
                     setattr(q, field, part)
-
-    def _lp_all(self):
-        """The stacked positional projections as long as every block's layer is its part of them, else None."""
-        whole, n = self._positions, self.cfg.blocks
-        if whole is None or whole.rows != n * self.cfg.d_model:
-            return None
-        for i in range(n):
-            layer = self.p[f"b{i}.lp"]
-            if layer.bias is not None:
-                return None
-            for field in ("codes", "scales", "sf"):
-                t, part = getattr(whole, field), getattr(layer.q, field)
-                if t is None and part is None:
-                    continue
-                if t is None or part is None or part.shape != (t.shape[0] // n, *t.shape[1:]) or \
-                        part.data_ptr() != t.data_ptr() + i * part.numel() * part.element_size():
-                    return None
-        return whole
 
     # ---- forward
     def forward(self, x: torch.Tensor, pos: Optional[torch.Tensor] = None, *, return_hidden: bool = False,
