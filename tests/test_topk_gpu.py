@@ -28,8 +28,9 @@ def _check(ops, a, b, bias, k):
 
 @pytest.mark.parametrize("N", [64, 264, 5538])
 @pytest.mark.parametrize("masked", ["first_piece", "lane", "all_but_16", "tail"])
-def test_masked_columns(ops, N, masked):
-    """A bias of -inf masks tokens.  The selection kernel reads 8 columns per lane and step of 256: masked are the first
+@pytest.mark.parametrize("by", [float("-inf"), torch.finfo(torch.bfloat16).min, -1e10])
+def test_masked_columns(ops, N, masked, by):
+    """A bias of -inf, of the lowest bf16 value or of some large negative one masks tokens.  The selection kernel reads 8 columns per lane and step of 256: masked are the first
     8, everything that lane 0 reads, all but 16 columns, everything from the second step on."""
     torch.manual_seed(N)
     M, K = 9, 512
@@ -38,8 +39,23 @@ def test_masked_columns(ops, N, masked):
     bias = torch.randn(N, device="cuda")
     col = torch.arange(N, device="cuda")
     mask = {"first_piece": col < 8, "lane": (col % 256) < 8, "all_but_16": (col % (N // 16)) != 3, "tail": col >= 256}[masked]
-    bias[mask] = float("-inf")
+    bias[mask] = by
     _check(ops, a, b, bias, 4)
+
+
+@pytest.mark.parametrize("by", [torch.finfo(torch.bfloat16).min, -1e10, -1e9])
+def test_rows_of_masked_columns_only(ops, by):
+    """Every logit is the same large negative value: log_softmax is -log N for each."""
+    M, N, K = 5, 520, 512
+    a = ops.quantize(torch.randn(M, K, device="cuda"), "mx32", natural=False)
+    b = ops.quantize(0.05 * torch.randn(N, K, device="cuda"), "mx32")
+    bias = torch.full((N,), by, device="cuda")
+    z = ops.bsgemm(a, b, epilogue=ops.EPI_BIAS, bias=bias, out_dtype=torch.bfloat16)
+    assert (z == z[0, 0]).all()
+    logp, ids = ops.bsgemm_topk(a, b, bias, 4)
+    assert torch.equal(ids, torch.arange(4, device="cuda").expand(M, 4))
+    # the log-sum-exp is an fp32 number of the logits' magnitude: half a unit in its last place
+    assert (logp + torch.log(torch.tensor(float(N)))).abs().max().item() <= max(2.0 ** -24 * abs(float(z[0, 0])), 1e-5)
 
 
 def test_per_16_format(ops):
