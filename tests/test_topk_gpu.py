@@ -43,6 +43,27 @@ def test_masked_columns(ops, N, masked, by):
     _check(ops, a, b, bias, 4)
 
 
+@pytest.mark.parametrize("masked", ["first_chunk", "second_chunk", "group", "half"])
+@pytest.mark.parametrize("by", [float("-inf"), torch.finfo(torch.bfloat16).min, -1e10])
+@pytest.mark.parametrize("N", [96, 1000, 5538])
+def test_log_sum_exp_of_the_arg_max_head_with_masked_columns(ops, N, masked, by):
+    """The epilogue sums 32 columns at a time and two such chunks per partial: masked are either chunk, a whole group of 64, and
+    every other chunk of the row."""
+    torch.manual_seed(N)
+    M, K = 140, 512
+    a = ops.quantize(torch.randn(M, K, device="cuda"), "mx32", natural=False)
+    b = ops.quantize(0.05 * torch.randn(N, K, device="cuda"), "mx32")
+    bias = torch.randn(N, device="cuda")
+    col = torch.arange(N, device="cuda")
+    bias[{"first_chunk": col < 32, "second_chunk": (col // 32) == 1, "group": col < 64, "half": (col // 32) % 2 == 0}[masked]] = by
+    ids, lse, logp = ops.bsgemm_argmax(a, b, bias, return_logp=True)
+    z = ops.bsgemm(a, b, epilogue=ops.EPI_BIAS, bias=bias, out_dtype=torch.bfloat16).double()
+    assert torch.equal(ids.long(), z.argmax(1))
+    want = torch.logsumexp(z, 1)  # (ex2 to 2 ulp, |lse| below 16, as above)
+    assert (lse.double() - want).abs().max().item() < 4e-5
+    assert (logp.double() - (z.max(1).values - want)).abs().max().item() < 4e-5
+
+
 @pytest.mark.parametrize("by", [torch.finfo(torch.bfloat16).min, -1e10, -1e9])
 def test_rows_of_masked_columns_only(ops, by):
     """Every logit is the same large negative value: log_softmax is -log N for each."""

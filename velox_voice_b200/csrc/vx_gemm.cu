@@ -1455,13 +1455,22 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
               // log-sum-exp of the bf16-rounded logits, streaming: the chunk's sum relative to its maximum,
               // merged into the running pair of this 64-column group
               constexpr float L2E = 1.4426950408889634f;
-              const float nb2 = -cm * L2E;
-              float cs = 0.0f;
+              if (cm > -INFINITY) {  // (32 columns masked by -inf add nothing; their sum would be of -inf + inf)
+                const float nb2 = -cm * L2E;
+                float cs = 0.0f;
 #pragma unroll
-              for (int i = 0; i < 32; ++i) cs += ex2_ftz(fmaf(zr[i], L2E, nb2));
-              const float nm = fmaxf(lse_m, cm);
-              lse_s = lse_s * ex2_ftz((lse_m - nm) * L2E) + cs * ex2_ftz((cm - nm) * L2E);
-              lse_m = nm;
+                for (int i = 0; i < 32; ++i) cs += ex2_ftz(fmaf(zr[i], L2E, nb2));
+                // (32 columns masked by a large negative value: the rounding of cm log2 e is no longer small against 1, or the
+                // product overflows, and cs is not the sum of 1 to 32 ones: formed again from the exact differences)
+                if (!(cs >= 0.5f && cs <= 64.0f)) {
+                  cs = 0.0f;
+#pragma unroll
+                  for (int i = 0; i < 32; ++i) cs += ex2_ftz((zr[i] - cm) * L2E);
+                }
+                const float nm = fmaxf(lse_m, cm);
+                lse_s = lse_s * ex2_ftz((lse_m - nm) * L2E) + cs * ex2_ftz((cm - nm) * L2E);
+                lse_m = nm;
+              }
               if (TOPK && row_ok) {
                 // candidate pass of the top-k: append every logit of this chunk that reaches the row's threshold
                 // (few chunks of a row hold one; the chunk maximum decides whether to look at all)
