@@ -69,3 +69,16 @@ def test_the_wait_for_the_other_ctas_sums_acquires_at_cluster_scope():
     text = source("vx_gemm_ln.cu")
     assert re.findall(r"mbar_wait\w*\(&sm\.xch", text) == ["mbar_wait_spin_cluster(&sm.xch"]
     assert "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64" in source("vx_ptx.cuh")
+
+
+def test_what_writes_weights_does_not_trigger_the_next_launch():
+    """A GEMM may read a constant weight and its scale factors ahead of its wait, and the launches between may all have triggered
+    before their own: the kernels that write them must not.  (Scale factors of a single operand are a weight's: PackedLinear, or
+    a C caller before VX_GEMM_CONST_B.)"""
+    text = source("vx_quant.cu")
+    body = text[text.index("sf_relayout_kernel(RelayoutSide"):]
+    body = body[:body.index("pdl_wait()")]
+    assert re.findall(r"[^\n]*pdl_launch_dependents\(\);", body) == ["  if (early) pdl_launch_dependents();"]
+    pair = text[text.index("int vx_sf_from_natural_pair("):]
+    assert re.search(r"launch_dependent\(sf_relayout_kernel.*?side\[1\]\.words != 0 \? 1 : 0\)\)", pair, re.S)
+    assert "vx_sf_from_natural_pair(fmt, scales, R, scales_sf, fmt, nullptr, 0, nullptr, K, stream)" in pair

@@ -932,8 +932,9 @@ struct RelayoutSide {
   int64_t R, words;  // rows, 4-byte words of all atoms
   int fmt;
 };
-__global__ void __launch_bounds__(256) sf_relayout_kernel(RelayoutSide a, RelayoutSide b, int nkb, int sf_kg) {
-  pdl_launch_dependents();
+// early: the scales of both operands of a product that follows; those of one operand may be a weight's (see launch_dependent)
+__global__ void __launch_bounds__(256) sf_relayout_kernel(RelayoutSide a, RelayoutSide b, int nkb, int sf_kg, int early) {
+  if (early) pdl_launch_dependents();
   pdl_wait();
   const int64_t total = a.words + b.words;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -1208,7 +1209,7 @@ int vx_sf_from_natural_pair(int fmt_a, const void* scales_a, int64_t Ra, void* s
   int64_t grid = (words + 255) / 256;
   if (grid > 148 * 8) grid = 148 * 8;
   VX_CUDA_OK(launch_dependent(sf_relayout_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, static_cast<cudaStream_t>(stream), side[0],
-                              side[1], static_cast<int>(K / fmt_block(fmt_a)), static_cast<int>(sf_kgroups(fmt_a, K))));
+                              side[1], static_cast<int>(K / fmt_block(fmt_a)), static_cast<int>(sf_kgroups(fmt_a, K)), side[1].words != 0 ? 1 : 0));
   return 0;
 }
 
