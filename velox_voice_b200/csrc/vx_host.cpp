@@ -657,6 +657,7 @@ PyObject* py_power_mel_log(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
 // issues every launch of the pass; its intermediate tensors live in one workspace block.
 struct Lin {
   const void* codes; int64_t ld; const void* scales; const float* amax; const float* bias; int64_t N, K;
+  int flags;  // VX_GEMM_CONST_B for what PackedLinear packs: see PackedLinear._const
 };
 struct Norm { const float *g, *b; };
 enum { L_FFM1, L_FFM2, L_QKV, L_LO, L_LP, L_PW1, L_PW2, L_FF1, L_FF2, L_COUNT };
@@ -701,9 +702,9 @@ struct Plan {
       if (k.t.data_ptr() != k.ptr || k.t.numel() != k.numel || row_stride(k.t) != k.ld) return false;
     return true;
   }
-  Lin layer(const Operand& w, const float* bias) {
+  Lin layer(const Operand& w, const float* bias, int flags) {
     for (const at::Tensor& t : {w.codes, w.scales, w.amax}) keep(t);
-    return {w.codes.data_ptr(), w.codes.stride(0), w.scales.data_ptr(), f32_ptr(w.amax), bias, w.rows, w.k};
+    return {w.codes.data_ptr(), w.codes.stride(0), w.scales.data_ptr(), f32_ptr(w.amax), bias, w.rows, w.k, flags};
   }
   const float* amax(size_t i) const { return am.empty() ? nullptr : am[i]; }
 };
@@ -752,7 +753,7 @@ struct Pass {
     d.a_scales = a.scales; d.b_scales = w.scales;
     d.a_amax = a.amax; d.b_amax = w.amax;
     d.epilogue = epi == VX_EPI_BIAS && !w.bias ? VX_EPI_NONE : epi;
-    d.flags = VX_GEMM_CONST_B;
+    d.flags = w.flags;
     d.bias = w.bias;
     return d;
   }
@@ -883,7 +884,8 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (l == L_FFM1 || l == L_FF1) plan->ffn = std::max(plan->ffn, w.rows);
     if (l == L_PW1) plan->glu = std::max(plan->glu, w.rows / 2);
     if (head) plan->vocab = w.rows;
-    plan->lin.push_back(plan->layer(w, y.bias == Py_None ? nullptr : f32(y.bias, w.rows)));
+    const bool packed = plan->own(PyObject_GetAttr(y.q, s_scales)) != Py_None;
+    plan->lin.push_back(plan->layer(w, y.bias == Py_None ? nullptr : f32(y.bias, w.rows), packed ? VX_GEMM_CONST_B : 0));
     plan->layers.push_back(y);
   }
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[6]); ++i) {
@@ -909,7 +911,7 @@ PyObject* py_stack_plan(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       parts = !L.bias && L.ld == w.codes.stride(0) && L.codes == static_cast<uint8_t*>(w.codes.data_ptr()) + i * plan->d * L.ld &&
               L.scales == static_cast<uint8_t*>(w.scales.data_ptr()) + i * scale_bytes;
     }
-    if (parts) plan->lp_all = plan->layer(w, nullptr);
+    if (parts) plan->lp_all = plan->layer(w, nullptr, VX_GEMM_CONST_B);
   }
   PyObject* cap = PyCapsule_New(plan.get(), "velox_stack_plan", plan_free);
   if (!cap) return nullptr;

@@ -74,6 +74,12 @@ class PackedLinear:
         self.q: Quantized = ops.quantize(w.contiguous(), self.fmt_b, natural=True, sf=True, amax_t=weight_amax)
         self.bias = None if b is None else b.contiguous()
 
+    def _const(self) -> int:
+        """GEMM flag for a weight that may be read under the tail of the launches before: what the constructor packs.  A program
+        may assign another ``q``; one without natural-layout scales comes from a quantizer that lets the next launch start
+        before it has written its output."""
+        return GEMM_CONST_B if self.q.scales is not None else 0
+
     def forward(self, a: Quantized, *, act: Optional[str] = None, residual: Optional[torch.Tensor] = None,
                 alpha: float = 1.0, out_dtype=torch.bfloat16, out: Optional[torch.Tensor] = None,
                 out_fmt=None, out_amax: Optional[torch.Tensor] = None):
@@ -88,7 +94,7 @@ class PackedLinear:
         else:
             epi = EPI_NONE
         r = ops._host().bsgemm(a, self.q, epi, self.bias, residual, alpha, out_dtype, out,
-                               None if out_fmt is None else ops._fmt(out_fmt), out_amax, False, GEMM_CONST_B)
+                               None if out_fmt is None else ops._fmt(out_fmt), out_amax, False, self._const())
         if r is not None:
             return r
         return ops.bsgemm(a, self.q, epilogue=epi, bias=self.bias, residual=residual, alpha=alpha,
@@ -106,7 +112,7 @@ class PackedLinear:
         """``x = alpha (a W^T + bias) + residual`` and ``ln_quantize(x, gamma, beta, eps)`` in one launch:
         ``(x, q)`` with the bits of the two separate calls.  With ``gamma2`` / ``beta2``: ``(LN(x), q)`` with
         ``q = ln_quantize(LN(x), gamma2, beta2)`` -- the end of a block (``ops.ln2_quantize``)."""
-        r = ops._host().residual_ln(a, self.q, self.bias, residual, gamma, beta, eps, alpha, out, gamma2, beta2, GEMM_CONST_B)
+        r = ops._host().residual_ln(a, self.q, self.bias, residual, gamma, beta, eps, alpha, out, gamma2, beta2, self._const())
         if r is not None:
             return r
         return ops.bsgemm_residual_ln(a, self.q, bias=self.bias, residual=residual, gamma=gamma, beta=beta,
