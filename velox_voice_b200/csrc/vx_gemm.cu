@@ -2152,7 +2152,7 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
     const int64_t stages = (K / 2 + STAGE_ROW_BYTES - 1) / STAGE_ROW_BYTES;
     const int64_t wide_tiles = ((M + BM - 1) / BM) * ((N + 255) / 256);
     bool narrow = stages <= 2 && epi != VX_EPI_BIAS_SWISH && epi != VX_EPI_BIAS_GLU &&
-                  (epi == VX_EPI_BIAS_RESIDUAL || wide_tiles < 148);
+                  (epi == VX_EPI_BIAS_RESIDUAL || wide_tiles < sm_count());
     // Few rows (a shard of a job cut over several GPUs): CTAs own column blocks and walk the row
     // blocks in rounds of sms / column-blocks, so what counts is the number of rounds times the cost of
     // a tile -- a narrow tile costs about 0.55 of a wide one.  88 row blocks, N = 512: the wide tiling

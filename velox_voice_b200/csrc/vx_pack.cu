@@ -87,7 +87,7 @@ extern "C" int vx_qkv_pack(const void* qkv, int64_t ld_qkv, const void* p0, int6
     if (reinterpret_cast<uintptr_t>(p) & 15) return fail(-1, "pointers must be 16-byte aligned");
   const int64_t total = static_cast<int64_t>(heads) * T * (head_dim >> 3);
   int64_t blocks = (total + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
+  if (blocks > sm_count() * 16) blocks = sm_count() * 16;
   qkv_pack_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(qkv), ld_qkv, static_cast<const __nv_bfloat16*>(p0), ld_p0,
       static_cast<const __nv_bfloat16*>(pos_u), static_cast<const __nv_bfloat16*>(pos_v), scale, T, heads, head_dim,

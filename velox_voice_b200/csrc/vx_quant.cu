@@ -1207,7 +1207,7 @@ int vx_sf_from_natural_pair(int fmt_a, const void* scales_a, int64_t Ra, void* s
   const int64_t words = side[0].words + side[1].words;
   if (words == 0) return 0;
   int64_t grid = (words + 255) / 256;
-  if (grid > 148 * 8) grid = 148 * 8;
+  if (grid > sm_count() * 8) grid = sm_count() * 8;
   VX_CUDA_OK(launch_dependent(sf_relayout_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, static_cast<cudaStream_t>(stream), side[0],
                               side[1], static_cast<int>(K / fmt_block(fmt_a)), static_cast<int>(sf_kgroups(fmt_a, K)), side[1].words != 0 ? 1 : 0));
   return 0;
