@@ -393,8 +393,8 @@ def test_wide_and_narrow_tiles_give_the_same_bytes(ops, fmt, M, N, K, epi):
 @pytest.mark.parametrize("fmt", [F.FMT_MX32, F.FMT_NV16])
 @pytest.mark.parametrize("M,k", [(300, 5), (1, 1), (129, 8), (2000, 16)])
 def test_ctc_topk_without_logits(ops, fmt, M, k):
-    """torch.topk(log_softmax(bf16 logits), k) from two launches of the head and two small kernels, no [M, N]
-    matrix: values within 1e-3 (the log-sum-exp is summed in another order), ids equal wherever the k-th and
+    """torch.topk(log_softmax(bf16 logits), k) from a launch of the head and one of the selection kernel per block of rows, no
+    [M, N] matrix: values within 1e-3 (the log-sum-exp is summed in another order), ids equal wherever the k-th and
     (k+1)-th logits differ (equal bf16 logits may come in either order from torch.topk; here: lowest column first)."""
     torch.manual_seed(M + k)
     N, K = 5538, 512
@@ -418,8 +418,8 @@ def test_ctc_topk_without_logits(ops, fmt, M, k):
 
 
 def test_ctc_topk_overflowing_rows_fall_back_to_logits(ops):
-    """All-equal logits: every column reaches the threshold, the candidate lists overflow, and the rows are redone
-    from explicit logits."""
+    """All-equal logits: every column reaches the threshold, far more than k and than the `capacity` that is accepted for
+    callers of an earlier route."""
     M, N, K = 40, 512, 256
     x = torch.zeros(M, K, device="cuda").bfloat16()
     w = torch.randn(N, K, device="cuda").bfloat16()

@@ -20,8 +20,9 @@
 //               buffer + TMA store (clipped at the tensor edge by hardware) or direct vector
 //               stores; optional re-quantization of the result to FP4.  Sixteen warps (four
 //               per scheduler) hide the TMEM-load, shared-memory and MUFU latencies of each other.
-// FP4: a 128 x 256 tile with one accumulator, drained into registers right after the commit,
-// or a 128 x 128 tile with two accumulators (epilogue of tile i under the MMAs of tile i + 1).
+// FP4: tiles of 128 x 256 or 128 x 128 on a ring of two or three 128-column accumulators, each
+// published and handed back by itself, so the MMAs run ahead of the epilogue; the wide tile of the
+// residual, GLU and arg-max epilogues is one 256-column accumulator, read right after its commit.
 // FP8: rounds of four K blocks into four accumulators, published per round and handed back in
 // pairs, so the MMAs of the next round run while the epilogue promotes.
 //
@@ -67,9 +68,9 @@ constexpr int FP8_SB_BYTES_PER_KB = 16 * 32 * 4;  // epilogue tables of B scales
 constexpr int TM_ACC0 = 0, TM_COLS = 512;
 __host__ __device__ constexpr int tm_sfa_col(int accs) { return accs == 3 ? 384 : 256; }
 
-// FP4 kinds come in two tile shapes: 128 x 256 with one accumulator (fewest MMA instructions
-// and least operand traffic per output) and 128 x 128 with two accumulators (the epilogue of
-// tile i overlaps the MMAs of tile i + 1; best when K is short and B stays in shared memory).
+// FP4 kinds come in two tile shapes: 128 x 256 (fewest MMA instructions and least operand traffic
+// per output) and 128 x 128 (more tiles, and always on the ring of 128-column accumulators, see
+// UNITS; best when K is short and B stays in shared memory).
 enum Kind { KIND_FP4_VEC2 = 0, KIND_FP4_VEC4 = 1, KIND_FP8 = 2, KIND_FP4_VEC2_N128 = 3, KIND_FP4_VEC4_N128 = 4 };
 // rows of B per tile = accumulator columns
 __host__ __device__ constexpr int kind_bn(int kind) {
@@ -594,9 +595,8 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   constexpr int VEC = kind_vec4(KIND) ? 4 : 2;
   constexpr int APS = kind_vec4(KIND) ? 4 : 2;  // SF atoms per 128 rows per stage
   constexpr bool GLU = (EPI == VX_EPI_BIAS_GLU);
-  // FP4 wide: one 128 x 256 accumulator (a single N = 256 MMA does twice the work per issued
-  // instruction).  FP4 narrow: two 128 x 128 accumulators.  FP8: 128 x 128, four accumulators,
-  // one per 128-wide K block of a round.
+  // FP4 wide: one 128 x 256 accumulator, or its two halves in the ring (SEQ below).  FP4 narrow: 128 x 128 accumulators in the
+  // ring.  FP8: 128 x 128, four accumulators, one per 128-wide K block of a round.
   constexpr bool WIDE = kind_bn(KIND) == 256;
   constexpr int BNT = kind_bn(KIND);         // accumulator columns = B rows per tile
   constexpr int NRT = BNT / 128;             // 128-row scale-factor tiles of B per tile
@@ -2142,10 +2142,10 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
   const bool vec2 = fmt == VX_FMT_ROWSCALE || fmt == VX_FMT_MX32;
   int kind = fp8 ? KIND_FP8 : (vec2 ? KIND_FP4_VEC2 : KIND_FP4_VEC4);
   if (!fp8) {
-    // Two 128-wide accumulators overlap the epilogue of one tile with the MMAs of the next.
-    // Measured at M = 90000, K = 512: that wins for the residual epilogue (N = 512: 52 vs
-    // 57 us) and loses where the output is wide (N = 1536: 83 vs 78 us; N = 5538 argmax: 388 vs
-    // 327 us), because every 128-wide column block re-reads A.  It also wins whenever the
+    // Narrow tiles overlap the residual epilogue with the MMAs of the next tile, which the wide tile's one accumulator
+    // does not.  Measured at M = 90000, K = 512: that wins for the residual epilogue (N = 512: 44.0 vs
+    // 50.2 us) and loses where the output is wide (plain bias, where both ring their accumulators: N = 1536 66.6 vs 64.5 us,
+    // N = 5538 248.8 vs 239.6 us), because every 128-wide column block re-reads A.  It also wins whenever the
     // wide tiling would leave SMs without a tile.  Swish (bound by its own epilogue
     // arithmetic) and GLU (weights interleaved per 256 rows) stay on the wide tile, and so
     // does a long K, where the wide tile halves the re-reads of A.

@@ -157,7 +157,8 @@ __global__ void __launch_bounds__(LN_THREADS, 1)
 bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                           const __grid_constant__ CUtensorMap tmap_res, const __grid_constant__ CUtensorMap tmap_out,
                           const LnParams p) {
-  // (no early trigger: with one, 1 in 30 passes over 24,000 frames had a 32-row block that a later launch had read too early)
+  // (No early trigger of the next launch: 24,000 frames take 1 % less with one.  The 32-row blocks that differed in passes with it
+  // came from the staged stores of bsgemm_kernel, see store_count there; it has not been tried since that was mended.)
   extern __shared__ uint8_t smem_raw[];
   // (the same offset in both CTAs of the cluster: map_to_cta relies on it)
   LnSmem& sm = *reinterpret_cast<LnSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));

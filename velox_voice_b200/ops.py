@@ -387,8 +387,8 @@ def bsgemm(
     ``out_fmt`` (MX32 or NV16) re-quantizes the result in the epilogue and returns a
     :class:`Quantized` ready to be the A operand of the next GEMM; otherwise a tensor of
     ``out_dtype`` (float32 / bfloat16) [M, N] ([M, N/2] for the GLU epilogue) is returned.
-    ``tiles`` overrides the FP4 tile shape the library would pick ("wide" 128 x 256, one
-    accumulator; "narrow" 128 x 128, two accumulators); results do not depend on it.
+    ``tiles`` overrides the FP4 tile shape the library would pick ("wide" 128 x 256,
+    "narrow" 128 x 128); results do not depend on it.
     """
     if not (direct_store or stream_b or tiles):
         r = (_native or _host()).bsgemm(a, b, epilogue, bias, residual, alpha, out_dtype, out,
