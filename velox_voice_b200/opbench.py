@@ -75,7 +75,9 @@ def op_breakdown(stack, T, fmt_name, only=""):
         T * d * 2 + qbytes(T, d), 0)
     add("ln2_quantize [T,512] (norm_final + next LayerNorm + quantize)", 0 if fused else nb,
         lambda: ops.ln2_quantize(x, g, b, g, b, cfg.eps, fmt, y=x, amax_t=am), T * d * 4 + qbytes(T, d), 0)
-    add("quantize [T,512]", 2 * nb + 1, lambda: ops.quantize(x, fmt, natural=fmt_name == "fp8_1x128", amax_t=am),
+    # (FP4: a step quantizes the value third of q | k | v and the GLU output in their GEMMs' epilogues)
+    fp4 = fmt_name != "fp8_1x128"
+    add("quantize [T,512]", 1 if fp4 else 2 * nb + 1, lambda: ops.quantize(x, fmt, natural=fmt_name == "fp8_1x128", amax_t=am),
         T * d * 2 + qbytes(T, d), 0)
     w1, w2 = stack.p["b0.ffm.w1"], stack.p["b0.ffm.w2"]
     if stack.fuse_ffn:
@@ -107,8 +109,13 @@ def op_breakdown(stack, T, fmt_name, only=""):
     add("gemm lo/pw2 512->512 +residual", 0 if fused else 2 * nb, lambda: stack.p["b0.lo"](xq, residual=res, alpha=1.0, out=res),
         qbytes(T, d) + qbytes(d, d) + T * d * 4, 2 * T * d * d)
     add("gemm lp 512->512", nb, lambda: stack.p["b0.lp"](xq), qbytes(T, d) + qbytes(d, d) + T * d * 2, 2 * T * d * d)
-    add("gemm pw1 512->1024 GLU", nb, lambda: stack.p["b0.pw1"](xq), qbytes(T, d) + qbytes(2 * d, d) + T * d * 2,
-        2 * T * d * 2 * d)
+    if fp4:
+        glu_am = stack.amax.get("b0.glu")
+        add("gemm pw1 512->1024 GLU, FP4 out", nb, lambda: stack.p["b0.pw1"](xq, out_fmt=fmt, out_amax=glu_am),
+            qbytes(T, d) + qbytes(2 * d, d) + qbytes(T, d), 2 * T * d * 2 * d)
+    else:
+        add("gemm pw1 512->1024 GLU", nb, lambda: stack.p["b0.pw1"](xq), qbytes(T, d) + qbytes(2 * d, d) + T * d * 2,
+            2 * T * d * 2 * d)
     add("gemm ctc 512->5538 bias + argmax (no logits written)", 1, lambda: stack.p["ctc"].argmax(xq),
         qbytes(T, d) + qbytes(V, d) + T * 12, 2 * T * d * V)
     if only and "mel" in only:
