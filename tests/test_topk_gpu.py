@@ -64,7 +64,7 @@ def test_log_sum_exp_of_the_arg_max_head_with_masked_columns(ops, N, masked, by)
     assert (logp.double() - (z.max(1).values - want)).abs().max().item() < 4e-5
 
 
-@pytest.mark.parametrize("by", [torch.finfo(torch.bfloat16).min, -1e10, -1e9])
+@pytest.mark.parametrize("by", [torch.finfo(torch.bfloat16).min, -1e10, -1e9, -1e8])
 def test_rows_of_masked_columns_only(ops, by):
     """Every logit is the same large negative value: log_softmax is -log N for each."""
     M, N, K = 5, 520, 512
@@ -75,6 +75,9 @@ def test_rows_of_masked_columns_only(ops, by):
     assert (z == z[0, 0]).all()
     logp, ids = ops.bsgemm_topk(a, b, bias, 4)
     assert torch.equal(ids, torch.arange(4, device="cuda").expand(M, 4))
+    first, lse, best = ops.bsgemm_argmax(a, b, bias, return_logp=True)
+    assert (first == 0).all() and torch.isfinite(best).all()
+    assert (lse.double() - torch.logsumexp(z.double(), 1)).abs().max().item() <= 2.0 ** -23 * abs(float(z[0, 0]))
     # the log-sum-exp is an fp32 number of the logits' magnitude: half a unit in its last place
     assert (logp + torch.log(torch.tensor(float(N)))).abs().max().item() <= max(2.0 ** -24 * abs(float(z[0, 0])), 1e-5)
 
