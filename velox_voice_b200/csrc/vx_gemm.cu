@@ -630,7 +630,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   const int out_fmt = OUT == 2 || OUT == 4 ? static_cast<int>(kind_vec4(KIND) ? VX_FMT_NV16 : VX_FMT_MX32) : p.out_fmt;
   const bool tr_on = kPhaseTrace && p.trace != nullptr && blockIdx.x == 0;  // phase trace requested (CTA 0 only)
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   // (The waits below take no abort flag: a flag that the roles poll was built and measured -- the
   // extra exits from every wait loop cost the 96-register epilogues spills, the fused-QKV kernel went

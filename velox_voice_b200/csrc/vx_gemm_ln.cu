@@ -162,7 +162,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   extern __shared__ uint8_t smem_raw[];
   // (the same offset in both CTAs of the cluster: map_to_cta relies on it)
   LnSmem& sm = *reinterpret_cast<LnSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();  // column half of this CTA
   const int cluster = static_cast<int>(blockIdx.x >> 1), nclusters = static_cast<int>(gridDim.x >> 1);
   const int my_tiles = cluster < p.m_tiles ? (p.m_tiles - cluster + nclusters - 1) / nclusters : 0;
