@@ -292,6 +292,49 @@ int vx_ctc_topk_finish(const void* candidates, const int32_t* count, int capacit
 int64_t vx_ctc_topk_rows(int64_t N);
 int vx_ctc_topk(const vx_gemm_desc* desc, int k, void* logits, int64_t rows, float* logp, int64_t* ids, void* stream);
 
+/* All layers of a run of Conformer blocks in one launch, for passes of few frames: what
+ *   for every block (veloxvoice/models/wenet/torch_conformer.py:705-713, linears, LayerNorms and quantizers only)
+ *     x += 0.5 w2(swish(w1(LN_ffm(x))));  q|k|v = qkv(LN_mha(x));  x += lo(v);  x += pw2(glu(pw1(LN_conv(x))));
+ *     x += 0.5 w2(swish(w1(LN_ff(x))));   x = LN_final(x)
+ * followed by the LayerNorm `after` and the quantizer in front of the head does, with the bits of the separate
+ * entry points above (vx_ln_quantize_pack, vx_bsgemm with its quantizing epilogues, vx_ln2_quantize_pack), MX32.
+ * d_model 512, a GLU of 512 outputs, ffn 1,024 or 2,048, 1 to 16 blocks: vx_conformer_pass_supported.
+ * Each row block of 128 frames runs on a cluster of CTAs that passes the activations on without a launch between layers;
+ * vx_conformer_pass_frames() is the number of frames up to which that is faster than the separate launches on the current device
+ * (0: it has no room for such clusters).
+ *   lin: E2M1 codes u8 [N, K/2] (row stride ld bytes), scale-factor atoms, bias f32 [N] (16-byte aligned), in the order
+ *        ffm.w1, ffm.w2, qkv, lo, pw1 (rows interleaved per vx_glu_tile), pw2, ff.w1, ff.w2;
+ *   gamma, beta: f32 [512], 16-byte aligned, of LN_ffm, LN_mha, LN_conv, LN_ff, LN_final;
+ *   const_weights: nonzero when no launch just before this one writes the weights (VX_GEMM_CONST_B of every GEMM);
+ *   src: features bf16 [M, 512]; x: the residual stream after the last block, bf16 [M, 512] (may be src);
+ *   qkv: bf16 [M, 1536], left with the last block's q | k | v; scratch: vx_conformer_pass_scratch(M, ffn) bytes;
+ *   codes u8 [M, 256], scales_sf: quantize(LN_after(x)) as vx_ln_quantize_pack leaves it. */
+#define VX_PASS_LINEARS 8
+typedef struct { const void* codes; int64_t ld; const void* scales_sf; const float* bias; } vx_pass_linear;
+typedef struct { vx_pass_linear lin[VX_PASS_LINEARS]; const float* gamma[5]; const float* beta[5]; } vx_pass_block;
+typedef struct {
+  int32_t struct_size;  /* sizeof(vx_pass_desc) */
+  int32_t blocks;
+  int64_t M, ffn;
+  float eps;
+  int32_t const_weights;
+  const vx_pass_block* block;
+  const float* after_gamma;
+  const float* after_beta;
+  const void* src;
+  int64_t ld_src;
+  void* x;
+  int64_t ldx;
+  void* qkv;
+  void* scratch;
+  void* codes;
+  void* scales_sf;
+} vx_pass_desc;
+int vx_conformer_pass_supported(int fmt, int64_t d_model, int64_t ffn, int64_t conv_pw, int64_t blocks);
+int64_t vx_conformer_pass_frames(void);
+int64_t vx_conformer_pass_scratch(int64_t M, int64_t ffn);
+int vx_conformer_pass(const vx_pass_desc* desc, void* stream);
+
 /* Attention fold pack in one pass: replaces velox_qkv_pack
  * (veloxvoice/kernels/csrc/velox_qkv_pack.cu:34-97; Python wrapper qkv_pack in
  * veloxvoice/kernels/ops/cuda_ops.py:554-581), i.e. the torch fold chain of

@@ -1,0 +1,27 @@
+"""The one-launch pass: argument checks without a device, and the rule for waits in front of warp-wide tensor-memory accesses."""
+
+import ctypes as C
+
+from test_device_sources_cpu import test_waits_before_warp_wide_tensor_memory_accesses_end_in_a_vote as vote_rule
+from velox_voice_b200 import _lib
+
+
+def test_arguments_are_checked_before_any_launch():
+    lib = _lib.load()
+    assert lib.vx_conformer_pass(None, None) == -1
+    desc = (C.c_int32 * 64)()
+    desc[0] = 8  # struct_size
+    assert lib.vx_conformer_pass(C.cast(desc, C.c_void_p), None) == -1 and b"struct_size" in lib.vx_last_error()
+
+
+def test_shapes_it_covers():
+    ok = _lib.load().vx_conformer_pass_supported
+    assert ok(_lib.FMT_MX32, 512, 2048, 1024, 12) == 1 and ok(_lib.FMT_MX32, 512, 1024, 1024, 16) == 1
+    for args in ((_lib.FMT_NV16, 512, 2048, 1024, 12), (_lib.FMT_MX32, 256, 2048, 1024, 12), (_lib.FMT_MX32, 512, 1536, 1024, 12),
+                 (_lib.FMT_MX32, 512, 4096, 1024, 12), (_lib.FMT_MX32, 512, 2048, 512, 12), (_lib.FMT_MX32, 512, 2048, 1024, 17),
+                 (_lib.FMT_MX32, 512, 2048, 1024, 0)):
+        assert ok(*args) == 0
+
+
+def test_waits_end_in_a_vote():
+    vote_rule("vx_pass.cu", "conformer_pass_kernel(")

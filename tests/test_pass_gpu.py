@@ -1,0 +1,107 @@
+"""All blocks of a short pass in one launch (``vx_pass.cu``) against the separate launches, bit for bit."""
+
+import pytest
+import torch
+
+from test_stack_routes_gpu import build
+
+pytestmark = pytest.mark.gpu
+
+
+def both(stack, x, pos=None, **kw):
+    """(logits, hidden) by the one launch and by separate launches, and the launches of each."""
+    from velox_voice_b200 import _lib, ops
+
+    limit, out = stack.one_launch_frames, []
+    for frames in (limit, 0):
+        stack.one_launch_frames = frames
+        ops.reset_launch_count()
+        out.append((*stack.forward(x.clone(), pos, return_hidden=True, **kw), ops.launch_count()))
+    stack.one_launch_frames = limit
+    assert _lib.device_status() == 0
+    return out
+
+
+# row blocks of 128: their edges, one and several clusters, the widest pass of eight-CTA clusters or beyond it, the longest pass
+@pytest.mark.parametrize("T", [1, 127, 128, 129, 1000, 1800, 2047, 2500, None])
+@pytest.mark.parametrize("ffn", [2048, 1024])
+def test_one_launch_has_the_bits_of_the_separate_ones(T, ffn):
+    stack = build(blocks=2, ffn=ffn)
+    T = stack.one_launch_frames if T is None else T
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, 512, generator=g, device="cuda").bfloat16()
+    x[T // 2] = 0.0                      # a row without variance
+    x[T // 3] *= 1e4
+    (got, h, n1), (want, hidden, n0) = both(stack, x)
+    assert torch.equal(got, want) and torch.equal(h, hidden)
+    assert n1 == 2 and n0 > 20           # the blocks, the head
+
+
+@pytest.mark.parametrize("blocks", [1, 16, 17])
+def test_number_of_blocks(blocks):
+    stack = build(blocks=blocks, vocab=64)
+    x = torch.randn(200, 512, device="cuda").bfloat16()
+    (got, h, n1), (want, hidden, n0) = both(stack, x)
+    assert torch.equal(got, want) and torch.equal(h, hidden) and (n1 == n0) == (blocks == 17)
+
+
+def test_rows_that_are_not_finite_stay_to_themselves():
+    stack = build(blocks=2)
+    x = torch.randn(300, 512, device="cuda").bfloat16()
+    clean = stack.forward(x.clone())
+    x[5, 7], x[140, 0], x[299, 511] = float("nan"), float("inf"), float("-inf")
+    got = stack.forward(x.clone())
+    keep = torch.ones(300, dtype=torch.bool, device="cuda")
+    keep[[5, 140, 299]] = False
+    assert torch.equal(got[keep], clean[keep])
+
+
+@pytest.mark.parametrize("offset,pitch", [(8, 528), (4, 520), (0, 516)])
+def test_rows_of_any_address_and_pitch(offset, pitch):
+    """Rows of 16-byte pieces take the one launch; what others do is what the separate launches do."""
+    stack = build(blocks=1)
+    x = torch.randn(150, 512, device="cuda").bfloat16()
+    limit, out = stack.one_launch_frames, []
+    for stack.one_launch_frames in (limit, 0):
+        wide = torch.zeros(150 * pitch + offset, device="cuda", dtype=torch.bfloat16)
+        view = wide[offset:].view(150, pitch)[:, :512]
+        view.copy_(x)
+        try:
+            out.append(stack.forward(view).clone())
+        except Exception as e:
+            out.append(str(e))
+    assert torch.equal(*out) if torch.is_tensor(out[0]) else out[0] == out[1]
+    if offset % 8 == 0 and pitch % 8 == 0:
+        assert torch.equal(out[0], stack.forward(x.clone()))
+
+
+def test_a_layer_without_bias_runs_separately():
+    from velox_voice_b200 import ops
+    from velox_voice_b200._lib import VeloxError
+
+    stack = build(blocks=1)
+    x = torch.randn(150, 512, device="cuda").bfloat16()
+    want = stack.forward(x.clone())
+    odd = torch.zeros(513, device="cuda")[1:]
+    odd.copy_(stack.p["b0.lo"].bias)
+    stack.p["b0.lo"].bias = odd
+    with pytest.raises(VeloxError, match="16-byte aligned"):  # as the separate launches refuse it
+        stack.forward(x.clone())
+    stack.p["b0.lo"].bias = None
+    ops.reset_launch_count()
+    assert not torch.equal(stack.forward(x.clone()), want) and ops.launch_count() > 10
+
+
+def test_passes_on_two_streams():
+    stack = build(blocks=3)
+    xs = [torch.randn(T, 512, device="cuda").bfloat16() for T in (375, 1300)]
+    want = [stack.forward(x.clone()) for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    got = [[], []]
+    for _ in range(20):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(stack.forward(xs[i].clone()))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want[i]) for i in range(2) for o in got[i])

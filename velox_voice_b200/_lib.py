@@ -69,6 +69,10 @@ EXPORTS = (
     "vx_rowscale_linear_scratch",
     "vx_ctc_topk_rows",
     "vx_ctc_topk",
+    "vx_conformer_pass_supported",
+    "vx_conformer_pass_frames",
+    "vx_conformer_pass_scratch",
+    "vx_conformer_pass",
 )
 
 
@@ -201,6 +205,14 @@ def load(build_if_missing: bool = True) -> C.CDLL:
         lib.vx_bsgemm_residual_ln.argtypes = [vp, vp, vp, C.c_float, vp, i64, vp, vp]
         lib.vx_bsgemm_residual_ln2.restype = i32
         lib.vx_bsgemm_residual_ln2.argtypes = [vp, vp, vp, vp, vp, C.c_float, vp, i64, vp, vp]
+        lib.vx_conformer_pass_supported.restype = i32
+        lib.vx_conformer_pass_supported.argtypes = [i32, i64, i64, i64, i64]
+        lib.vx_conformer_pass_frames.restype = i64
+        lib.vx_conformer_pass_frames.argtypes = []
+        lib.vx_conformer_pass_scratch.restype = i64
+        lib.vx_conformer_pass_scratch.argtypes = [i64, i64]
+        lib.vx_conformer_pass.restype = i32
+        lib.vx_conformer_pass.argtypes = [vp, vp]
         lib.vx_ctc_topk_threshold.restype = i32
         lib.vx_ctc_topk_threshold.argtypes = [vp, i64, i64, i32, vp, vp]
         lib.vx_ctc_topk_finish.restype = i32

@@ -18,7 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libvelox_b200.so")
 STAMP = os.path.join(LIB_DIR, "libvelox_b200.stamp")
-SOURCES = ("vx_api.cu", "vx_quant.cu", "vx_gemm.cu", "vx_noalloc.cu", "vx_pack.cu", "vx_mel.cu", "vx_attn.cu", "vx_gemm_ln.cu", "vx_topk.cu", "vx_rowscale.cu")
+SOURCES = ("vx_api.cu", "vx_quant.cu", "vx_gemm.cu", "vx_noalloc.cu", "vx_pack.cu", "vx_mel.cu", "vx_attn.cu", "vx_gemm_ln.cu", "vx_pass.cu", "vx_topk.cu", "vx_rowscale.cu")
 # native host path of the Python operators: a CPython extension against torch's headers (g++, no device code)
 HOST_SOURCE = "vx_host.cpp"
 HOST_PATH = os.path.join(LIB_DIR, "_vx_host.so")

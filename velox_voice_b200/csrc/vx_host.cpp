@@ -30,7 +30,8 @@ namespace {
 #define VX_FUNCS(X)                                                                                                 \
   X(vx_last_error) X(vx_quantize_pack) X(vx_ln_quantize_pack) X(vx_ln2_quantize_pack) X(vx_amax) X(vx_bsgemm)        \
   X(vx_bsgemm_residual_ln_supported) X(vx_bsgemm_residual_ln) X(vx_bsgemm_residual_ln2) X(vx_argmax_ids) X(vx_relpos_attention)   \
-  X(vx_power_mel_log) X(vx_power_mel_log_supported) X(vx_sf_from_natural_pair) X(vx_rowscale_linear) X(vx_rowscale_linear_scratch) X(vx_ctc_topk_rows) X(vx_ctc_topk)
+  X(vx_power_mel_log) X(vx_power_mel_log_supported) X(vx_sf_from_natural_pair) X(vx_rowscale_linear) X(vx_rowscale_linear_scratch) X(vx_ctc_topk_rows) X(vx_ctc_topk)        \
+  X(vx_conformer_pass_supported) X(vx_conformer_pass_scratch) X(vx_conformer_pass)
 struct Api {
 #define X(f) decltype(&::f) f = nullptr;
   VX_FUNCS(X)
@@ -803,6 +804,10 @@ struct Pass {
   }
 };
 
+// How a pass runs its residual GEMMs and LayerNorms: separate launches, with the LayerNorm + quantizer in the GEMM, or all
+// blocks in one launch where the shapes and addresses allow it (separate launches where not).
+enum { ROUTE_SEPARATE, ROUTE_FUSED, ROUTE_WHOLE };
+
 void plan_free(PyObject* cap) {
   delete static_cast<Plan*>(PyCapsule_GetPointer(cap, "velox_stack_plan"));
 }
@@ -955,14 +960,29 @@ PyObject* py_stack_plan_current(PyObject*, PyObject* const* a, Py_ssize_t nargs)
   VX_END
 }
 
+// Whether the blocks of a pass can run as one launch (vx_conformer_pass): the model's own widths, unit pieces of 16 bytes.
+bool one_launch(const Plan& p, const void* x, int64_t ldx, const void* src, int64_t ld_src) {
+  if (p.blocks == 0 || !p.fuse_ffn || !g.vx_conformer_pass_supported(p.fmt, p.d, p.lin[L_FFM1].N, p.lin[L_PW1].N, p.blocks)) return false;
+  for (int i = 0; i < p.blocks; ++i) {
+    const Lin* L = &p.lin[i * L_COUNT];
+    if (L[L_FFM1].N != p.lin[L_FFM1].N || L[L_FF1].N != p.lin[L_FFM1].N || L[L_PW1].N != p.lin[L_PW1].N) return false;
+    for (int l = 0; l < L_COUNT; ++l)
+      if ((l != L_LP && (!L[l].bias || (reinterpret_cast<uintptr_t>(L[l].bias) & 15))) || ((reinterpret_cast<uintptr_t>(L[l].codes) | reinterpret_cast<uintptr_t>(L[l].scales) | L[l].ld) & 15) != 0) return false;
+  }
+  for (const Norm& n : p.norm)
+    if (((reinterpret_cast<uintptr_t>(n.g) | reinterpret_cast<uintptr_t>(n.b)) & 15) != 0) return false;
+  return ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(src)) & 15) == 0 && ((ldx | ld_src) & 7) == 0;
+}
+
 // Every launch of one pass.  `src` (row stride ld_src): the features, where they are not in x; `pt`: the positions, or not
 // defined; of the outputs those that the caller did not bring are made.
-void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld_src, const at::Tensor& pt, bool fused, bool greedy,
+void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld_src, const at::Tensor& pt, int route, bool greedy,
                 at::Tensor& keys, at::Tensor& ids, at::Tensor& logits) {
   const at::Device dev = xt.device();
   const int64_t M = xt.size(0), ldx = xt.stride(0), d = p.d;
   void* const x = xt.data_ptr();
-  const bool with_pos = pt.defined();
+  const bool with_pos = pt.defined(), fused = route == ROUTE_FUSED;
+  const bool whole = route == ROUTE_WHOLE && M > 0 && one_launch(p, x, ldx, src ? src : x, src ? ld_src : ldx);
   Pass s{p, M, stream()};
   Pass sp{p, with_pos ? pt.size(0) : 0, s.st};  // the positions' own rows
 
@@ -971,6 +991,7 @@ void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld
   const int64_t bh = p.fuse_ffn ? s.act_bytes(p.ffn) : s.act_bytes(p.ffn) + (M * p.ffn * 2 + 255) / 256 * 256;
   int64_t big = bh > M * 3 * d * 2 ? bh : M * 3 * d * 2;
   if (big < M * p.glu * 2) big = M * p.glu * 2;
+  if (whole) big = M * 3 * d * 2 + 256 + g.vx_conformer_pass_scratch(M, p.ffn);  // q|k|v, then the kernel's scratch
   big = (big + 255) / 256 * 256;
   const int64_t bp = sp.act_bytes(d);
   const bool lp_batched = with_pos && p.lp_all.codes && sp.M <= LP_BATCH_MAX;
@@ -1004,8 +1025,36 @@ void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld
     s.residual(h, w2, x, ldx, 0.5f, n, n2, q_next, fused, from, ld_src);
   };
   Act q = s.act(w_act, d, p.amax(p.blocks > 0 ? A_FFM : 0));
-  s.ln_quantize(src ? src : x, src ? ld_src : ldx, p.norm[p.blocks > 0 ? N_FFM : 0], q);
-  for (int i = 0; i < p.blocks; ++i) {
+  if (whole) {
+    std::vector<vx_pass_block> blocks(p.blocks);
+    vx_pass_desc c{};
+    c.struct_size = sizeof(c);
+    c.const_weights = 1;
+    for (int i = 0; i < p.blocks; ++i) {
+      constexpr int order[VX_PASS_LINEARS] = {L_FFM1, L_FFM2, L_QKV, L_LO, L_PW1, L_PW2, L_FF1, L_FF2};
+      for (int l = 0; l < VX_PASS_LINEARS; ++l) {
+        const Lin& w = p.lin[i * L_COUNT + order[l]];
+        blocks[i].lin[l] = {w.codes, w.ld, w.scales, w.bias};
+        if (!(w.flags & VX_GEMM_CONST_B)) c.const_weights = 0;
+      }
+      for (int n = 0; n < N_COUNT; ++n) {
+        blocks[i].gamma[n] = p.norm[i * N_COUNT + n].g;
+        blocks[i].beta[n] = p.norm[i * N_COUNT + n].b;
+      }
+    }
+    c.blocks = p.blocks; c.M = M; c.ffn = p.ffn; c.eps = p.eps;
+    c.block = blocks.data();
+    c.after_gamma = p.norm[p.blocks * N_COUNT].g; c.after_beta = p.norm[p.blocks * N_COUNT].b;
+    c.src = src ? src : x; c.ld_src = src ? ld_src : ldx;
+    c.x = x; c.ldx = ldx;
+    c.qkv = w_big;
+    c.scratch = w_big + (M * 3 * d * 2 + 255) / 256 * 256;
+    c.codes = q.codes; c.scales_sf = q.scales;
+    check(g.vx_conformer_pass(&c, s.st), "vx_conformer_pass");
+    ++s.launches;
+  } else
+    s.ln_quantize(src ? src : x, src ? ld_src : ldx, p.norm[p.blocks > 0 ? N_FFM : 0], q);
+  for (int i = 0; i < p.blocks && !whole; ++i) {
     const Lin* L = &p.lin[i * L_COUNT];
     const Norm* n = &p.norm[i * N_COUNT];
     const float* const* am = p.am.empty() ? nullptr : &p.am[i * A_COUNT];
@@ -1052,7 +1101,7 @@ void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld
   count(s.launches + sp.launches);
 }
 
-// stack_forward(plan, x, pos | None, fused_ln, head, keys | None, ids | None, logits | None, source | None) -> logits / ids
+// stack_forward(plan, x, pos | None, route, head, keys | None, ids | None, logits | None, source | None) -> logits / ids
 //   x bf16 [T, d] (overwritten; with `source`, bf16 [T, d], the features are read there and x only receives the residual
 //   stream); head 0: bf16 logits [T, vocab], 1: greedy ids i32 [T]
 PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
@@ -1088,7 +1137,8 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (!rows2d(pt) || pt.size(1) != d || pt.device() != dev || dtype_code(pt) < 0)
       bad("pos must be a float32 or bf16 [frames, d_model] tensor on x's device with unit column stride");
   }
-  const bool fused = as_bool(a[3]), greedy = as_long(a[4]) != 0;
+  const int route = static_cast<int>(as_long(a[3]));
+  const bool greedy = as_long(a[4]) != 0;
   auto out_vec = [&](PyObject* o, at::ScalarType dt, const char* what, at::Tensor& t) {
     if (o == Py_None) return;
     if (!is_cuda_tensor(o)) bad(what);
@@ -1105,7 +1155,7 @@ PyObject* py_stack_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   }
   {
     NoGil nogil;
-    stack_pass(p, xt, src, ld_src, pt, fused, greedy, keys, ids, logits);
+    stack_pass(p, xt, src, ld_src, pt, route, greedy, keys, ids, logits);
   }
   PyObject* given = a[greedy ? 6 : 7];
   return given == Py_None ? wrap(greedy ? ids : logits) : Py_NewRef(given);

@@ -451,6 +451,12 @@ def residual_ln_supported(fmt, N: int, K: int) -> bool:
     return bool(_lib.load().vx_bsgemm_residual_ln_supported(_fmt(fmt), int(N), int(K)))
 
 
+def conformer_pass_frames(device) -> int:
+    """Frames up to which the stack runs all its MX32 blocks in one launch on ``device`` (``vx_conformer_pass``)."""
+    with torch.cuda.device(device):
+        return int(_lib.load().vx_conformer_pass_frames())
+
+
 def bsgemm_residual_ln(a: Quantized, b: Quantized, *, bias: Optional[torch.Tensor], residual: torch.Tensor,
                        gamma: torch.Tensor, beta: torch.Tensor, eps: float, alpha: float = 1.0,
                        out: Optional[torch.Tensor] = None, gamma2: Optional[torch.Tensor] = None,

@@ -13,7 +13,8 @@ convolution and its norm/activation are NOT linear layers and are outside this l
 stack passes the value projection straight to ``lo`` and the GLU output straight to ``pw2``,
 so it measures and validates every linear of the encoder with the real operand shapes.
 
-Kernel sequence per block (13 launches, 9 where the residual GEMMs also run the LayerNorm + quantizer behind
+Short MX32 passes (up to ``one_launch_frames``, 4,224 on a B200) run all blocks in one launch (``csrc/vx_pass.cu``), with the same bits.
+Kernel sequence per block of the others (13 launches, 9 where the residual GEMMs also run the LayerNorm + quantizer behind
 them; issued by the native host path ``csrc/vx_host.cpp``; the reference issues >= 4 per linear):
 ``GEMM(bias, swish, FP4 out) -> GEMM(bias, 0.5 residual)`` for each FFN (the second one behind its ``ln_quant``),
 ``ln_quant -> GEMM(bias, value third also quantized) [qkv] -> GEMM(bias, residual) [lo]``, ``GEMM [lp]`` (one launch
@@ -118,7 +119,11 @@ class ConformerLinearStack:
                         and ops.residual_ln_supported(self.fmt, cfg.d_model, cfg.d_model))
         dev = self.device
         least = os.environ.get("VELOX_B200_FUSE_LN_MIN_FRAMES", cfg.fuse_ln_min_frames)
+        # frames up to which all blocks run in one launch (not where the caller draws the line between separate and fused launches)
+        self.one_launch_frames = 0
         if least is None:
+            if self.fmt == FMT_MX32:
+                self.one_launch_frames = ops.conformer_pass_frames(dev)
             least = fuse_ln_frames(torch.cuda.get_device_properties(dev).multi_processor_count, cfg.d_model)
         self.fuse_ln_min_frames = int(least)
         self.p: Dict[str, PackedLinear] = {}
@@ -217,8 +222,10 @@ class ConformerLinearStack:
             self._amax("pos", pos)  # must have been calibrated
         if pos is not None and pos.stride(1) != 1:
             pos = pos.contiguous()
-        fused = self.fuse_ln and x.shape[0] >= self.fuse_ln_min_frames
-        out = ops._host().stack_forward(self._host_plan(), x, pos, fused, 1 if ids_only else 0, keys, ids, out_logits,
+        route = 0
+        if self.fuse_ln:
+            route = 2 if x.shape[0] <= self.one_launch_frames else int(x.shape[0] >= self.fuse_ln_min_frames)
+        out = ops._host().stack_forward(self._host_plan(), x, pos, route, 1 if ids_only else 0, keys, ids, out_logits,
                                          source)
         return (out, x) if return_hidden and not ids_only else out
 
