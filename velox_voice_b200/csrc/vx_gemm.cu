@@ -1808,8 +1808,8 @@ int dispatch_epi(int epi, int out, const CUtensorMap& ta, const CUtensorMap& tb,
 }  // namespace
 
 int make_tmap_2d(CUtensorMap* m, CUtensorMapDataType dt, const void* ptr, int64_t rows, int64_t cols, int64_t pitch_bytes,
-                 int box_cols, int box_rows) {
-  return make_tmap(m, dt, 0, ptr, rows, cols, pitch_bytes, box_cols, box_rows);
+                 int box_cols, int box_rows, bool swizzle64) {
+  return make_tmap(m, dt, 0, ptr, rows, cols, pitch_bytes, box_cols, box_rows, swizzle64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 }  // namespace vx

@@ -7,13 +7,14 @@
 // factors of a block-scaled MMA in tensor memory.  So a CLUSTER OF TWO CTAs owns each block of 128 rows:
 // CTA r computes columns [256 r, 256 r + 256) with 128 x 256 x 64 MXF4 MMAs, and the two exchange the
 // per-row partial sums of the LayerNorm statistics through distributed shared memory (st.async with
-// mbarrier completion into a table double-buffered per tile, one barrier per lane quadrant).  Per CTA, 18 warps:
+// mbarrier completion into a table double-buffered per tile, one barrier per lane quadrant).  Per CTA, 19 warps:
 //   warp 0      TMA producer: A tiles (128-byte swizzle) + scale-factor atoms into a ring; the CTA's half of B stays
-//               resident in shared memory when K <= 512, else it streams through the ring with A;
+//               resident in shared memory when K <= 512;
+//   warp 18     otherwise streams B through a ring of its own;
 //   warp 1      owns tensor memory, copies scale factors shared -> tensor memory and issues the MMAs;
 //   warps 2..17 epilogue, warp (q, g) = TMEM lane quadrant q, 32-column blocks 2 g and 2 g + 1 of the CTA:
 //     pass 1  accumulator -> + bias, alpha, residual (its 32 x 64 block prefetched by TMA into the warp's
-//             staging buffer) -> bf16, formed in place and stored by TMA; the bf16 pairs also go back to
+//             staging buffer) -> bf16, formed in place and stored from there; the bf16 pairs also go back to
 //             tensor memory (128 columns next to the accumulator), the accumulator is released to the
 //             MMAs of the next tile; per-block (sum, sum of squares) sent to both CTAs;
 //     pass 2  after the exchange: mean / rstd, normalise the bf16 values read back from tensor memory,
@@ -50,15 +51,20 @@ constexpr int LN_SFB = 2 * 2 * 512;           // two 128-row tiles x two atoms
 constexpr int LN_B_OFF = LN_A_TILE + LN_SFA;  // 17 KB: keeps the B tile 1024-byte aligned
 constexpr int LN_A_SLOT = LN_B_OFF;                     // 17 KB: A tile + its scale factors
 constexpr int LN_B_SLOT = LN_B_TILE + LN_SFB;           // 34 KB: B tile + its scale factors
-constexpr int LN_SLOT = LN_A_SLOT + LN_B_SLOT;          // 51 KB
+constexpr int LN_HB_TILE = LN_BN * 64;                  // 16 KB: B rows of half a stage (128 FP4 elements of K)
+constexpr int LN_HB_SLOT = LN_HB_TILE + 2 * 512;        // 17 KB: and their scale factors (an atom per 128 rows)
+constexpr int LN_HB_SLOTS = 4;
 // Operand arena, two plans (as in vx_gemm.cu):
 //   B resident (K <= 512)  [B stage 0 | B stage 1] then three ring slots [A | SFA];
-//   streaming              two ring slots [A | SFA | B | SFB].
+//   streaming              four ring slots of half a stage of B [B | SFB], then three of A [A | SFA], each with a loader of its own.
+//                          (One ring of two slots [A | SFA | B | SFB], 102 KB in flight by one loader: the MMAs waited for it, 1,500 cycles a
+//                          stage where they take 600; 90,000 rows x 2048: 86 us, 82 like this.)
 constexpr int LN_RESIDENT_MAX_STAGES = 2;
 constexpr int LN_ARENA = LN_RESIDENT_MAX_STAGES * LN_B_SLOT + 3 * LN_A_SLOT;  // 119 KB
-constexpr int LN_MAX_SLOTS = 3;
+constexpr int LN_A_SLOTS = 3;
+static_assert(LN_HB_SLOTS * LN_HB_SLOT + LN_A_SLOTS * LN_A_SLOT <= LN_ARENA, "streaming plan");
 constexpr int LN_STAGING = 32 * 128;                    // per epilogue warp: 32 rows x 64 bf16 columns, 128-byte swizzle
-constexpr int LN_THREADS = 18 * 32;
+constexpr int LN_THREADS = 19 * 32;
 constexpr uint32_t LN_XCH_BYTES = 2 * 4 * 32 * 16;  // per CTA, tile and lane quadrant: 2 CTAs x 4 warps x 32 lanes x 16 bytes
 // tensor-memory columns
 constexpr uint32_t LN_TM_ACC = 0, LN_TM_XP = 256, LN_TM_SFA = 384, LN_TM_SFB = 448;
@@ -93,7 +99,7 @@ struct __align__(1024) LnSmem {
   uint8_t staging[16][LN_STAGING];  // residual block in (TMA), x block out (TMA), per epilogue warp
   float4 part[2][8][LN_BM];  // [tile parity][block pair of the row][row] = (S, Q) of blocks 2 i and 2 i + 1
   float bias[LN_BN], gamma[LN_BN], beta[LN_BN], gamma2[LN_BN], beta2[LN_BN];
-  uint64_t full[LN_MAX_SLOTS], empty[LN_MAX_SLOTS];
+  uint64_t full[LN_A_SLOTS], empty[LN_A_SLOTS], hb_full[LN_HB_SLOTS], hb_empty[LN_HB_SLOTS];
   uint64_t tmem_full, tmem_empty, b_full;
   uint64_t res_full[16];
   uint64_t xch[2][4];  // [tile parity][lane quadrant]: the rows of a quadrant depend on that quadrant's warps only
@@ -123,16 +129,12 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   const int cluster = static_cast<int>(blockIdx.x >> 1), nclusters = static_cast<int>(gridDim.x >> 1);
   const int my_tiles = cluster < p.m_tiles ? (p.m_tiles - cluster + nclusters - 1) / nclusters : 0;
   const bool resident = p.b_resident != 0;
-  const int nslots = resident ? 3 : 2;
-  const uint32_t slot_bytes = resident ? LN_A_SLOT : LN_SLOT;
-  const uint32_t ring_off = resident ? p.k_stages * LN_B_SLOT : 0;
+  const uint32_t ring_off = resident ? p.k_stages * LN_B_SLOT : LN_HB_SLOTS * LN_HB_SLOT;  // ring of A
 
   // ---- set-up
   if (threadIdx.x == 0) {
-    for (int s = 0; s < LN_MAX_SLOTS; ++s) {
-      mbar_init(&sm.full[s], 1);
-      mbar_init(&sm.empty[s], 1);
-    }
+    for (int s = 0; s < LN_A_SLOTS; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
+    for (int s = 0; s < LN_HB_SLOTS; ++s) { mbar_init(&sm.hb_full[s], 1); mbar_init(&sm.hb_empty[s], 1); }
     mbar_init(&sm.tmem_full, 1);
     mbar_init(&sm.tmem_empty, 16);  // one arrival per epilogue warp
     mbar_init(&sm.b_full, 1);
@@ -167,7 +169,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   tc_fence_after();
   cluster_sync_all();  // the peer's barriers exist before anything is sent to them
   const uint32_t tmem_base = sm.tmem_base;
-  const bool producer_thread = warp == 0 && lane == 0 && my_tiles > 0;
+  const bool producer_thread = (warp == 0 || warp == 18) && lane == 0 && my_tiles > 0;
   if (!producer_thread) pdl_wait();
 
   if (warp == 0) {
@@ -194,12 +196,31 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         const uint8_t* sfa_row = p.sfa + (static_cast<int64_t>(mb) * p.sf_kg) * 512;
         for (int ks = 0; ks < p.k_stages; ++ks) {
           if (!mbar_wait(&sm.empty[s], ph ^ 1, p.status, 21)) { ok = false; break; }
-          uint8_t* dst = sm.arena + ring_off + s * slot_bytes;
-          mbar_expect_tx(&sm.full[s], slot_bytes);
+          uint8_t* dst = sm.arena + ring_off + s * LN_A_SLOT;
+          mbar_expect_tx(&sm.full[s], LN_A_SLOT);
           tma_load_2d(dst, &tmap_a, ks * 128, mb * LN_BM, &sm.full[s]);
           bulk_load(dst + LN_A_TILE, sfa_row + static_cast<int64_t>(ks) * LN_SFA, LN_SFA, &sm.full[s]);
-          if (!resident) load_b(dst + LN_A_SLOT, ks, &sm.full[s]);
-          if (++s == static_cast<uint32_t>(nslots)) { s = 0; ph ^= 1; }
+          if (++s == LN_A_SLOTS) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 18) {
+    // =========================== loader of B, streaming plan ===========================
+    if (lane == 0 && my_tiles > 0 && !resident) {
+      uint32_t s = 0, ph = 0;
+      bool ok = true;
+      if (!p.b_const) pdl_wait();
+      const uint8_t* const sf0 = p.sfb + static_cast<int64_t>(rank * 2) * p.sf_kg * 512;
+      const int64_t sf_tile = p.sf_kg * 512;
+      for (int i = 0; i < my_tiles && ok; ++i) {
+        for (int kh = 0; kh < 2 * p.k_stages; ++kh) {
+          if (!mbar_wait(&sm.hb_empty[s], ph ^ 1, p.status, 28)) { ok = false; break; }
+          uint8_t* dst = sm.arena + s * LN_HB_SLOT;
+          mbar_expect_tx(&sm.hb_full[s], LN_HB_SLOT);
+          tma_load_2d(dst, &tmap_b, kh * 64, static_cast<int>(rank) * LN_BN, &sm.hb_full[s]);
+          bulk_load(dst + LN_HB_TILE, sf0 + kh * 512, 512, &sm.hb_full[s]);
+          bulk_load(dst + LN_HB_TILE + 512, sf0 + sf_tile + kh * 512, 512, &sm.hb_full[s]);
+          if (++s == LN_HB_SLOTS) { s = 0; ph ^= 1; }
         }
       }
     }
@@ -207,10 +228,11 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     // =========================== MMA issuer ===========================
     if (my_tiles > 0) {
       const bool leader = elect_one();
-      uint32_t s = 0, ph = 0, sfsel = 0;
+      uint32_t s = 0, ph = 0, bs = 0, bph = 0, sfsel = 0;
       bool ok = true;
       const uint32_t idesc_base = make_idesc_mxf4(LN_BM, LN_BN, true);
       const uint32_t k128_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+      const uint32_t k64_hi = (512u >> 4) | (1u << 14) | (4u << 29);  // rows of 64 bytes, 64-byte swizzle
       const uint32_t sf_hi = (128u >> 4) | (1u << 14);
       auto desc = [](uint32_t lo, uint32_t hi) -> uint64_t { return (static_cast<uint64_t>(hi) << 32) | (lo & 0x3fffu); };
       const uint32_t arena_lo = smem_u32(sm.arena) >> 4;
@@ -234,35 +256,58 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         // the epilogue has read the previous accumulator out (pass 1 of tile i - 1)
         if (!mbar_wait_spin(&sm.tmem_empty, (i & 1) ^ 1, p.status, 22)) { ok = false; break; }
         tc_fence_after();
-        for (int ks = 0; ks < p.k_stages; ++ks) {
+        for (int ks = 0; ks < p.k_stages && ok; ++ks) {
           if (!mbar_wait_spin(&sm.full[s], ph, p.status, 23)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a_lo = ring_lo + s * (slot_bytes >> 4);
-          const uint32_t b_lo = resident ? arena_lo + ks * (LN_B_SLOT >> 4) : a_lo + (LN_A_SLOT >> 4);
+          const uint32_t a_lo = ring_lo + s * (LN_A_SLOT >> 4);
           const uint32_t sfa_buf = tmem_base + LN_TM_SFA + sfsel * 32;
-          const uint32_t sfb_buf = tmem_base + LN_TM_SFB + (resident ? ks * 16 : sfsel * 32);
           if (leader) {
 #pragma unroll
             for (int a = 0; a < 2; ++a) tc_cp_32x128b_warpx4(sfa_buf + a * 4, desc(a_lo + (LN_A_TILE >> 4) + a * 32, sf_hi));
-            if (!resident) cp_sfb(b_lo, sfb_buf);
+          }
+          if (resident) {
+            const uint32_t b_lo = arena_lo + ks * (LN_B_SLOT >> 4), sfb_buf = tmem_base + LN_TM_SFB + ks * 16;
+            if (leader) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint32_t atom = j >> 1, sf_id = (j & 1) * 2;
-              mma_mxf4<2>(tmem_base + LN_TM_ACC, desc(a_lo + 2 * j, k128_hi), desc(b_lo + 2 * j, k128_hi),
-                          idesc_with_sf_id(idesc_base, sf_id, sf_id), sfa_buf + atom * 4, sfb_buf + atom * 8,
-                          static_cast<uint32_t>((ks | j) != 0));
+              for (int j = 0; j < 4; ++j) {
+                const uint32_t atom = j >> 1, sf_id = (j & 1) * 2;
+                mma_mxf4<2>(tmem_base + LN_TM_ACC, desc(a_lo + 2 * j, k128_hi), desc(b_lo + 2 * j, k128_hi),
+                            idesc_with_sf_id(idesc_base, sf_id, sf_id), sfa_buf + atom * 4, sfb_buf + atom * 8,
+                            static_cast<uint32_t>((ks | j) != 0));
+              }
             }
+          } else {
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+              if (!mbar_wait_spin(&sm.hb_full[bs], bph, p.status, 29)) { ok = false; break; }
+              tc_fence_after();
+              const uint32_t b_lo = arena_lo + bs * (LN_HB_SLOT >> 4), sfb_buf = tmem_base + LN_TM_SFB + bs * 16;
+              if (leader) {
+#pragma unroll
+                for (int rt = 0; rt < 2; ++rt) tc_cp_32x128b_warpx4(sfb_buf + rt * 4, desc(b_lo + (LN_HB_TILE >> 4) + rt * 32, sf_hi));
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                  mma_mxf4<2>(tmem_base + LN_TM_ACC, desc(a_lo + 4 * hf + 2 * j, k128_hi), desc(b_lo + 2 * j, k64_hi),
+                              idesc_with_sf_id(idesc_base, 2 * j, 2 * j), sfa_buf + hf * 4, sfb_buf, static_cast<uint32_t>((ks | hf | j) != 0));
+                tc_commit(&sm.hb_empty[bs]);
+              }
+              __syncwarp();
+              if (++bs == LN_HB_SLOTS) { bs = 0; bph ^= 1; }
+            }
+            if (!ok) break;
+          }
+          if (leader) {
             tc_commit(&sm.empty[s]);
             if (ks == p.k_stages - 1) tc_commit(&sm.tmem_full);
           }
           __syncwarp();
           sfsel ^= 1;
-          if (++s == static_cast<uint32_t>(nslots)) { s = 0; ph ^= 1; }
+          if (++s == LN_A_SLOTS) { s = 0; ph ^= 1; }
         }
       }
     }
   } else {
-    // =========================== epilogue ===========================
+    // =========================== epilogue (warps 2..17) ===========================
     const int q = warp & 3, g = (warp - 2) >> 2;  // TMEM lane quadrant; blocks 2 g, 2 g + 1 of this CTA's eight
     const int ew = warp - 2;
     const int row_in = q * 32 + lane;
@@ -298,24 +343,25 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       ok = __all_sync(0xffffffffu, mbar_wait(&sm.tmem_full, i & 1, p.status, 24));
       if (!ok) break;
       tc_fence_after();
-      ok = __all_sync(0xffffffffu, mbar_wait(&sm.res_full[ew], i & 1, p.status, 27));
-      if (!ok) break;
       // ---- pass 1: x = bf16(alpha (acc + bias) + residual), block statistics
       float SQ[4];
+      // (both blocks at once: the accumulator is free after 700 cycles instead of 2,500, 90,000 rows x 2048: 92 us -> 86 with the stores below)
+      uint32_t acc[2][4][8];
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tc_ld_x8(lane_addr + LN_TM_ACC + (2 * g + t) * 32 + piece[c] * 8, acc[t][c]);
+      tc_wait_ld();
+      // the warp's part of the accumulator is in registers: free it for the MMAs of the next tile now, not behind the arithmetic
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.tmem_empty);
+      ok = __all_sync(0xffffffffu, mbar_wait(&sm.res_full[ew], i & 1, p.status, 27));
+      if (!ok) break;
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const int k = 2 * g + t;
-        uint32_t z[4][8];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tc_ld_x8(lane_addr + LN_TM_ACC + k * 32 + piece[c] * 8, z[c]);
-        tc_wait_ld();
-        if (t == 1) {
-          // the warp's part of the accumulator is in registers: free it for the MMAs of the next tile now, not
-          // after the arithmetic below (with K = 2048 those MMAs are what the next tile waits for)
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.tmem_empty);
-        }
+        const uint32_t (&z)[4][8] = acc[t];
         uint32_t xp[16];
         uint64_t S = pack_f32x2(0.0f, 0.0f), Q = S;
 #pragma unroll
@@ -357,8 +403,22 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 #pragma unroll
         for (int d = 0; d < 2; ++d) st_async_f4(dst_part[d] + b * PART_STRIDE, sq[0], sq[1], sq[2], sq[3], dst_bar[d] + b * 32);
       };
-      // x (or y) leaves by TMA from the staging block
+      // x (or y) leaves from the staging block: by TMA, or, where operands stream, by ordinary stores of whole 128-byte rows (as
+      // TMA stores its 64 KB held up the loads of the next stages for 2,500 of a tile's 15,400 cycles)
       auto store_block = [&]() {
+        if (!resident) {
+          __syncwarp();
+#pragma unroll
+          for (int v = 0; v < 8; ++v) {
+            const int r = 4 * v + (lane >> 3), u = lane & 7;
+            const int64_t orow = static_cast<int64_t>(mb) * LN_BM + q * 32 + r;
+            const uint4 w = *reinterpret_cast<const uint4*>(sm.staging[ew] + r * 128 + ((u ^ (r & 7)) << 4));
+            if (orow < p.M) *reinterpret_cast<uint4*>(p.out + orow * p.ldo + tile_col + u * 8) = w;
+          }
+          fence_proxy_async_smem();  // read before the next residual block may land here
+          __syncwarp();
+          return;
+        }
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
@@ -592,7 +652,8 @@ int launch_residual_ln(const vx_gemm_desc* d, const float* gamma, const float* b
   CUtensorMap ta, tb, tr, to;
   int rc = make_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, d->a_codes, M, row_bytes, d->lda, 128, LN_BM);
   if (rc) return rc;
-  rc = make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, d->b_codes, LN_D, row_bytes, d->ldb, 128, LN_BN);
+  rc = p.b_resident ? make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, d->b_codes, LN_D, row_bytes, d->ldb, 128, LN_BN)
+                    : make_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, d->b_codes, LN_D, row_bytes, d->ldb, 64, LN_BN, true);
   if (rc) return rc;
   // residual in / x out: blocks of 32 rows x 64 bf16 columns (128-byte rows), one per epilogue warp and tile
   rc = make_tmap_2d(&tr, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d->residual, M, LN_D, d->ldr * 2, 64, 32);
