@@ -119,8 +119,6 @@ __global__ void __launch_bounds__(LN_THREADS, 1)
 bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                           const __grid_constant__ CUtensorMap tmap_res, const __grid_constant__ CUtensorMap tmap_out,
                           const LnParams p) {
-  // (No early trigger of the next launch: 24,000 frames take 1 % less with one.  The 32-row blocks that differed in passes with it
-  // came from the staged stores of bsgemm_kernel, see store_count there; it has not been tried since that was mended.)
   extern __shared__ uint8_t smem_raw[];
   // (the same offset in both CTAs of the cluster: map_to_cta relies on it)
   LnSmem& sm = *reinterpret_cast<LnSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -170,7 +168,12 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   cluster_sync_all();  // the peer's barriers exist before anything is sent to them
   const uint32_t tmem_base = sm.tmem_base;
   const bool producer_thread = (warp == 0 || warp == 18) && lane == 0 && my_tiles > 0;
-  if (!producer_thread) pdl_wait();
+  // (The next launch is triggered behind the wait, by threads that have waited, as in vx_gemm.cu: its set-up and weights come in under
+  // the last round, which leaves clusters idle.  12 blocks, 24,000 frames: 2,650 us without, 2,577 like this.)
+  if (!producer_thread) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
 
   if (warp == 0) {
     // =========================== TMA producer ===========================
