@@ -127,3 +127,26 @@ def test_entry_points_without_logits(ops, M, k, capacity):
     # two summation orders of the fp32 log-sum-exp of one row (see _check)
     assert torch.allclose(logp[~full], want_logp[~full], rtol=0, atol=4e-5)
     del keep
+
+
+@pytest.mark.parametrize("N", [1024, 1032, 1500, 4096, 6137, 6144, 6152])
+@pytest.mark.parametrize("k", [1, 7, 16])
+def test_widths_around_the_kernels_ranges(ops, N, k):
+    """Rows of more than 1,024 and up to 6,144 columns are held in registers, others read twice; equal logits
+    (more than a row's candidate list holds) and rows whose columns are masked but for fewer than k."""
+    torch.manual_seed(N + k)
+    M, K = 67, 512
+    a = ops.quantize(torch.randn(M, K, device="cuda"), "mx32", natural=False)
+    b = ops.quantize(0.05 * torch.randn(N, K, device="cuda"), "mx32")
+    bias = torch.randn(N, device="cuda")
+    _check(ops, a, b, bias, k)
+    few = torch.full((N,), float("-inf"), device="cuda")
+    few[torch.randperm(N, device="cuda")[: k + 3]] = 0.5
+    _check(ops, a, b, few, k)
+    zero = ops.quantize(torch.zeros(N, K, device="cuda"), "mx32")
+    logp, ids = ops.bsgemm_topk(a, zero, torch.full((N,), 2.0, device="cuda"), k)  # all equal: the lowest columns
+    assert torch.equal(ids, torch.arange(k, device="cuda").expand(M, k))
+    assert (logp + torch.log(torch.tensor(float(N)))).abs().max().item() < 4e-5
+    bias[N // 2] = float("nan")  # no column is a NaN's winner, and every log-probability of the row is one
+    logp, ids = ops.bsgemm_topk(a, b, bias, k)
+    assert torch.isnan(logp).all() and (ids != N // 2).all()

@@ -2,7 +2,7 @@
 //
 // The prefix beam search takes torch.topk(log_softmax(ctc_lo(x)), k).  The head's GEMM writes the bf16 logits of a block
 // of rows (vx_ctc_topk_rows, about 60 MB: half of the L2) into a scratch buffer, and the kernel below reads them back from
-// L2, one warp per row: log-sum-exp and the k largest values in two passes over the row.  Against the route without
+// L2, one warp per row: log-sum-exp and the k largest values.  Against the route without
 // logits (two launches of the head, the second with a candidate test in its epilogue, a threshold kernel, a finish
 // kernel and a host check for overflowed candidate lists) that is half the matrix work and no synchronisation.
 
@@ -173,6 +173,172 @@ __global__ void __launch_bounds__(TK_WARPS * 32) topk_rows_kernel(const __nv_bfl
   }
 }
 
+// The same for rows of 1,025 to 6,144 columns, which a warp holds in registers (up to 24 pieces of 16 bytes a lane): the row is read
+// once, with all loads of a lane in flight, maxima are taken on packed bf16 pairs, the log-sum-exp against the row's maximum
+// without running rescales.  The threshold is found by one integer reduction per rank; the pieces that hold a value reaching it
+// (few more than k) are listed, and only their values are looked at one by one.  About 1,100 warp instructions per row of 5,538
+// where two passes over the row with a running maximum issued 3,300.  Head's GEMM, selection and LayerNorm quantizer of 3,750 rows:
+// 49 us with two passes, 37.6 like this.  (Four warps per row, 40 us: what each repeats costs more than the shorter chain gives.)
+constexpr int TR_WARPS = 8, TR_PIECES = 24, TR_LIST = 64, TR_MIN_N = 1024;
+__global__ void __launch_bounds__(TR_WARPS * 32, 2) topk_regs_kernel(const __nv_bfloat16* logits, int64_t ld, int N, int M, int k, float* logp,
+                                                                    int64_t* ids) {
+  __shared__ unsigned long long cand_s[TR_WARPS][TK_CAND];
+  __shared__ int list_s[TR_WARPS][TR_LIST];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * TR_WARPS + w;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (row >= M) return;
+  constexpr float L2E = 1.4426950408889634f;
+  const __nv_bfloat16* const z0 = logits + row * ld;
+  const uint4* const src = reinterpret_cast<const uint4*>(z0);
+  const int pieces = (N + 7) >> 3;
+  constexpr uint32_t NONE = 0xff80ff80u;  // two bf16 -inf
+  uint4 u[TR_PIECES];
+#pragma unroll
+  for (int j = 0; j < TR_PIECES; ++j) {
+    u[j] = make_uint4(NONE, NONE, NONE, NONE);
+    if (j * 32 + lane < pieces) u[j] = src[j * 32 + lane];
+  }
+  if (N & 7) {  // columns beyond N in the last piece
+#pragma unroll
+    for (int j = 0; j < TR_PIECES; ++j)
+      if (j * 32 + lane == pieces - 1) {
+        uint32_t* const x = reinterpret_cast<uint32_t*>(&u[j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int valid = N - 8 * (pieces - 1) - 2 * i;
+          if (valid <= 0) x[i] = NONE;
+          else if (valid == 1) x[i] = (x[i] & 0xffffu) | (NONE & 0xffff0000u);
+        }
+      }
+  }
+  auto b2 = [](const uint32_t& x) { return *reinterpret_cast<const __nv_bfloat162*>(&x); };
+  __nv_bfloat162 m4[4] = {b2(u[0].x), b2(u[0].y), b2(u[0].z), b2(u[0].w)};
+#pragma unroll
+  for (int j = 1; j < TR_PIECES; ++j) {
+    if (j * 32 < pieces) {
+      m4[0] = __hmax2(m4[0], b2(u[j].x));
+      m4[1] = __hmax2(m4[1], b2(u[j].y));
+      m4[2] = __hmax2(m4[2], b2(u[j].z));
+      m4[3] = __hmax2(m4[3], b2(u[j].w));
+    }
+  }
+  const __nv_bfloat162 mm = __hmax2(__hmax2(m4[0], m4[1]), __hmax2(m4[2], m4[3]));
+  const float m = fmaxf(fmaxf(__low2float(mm), __high2float(mm)), -INFINITY);  // (a lane of NaNs only: -inf)
+  // order-preserving bits of the lane's maximum in the high half, the lane below: all different
+  uint32_t key, top = 0, kth = 0;
+  {
+    const uint32_t x = __float_as_uint(__fadd_rn(m, 0.0f));
+    key = ((x ^ (static_cast<uint32_t>(static_cast<int32_t>(x) >> 31) | 0x80000000u)) & 0xffff0000u) | static_cast<uint32_t>(31 - lane);
+  }
+  for (int r = 0; r < k; ++r) {
+    kth = __reduce_max_sync(0xffffffffu, key);
+    if (r == 0) top = kth;
+    if (key == kth) key = 0;
+  }
+  auto value = [](uint32_t kk) {
+    const uint32_t x = kk & 0xffff0000u;
+    return __uint_as_float((x & 0x80000000u) ? (x ^ 0x80000000u) : ~x & 0xffff0000u);
+  };
+  const float rm = value(top), thr = value(kth);
+  const uint64_t l2 = pack_f32x2(L2E, L2E), nb2 = pack_f32x2(-rm * L2E, -rm * L2E);
+  uint64_t sa = pack_f32x2(0.0f, 0.0f), sb = sa;
+  int listed = 0;  // pieces that reach the threshold
+#pragma unroll
+  for (int j = 0; j < TR_PIECES; ++j) {
+    if (j * 32 < pieces) {
+      const uint32_t x[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float a, b;
+        unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(x[i] << 16), __uint_as_float(x[i] & 0xffff0000u)), l2, nb2), a, b);
+        const uint64_t e = pack_f32x2(ex2_approx(a), ex2_approx(b));
+        if (i & 1) sb = add_f32x2(sb, e); else sa = add_f32x2(sa, e);
+      }
+      const __nv_bfloat162 pm = __hmax2(__hmax2(b2(x[0]), b2(x[1])), __hmax2(b2(x[2]), b2(x[3])));
+      const bool hit = j * 32 + lane < pieces && fmaxf(__low2float(pm), __high2float(pm)) >= thr;
+      const uint32_t who = __ballot_sync(0xffffffffu, hit);
+      if (who) {
+        const int at = listed + __popc(who & ((1u << lane) - 1u));
+        if (hit && at < TR_LIST) list_s[w][at] = j * 32 + lane;
+        listed += __popc(who);
+      }
+    }
+  }
+  float s0, s1;
+  unpack_f32x2(add_f32x2(sa, sb), s0, s1);
+  float rs = s0 + s1;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);
+  // (as there: a sum that is not one of at most N ones is formed again from the exact differences)
+  if (rm > -INFINITY && !(rs >= 0.5f && rs <= 2.0f * static_cast<float>(N))) {
+    rs = 0.0f;
+    for (int c = lane; c < pieces; c += 32) {
+      float z[8];
+      unpack8(src[c], z);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (8 * c + i < N) rs += ex2_approx((z[i] - rm) * L2E);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);
+  }
+  if (!(rm > -INFINITY)) rs = 0.0f;
+  const float lse = rm + logf(rs);
+  // the listed pieces value by value, four pieces at a time
+  __syncwarp();
+  int n = listed <= TR_LIST ? 0 : TK_CAND + 1;
+  if (listed <= TR_LIST)
+    for (int p0 = 0; p0 < listed; p0 += 4) {
+      const int p = p0 + (lane >> 3);
+      const int col = p < listed ? 8 * list_s[w][p] + (lane & 7) : N;
+      const float z = col < N ? __bfloat162float(z0[col]) : 0.0f;
+      const bool hit = col < N && z >= thr;
+      const uint32_t who = __ballot_sync(0xffffffffu, hit);
+      const int at = n + __popc(who & ((1u << lane) - 1u));
+      if (hit && at < TK_CAND) cand_s[w][at] = topk_key(z, col);
+      n += __popc(who);
+    }
+  __syncwarp();
+  auto put = [&](int j, unsigned long long e) {
+    const uint32_t x = static_cast<uint32_t>(e >> 32);
+    const float z = __uint_as_float((x & 0x80000000u) ? (x ^ 0x80000000u) : ~x);
+    ids[row * k + j] = e ? static_cast<int64_t>(0xffffffffu - static_cast<uint32_t>(e)) : -1;
+    logp[row * k + j] = e ? z - lse : -INFINITY;
+  };
+  if (n <= 32 && n >= k) {  // as a rule: every lane counts the entries above its own and writes it where that says
+    const unsigned long long mine = lane < n ? cand_s[w][lane] : 0ull;
+    int rank = 0;
+    for (int i = 0; i < n; ++i) rank += cand_s[w][i] > mine ? 1 : 0;
+    if (lane < n && rank < k) put(rank, mine);
+    return;
+  }
+  unsigned long long last = ~0ull;
+  for (int j = 0; j < k; ++j) {
+    unsigned long long best = 0;
+    if (n <= TK_CAND) {
+      for (int t = lane; t < n; t += 32) {
+        const unsigned long long e = cand_s[w][t];
+        if (e < last && e > best) best = e;
+      }
+    } else {
+      for (int c = lane; c < pieces; c += 32) {
+        float z[8];
+        unpack8(src[c], z);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const unsigned long long e = topk_key(z[i], 8 * c + i);
+          if (8 * c + i < N && e < last && e > best) best = e;
+        }
+      }
+    }
+    best = warp_max_u64(best);
+    last = best;
+    if (lane == 0) put(j, best);
+  }
+}
+
 }  // namespace
 }  // namespace vx
 
@@ -210,6 +376,14 @@ int vx_ctc_topk(const vx_gemm_desc* desc, int k, void* logits, int64_t rows, flo
     d.out_dtype = VX_BF16; d.out = logits; d.ldo = ld;
     const int rc = vx_bsgemm(&d, stream);
     if (rc) return rc;
+    // (Short rows leave most of the registers empty, and half the warps per SM to wait for them: N = 300, 15,000 rows 29 us with two
+    // passes, 42 in registers; N = 1,032 42 and 40, N = 4,096 89 and 75, N = 5,538 148 and 122.)
+    if (N > TR_MIN_N && N <= TR_PIECES * 32 * 8) {
+      VX_CUDA_OK(launch_dependent(topk_regs_kernel, dim3(static_cast<unsigned>((m + TR_WARPS - 1) / TR_WARPS)), dim3(TR_WARPS * 32), 0,
+                                  static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(logits), ld, static_cast<int>(N),
+                                  static_cast<int>(m), k, logp + r0 * k, ids + r0 * k));
+      continue;
+    }
     VX_CUDA_OK(launch_dependent(topk_rows_kernel, dim3(static_cast<unsigned>((m + TK_WARPS - 1) / TK_WARPS)), dim3(TK_WARPS * 32), 0,
                                 static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(logits), ld, static_cast<int>(N),
                                 static_cast<int>(m), k, logp + r0 * k, ids + r0 * k));
