@@ -1052,6 +1052,7 @@ void stack_pass(const Plan& p, const at::Tensor& xt, const void* src, int64_t ld
     c.codes = q.codes; c.scales_sf = q.scales;
     check(g.vx_conformer_pass(&c, s.st), "vx_conformer_pass");
     ++s.launches;
+    for (int i = 0; i < p.blocks && with_pos && !lp_batched; ++i) sp.gemm(pos_q, p.lin[i * L_COUNT + L_LP], VX_EPI_BIAS, w_lp, d);
   } else
     s.ln_quantize(src ? src : x, src ? ld_src : ldx, p.norm[p.blocks > 0 ? N_FFM : 0], q);
   for (int i = 0; i < p.blocks && !whole; ++i) {
