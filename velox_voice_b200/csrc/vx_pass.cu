@@ -25,7 +25,7 @@
 // nothing and run ahead through rings of four and three slots.  Accumulators: a ring of three times 128 columns.
 //
 // Measured, whole greedy pass of 12 blocks, separate launches against this: 375 frames 752 us -> 581, 1,920 frames (the most for
-// clusters of eight) 836 -> 594, 4,200 frames (the most for clusters of four) 1,035 -> 700.  What bounds it now, of 83,000 cycles a
+// clusters of eight) 836 -> 594, 4,000 frames (clusters of four) 986 -> 717, 4,200 frames 1,036 -> 756 (its twelve positional projections are launches of their own).  What bounds it now, of 83,000 cycles a
 // block (clusters of eight): the hand-over of an operand, 4,000 a phase -- the release waits 1,750 for the stores, fence and loads take
 // 1,900 --, the issue of the MMAs, 500 to 700 cycles per stage of four, and the chain accumulator -> sums -> exchange -> quantize of
 // the four LayerNorms, 4,000 each.  Tried and not kept: operands pushed to the other CTAs' shared memory by st.async (630 us) or bulk
@@ -745,8 +745,8 @@ int vx_conformer_pass_supported(int fmt, int64_t d_model, int64_t ffn, int64_t c
          blocks <= PS_MAX_BLOCKS;
 }
 
-// One round of clusters of four.  4,200 frames: separate launches 1,035 us, one launch 700; a second round takes as long again, and
-// the launches that pipeline over many row blocks are as fast (4,608 frames: 1,075 and about 1,400).
+// One round of clusters of four.  4,200 frames: separate launches 1,036 us, one launch 756; a second round takes as long again, and
+// the launches that pipeline over many row blocks are as fast (4,608 frames: 1,075 and about 1,450).
 int64_t vx_conformer_pass_frames(void) {
   return static_cast<int64_t>(vx::max_clusters<4>()) * vx::PS_BM;
 }
