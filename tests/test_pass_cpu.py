@@ -25,3 +25,17 @@ def test_shapes_it_covers():
 
 def test_waits_end_in_a_vote():
     vote_rule("vx_pass.cu", "conformer_pass_kernel(")
+
+
+def test_a_line_for_the_fused_launches_takes_passes_off_the_one_launch():
+    """``fuse_ln_min_frames`` chooses between separate and fused launches for passes of every length, whenever it is assigned."""
+    from velox_voice_b200.stack import ConformerLinearStack
+
+    stack = object.__new__(ConformerLinearStack)  # (the route only: a stack's weights need a GPU)
+    stack.fuse_ln, stack.fuse_ln_min_frames = True, 4737
+    stack.one_launch_frames = 4224
+    assert [stack._route(t) for t in (1, 4224, 4225, 4736, 4737)] == [2, 2, 0, 0, 1]
+    stack.fuse_ln_min_frames = 375
+    assert [stack._route(t) for t in (1, 374, 375, 4224)] == [0, 0, 1, 1]
+    stack.fuse_ln = False
+    assert stack._route(375) == 0

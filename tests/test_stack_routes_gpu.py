@@ -103,6 +103,25 @@ def test_frames_of_the_fused_launches_are_the_callers_to_choose():
     assert count[1] == count[5000] == count[None] < count[5001] == count[1 << 30]
 
 
+@pytest.mark.parametrize("frames", [375, 5000])
+def test_frames_of_the_fused_launches_may_be_chosen_on_a_built_stack(frames):
+    """Assigned later the line holds for passes of every length, as it does when given with the configuration."""
+    from velox_voice_b200 import ops
+
+    torch.manual_seed(12)
+    x = torch.randn(frames, 512, device="cuda").bfloat16()
+    stack = build(blocks=1)
+    want = stack.forward(x.clone())
+    for least in (0, frames, frames + 1):
+        count = []
+        for given in (build(blocks=1, fuse_ln_min_frames=least), stack):
+            given.fuse_ln_min_frames = least
+            ops.reset_launch_count()
+            assert torch.equal(given.forward(x.clone()), want)
+            count.append(ops.launch_count())
+        assert count[0] == count[1] == (14 if least > frames else 10)
+
+
 def test_what_a_program_replaces_takes_effect():
     """Layers, their weights and biases, LayerNorm parameters and calibrated maxima may be replaced between passes."""
     torch.manual_seed(8)

@@ -119,13 +119,12 @@ class ConformerLinearStack:
                         and ops.residual_ln_supported(self.fmt, cfg.d_model, cfg.d_model))
         dev = self.device
         least = os.environ.get("VELOX_B200_FUSE_LN_MIN_FRAMES", cfg.fuse_ln_min_frames)
-        # frames up to which all blocks run in one launch (not where the caller draws the line between separate and fused launches)
-        self.one_launch_frames = 0
         if least is None:
+            self.fuse_ln_min_frames = fuse_ln_frames(torch.cuda.get_device_properties(dev).multi_processor_count, cfg.d_model)
             if self.fmt == FMT_MX32:
-                self.one_launch_frames = ops.conformer_pass_frames(dev)
-            least = fuse_ln_frames(torch.cuda.get_device_properties(dev).multi_processor_count, cfg.d_model)
-        self.fuse_ln_min_frames = int(least)
+                self.one_launch_frames = ops.conformer_pass_frames(dev)  # frames up to which all blocks run in one launch
+        else:
+            self.fuse_ln_min_frames = least
         self.p: Dict[str, PackedLinear] = {}
         self.ln: Dict[str, Tuple[torch.Tensor, torch.Tensor]] = {}
 
@@ -155,6 +154,26 @@ class ConformerLinearStack:
         if amax:
             for k, v in amax.items():
                 self.amax[k] = torch.tensor([v], dtype=torch.float32, device=dev)
+
+    # ---- route
+    @property
+    def fuse_ln_min_frames(self) -> int:
+        """Frames from which the residual GEMMs run the LayerNorm + quantizer behind them.  Assigning it, when the stack is built or
+        later, draws the line between separate and fused launches for passes of every length, so none runs its blocks in
+        one launch any more (``one_launch_frames`` = 0; assign that one afterwards to have both)."""
+        return self._fuse_ln_min_frames
+
+    @fuse_ln_min_frames.setter
+    def fuse_ln_min_frames(self, frames: int):
+        self._fuse_ln_min_frames = int(frames)
+        self.one_launch_frames = 0
+
+    def _route(self, frames: int) -> int:
+        """How a pass of that many frames runs its blocks, as ``vx_host.cpp`` names it: 0 separate launches, 1 LayerNorm and
+        quantizer in the residual GEMMs, 2 one launch."""
+        if not self.fuse_ln:
+            return 0
+        return 2 if frames <= self.one_launch_frames else int(frames >= self.fuse_ln_min_frames)
 
     # ---- helpers
     def _amax(self, key: str, x: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -222,11 +241,8 @@ class ConformerLinearStack:
             self._amax("pos", pos)  # must have been calibrated
         if pos is not None and pos.stride(1) != 1:
             pos = pos.contiguous()
-        route = 0
-        if self.fuse_ln:
-            route = 2 if x.shape[0] <= self.one_launch_frames else int(x.shape[0] >= self.fuse_ln_min_frames)
-        out = ops._host().stack_forward(self._host_plan(), x, pos, route, 1 if ids_only else 0, keys, ids, out_logits,
-                                         source)
+        out = ops._host().stack_forward(self._host_plan(), x, pos, self._route(x.shape[0]), 1 if ids_only else 0, keys, ids,
+                                         out_logits, source)
         return (out, x) if return_hidden and not ids_only else out
 
     def forward_ids(self, x: torch.Tensor, pos: Optional[torch.Tensor] = None, *, keys=None, ids=None):
