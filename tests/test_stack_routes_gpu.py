@@ -269,3 +269,18 @@ def test_first_pass_on_another_stream_and_in_a_capture():
     buf.copy_(x)
     graph.replay()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("fmt,frames", [("mx32", 375), ("mx32", 4200), ("mx32", 4500), ("mx32", 5000), ("nv16", 375)])
+def test_the_launches_of_the_benchmark_are_those_of_a_pass(fmt, frames):
+    from velox_voice_b200 import opbench, ops
+
+    stack = build(fmt, blocks=2)
+    x = torch.randn(frames, 512, device="cuda").bfloat16()
+    cases = opbench.op_breakdown(stack, frames, fmt)
+    ops.reset_launch_count()
+    stack.forward_ids(x.clone(), x)
+    # the entry for all blocks holds the head and, as the head's own entry, the launch that turns keys into ids
+    whole = any(n.startswith("all blocks") for n, *_ in cases)
+    assert whole == (fmt == "mx32" and frames <= stack.one_launch_frames)
+    assert sum(c for _, c, *_ in cases) + (2 if whole else 1) == ops.launch_count()

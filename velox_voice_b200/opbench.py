@@ -38,6 +38,15 @@ def _timed(fn, flush, n=5, warm=2):
     return ts[len(ts) // 2]
 
 
+def _blocks_in_one_launch(stack, T) -> bool:
+    """Whether a pass over T aligned frames runs all blocks of ``stack`` in one launch."""
+    from . import _lib
+
+    cfg = stack.cfg
+    return stack._route(T) == 2 and stack.fuse_ffn and bool(
+        _lib.load().vx_conformer_pass_supported(stack.fmt, cfg.d_model, cfg.ffn, cfg.conv_pw, cfg.blocks))
+
+
 def op_breakdown(stack, T, fmt_name, only=""):
     """Times every distinct launch of one block (+ CTC) alone, L2 flushed before each timed
     launch, and returns [(name, count_per_step, us, algorithmic_bytes, flops)]."""
@@ -69,11 +78,20 @@ def op_breakdown(stack, T, fmt_name, only=""):
             return
         cases.append((name, count, _timed(fn, flush), nbytes, flops))
 
-    # the LayerNorms behind residual GEMMs run in those GEMMs (long inputs only, see StackConfig)
-    fused = bool(getattr(stack, "fuse_ln", False)) and T >= stack.fuse_ln_min_frames
-    add("ln_quantize [T,512]", 1 if fused else 3 * nb + 1, lambda: ops.ln_quantize(x, g, b, cfg.eps, fmt, amax_t=am),
+    # the LayerNorms behind residual GEMMs run in those GEMMs (long inputs), or all blocks are one launch (short MX32 passes)
+    whole = _blocks_in_one_launch(stack, T)
+    fused = stack._route(T) == 1
+    steps = 0 if whole else nb  # blocks whose layers are launches of their own
+    if whole:
+        keys, ids = torch.empty(T, dtype=torch.int64, device=dev), torch.empty(T, dtype=torch.int32, device=dev)
+        buf = torch.empty_like(x)
+        add("all blocks in one launch, arg-max head", 1,
+            lambda: stack.forward(buf, ids_only=True, keys=keys, ids=ids, source=x),
+            T * d * 2 + nb * (2 * (qbytes(f, d) + qbytes(d, f)) + qbytes(7 * d, d)) + qbytes(V, d) + T * 12,
+            T * (cfg.flops_per_frame() - nb * 2 * d * d))
+    add("ln_quantize [T,512]", 0 if whole else 1 if fused else 3 * nb + 1, lambda: ops.ln_quantize(x, g, b, cfg.eps, fmt, amax_t=am),
         T * d * 2 + qbytes(T, d), 0)
-    add("ln2_quantize [T,512] (norm_final + next LayerNorm + quantize)", 0 if fused else nb,
+    add("ln2_quantize [T,512] (norm_final + next LayerNorm + quantize)", 0 if fused else steps,
         lambda: ops.ln2_quantize(x, g, b, g, b, cfg.eps, fmt, y=x, amax_t=am), T * d * 4 + qbytes(T, d), 0)
     # (FP4: a step quantizes the value third of q | k | v and the GLU output in their GEMMs' epilogues)
     fp4 = fmt_name != "fp8_1x128"
@@ -82,7 +100,7 @@ def op_breakdown(stack, T, fmt_name, only=""):
     w1, w2 = stack.p["b0.ffm.w1"], stack.p["b0.ffm.w2"]
     if stack.fuse_ffn:
         hq = w1(xq, act="swish", out_fmt=fmt, out_amax=stack.amax.get("b0.ffm.h"))
-        add("gemm ffn-up 512->2048 swish, FP4 out", 2 * nb,
+        add("gemm ffn-up 512->2048 swish, FP4 out", 2 * steps,
             lambda: w1(xq, act="swish", out_fmt=fmt, out_amax=stack.amax.get("b0.ffm.h")),
             qbytes(T, d) + qbytes(f, d) + qbytes(T, f), 2 * T * d * f)
     else:
@@ -92,9 +110,9 @@ def op_breakdown(stack, T, fmt_name, only=""):
             qbytes(T, d) + qbytes(f, d) + T * f * 2, 2 * T * d * f)
         add("quantize [T,2048]", 2 * nb, lambda: ops.quantize(h, fmt, natural=fmt_name == "fp8_1x128"),
             T * f * 2 + qbytes(T, f), 0)
-    add("gemm ffn-down 2048->512 +0.5 residual", 0 if fused else 2 * nb, lambda: w2(hq, residual=res, alpha=0.5, out=res),
+    add("gemm ffn-down 2048->512 +0.5 residual", 0 if fused else 2 * steps, lambda: w2(hq, residual=res, alpha=0.5, out=res),
         qbytes(T, f) + qbytes(d, f) + T * d * 4, 2 * T * d * f)
-    add("gemm qkv 512->1536 bias", nb, lambda: stack.p["b0.qkv"](xq), qbytes(T, d) + qbytes(3 * d, d) + T * 3 * d * 2,
+    add("gemm qkv 512->1536 bias", steps, lambda: stack.p["b0.qkv"](xq), qbytes(T, d) + qbytes(3 * d, d) + T * 3 * d * 2,
         2 * T * d * 3 * d)
     if fused:
         add("gemm ffn-down 2048->512 +0.5 residual + LayerNorm + quantize (2-CTA clusters)", nb,
@@ -106,17 +124,23 @@ def op_breakdown(stack, T, fmt_name, only=""):
         add("gemm lo/pw2 512->512 +residual + LayerNorm + quantize (2-CTA clusters)", 2 * nb,
             lambda: stack.p["b0.lo"].residual_ln(xq, residual=res, gamma=g, beta=b, eps=cfg.eps, alpha=1.0, out=res),
             qbytes(T, d) + qbytes(d, d) + T * d * 4 + qbytes(T, d), 2 * T * d * d)
-    add("gemm lo/pw2 512->512 +residual", 0 if fused else 2 * nb, lambda: stack.p["b0.lo"](xq, residual=res, alpha=1.0, out=res),
+    add("gemm lo/pw2 512->512 +residual", 0 if fused else 2 * steps, lambda: stack.p["b0.lo"](xq, residual=res, alpha=1.0, out=res),
         qbytes(T, d) + qbytes(d, d) + T * d * 4, 2 * T * d * d)
-    add("gemm lp 512->512", nb, lambda: stack.p["b0.lp"](xq), qbytes(T, d) + qbytes(d, d) + T * d * 2, 2 * T * d * d)
+    # (positional projections of all blocks as one weight up to this many rows: LP_BATCH_MAX of vx_host.cpp)
+    together = stack._positions is not None and T <= 4096
+    add("gemm lp 512->512", 0 if together else nb, lambda: stack.p["b0.lp"](xq), qbytes(T, d) + qbytes(d, d) + T * d * 2,
+        2 * T * d * d)
+    if together:
+        add(f"gemm lp of all blocks 512->{nb * d}", 1, lambda: ops.bsgemm(xq, stack._positions),
+            qbytes(T, d) + qbytes(nb * d, d) + T * nb * d * 2, 2 * T * d * nb * d)
     if fp4:
         glu_am = stack.amax.get("b0.glu")
-        add("gemm pw1 512->1024 GLU, FP4 out", nb, lambda: stack.p["b0.pw1"](xq, out_fmt=fmt, out_amax=glu_am),
+        add("gemm pw1 512->1024 GLU, FP4 out", steps, lambda: stack.p["b0.pw1"](xq, out_fmt=fmt, out_amax=glu_am),
             qbytes(T, d) + qbytes(2 * d, d) + qbytes(T, d), 2 * T * d * 2 * d)
     else:
         add("gemm pw1 512->1024 GLU", nb, lambda: stack.p["b0.pw1"](xq), qbytes(T, d) + qbytes(2 * d, d) + T * d * 2,
             2 * T * d * 2 * d)
-    add("gemm ctc 512->5538 bias + argmax (no logits written)", 1, lambda: stack.p["ctc"].argmax(xq),
+    add("gemm ctc 512->5538 bias + argmax (no logits written)", 0 if whole else 1, lambda: stack.p["ctc"].argmax(xq),
         qbytes(T, d) + qbytes(V, d) + T * 12, 2 * T * d * V)
     if only and "mel" in only:
         # the audio front-end's filterbank projection (not part of the encoder step): one hour of 10 ms frames
