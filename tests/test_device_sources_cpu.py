@@ -63,6 +63,18 @@ def test_the_gemm_triggers_the_next_launch_only_behind_its_own_wait():
     assert re.search(r"if \(warp != 0 \|\| my_tiles == 0\) {\s*pdl_wait\(\);\s*pdl_launch_dependents\(\);\s*}", text)
 
 
+@pytest.mark.parametrize("name,barrier", [("vx_gemm.cu", "empty"), ("vx_gemm_ln.cu", "empty"), ("vx_gemm_ln.cu", "hb_empty"),
+                                          ("vx_pass.cu", "b_empty")])
+def test_loaders_that_run_ahead_wait_for_the_previous_launch_before_a_bounded_wait(name, barrier):
+    """A ring that is full empties only when the MMAs start, behind the previous launch: the limit of a wait is for this kernel's
+    own progress, so whoever loads constant weights ahead waits for that launch once before waiting for a slot to be free."""
+    text = source(name)
+    wait = re.search(r"mbar_wait\w*(<\w+>)?\(&sm\.%s\[" % barrier, text).start()
+    role = text[text.rindex("if (warp == ", 0, wait):wait]
+    waits = re.findall(r"if \(([^\n]*)\) (?:\{ )?pdl_wait\(\)", role)
+    assert "p.b_const" in waits or any(w in ("ph && !waited", "!par && !waited") for w in waits), (name, waits)
+
+
 def test_the_wait_for_the_other_ctas_sums_acquires_at_cluster_scope():
     """st.async of the peer completes the exchange barrier with a release at cluster scope; a wait that acquires at the default
     scope, the CTA, does not pair with it."""

@@ -211,12 +211,13 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     // =========================== loader of B, streaming plan ===========================
     if (lane == 0 && my_tiles > 0 && !resident) {
       uint32_t s = 0, ph = 0;
-      bool ok = true;
-      if (!p.b_const) pdl_wait();
+      bool ok = true, waited = !p.b_const;
+      if (waited) pdl_wait();
       const uint8_t* const sf0 = p.sfb + static_cast<int64_t>(rank * 2) * p.sf_kg * 512;
       const int64_t sf_tile = p.sf_kg * 512;
       for (int i = 0; i < my_tiles && ok; ++i) {
         for (int kh = 0; kh < 2 * p.k_stages; ++kh) {
+          if (ph && !waited) { pdl_wait(); waited = true; }  // a ring ahead; the limit of the waits is not for the previous launch
           if (!mbar_wait(&sm.hb_empty[s], ph ^ 1, p.status, 28)) { ok = false; break; }
           uint8_t* dst = sm.arena + s * LN_HB_SLOT;
           mbar_expect_tx(&sm.hb_full[s], LN_HB_SLOT);

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) conformer_pass_kernel(const __g
     // =========================== weights ===========================
     if (lane == 0) {
       uint32_t s = 0, par = 1;
-      bool ok = true;
+      bool ok = true, waited = !p.b_const;
 #pragma unroll 1
       for (int mt = cluster; mt < p.m_tiles && ok; mt += nclusters)
 #pragma unroll 1
@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) conformer_pass_kernel(const __g
               const uint8_t* const sf_row = sf + static_cast<int64_t>(row0 >> 7) * stages * 1024;
 #pragma unroll 1
               for (int ks = 0; ks < stages; ks += n) {
+                if (!par && !waited) { pdl_wait(); waited = true; }  // a ring ahead; the limit of the waits is not for the previous launch
                 if (!mbar_wait(&sm.b_empty[s], par, p.status, 41)) { ok = false; break; }
                 mbar_expect_tx(&sm.b_full[s], n * (tile + 1024));
                 tma_load_2d(sm.b[s], map, ks * 128, row0, &sm.b_full[s]);
