@@ -305,7 +305,8 @@ int vx_ctc_topk(const vx_gemm_desc* desc, int k, void* logits, int64_t rows, flo
  *   lin: E2M1 codes u8 [N, K/2] (row stride ld bytes), scale-factor atoms, bias f32 [N] (16-byte aligned), in the order
  *        ffm.w1, ffm.w2, qkv, lo, pw1 (rows interleaved per vx_glu_tile), pw2, ff.w1, ff.w2;
  *   gamma, beta: f32 [512], 16-byte aligned, of LN_ffm, LN_mha, LN_conv, LN_ff, LN_final;
- *   const_weights: nonzero when no launch just before this one writes the weights (VX_GEMM_CONST_B of every GEMM);
+ *   const_weights: nonzero when no launch just before this one writes the weights' codes and scale factors (VX_GEMM_CONST_B of every
+ *        GEMM); biases and LayerNorm parameters are read behind the wait for that launch either way;
  *   src: features bf16 [M, 512]; x: the residual stream after the last block, bf16 [M, 512] (may be src);
  *   qkv: bf16 [M, 1536], left with the last block's q | k | v; scratch: vx_conformer_pass_scratch(M, ffn) bytes;
  *   codes u8 [M, 256], scales_sf: quantize(LN_after(x)) as vx_ln_quantize_pack leaves it. */

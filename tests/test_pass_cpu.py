@@ -1,7 +1,9 @@
 """The one-launch pass: argument checks without a device, and the rule for waits in front of warp-wide tensor-memory accesses."""
 
 import ctypes as C
+import re
 
+from test_device_sources_cpu import source
 from test_device_sources_cpu import test_waits_before_warp_wide_tensor_memory_accesses_end_in_a_vote as vote_rule
 from velox_voice_b200 import _lib
 
@@ -39,3 +41,11 @@ def test_a_line_for_the_fused_launches_takes_passes_off_the_one_launch():
     assert [stack._route(t) for t in (1, 374, 375, 4224)] == [0, 0, 1, 1]
     stack.fuse_ln = False
     assert stack._route(375) == 0
+
+
+def test_only_constant_weights_are_read_ahead_of_the_previous_launch():
+    """The launch before may have written a bias or a LayerNorm parameter; the flag speaks of weights.  Whoever triggers the next
+    launch has waited."""
+    text = source("vx_pass.cu")
+    assert re.search(r"if \(warp != PS_WARP_B\) {\s*pdl_wait\(\);\s*pdl_launch_dependents\(\);\s*} else if \(!p.b_const\) {\s*pdl_wait\(\);\s*}", text)
+    assert text.count("pdl_launch_dependents()") == 1

@@ -105,3 +105,26 @@ def test_passes_on_two_streams():
                 got[i].append(stack.forward(xs[i].clone()))
     torch.cuda.synchronize()
     assert all(torch.equal(o, want[i]) for i in range(2) for o in got[i])
+
+
+def test_a_bias_that_the_launch_before_wrote():
+    """A library GEMM triggers the launch behind it early; the pass reads its biases behind that GEMM's end."""
+    from velox_voice_b200 import ops
+
+    stack = build(blocks=1, vocab=64)
+    x = torch.randn(100, 512, device="cuda").bfloat16()
+    w = ops.quantize(torch.randn(2048, 512, device="cuda"), "mx32")
+    bias = stack.p["b0.ffm.w1"].bias = torch.zeros(1, 2048, device="cuda")[0]
+    acts = [ops.quantize(torch.randn(1, 512, device="cuda"), "mx32") for _ in range(8)]
+    want = []
+    for a in acts:
+        ops.bsgemm(a, w, out=bias[None])
+        torch.cuda.synchronize()
+        want.append(stack.forward(x.clone()))
+    assert not torch.equal(want[0], want[1])
+    for _ in range(10):
+        got, xs = [], [x.clone() for _ in acts]
+        for a, xx in zip(acts, xs):
+            ops.bsgemm(a, w, out=bias[None])
+            got.append(stack.forward(xx))
+        assert all(torch.equal(g, v) for g, v in zip(got, want))

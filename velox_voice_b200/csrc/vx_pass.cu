@@ -22,7 +22,7 @@
 //
 // Warps: 0..15 epilogue, warp (q, g) = tensor-memory lane quadrant q, 32-column unit g of a job (a thread is a row); 16 loads
 // activations, 17 issues the MMAs (one elected lane), 18 and 19 load weights and the biases and LayerNorm parameters, which depend on
-// nothing and run ahead through rings of four and three slots.  Accumulators: a ring of three times 128 columns.
+// no layer and run ahead of them through rings of four and three slots.  Accumulators: a ring of three times 128 columns.
 //
 // Measured, whole greedy pass of 12 blocks, separate launches against this: 375 frames 752 us -> 581, 1,920 frames (the most for
 // clusters of eight) 836 -> 594, 4,000 frames (clusters of four) 986 -> 717, 4,200 frames 1,036 -> 756 (its twelve positional projections are launches of their own).  What bounds it now, of 83,000 cycles a
@@ -187,9 +187,10 @@ __global__ void __launch_bounds__(PS_THREADS, 1) conformer_pass_kernel(const __g
   tc_fence_after();
   cluster_sync_all();  // every CTA's barriers exist before anything is sent to them
   const uint32_t tmem_base = sm.tmem_base;
-  // (The loaders of weights and parameters run ahead; the weights' loader waits if the weights may just have been written.  The
-  // trigger: behind the wait, by warps that have waited, as in vx_gemm.cu; the head's CTAs set up on the SMs this grid leaves idle.)
-  if (warp != PS_WARP_B && warp != PS_WARP_P) {
+  // (Only weights are read ahead, if the caller calls them constant: biases and LayerNorm parameters may be what the launch before
+  // wrote, as for the separate launches.  The trigger: behind the wait, by warps that have waited, as in vx_gemm.cu; the head's
+  // CTAs set up on the SMs this grid leaves idle.)
+  if (warp != PS_WARP_B) {
     pdl_wait();
     pdl_launch_dependents();
   } else if (!p.b_const) {
