@@ -42,6 +42,27 @@ def test_waits_before_warp_wide_tensor_memory_accesses_end_in_a_vote(name, kerne
             assert open_wait is None, f"{name}: {t} can be reached by a part of a warp behind {open_wait!r}"
 
 
+@pytest.mark.parametrize("name,kernel", [("vx_gemm_ln.cu", "bsgemm_residual_ln_kernel("), ("vx_pass.cu", "conformer_pass_kernel(")])
+def test_no_lane_of_a_warp_stays_behind_when_a_limit_runs_out(name, kernel):
+    """The kernels of clusters end in a barrier that every thread has to reach.  A limit that runs out for some lanes of a warp while
+    the barrier completes for the others must not part them at a __syncwarp: each wait is one thread's, or a vote, or its
+    outcome ends no loop (no MMA is issued for a lane that gave up, and it waits for nothing more)."""
+    text = source(name)
+    text = text[text.index(kernel):]
+    text = text[:re.search(r"\n}\n", text).end()]
+    start, end = text.index("elect_one()"), text.rindex("  } else {\n", 0, text.index("const int row_in"))
+    mma = text[start:end]
+    together = "__syncwarp" in mma
+    if together:
+        assert "break" not in mma and not re.search(r"for \([^\n]*\bok\b", mma)
+        assert len(re.findall(r"if \(leader && ok\)", mma)) == mma.count("if (leader")
+    for m in re.finditer(r"\bmbar_wait\w*\(", text):
+        line = text[text.rfind("\n", 0, m.start()):text.index("\n", m.start())]
+        role = text[text.rindex("if (warp == ", 0, m.start()):m.start()]
+        alone = re.match(r"[^{]*{\s*if \((lane == 0\b[^\n]*|elect_one\(\)\)) {", role)
+        assert alone or "__all_sync" in line or (together and start < m.start() < end), f"{name}: {line.strip()}"
+
+
 @pytest.mark.parametrize("name", ["vx_gemm_ln.cu", "vx_gemm.cu"])
 def test_stores_are_complete_before_a_kernel_ends(name):
     """Writes of a bulk store are ordered by waiting for its group, not by the end of the thread that issued it; the `.read`

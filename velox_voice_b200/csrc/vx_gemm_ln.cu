@@ -233,7 +233,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     if (my_tiles > 0) {
       const bool leader = elect_one();
       uint32_t s = 0, ph = 0, bs = 0, bph = 0, sfsel = 0;
-      bool ok = true;
+      bool ok = true;  // a lane whose limit ran out goes on without waits or MMAs: none stays behind at a __syncwarp
       const uint32_t idesc_base = make_idesc_mxf4(LN_BM, LN_BN, true);
       const uint32_t k128_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
       const uint32_t k64_hi = (512u >> 4) | (1u << 14) | (4u << 29);  // rows of 64 bytes, 64-byte swizzle
@@ -250,28 +250,28 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             tc_cp_32x128b_warpx4(col0 + a * 8 + rt * 4, desc(b_lo + (LN_B_TILE >> 4) + (rt * 2 + a) * 32, sf_hi));
       };
       if (resident) {
-        if (!mbar_wait(&sm.b_full, 0, p.status, 26)) ok = false;
+        ok = mbar_wait(&sm.b_full, 0, p.status, 26);
         tc_fence_after();
-        if (ok && leader)  // B's scale factors stay in tensor memory for the whole kernel
+        if (leader && ok)  // B's scale factors stay in tensor memory for the whole kernel
           for (int ks = 0; ks < p.k_stages; ++ks) cp_sfb(arena_lo + ks * (LN_B_SLOT >> 4), tmem_base + LN_TM_SFB + ks * 16);
         __syncwarp();
       }
-      for (int i = 0; i < my_tiles && ok; ++i) {
+      for (int i = 0; i < my_tiles; ++i) {
         // the epilogue has read the previous accumulator out (pass 1 of tile i - 1)
-        if (!mbar_wait_spin(&sm.tmem_empty, (i & 1) ^ 1, p.status, 22)) { ok = false; break; }
+        if (ok) ok = mbar_wait_spin(&sm.tmem_empty, (i & 1) ^ 1, p.status, 22);
         tc_fence_after();
-        for (int ks = 0; ks < p.k_stages && ok; ++ks) {
-          if (!mbar_wait_spin(&sm.full[s], ph, p.status, 23)) { ok = false; break; }
+        for (int ks = 0; ks < p.k_stages; ++ks) {
+          if (ok) ok = mbar_wait_spin(&sm.full[s], ph, p.status, 23);
           tc_fence_after();
           const uint32_t a_lo = ring_lo + s * (LN_A_SLOT >> 4);
           const uint32_t sfa_buf = tmem_base + LN_TM_SFA + sfsel * 32;
-          if (leader) {
+          if (leader && ok) {
 #pragma unroll
             for (int a = 0; a < 2; ++a) tc_cp_32x128b_warpx4(sfa_buf + a * 4, desc(a_lo + (LN_A_TILE >> 4) + a * 32, sf_hi));
           }
           if (resident) {
             const uint32_t b_lo = arena_lo + ks * (LN_B_SLOT >> 4), sfb_buf = tmem_base + LN_TM_SFB + ks * 16;
-            if (leader) {
+            if (leader && ok) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 const uint32_t atom = j >> 1, sf_id = (j & 1) * 2;
@@ -283,10 +283,10 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           } else {
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-              if (!mbar_wait_spin(&sm.hb_full[bs], bph, p.status, 29)) { ok = false; break; }
+              if (ok) ok = mbar_wait_spin(&sm.hb_full[bs], bph, p.status, 29);
               tc_fence_after();
               const uint32_t b_lo = arena_lo + bs * (LN_HB_SLOT >> 4), sfb_buf = tmem_base + LN_TM_SFB + bs * 16;
-              if (leader) {
+              if (leader && ok) {
 #pragma unroll
                 for (int rt = 0; rt < 2; ++rt) tc_cp_32x128b_warpx4(sfb_buf + rt * 4, desc(b_lo + (LN_HB_TILE >> 4) + rt * 32, sf_hi));
 #pragma unroll
@@ -298,9 +298,8 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
               __syncwarp();
               if (++bs == LN_HB_SLOTS) { bs = 0; bph ^= 1; }
             }
-            if (!ok) break;
           }
-          if (leader) {
+          if (leader && ok) {
             tc_commit(&sm.empty[s]);
             if (ks == p.k_stages - 1) tc_commit(&sm.tmem_full);
           }

@@ -296,39 +296,39 @@ __global__ void __launch_bounds__(PS_THREADS, 1) conformer_pass_kernel(const __g
     }
   } else if (warp == PS_WARP_MMA) {
     // =========================== MMA issuer ===========================
-    const bool leader = elect_one();
-    const uint32_t b_hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // rows of 128 bytes, 128-byte swizzle
-    const uint32_t a_hi = (128u >> 4) | (1u << 14);                // no swizzle: 128 bytes to the next eight rows ...
-    const uint32_t a_lbo = static_cast<uint32_t>(PS_BLOCK >> 4) << 16;  // ... and a block to the next 16 bytes of K
-    const uint32_t sf_hi = (128u >> 4) | (1u << 14);
-    auto desc = [](uint32_t lo, uint32_t hi) -> uint64_t { return (static_cast<uint64_t>(hi) << 32) | lo; };
-    const uint32_t a_lo0 = smem_u32(sm.a) >> 4, b_lo0 = smem_u32(sm.b) >> 4;
-    uint32_t as = 0, apar = 0, bs = 0, bpar = 0, acc = 0, accpar = 1, sfsel = 0;
-    bool ok = true;
+    // (one thread: lanes that wait together could part where a limit runs out, unless they vote, 587 us for 375 frames against 580)
+    if (elect_one()) {
+      const uint32_t b_hi = (1024u >> 4) | (1u << 14) | (2u << 29);  // rows of 128 bytes, 128-byte swizzle
+      const uint32_t a_hi = (128u >> 4) | (1u << 14);                // no swizzle: 128 bytes to the next eight rows ...
+      const uint32_t a_lbo = static_cast<uint32_t>(PS_BLOCK >> 4) << 16;  // ... and a block to the next 16 bytes of K
+      const uint32_t sf_hi = (128u >> 4) | (1u << 14);
+      auto desc = [](uint32_t lo, uint32_t hi) -> uint64_t { return (static_cast<uint64_t>(hi) << 32) | lo; };
+      const uint32_t a_lo0 = smem_u32(sm.a) >> 4, b_lo0 = smem_u32(sm.b) >> 4;
+      uint32_t as = 0, apar = 0, bs = 0, bpar = 0, acc = 0, accpar = 1, sfsel = 0;
+      bool ok = true;
 #pragma unroll 1
-    for (int mt = cluster; mt < p.m_tiles && ok; mt += nclusters)
+      for (int mt = cluster; mt < p.m_tiles && ok; mt += nclusters)
 #pragma unroll 1
-      for (int i = 0; i < PH_COUNT * p.blocks && ok; ++i) {
-        const int ph = i & (PH_COUNT - 1);
-        const int stages = phase_stages(ph, ffn), jobs = G::jobs(ph, ffn), n = G::slot_stages(ph);
-        const uint32_t tile = G::cols(ph) * 128 >> 4, idesc = make_idesc_mxf4(PS_BM, G::cols(ph), true);
+        for (int i = 0; i < PH_COUNT * p.blocks && ok; ++i) {
+          const int ph = i & (PH_COUNT - 1);
+          const int stages = phase_stages(ph, ffn), jobs = G::jobs(ph, ffn), n = G::slot_stages(ph);
+          const uint32_t tile = G::cols(ph) * 128 >> 4, idesc = make_idesc_mxf4(PS_BM, G::cols(ph), true);
 #pragma unroll 1
-        for (int j = 0; j < jobs && ok; ++j) {
-          // a job's weight rows may be part of a 128-row scale-factor tile: column of their first group of 32 rows
-          const uint32_t sfc = static_cast<uint32_t>(G::row0(ph, j, rank, ffn) & 127) >> 5;
-          if (!mbar_wait(&sm.tm_empty[acc], accpar, p.status, 44)) { ok = false; break; }
-          uint32_t s = as, par = apar, in_slot = 0;
+          for (int j = 0; j < jobs && ok; ++j) {
+            // a job's weight rows may be part of a 128-row scale-factor tile: column of their first group of 32 rows
+            const uint32_t sfc = static_cast<uint32_t>(G::row0(ph, j, rank, ffn) & 127) >> 5;
+            if (!mbar_wait(&sm.tm_empty[acc], accpar, p.status, 44)) { ok = false; break; }
+            uint32_t s = as, par = apar, in_slot = 0;
 #pragma unroll 1
-          for (int ks = 0; ks < stages; ++ks) {
-            if (in_slot == 0 && !mbar_wait(&sm.b_full[bs], bpar, p.status, 45)) { ok = false; break; }
-            // (jobs behind the first find the phase's two stages in place; the last one releases them)
-            if (j == 0 && !mbar_wait(&sm.a_full[s], par, p.status, 46)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t a_lo = a_lo0 + s * (PS_STAGE >> 4);
-            const uint32_t slot_lo = b_lo0 + bs * (PS_B_SLOT >> 4), b_lo = slot_lo + in_slot * tile, b_sf = slot_lo + n * tile + in_slot * 64;
-            const uint32_t sfa = tmem_base + PS_TM_SFA + (ks & 1) * 16, sfb = tmem_base + PS_TM_SFB + sfsel * 8;
-            const bool slot_done = in_slot + 1 == static_cast<uint32_t>(n);
-            if (leader) {
+            for (int ks = 0; ks < stages; ++ks) {
+              if (in_slot == 0 && !mbar_wait(&sm.b_full[bs], bpar, p.status, 45)) { ok = false; break; }
+              // (jobs behind the first find the phase's two stages in place; the last one releases them)
+              if (j == 0 && !mbar_wait(&sm.a_full[s], par, p.status, 46)) { ok = false; break; }
+              tc_fence_after();
+              const uint32_t a_lo = a_lo0 + s * (PS_STAGE >> 4);
+              const uint32_t slot_lo = b_lo0 + bs * (PS_B_SLOT >> 4), b_lo = slot_lo + in_slot * tile, b_sf = slot_lo + n * tile + in_slot * 64;
+              const uint32_t sfa = tmem_base + PS_TM_SFA + (ks & 1) * 16, sfb = tmem_base + PS_TM_SFB + sfsel * 8;
+              const bool slot_done = in_slot + 1 == static_cast<uint32_t>(n);
               if (j == 0) {  // (scale factors of the two stages of K = 512 stay in tensor memory for the other jobs)
 #pragma unroll
                 for (int t = 0; t < 4; ++t) tc_cp_32x128b_warpx4(sfa + t * 4, desc((a_lo + (PS_STAGE_SF >> 4) + t * 32) & 0x3fffu, sf_hi));
@@ -343,20 +343,19 @@ __global__ void __launch_bounds__(PS_THREADS, 1) conformer_pass_kernel(const __g
               if (slot_done) tc_commit(&sm.b_empty[bs]);
               if (j == jobs - 1) tc_commit(&sm.a_empty[s]);
               if (ks == stages - 1) tc_commit(&sm.tm_full[acc]);
+              sfsel = (sfsel + 1) & 3;
+              ++in_slot;
+              if (slot_done) {
+                in_slot = 0;
+                if (++bs == PS_B_SLOTS) { bs = 0; bpar ^= 1; }
+              }
+              if (++s == PS_A_SLOTS) { s = 0; par ^= 1; }
             }
-            __syncwarp();
-            sfsel = (sfsel + 1) & 3;
-            ++in_slot;
-            if (slot_done) {
-              in_slot = 0;
-              if (++bs == PS_B_SLOTS) { bs = 0; bpar ^= 1; }
-            }
-            if (++s == PS_A_SLOTS) { s = 0; par ^= 1; }
+            if (j == jobs - 1) { as = s; apar = par; }
+            if (++acc == PS_ACCS) { acc = 0; accpar ^= 1; }
           }
-          if (j == jobs - 1) { as = s; apar = par; }
-          if (++acc == PS_ACCS) { acc = 0; accpar ^= 1; }
         }
-      }
+    }
   } else {
     // =========================== epilogue ===========================
     const int q = warp & 3, g = warp >> 2;
