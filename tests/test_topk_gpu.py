@@ -150,3 +150,17 @@ def test_widths_around_the_kernels_ranges(ops, N, k):
     bias[N // 2] = float("nan")  # no column is a NaN's winner, and every log-probability of the row is one
     logp, ids = ops.bsgemm_topk(a, b, bias, k)
     assert torch.isnan(logp).all() and (ids != N // 2).all()
+
+
+@pytest.mark.parametrize("equal", [60, 100, 200])
+def test_a_nan_is_no_winner_among_many_equal_logits(ops, equal):
+    """Fewer equal winners than a row's lists hold, more pieces than listed, more columns than listed: the rescans leave a NaN out as
+    the lists do."""
+    M, N, k = 5, 5538, 6
+    a = ops.quantize(torch.randn(M, 512, device="cuda"), "mx32", natural=False)
+    zero = ops.quantize(torch.zeros(N, 512, device="cuda"), "mx32")
+    bias = torch.zeros(N, device="cuda")
+    top = 11 + 24 * torch.arange(equal, device="cuda")  # a piece of its own each
+    bias[top], bias[1000] = 2.0, float("nan")
+    logp, ids = ops.bsgemm_topk(a, zero, bias, k)
+    assert torch.equal(ids, top[:k].expand(M, k)) and torch.isnan(logp).all()

@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(TR_WARPS * 32, 2) topk_regs_kernel(const __nv_
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const unsigned long long e = topk_key(z[i], 8 * c + i);
-          if (8 * c + i < N && e < last && e > best) best = e;
+          if (8 * c + i < N && z[i] >= thr && e < last && e > best) best = e;  // (no NaN, as in the list)
         }
       }
     }
