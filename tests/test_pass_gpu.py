@@ -56,23 +56,31 @@ def test_rows_that_are_not_finite_stay_to_themselves():
     assert torch.equal(got[keep], clean[keep])
 
 
-@pytest.mark.parametrize("offset,pitch", [(8, 528), (4, 520), (0, 516)])
-def test_rows_of_any_address_and_pitch(offset, pitch):
-    """Rows of 16-byte pieces take the one launch; what others do is what the separate launches do."""
+@pytest.mark.parametrize("offset,pitch,refused", [(8, 528, None), (0, 512, None), (4, 520, "x rows must be 16-byte aligned"),
+                                                  (0, 516, "x rows must be 16-byte aligned"), (0, 256, "x rows must be 16-byte aligned"),
+                                                  (0, 0, "x rows must be 16-byte aligned")])
+def test_rows_of_any_address_and_pitch(offset, pitch, refused):
+    """Rows of 16-byte pieces take the one launch; others are refused in the words of the separate launches."""
+    from velox_voice_b200 import ops
+    from velox_voice_b200._lib import VeloxError
+
     stack = build(blocks=1)
     x = torch.randn(150, 512, device="cuda").bfloat16()
-    limit, out = stack.one_launch_frames, []
-    for stack.one_launch_frames in (limit, 0):
-        wide = torch.zeros(150 * pitch + offset, device="cuda", dtype=torch.bfloat16)
-        view = wide[offset:].view(150, pitch)[:, :512]
-        view.copy_(x)
-        try:
-            out.append(stack.forward(view).clone())
-        except Exception as e:
-            out.append(str(e))
-    assert torch.equal(*out) if torch.is_tensor(out[0]) else out[0] == out[1]
-    if offset % 8 == 0 and pitch % 8 == 0:
-        assert torch.equal(out[0], stack.forward(x.clone()))
+    limit = stack.one_launch_frames
+    for frames in (limit, 0):
+        stack.one_launch_frames = frames
+        view = torch.zeros(150 * max(pitch, 512) + offset, device="cuda", dtype=torch.bfloat16).as_strided((150, 512), (pitch, 1), offset)
+        for source in (False, True):
+            call = (lambda: stack.forward(torch.empty_like(x), source=view)) if source else lambda: stack.forward(view)
+            if refused:
+                with pytest.raises(VeloxError, match=refused):
+                    call()
+                continue
+            view.copy_(x)
+            ops.reset_launch_count()
+            got = call()
+            assert ops.launch_count() == (2 if frames else 14)
+            assert torch.equal(got, stack.forward(x.clone()))
 
 
 def test_a_layer_without_bias_runs_separately():

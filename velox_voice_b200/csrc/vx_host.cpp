@@ -971,7 +971,8 @@ bool one_launch(const Plan& p, const void* x, int64_t ldx, const void* src, int6
   }
   for (const Norm& n : p.norm)
     if (((reinterpret_cast<uintptr_t>(n.g) | reinterpret_cast<uintptr_t>(n.b)) & 15) != 0) return false;
-  return ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(src)) & 15) == 0 && ((ldx | ld_src) & 7) == 0;
+  // (rows that overlap are for the separate launches to refuse)
+  return ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(src)) & 15) == 0 && ((ldx | ld_src) & 7) == 0 && ldx >= p.d && ld_src >= p.d;
 }
 
 // Every launch of one pass.  `src` (row stride ld_src): the features, where they are not in x; `pt`: the positions, or not
