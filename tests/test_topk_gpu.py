@@ -164,3 +164,17 @@ def test_a_nan_is_no_winner_among_many_equal_logits(ops, equal):
     bias[top], bias[1000] = 2.0, float("nan")
     logp, ids = ops.bsgemm_topk(a, zero, bias, k)
     assert torch.equal(ids, top[:k].expand(M, k)) and torch.isnan(logp).all()
+
+
+@pytest.mark.parametrize("N", [1500, 5538])
+def test_log_probability_of_two_equal_logits(ops, N):
+    """Rows held in registers: log(1/2) for logits c in [16, 32): the log-sum-exp c + log 2 is rounded once (2^-20), exponential and logarithm take up to
+    3.6e-7, and the rounding of c log2 e (up to 2^-19 log 2) must not come on top."""
+    a = ops.quantize(torch.randn(3, 512, device="cuda"), "mx32", natural=False)
+    zero = ops.quantize(torch.zeros(N, 512, device="cuda"), "mx32")
+    for c in torch.arange(16, 31, 0.125):
+        bias = torch.full((N,), float("-inf"), device="cuda")
+        bias[7], bias[N // 2] = c, c
+        logp, ids = ops.bsgemm_topk(a, zero, bias, 2)
+        assert torch.equal(ids, torch.tensor([7, N // 2], device="cuda").expand(3, 2))
+        assert (logp.double() + torch.log(torch.tensor(2.0, dtype=torch.float64))).abs().max().item() < 2.0**-20 + 3.6e-7, c
