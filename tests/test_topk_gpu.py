@@ -178,3 +178,20 @@ def test_log_probability_of_two_equal_logits(ops, N):
         logp, ids = ops.bsgemm_topk(a, zero, bias, 2)
         assert torch.equal(ids, torch.tensor([7, N // 2], device="cuda").expand(3, 2))
         assert (logp.double() + torch.log(torch.tensor(2.0, dtype=torch.float64))).abs().max().item() < 2.0**-20 + 3.6e-7, c
+
+
+@pytest.mark.parametrize("N", [1025, 1791, 1792, 1793, 1800, 2047, 2048, 2049, 3839, 3841, 4095, 4097, 5887, 5889, 6143])
+def test_ragged_last_pieces_of_rows_in_registers(ops, N):
+    """The ragged last 8 columns of a row go to the last slot of lane 0 unless another piece is there: both sides of that line for
+    rows of up to 8, 16 and 24 pieces a lane, the winner in and around those columns, and lists of one and two entries a lane."""
+    torch.manual_seed(N)
+    a = ops.quantize(torch.randn(21, 512, device="cuda"), "mx32", natural=False)
+    b = ops.quantize(0.05 * torch.randn(N, 512, device="cuda"), "mx32")
+    bias = torch.randn(N, device="cuda")
+    for k in (1, 5, 16):
+        _check(ops, a, b, bias, k)
+    for col in (0, N // 8 * 8 - 1, min(N // 8 * 8, N - 1), N - 1):
+        one = bias.clone()
+        one[col] = 50.0
+        assert (ops.bsgemm_topk(a, b, one, 3)[1][:, 0] == col).all()
+        _check(ops, a, b, one, 3)

@@ -173,15 +173,16 @@ __global__ void __launch_bounds__(TK_WARPS * 32) topk_rows_kernel(const __nv_bfl
   }
 }
 
-// The same for rows of 1,025 to 6,144 columns, which a warp holds in registers (up to 24 pieces of 16 bytes a lane): the row is read
+// The same for rows of 1,025 to 6,144 columns, which a warp holds in registers (8, 16 or 24 pieces of 16 bytes a lane): the row is read
 // once, with all loads of a lane in flight, maxima are taken on packed bf16 pairs, the log-sum-exp against the row's maximum
 // without running rescales.  The threshold is found by one integer reduction per rank; the pieces that hold a value reaching it
-// (few more than k) are listed, and only their values are looked at one by one.  About 1,100 warp instructions per row of 5,538
+// (few more than k) are listed, and only their values are looked at one by one.  About 1,670 warp instructions per row of 5,538
 // where two passes over the row with a running maximum issued 3,300.  Head's GEMM, selection and LayerNorm quantizer of 3,750 rows:
-// 49 us with two passes, 37.6 like this.  (Four warps per row, 40 us: what each repeats costs more than the shorter chain gives.)
-constexpr int TR_WARPS = 8, TR_PIECES = 24, TR_LIST = 64, TR_MIN_N = 1024;
-__global__ void __launch_bounds__(TR_WARPS * 32, 2) topk_regs_kernel(const __nv_bfloat16* logits, int64_t ld, int N, int M, int k, float* logp,
-                                                                    int64_t* ids) {
+// 49 us with two passes, 33.4 like this.  (Four warps per row, 2.5 us more: what each repeats costs more than the shorter chain gives.)
+constexpr int TR_WARPS = 8, TR_LIST = 64, TR_MIN_N = 1024;
+template <int PIECES, int BLOCKS>
+__global__ void __launch_bounds__(TR_WARPS * 32, BLOCKS) topk_regs_kernel(const __nv_bfloat16* logits, int64_t ld, int N, int M, int k,
+                                                                          float* logp, int64_t* ids) {
   __shared__ unsigned long long cand_s[TR_WARPS][TK_CAND];
   __shared__ int list_s[TR_WARPS][TR_LIST];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -192,32 +193,35 @@ __global__ void __launch_bounds__(TR_WARPS * 32, 2) topk_regs_kernel(const __nv_
   constexpr float L2E = 1.4426950408889634f;
   const __nv_bfloat16* const z0 = logits + row * ld;
   const uint4* const src = reinterpret_cast<const uint4*>(z0);
-  const int pieces = (N + 7) >> 3;
+  const int full = N >> 3, pieces = (N + 7) >> 3;
   constexpr uint32_t NONE = 0xff80ff80u;  // two bf16 -inf
-  uint4 u[TR_PIECES];
+  // Piece j * 32 + lane in slot j.  A ragged last piece goes to the last slot, lane 0, unless that holds it anyway: so only one slot
+  // is masked (all of them, 24 pieces: 15,000 rows of 1,025 columns 51 us, where 1,032 columns took 40).
+  constexpr int LAST = PIECES - 1;
+  const bool moved = pieces <= LAST * 32;
+  const int last_c = !moved ? LAST * 32 + lane : (lane == 0 ? full : pieces);  // (N a multiple of 8: full == pieces, none)
+  uint4 u[PIECES];
 #pragma unroll
-  for (int j = 0; j < TR_PIECES; ++j) {
+  for (int j = 0; j < PIECES; ++j) {
+    const int c = j == LAST ? last_c : j * 32 + lane;
     u[j] = make_uint4(NONE, NONE, NONE, NONE);
-    if (j * 32 + lane < pieces) u[j] = src[j * 32 + lane];
+    if (c < (j == LAST ? pieces : full)) u[j] = src[c];
   }
-  if (N & 7) {  // columns beyond N in the last piece
+  if (last_c == full && full < pieces) {
+    uint32_t* const x = reinterpret_cast<uint32_t*>(&u[LAST]);
 #pragma unroll
-    for (int j = 0; j < TR_PIECES; ++j)
-      if (j * 32 + lane == pieces - 1) {
-        uint32_t* const x = reinterpret_cast<uint32_t*>(&u[j]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int valid = N - 8 * (pieces - 1) - 2 * i;
-          if (valid <= 0) x[i] = NONE;
-          else if (valid == 1) x[i] = (x[i] & 0xffffu) | (NONE & 0xffff0000u);
-        }
-      }
+    for (int i = 0; i < 4; ++i) {
+      const int valid = (N & 7) - 2 * i;
+      if (valid <= 0) x[i] = NONE;
+      else if (valid == 1) x[i] = (x[i] & 0xffffu) | (NONE & 0xffff0000u);
+    }
   }
+  auto used = [&](int j) { return j == LAST ? !moved || full < pieces : j * 32 < pieces; };  // (the same for all lanes)
   auto b2 = [](const uint32_t& x) { return *reinterpret_cast<const __nv_bfloat162*>(&x); };
   __nv_bfloat162 m4[4] = {b2(u[0].x), b2(u[0].y), b2(u[0].z), b2(u[0].w)};
 #pragma unroll
-  for (int j = 1; j < TR_PIECES; ++j) {
-    if (j * 32 < pieces) {
+  for (int j = 1; j < PIECES; ++j) {
+    if (used(j)) {
       m4[0] = __hmax2(m4[0], b2(u[j].x));
       m4[1] = __hmax2(m4[1], b2(u[j].y));
       m4[2] = __hmax2(m4[2], b2(u[j].z));
@@ -251,8 +255,8 @@ __global__ void __launch_bounds__(TR_WARPS * 32, 2) topk_regs_kernel(const __nv_
   uint64_t sa = pack_f32x2(0.0f, 0.0f), sb = sa;
   int listed = 0;  // pieces that reach the threshold
 #pragma unroll
-  for (int j = 0; j < TR_PIECES; ++j) {
-    if (j * 32 < pieces) {
+  for (int j = 0; j < PIECES; ++j) {
+    if (used(j)) {
       const uint32_t x[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -262,11 +266,12 @@ __global__ void __launch_bounds__(TR_WARPS * 32, 2) topk_regs_kernel(const __nv_
         if (i & 1) sb = add_f32x2(sb, e); else sa = add_f32x2(sa, e);
       }
       const __nv_bfloat162 pm = __hmax2(__hmax2(b2(x[0]), b2(x[1])), __hmax2(b2(x[2]), b2(x[3])));
-      const bool hit = j * 32 + lane < pieces && fmaxf(__low2float(pm), __high2float(pm)) >= thr;
+      const int c = j == LAST ? last_c : j * 32 + lane;
+      const bool hit = c < (j == LAST ? pieces : full) && fmaxf(__low2float(pm), __high2float(pm)) >= thr;
       const uint32_t who = __ballot_sync(0xffffffffu, hit);
       if (who) {
         const int at = listed + __popc(who & ((1u << lane) - 1u));
-        if (hit && at < TR_LIST) list_s[w][at] = j * 32 + lane;
+        if (hit && at < TR_LIST) list_s[w][at] = c;
         listed += __popc(who);
       }
     }
@@ -312,11 +317,13 @@ __global__ void __launch_bounds__(TR_WARPS * 32, 2) topk_regs_kernel(const __nv_
     ids[row * k + j] = e ? static_cast<int64_t>(0xffffffffu - static_cast<uint32_t>(e)) : -1;
     logp[row * k + j] = e ? z - lse : -INFINITY;
   };
-  if (n <= 32 && n >= k) {  // as a rule: every lane counts the entries above its own and writes it where that says
-    const unsigned long long mine = lane < n ? cand_s[w][lane] : 0ull;
-    int rank = 0;
-    for (int i = 0; i < n; ++i) rank += cand_s[w][i] > mine ? 1 : 0;
-    if (lane < n && rank < k) put(rank, mine);
+  if (n <= 64 && n >= k) {  // as a rule: every lane counts the entries above its own one or two and writes them where that says
+    for (int t = lane; t < n; t += 32) {
+      const unsigned long long mine = cand_s[w][t];
+      int rank = 0;
+      for (int i = 0; i < n; ++i) rank += cand_s[w][i] > mine ? 1 : 0;
+      if (rank < k) put(rank, mine);
+    }
     return;
   }
   unsigned long long last = ~0ull;
@@ -381,12 +388,15 @@ int vx_ctc_topk(const vx_gemm_desc* desc, int k, void* logits, int64_t rows, flo
     d.out_dtype = VX_BF16; d.out = logits; d.ldo = ld;
     const int rc = vx_bsgemm(&d, stream);
     if (rc) return rc;
-    // (Short rows leave most of the registers empty, and half the warps per SM to wait for them: N = 300, 15,000 rows 29 us with two
-    // passes, 42 in registers; N = 1,032 42 and 40, N = 4,096 89 and 75, N = 5,538 148 and 122.)
-    if (N > TR_MIN_N && N <= TR_PIECES * 32 * 8) {
-      VX_CUDA_OK(launch_dependent(topk_regs_kernel, dim3(static_cast<unsigned>((m + TR_WARPS - 1) / TR_WARPS)), dim3(TR_WARPS * 32), 0,
-                                  static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(logits), ld, static_cast<int>(N),
-                                  static_cast<int>(m), k, logp + r0 * k, ids + r0 * k));
+    auto regs = [&](auto kernel) {
+      return launch_dependent(kernel, dim3(static_cast<unsigned>((m + TR_WARPS - 1) / TR_WARPS)), dim3(TR_WARPS * 32), 0,
+                              static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(logits), ld, static_cast<int>(N),
+                              static_cast<int>(m), k, logp + r0 * k, ids + r0 * k);
+    };
+    // As many pieces a lane as the row needs, in steps of 8, so that 32, 24 or 16 warps per SM wait for them (15,000 rows, k = 1: N = 1,032
+    // 36 us with 24 pieces, 25 with 8, 30 with two passes; N = 2,049 46, 39 with 16, 44).  Two passes below: N = 300 29 us, 42 with 24 pieces.
+    if (N > TR_MIN_N && N <= 24 * 256) {
+      VX_CUDA_OK(N <= 8 * 256 ? regs(topk_regs_kernel<8, 4>) : N <= 16 * 256 ? regs(topk_regs_kernel<16, 3>) : regs(topk_regs_kernel<24, 2>));
       continue;
     }
     VX_CUDA_OK(launch_dependent(topk_rows_kernel, dim3(static_cast<unsigned>((m + TK_WARPS - 1) / TK_WARPS)), dim3(TK_WARPS * 32), 0,
