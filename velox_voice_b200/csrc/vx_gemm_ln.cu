@@ -14,7 +14,7 @@
 //   warp 1      owns tensor memory, copies scale factors shared -> tensor memory and issues the MMAs;
 //   warps 2..17 epilogue, warp (q, g) = TMEM lane quadrant q, 32-column blocks 2 g and 2 g + 1 of the CTA:
 //     pass 1  accumulator -> + bias, alpha, residual (its 32 x 64 block prefetched by TMA into the warp's
-//             staging buffer) -> bf16, formed in place and stored from there; the bf16 pairs also go back to
+//             staging buffer) -> bf16, formed in place and stored by TMA; the bf16 pairs also go back to
 //             tensor memory (128 columns next to the accumulator), the accumulator is released to the
 //             MMAs of the next tile; per-block (sum, sum of squares) sent to both CTAs;
 //     pass 2  after the exchange: mean / rstd, normalise the bf16 values read back from tensor memory,
@@ -348,7 +348,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       tc_fence_after();
       // ---- pass 1: x = bf16(alpha (acc + bias) + residual), block statistics
       float SQ[4];
-      // (both blocks at once: the accumulator is free after 700 cycles instead of 2,500, 90,000 rows x 2048: 92 us -> 86 with the stores below)
+      // (both blocks at once: the accumulator is free after 700 cycles instead of 2,500)
       uint32_t acc[2][4][8];
 #pragma unroll
       for (int t = 0; t < 2; ++t)
@@ -406,22 +406,10 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 #pragma unroll
         for (int d = 0; d < 2; ++d) st_async_f4(dst_part[d] + b * PART_STRIDE, sq[0], sq[1], sq[2], sq[3], dst_bar[d] + b * 32);
       };
-      // x (or y) leaves from the staging block: by TMA, or, where operands stream, by ordinary stores of whole 128-byte rows (as
-      // TMA stores its 64 KB held up the loads of the next stages for 2,500 of a tile's 15,400 cycles)
+      // x (or y) leaves by TMA from the staging block.  (By ordinary stores, where operands stream, as long as one ring held A and B: its
+      // loads queued behind the TMA stores.  With a loader for each, ordinary stores against this, captured calls in a row, 90,000 rows: K = 2048 82.3
+      // and 81.4 us, two LayerNorms 100.9 and 88.4, K = 1024 62.7 and 60.4, two LayerNorms 88.1 and 76.0.)
       auto store_block = [&]() {
-        if (!resident) {
-          __syncwarp();
-#pragma unroll
-          for (int v = 0; v < 8; ++v) {
-            const int r = 4 * v + (lane >> 3), u = lane & 7;
-            const int64_t orow = static_cast<int64_t>(mb) * LN_BM + q * 32 + r;
-            const uint4 w = *reinterpret_cast<const uint4*>(sm.staging[ew] + r * 128 + ((u ^ (r & 7)) << 4));
-            if (orow < p.M) *reinterpret_cast<uint4*>(p.out + orow * p.ldo + tile_col + u * 8) = w;
-          }
-          fence_proxy_async_smem();  // read before the next residual block may land here
-          __syncwarp();
-          return;
-        }
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
