@@ -380,7 +380,12 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   const int out_fmt = OUT == 2 || OUT == 4 ? static_cast<int>(kind_vec4(KIND) ? VX_FMT_NV16 : VX_FMT_MX32) : p.out_fmt;
   const bool tr_on = kPhaseTrace && p.trace != nullptr && blockIdx.x == 0;  // phase trace requested (CTA 0 only)
 
-  const int warp = warp_index();
+  // The roles by a uniform warp index (warp_index) gain where registers or issue are short, and cost the others: captured calls in a
+  // row, per-lane against uniform, MX32: GLU 24,000 rows 15.3 and 13.9 us, residual 9.38 and 9.26, fold pack 63.6 and 62.0; but FFN-up
+  // (Swish, FP4) 26.0 and 26.7, arg-max 3,750 rows 17.5 and 17.9, fp32 result 1,537 x 2,048 6.50 and 6.87, plain bias 375 rows 4.04 and 4.15.
+  // (NV16: +4 to -10 % uniform, -5 % only for fp32 results of some sizes.)
+  constexpr bool LANE_ROLES = kind_pow2_scales(KIND) && (SWQ || EPI == VX_EPI_BIAS_ARGMAX || (EPI == VX_EPI_BIAS && OUT < 2));
+  const int warp = LANE_ROLES ? static_cast<int>(threadIdx.x >> 5) : warp_index();
   const int lane = threadIdx.x & 31;
   // (The waits below take no abort flag: a flag that the roles poll was built and measured -- the
   // extra exits from every wait loop cost the 96-register epilogues spills, the fused-QKV kernel went
