@@ -119,7 +119,7 @@ relpos_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   uint8_t* const k_s = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* const v_s = k_s + AT_NS * AT_K_BYTES;
   __shared__ AttnBarriers bar;
-  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.y;
   const int64_t q0 = static_cast<int64_t>(blockIdx.x) * AT_BM;
   const int steps = static_cast<int>((p.kv_len + AT_BN - 1) / AT_BN);

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(MEL_THREADS, 1) power_mel_log_kernel(const Mel
   uint8_t* const ring = base;                                  // p.ring x 16 KB
   uint8_t* const bres = base + p.ring * MEL_SLOT;              // stages x n_pad x 128 B (n_pad % 8 == 0: 1 KB atoms hold)
   __shared__ MelBarriers bar;
-  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* const abortp = &bar.abort_flag;
   const int my_tiles = static_cast<int>(blockIdx.x) < p.tiles ? (p.tiles - static_cast<int>(blockIdx.x) + gridDim.x - 1) / gridDim.x : 0;
   const uint32_t b_stage_bytes = static_cast<uint32_t>(p.n_pad) * 128u;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
   uint8_t* const ring = tiles_s + 2 * tile_bytes;
   const uint32_t row_bytes = static_cast<uint32_t>(p.F) * 8u, chunk_bytes = MT_ROWS * row_bytes;
   __shared__ MtBarriers bar;
-  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* const abortp = &bar.abort_flag;
   const int my_tiles = static_cast<int>(blockIdx.x) < p.tiles ? (p.tiles - static_cast<int>(blockIdx.x) + gridDim.x - 1) / gridDim.x : 0;
   const int F = static_cast<int>(p.F), M = static_cast<int>(p.M), ksteps = (F + 7) / 8;
