@@ -74,14 +74,19 @@ def test_stores_are_complete_before_a_kernel_ends(name):
     assert text.rindex("tma_store_commit()") < last < text.index("tmem_dealloc(tmem_base", last)
 
 
-def test_the_gemm_triggers_the_next_launch_only_behind_its_own_wait():
-    """One thread that triggers counts for its CTA.  The producer's lane reads weights ahead of its wait, so the trigger must
-    not be reachable for it, nor for any thread, without the wait in front."""
-    text = source("vx_gemm.cu")
-    text = text[text.index("bsgemm_kernel("):]
+@pytest.mark.parametrize("name,kernel,waits", [("vx_gemm.cu", "bsgemm_kernel(", r"warp != 0 \|\| my_tiles == 0"),
+                                               ("vx_gemm_ln.cu", "bsgemm_residual_ln_kernel(", "!producer_thread"),
+                                               ("vx_pass.cu", "conformer_pass_kernel(", "warp != PS_WARP_B")])
+def test_a_gemm_triggers_the_next_launch_only_behind_its_own_wait(name, kernel, waits):
+    """One thread that triggers counts for its CTA.  A loader reads weights ahead of its wait, so the trigger must not be reachable for
+    it, nor for any thread, without the wait in front."""
+    text = source(name)
+    text = text[text.index(kernel):]
     text = text[:re.search(r"\n}\n", text).end()]
     assert text.count("pdl_launch_dependents()") == 1
-    assert re.search(r"if \(warp != 0 \|\| my_tiles == 0\) {\s*pdl_wait\(\);\s*pdl_launch_dependents\(\);\s*}", text)
+    assert re.search(r"if \(%s\) {\s*pdl_wait\(\);\s*pdl_launch_dependents\(\);\s*}" % waits, text)
+    if name == "vx_gemm_ln.cu":
+        assert "const bool producer_thread = (warp == 0 || warp == 18) && lane == 0 && my_tiles > 0;" in text
 
 
 @pytest.mark.parametrize("name,barrier", [("vx_gemm.cu", "empty"), ("vx_gemm_ln.cu", "empty"), ("vx_gemm_ln.cu", "hb_empty"),

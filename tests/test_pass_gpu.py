@@ -45,15 +45,50 @@ def test_number_of_blocks(blocks):
     assert torch.equal(got, want) and torch.equal(h, hidden) and (n1 == n0) == (blocks == 17)
 
 
-def test_rows_that_are_not_finite_stay_to_themselves():
+def same(a, b):
+    """Equal bits, a NaN being equal to a NaN."""
+    return torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.nan_to_num(a, 0.0), torch.nan_to_num(b, 0.0))
+
+
+@pytest.mark.parametrize("T", [129, 300, 2100])
+def test_rows_that_are_not_finite(T):
+    """They have the values of the separate launches and stay to themselves."""
     stack = build(blocks=2)
-    x = torch.randn(300, 512, device="cuda").bfloat16()
+    x = torch.randn(T, 512, device="cuda").bfloat16()
     clean = stack.forward(x.clone())
-    x[5, 7], x[140, 0], x[299, 511] = float("nan"), float("inf"), float("-inf")
-    got = stack.forward(x.clone())
-    keep = torch.ones(300, dtype=torch.bool, device="cuda")
-    keep[[5, 140, 299]] = False
+    x[5, 7], x[T // 2, 0], x[T - 1, 511], x[17] = float("nan"), float("inf"), float("-inf"), 3e38
+    (got, h, _), (want, hidden, _) = both(stack, x)
+    assert same(got, want) and same(h, hidden)
+    keep = torch.ones(T, dtype=torch.bool, device="cuda")
+    keep[[5, T // 2, T - 1, 17]] = False
     assert torch.equal(got[keep], clean[keep])
+
+
+@pytest.mark.parametrize("T", [1, 300, 2100])
+def test_weights_that_may_have_just_been_written(T):
+    """Without the scales in natural layout a weight is not known to come from the packing quantizer: its loader waits."""
+    stack, other = build(blocks=2), build(blocks=2, seed=1)
+    x = torch.randn(T, 512, device="cuda").bfloat16()
+    for name, layer in stack.p.items():
+        layer.q.scales = None
+        layer.q.codes.copy_(other.p[name].q.codes)  # ... and this one was, right before the pass
+        layer.q.sf.copy_(other.p[name].q.sf)
+    (got, h, n1), (want, hidden, n0) = both(stack, x)
+    assert torch.equal(got, want) and torch.equal(h, hidden) and n1 == 2 and n0 > 20
+
+
+@pytest.mark.parametrize("T", [4300, 9000])
+@pytest.mark.parametrize("ffn", [2048, 1024])
+def test_more_row_blocks_than_clusters(T, ffn):
+    """A cluster takes several row blocks in turn: two rounds, and three of which the last is not full."""
+    stack = build(blocks=2, ffn=ffn)
+    assert T > stack.one_launch_frames
+    stack.one_launch_frames = T
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, 512, generator=g, device="cuda").bfloat16()
+    for _ in range(3):
+        (got, h, n1), (want, hidden, _) = both(stack, x)
+        assert torch.equal(got, want) and torch.equal(h, hidden) and n1 == 2
 
 
 @pytest.mark.parametrize("offset,pitch,refused", [(8, 528, None), (0, 512, None), (4, 520, "x rows must be 16-byte aligned"),

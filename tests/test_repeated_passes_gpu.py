@@ -27,12 +27,10 @@ def test_staged_stores_of_ragged_widths(fmt, M, N):
     assert bad == 0, f"{bad} of 160 launches differ"
 
 
-@pytest.mark.parametrize("fused", [True, False])
-@pytest.mark.parametrize("frames,passes", [(375, 400), (4800, 200), (21090, 200), (24000, 200)])
-def test_passes_of_the_stack(frames, passes, fused):
-    """Passes issued eight at a time without a pause between them, against a pass in which the residual GEMMs, LayerNorms and
-    quantizers run as separate kernels and the logits leave by per-thread stores."""
-    from velox_voice_b200 import _lib, ops
+def expected(frames):
+    """A stack, features, positions, and hidden states and logits of a pass in which the residual GEMMs, LayerNorms and quantizers run
+    as separate kernels and the logits leave by per-thread stores."""
+    from velox_voice_b200 import ops
     from velox_voice_b200.stack import ConformerLinearStack, StackConfig, make_weights
 
     cfg = StackConfig()
@@ -45,11 +43,43 @@ def test_passes_of_the_stack(frames, passes, fused):
     torch.cuda.synchronize()
     q = ops.ln_quantize(hidden, *stack.ln["after"], cfg.eps, "mx32")
     want = ops.bsgemm(q, stack.p["ctc"].q, epilogue=ops.EPI_BIAS, bias=stack.p["ctc"].bias, direct_store=True)
+    return stack, x, pos, hidden, want
+
+
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("frames,passes", [(375, 400), (4800, 200), (21090, 200), (24000, 200)])
+def test_passes_of_the_stack(frames, passes, fused):
+    """Passes issued eight at a time without a pause between them, against a pass in which the residual GEMMs, LayerNorms and
+    quantizers run as separate kernels and the logits leave by per-thread stores."""
+    from velox_voice_b200 import _lib, ops
+
+    stack, x, pos, hidden, want = expected(frames)
     stack.fuse_ln, stack.fuse_ln_min_frames = fused, 0
     bad = 0
+    ops.reset_launch_count()
     for _ in range(passes // 8):
         outs = [stack.forward(x.clone(), pos, return_hidden=True) for _ in range(8)]
         bad += sum(not (torch.equal(o, want) and torch.equal(h, hidden)) for o, h in outs)
         del outs
     assert bad == 0, f"{bad} of {passes} passes differ"
     assert _lib.device_status() == 0
+    lp = 1 if frames <= 4096 else 12
+    assert ops.launch_count() == passes // 8 * 8 * (2 + lp + (12 * 8 if fused else 12 * 12) + 1)
+
+
+@pytest.mark.parametrize("frames,passes", [(375, 400), (1920, 400), (4096, 200)])
+def test_passes_in_one_launch(frames, passes):
+    """The same where all blocks run in one launch (clusters of eight CTAs, all of them, and of four)."""
+    from velox_voice_b200 import _lib, ops
+
+    stack, x, pos, hidden, want = expected(frames)
+    stack.fuse_ln = True
+    bad = 0
+    ops.reset_launch_count()
+    for _ in range(passes // 8):
+        outs = [stack.forward(x.clone(), pos, return_hidden=True) for _ in range(8)]
+        bad += sum(not (torch.equal(o, want) and torch.equal(h, hidden)) for o, h in outs)
+        del outs
+    assert bad == 0, f"{bad} of {passes} passes differ"
+    assert _lib.device_status() == 0
+    assert ops.launch_count() == passes // 8 * 8 * 4  # positions (quantizer, projections), blocks, head
