@@ -24,9 +24,9 @@
 // activations, 17 issues the MMAs (one elected lane), 18 and 19 load weights and the biases and LayerNorm parameters, which depend on
 // no layer and run ahead of them through rings of four and three slots.  Accumulators: a ring of three times 128 columns.
 //
-// Measured, whole greedy pass of 12 blocks, separate launches against this: 375 frames 752 us -> 581, 1,920 frames (the most for
-// clusters of eight) 836 -> 594, 4,000 frames (clusters of four) 986 -> 717, 4,200 frames 1,036 -> 756 (its twelve positional projections are launches of their own).  What bounds it now, of 83,000 cycles a
-// block (clusters of eight): the hand-over of an operand, 4,000 a phase -- the release waits 1,750 for the stores, fence and loads take
+// Measured, whole greedy pass of 12 blocks, separate launches against this: 375 frames 752 us -> 579, 1,920 frames (the most for
+// clusters of eight) 838 -> 592, 4,000 frames (clusters of four) 988 -> 718, 4,200 frames 1,038 -> 760 (its twelve positional projections are launches of their own).  What bounds it now, of 92,000 cycles a
+// block (47 us, clusters of eight): the hand-over of an operand, 4,000 a phase -- the release waits 1,750 for the stores, fence and loads take
 // 1,900 --, the issue of the MMAs, 500 to 700 cycles per stage of four, and the chain accumulator -> sums -> exchange -> quantize of
 // the four LayerNorms, 4,000 each.  Tried and not kept: operands pushed to the other CTAs' shared memory by st.async (630 us) or bulk
 // copies (590; shared memory leaves an SM at 14 to 16 bytes a cycle, what L2 delivers enters at 90), jobs of 64 columns for the
@@ -731,7 +731,7 @@ int launch_pass(PassParams& p, const vx_pass_desc* d, cudaStream_t st) {
   return 0;
 }
 
-// CTAs per cluster for a pass of `tiles` row blocks: eight while all row blocks run at once (15 on a B200), as a block takes 49 us
+// CTAs per cluster for a pass of `tiles` row blocks: eight while all row blocks run at once (15 on a B200), as a Conformer block takes 47 us
 // instead of 58; four up to 33 row blocks.
 int pass_cluster(int64_t tiles) { return tiles <= max_clusters<8>() ? 8 : 4; }
 
@@ -746,7 +746,7 @@ int vx_conformer_pass_supported(int fmt, int64_t d_model, int64_t ffn, int64_t c
          blocks <= PS_MAX_BLOCKS;
 }
 
-// One round of clusters of four.  4,200 frames: separate launches 1,036 us, one launch 756; a second round takes as long again, and
+// One round of clusters of four.  4,200 frames: separate launches 1,038 us, one launch 760; a second round takes as long again, and
 // the launches that pipeline over many row blocks are as fast (4,608 frames: 1,075 and about 1,450).
 int64_t vx_conformer_pass_frames(void) {
   return static_cast<int64_t>(vx::max_clusters<4>()) * vx::PS_BM;

@@ -51,7 +51,7 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&z)[8]) {
 // One warp per row.  Pass 1: every lane's running (max, sum of 2^((z - max) log2 e)) over its 16-byte pieces, merged into the
 // row's log-sum-exp.  The k-th largest of the 32 lane maxima is a threshold that at least k logits reach and each of the k
 // largest does; pass 2 (the row again, from L1) collects what reaches it -- a few more than k -- and the k largest of the
-// list are taken in order.  Bound by instruction issue: about 900 warp instructions per row of 5,538.
+// list are taken in order.  Bound by instruction issue: 1,670 warp instructions per row of 1,000 columns.
 __global__ void __launch_bounds__(TK_WARPS * 32) topk_rows_kernel(const __nv_bfloat16* logits, int64_t ld, int N, int M,
                                                                   int k, float* logp, int64_t* ids) {
   __shared__ unsigned long long cand_s[TK_WARPS][TK_CAND];
