@@ -63,6 +63,19 @@ def test_no_lane_of_a_warp_stays_behind_when_a_limit_runs_out(name, kernel):
         assert alone or "__all_sync" in line or (together and start < m.start() < end), f"{name}: {line.strip()}"
 
 
+@pytest.mark.parametrize("name,kernel", [("vx_mel.cu", "power_mel_log_kernel("), ("vx_mel.cu", "power_mel_log_dense_kernel("),
+                                         ("vx_attn.cu", "relpos_attn_kernel("), ("vx_gemm.cu", "bsgemm_kernel(")])
+def test_lanes_that_meet_at_a_syncwarp_agree_on_their_waits(name, kernel):
+    """A lane of an MMA warp that gave up a wait leaves its loop.  Either the lanes meet nowhere in it, or whether the limit ran out is a
+    vote."""
+    text = source(name)
+    text = text[text.index(kernel):]
+    text = text[text.index("elect_one()"):]
+    mma = text[:re.search(r"\n  } else {\n", text).start()]
+    waits = [mma[mma.rfind("\n", 0, m.start()):m.start()] for m in re.finditer(r"\bmbar_wait\w*(<\w+>)?\(", mma)]
+    assert len(waits) >= 2 and ("__syncwarp" not in mma or all("__all_sync" in w for w in waits))
+
+
 @pytest.mark.parametrize("name", ["vx_gemm_ln.cu", "vx_gemm.cu"])
 def test_stores_are_complete_before_a_kernel_ends(name):
     """Writes of a bulk store are ordered by waiting for its group, not by the end of the thread that issued it; the `.read`
