@@ -46,10 +46,9 @@ from .ops import FMT_FP8_1X128, FMT_MX32, FMT_NV16
 def fuse_ln_frames(sms: int, d_model: int) -> int:
     """Frames from which the residual GEMMs run the LayerNorm + quantizer behind them (two-CTA clusters, a row block each) unless
     the caller chooses.  As long as the separate residual GEMM takes a single round -- a tile of 128 x 128 per SM, 37 row blocks
-    of four tiles on 148 SMs -- it is faster (12 blocks, captured, separate against fused: 3,750 frames 928 and 1,033 us, 4,736
-    1,040 and 1,134).  From 18,944 frames on the fused launches are (2,188 and 2,051 us; 40,000: 4,129 and 3,965).  In between the two stay
-    within 8 % of one another, in turn: the clusters take rounds of 74 row blocks (5,000: 1,121 and 1,157 us; 7,000: 1,227 and
-    1,235; 9,472: 1,461 and 1,349; 9,500: 1,559 and 1,604; 14,208: 1,817 and 1,834)."""
+    of four tiles on 148 SMs -- it is as fast or faster (12 blocks, captured, in turn, separate against fused: 3,750 frames 913 and
+    941 us, 4,736 1,033 and 1,031); beyond that the fused launches are (5,000: 1,102 and 1,049; 9,472, their last single round of 74 row
+    blocks: 1,439 and 1,296; 9,500: 1,549 and 1,478; 18,944: 2,154 and 1,961; 40,000: 4,045 and 3,744)."""
     return sms // max(d_model // 128, 1) * 128 + 1
 
 
