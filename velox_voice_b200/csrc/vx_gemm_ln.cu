@@ -7,10 +7,11 @@
 // factors of a block-scaled MMA in tensor memory.  So a CLUSTER OF TWO CTAs owns each block of 128 rows:
 // CTA r computes columns [256 r, 256 r + 256) with 128 x 256 x 64 MXF4 MMAs, and the two exchange the
 // per-row partial sums of the LayerNorm statistics through distributed shared memory (st.async with
-// mbarrier completion into a table double-buffered per tile, one barrier per lane quadrant).  Per CTA, 19 warps:
+// mbarrier completion into a table double-buffered per tile, one barrier per lane quadrant).  Per CTA, 20 warps:
 //   warp 0      TMA producer: A tiles (128-byte swizzle) + scale-factor atoms into a ring; the CTA's half of B stays
 //               resident in shared memory when K <= 512;
 //   warp 18     otherwise streams B through a ring of its own;
+//   warp 19     where B streams, moves the residual and x blocks of the epilogue warps;
 //   warp 1      owns tensor memory, copies scale factors shared -> tensor memory and issues the MMAs;
 //   warps 2..17 epilogue, warp (q, g) = TMEM lane quadrant q, 32-column blocks 2 g and 2 g + 1 of the CTA:
 //     pass 1  accumulator -> + bias, alpha, residual (its 32 x 64 block prefetched by TMA into the warp's
@@ -64,7 +65,9 @@ constexpr int LN_ARENA = LN_RESIDENT_MAX_STAGES * LN_B_SLOT + 3 * LN_A_SLOT;  //
 constexpr int LN_A_SLOTS = 3;
 static_assert(LN_HB_SLOTS * LN_HB_SLOT + LN_A_SLOTS * LN_A_SLOT <= LN_ARENA, "streaming plan");
 constexpr int LN_STAGING = 32 * 128;                    // per epilogue warp: 32 rows x 64 bf16 columns, 128-byte swizzle
-constexpr int LN_THREADS = 19 * 32;
+// (the instance with two LayerNorms has no warp 19: one more warp, idle, costs it 3 % at 24,000 rows x 1024)
+__host__ __device__ constexpr int ln_threads(bool two) { return (two ? 19 : 20) * 32; }
+constexpr int LN_PACED_STORES = 2;  // blocks of x that the pacing warp has with the TMA at a time
 constexpr uint32_t LN_XCH_BYTES = 2 * 4 * 32 * 16;  // per CTA, tile and lane quadrant: 2 CTAs x 4 warps x 32 lanes x 16 bytes
 // tensor-memory columns
 constexpr uint32_t LN_TM_ACC = 0, LN_TM_XP = 256, LN_TM_SFA = 384, LN_TM_SFB = 448;
@@ -101,7 +104,7 @@ struct __align__(1024) LnSmem {
   float bias[LN_BN], gamma[LN_BN], beta[LN_BN], gamma2[LN_BN], beta2[LN_BN];
   uint64_t full[LN_A_SLOTS], empty[LN_A_SLOTS], hb_full[LN_HB_SLOTS], hb_empty[LN_HB_SLOTS];
   uint64_t tmem_full, tmem_empty, b_full;
-  uint64_t res_full[16];
+  uint64_t res_full[16], out_ready[16];  // per staging block: residual landed, x formed
   uint64_t xch[2][4];  // [tile parity][lane quadrant]: the rows of a quadrant depend on that quadrant's warps only
   uint32_t tmem_base;
 };
@@ -115,7 +118,7 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
 // LN2 = true (the end of a Conformer block): out = y = bf16(LN(x; gamma, beta)) -- x itself is not stored -- and
 // codes = quantize(LN(y as stored; gamma2, beta2)): a second exchange of row statistics and a third pass.
 template <bool LN2>
-__global__ void __launch_bounds__(LN_THREADS, 1)
+__global__ void __launch_bounds__(ln_threads(LN2), 1)
 bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                           const __grid_constant__ CUtensorMap tmap_res, const __grid_constant__ CUtensorMap tmap_out,
                           const LnParams p) {
@@ -127,16 +130,26 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   const int cluster = static_cast<int>(blockIdx.x >> 1), nclusters = static_cast<int>(gridDim.x >> 1);
   const int my_tiles = cluster < p.m_tiles ? (p.m_tiles - cluster + nclusters - 1) / nclusters : 0;
   const bool resident = p.b_resident != 0;
+  // Warp 19 moves the residual and x blocks, two of x at a time, or each epilogue warp its own, sixteen of x at a time.  The sixteen hold up
+  // the loads of the operands (64 KB leave an SM at about 16 bytes a cycle, in front of the loads in the TMA's queue), which costs where
+  // operands stream: of 12,700 cycles a tile with K = 2048 the MMAs waited 3,000 for one stage of B.  One thread for sixteen blocks is
+  // slower where they don't, and nothing else than the epilogue bounds the kernel.  90,000 rows, captured calls in a row, own / paced:
+  // K = 2048 80.9 / 75.5 us, K = 512 53.8 / 56.0, two LayerNorms with K = 2048 88.7 / 88.8.
+  const bool paced = !LN2 && !resident;
   const uint32_t ring_off = resident ? p.k_stages * LN_B_SLOT : LN_HB_SLOTS * LN_HB_SLOT;  // ring of A
 
   // ---- set-up
+  // Warp 0 makes the barriers and goes straight to its loads, as do the loader of B, the MMA issuer and the storer once the barriers exist
+  // (named barrier); they meet the others only at the end.  The epilogue needs the cluster's barrier: tensor memory, parameters, the
+  // peer's barriers.
   if (threadIdx.x == 0) {
+    prefetch_tmap(&tmap_b);
     for (int s = 0; s < LN_A_SLOTS; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
     for (int s = 0; s < LN_HB_SLOTS; ++s) { mbar_init(&sm.hb_full[s], 1); mbar_init(&sm.hb_empty[s], 1); }
     mbar_init(&sm.tmem_full, 1);
     mbar_init(&sm.tmem_empty, 16);  // one arrival per epilogue warp
     mbar_init(&sm.b_full, 1);
-    for (int w = 0; w < 16; ++w) mbar_init(&sm.res_full[w], 1);
+    for (int w = 0; w < 16; ++w) { mbar_init(&sm.res_full[w], 1); mbar_init(&sm.out_ready[w], 1); }
     // exchange barriers: the one arrival is the arming below / after each use; the partial sums arrive as bytes
     for (int b = 0; b < 2; ++b)
       for (int qq = 0; qq < 4; ++qq) {
@@ -145,34 +158,48 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       }
     mbar_fence_init();
     prefetch_tmap(&tmap_a);
-    prefetch_tmap(&tmap_b);
-    prefetch_tmap(&tmap_res);
-    prefetch_tmap(&tmap_out);
-  }
-  for (int i = threadIdx.x; i < LN_BN; i += blockDim.x) {  // constants of the model
-    sm.bias[i] = p.bias ? __ldg(p.bias + rank * LN_BN + i) : 0.0f;
-    sm.gamma[i] = __ldg(p.gamma + rank * LN_BN + i);
-    sm.beta[i] = __ldg(p.beta + rank * LN_BN + i);
-    if constexpr (LN2) {
-      sm.gamma2[i] = __ldg(p.gamma2 + rank * LN_BN + i);
-      sm.beta2[i] = __ldg(p.beta2 + rank * LN_BN + i);
-    }
-  }
-  if (warp == 1) {
+  } else if (warp == 1) {
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
+  } else if (warp == 18) {
+    if (lane == 0) { prefetch_tmap(&tmap_res); prefetch_tmap(&tmap_out); }
+  } else if (warp >= 2 && warp < 18) {
+    const int i = threadIdx.x - 64;  // constants of the model
+    if (i < LN_BN) {
+      sm.bias[i] = p.bias ? __ldg(p.bias + rank * LN_BN + i) : 0.0f;
+      sm.gamma[i] = __ldg(p.gamma + rank * LN_BN + i);
+      sm.beta[i] = __ldg(p.beta + rank * LN_BN + i);
+      if constexpr (LN2) {
+        sm.gamma2[i] = __ldg(p.gamma2 + rank * LN_BN + i);
+        sm.beta2[i] = __ldg(p.beta2 + rank * LN_BN + i);
+      }
+    }
   }
+  __syncwarp();
   tc_fence_before();
-  __syncthreads();
+  cluster_arrive();
+  const bool epilogue_warp = warp >= 2 && warp < 18;
+  constexpr int SETUP_THREADS = ln_threads(LN2) - 16 * 32;
+  if (epilogue_warp) {
+    cluster_wait();  // tensor memory, parameters, and the peer's barriers before anything is sent to them
+  } else if (warp == 0) {
+    named_bar_arrive(1, SETUP_THREADS);
+  } else {
+    named_bar_sync(1, SETUP_THREADS);
+  }
   tc_fence_after();
-  cluster_sync_all();  // the peer's barriers exist before anything is sent to them
   const uint32_t tmem_base = sm.tmem_base;
+  // The loaders wait for the previous launch behind what they may read ahead of it; their other lanes do not wait here at all: they
+  // would hold up the loading lane at the end of the branch (as they once did: no weight was read ahead, 90,000 rows x 512 56.5 us, 53.8 like
+  // this).  The next launch is triggered behind the wait, by threads that have waited, as in vx_gemm.cu: its set-up and weights come in under
+  // the last round, which leaves clusters idle (12 blocks, 24,000 frames: 2,650 us without, 2,577 like this).
   const bool producer_thread = (warp == 0 || warp == 18) && lane == 0 && my_tiles > 0;
-  // (The next launch is triggered behind the wait, by threads that have waited, as in vx_gemm.cu: its set-up and weights come in under
-  // the last round, which leaves clusters idle.  12 blocks, 24,000 frames: 2,650 us without, 2,577 like this.)
-  if (!producer_thread) {
-    pdl_wait();
-    pdl_launch_dependents();
+  const bool idle_lane = (warp == 0 || warp == 18) && lane != 0;
+  if (!idle_lane) {
+    if (!producer_thread) {
+      pdl_wait();
+      pdl_launch_dependents();
+    }
   }
 
   if (warp == 0) {
@@ -227,6 +254,35 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           if (++s == LN_HB_SLOTS) { s = 0; ph ^= 1; }
         }
       }
+    }
+  } else if (warp == 19) {
+    // =========================== residual blocks in, x blocks out (paced) ===========================
+    if (lane == 0 && paced && my_tiles > 0) {
+      const int col0 = static_cast<int>(rank) * LN_BN;
+      auto load_res = [&](int w, int mb) {
+        mbar_expect_tx(&sm.res_full[w], LN_STAGING);
+        tma_load_2d(sm.staging[w], &tmap_res, col0 + (w >> 2) * 64, mb * LN_BM + (w & 3) * 32, &sm.res_full[w]);
+      };
+      int mb = cluster;
+      for (int w = 0; w < 16; ++w) load_res(w, mb);
+      bool ok = true;
+      for (int i = 0; i < my_tiles && ok; ++i, mb += nclusters) {
+        const bool more = i + 1 < my_tiles;
+        for (int w = 0; w < 16; ++w) {
+          if (!mbar_wait(&sm.out_ready[w], i & 1, p.status, 30)) { ok = false; break; }
+          tma_store_2d(&tmap_out, col0 + (w >> 2) * 64, mb * LN_BM + (w & 3) * 32, sm.staging[w]);
+          tma_store_commit();
+          // blocks that have been read: the next residual block may land there
+          tma_store_wait_read<LN_PACED_STORES - 1>();
+          if (more && w >= LN_PACED_STORES - 1) load_res(w - (LN_PACED_STORES - 1), mb + nclusters);
+        }
+        if (!ok) break;
+        if (more) {
+          tma_store_wait_read<0>();
+          for (int w = 17 - LN_PACED_STORES; w < 16; ++w) load_res(w, mb + nclusters);
+        }
+      }
+      tma_store_wait_all<0>();  // the writes, not only the reads of shared memory: the next launch may be waiting for this grid to end
     }
   } else if (warp == 1) {
     // =========================== MMA issuer ===========================
@@ -312,7 +368,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   } else {
     // =========================== epilogue (warps 2..17) ===========================
     const int q = warp & 3, g = (warp - 2) >> 2;  // TMEM lane quadrant; blocks 2 g, 2 g + 1 of this CTA's eight
-    const int ew = warp - 2;
+    const int sb = 4 * g + q;  // staging block of this warp
     const int row_in = q * 32 + lane;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     // piece (8 columns) handled at step c of a block: (c + rot) & 3, rot = (block >> 1) & 3 = g for both blocks
@@ -328,15 +384,15 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     // Staging block of this warp: rows [32 q, +32) x columns [256 rank + 64 g, +64) of the tile as bf16, rows of
     // 128 bytes with the 128-byte swizzle: 16-byte unit u of row r sits at unit u ^ (r & 7).  The residual block
     // lands here by TMA, x is formed in place and leaves by TMA (rows beyond M: zero-filled / clipped).
-    uint8_t* const stage_row = sm.staging[ew] + lane * 128;
+    uint8_t* const stage_row = sm.staging[sb] + lane * 128;
     const int sw = lane & 7;
     const int tile_col = static_cast<int>(rank) * LN_BN + g * 64;
     const uint64_t A2 = pack_f32x2(p.alpha, p.alpha);
     bool ok = true;
     int mb = cluster;
-    if (lane == 0 && my_tiles > 0) {
-      mbar_expect_tx(&sm.res_full[ew], LN_STAGING);
-      tma_load_2d(sm.staging[ew], &tmap_res, tile_col, mb * LN_BM + q * 32, &sm.res_full[ew]);
+    if (!paced && lane == 0 && my_tiles > 0) {
+      mbar_expect_tx(&sm.res_full[sb], LN_STAGING);
+      tma_load_2d(sm.staging[sb], &tmap_res, tile_col, mb * LN_BM + q * 32, &sm.res_full[sb]);
     }
     for (int i = 0; i < my_tiles && ok; ++i, mb += nclusters) {
       const int64_t row = static_cast<int64_t>(mb) * LN_BM + row_in;
@@ -359,7 +415,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.tmem_empty);
-      ok = __all_sync(0xffffffffu, mbar_wait(&sm.res_full[ew], i & 1, p.status, 27));
+      ok = __all_sync(0xffffffffu, mbar_wait(&sm.res_full[sb], i & 1, p.status, 27));
       if (!ok) break;
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
@@ -406,15 +462,17 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 #pragma unroll
         for (int d = 0; d < 2; ++d) st_async_f4(dst_part[d] + b * PART_STRIDE, sq[0], sq[1], sq[2], sq[3], dst_bar[d] + b * 32);
       };
-      // x (or y) leaves by TMA from the staging block.  (By ordinary stores, where operands stream, as long as one ring held A and B: its
-      // loads queued behind the TMA stores.  With a loader for each, ordinary stores against this, captured calls in a row, 90,000 rows: K = 2048 82.3
-      // and 81.4 us, two LayerNorms 100.9 and 88.4, K = 1024 62.7 and 60.4, two LayerNorms 88.1 and 76.0.)
+      // x (or y) leaves by TMA from the staging block
       auto store_block = [&]() {
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          tma_store_2d(&tmap_out, tile_col, mb * LN_BM + q * 32, sm.staging[ew]);
-          tma_store_commit();
+          if (paced) {
+            mbar_arrive(&sm.out_ready[sb]);
+          } else {
+            tma_store_2d(&tmap_out, tile_col, mb * LN_BM + q * 32, sm.staging[sb]);
+            tma_store_commit();
+          }
         }
       };
       // waits for the sums of exchange b, arms its barrier for the next use, fetches the next residual block when
@@ -426,12 +484,12 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         tc_wait_st_all();  // the bf16 copy is in tensor memory before the next pass reads it back
         if (!landed) return false;
         if (g == 0 && lane == 0) mbar_expect_tx(&sm.xch[b][q], LN_XCH_BYTES);  // armed for the next use
-        if (staging_free && lane == 0 && i + 1 < my_tiles) {
+        if (staging_free && !paced && lane == 0 && i + 1 < my_tiles) {
           // By now the store has read the staging block (waiting for that right behind the store would hold the
           // whole warp for the read): the residual block of the next tile may land in it.
           tma_store_wait_read<0>();
-          mbar_expect_tx(&sm.res_full[ew], LN_STAGING);
-          tma_load_2d(sm.staging[ew], &tmap_res, tile_col, (mb + nclusters) * LN_BM + q * 32, &sm.res_full[ew]);
+          mbar_expect_tx(&sm.res_full[sb], LN_STAGING);
+          tma_load_2d(sm.staging[sb], &tmap_res, tile_col, (mb + nclusters) * LN_BM + q * 32, &sm.res_full[sb]);
         }
         // block sums j and j ^ 8 first (blocks 2 e, 2 e + 1 sit in entry e: entries e and e + 4), then xor 4, 2, 1
         float s[8], qq[8];
@@ -562,10 +620,14 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         *reinterpret_cast<uint16_t*>(p.sf_out + off) = static_cast<uint16_t>(row_ok ? sf2 : 0u);
       }
     }
-    if (lane == 0) tma_store_wait_all<0>();  // the writes, not only the reads of shared memory: the next launch may be waiting for this grid to end
+    if (!paced && lane == 0) tma_store_wait_all<0>();  // the writes, not only the reads of shared memory: the next launch may be waiting for this grid to end
   }
 
   // ---- tear-down
+  if (!epilogue_warp) {
+    __syncwarp();
+    cluster_wait();  // of the arrival above
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -668,7 +730,7 @@ int launch_residual_ln(const vx_gemm_desc* d, const float* gamma, const float* b
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters);
-  cfg.blockDim = dim3(LN_THREADS);
+  cfg.blockDim = dim3(ln_threads(two));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = static_cast<cudaStream_t>(stream);
   cudaLaunchAttribute attr[2];

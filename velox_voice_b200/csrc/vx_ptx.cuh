@@ -306,6 +306,12 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Its halves, for warps that do not need the others yet: every thread that has arrived waits before it arrives again.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Named barrier of some warps of a CTA; `threads` counts those that arrive and those that wait.
+__device__ __forceinline__ void named_bar_arrive(int id, int threads) { asm volatile("barrier.cta.arrive.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void named_bar_sync(int id, int threads) { asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 // shared::cta address of this CTA -> shared::cluster address of the same variable in CTA `rank`
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
   uint32_t r;
