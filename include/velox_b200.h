@@ -186,8 +186,13 @@ int vx_glu_tile(int fmt);
                                   out_fmt = fmt, the bits of vx_quantize_pack on them: out_scales = codes u8 [M, (N - quant_col0) / 2]
                                   (dense), out_scales_sf = SF atoms.  The value third of a fused QKV projection that feeds the
                                   next linear needs no quantizer launch then */
+#define VX_GEMM_NATURAL_SF 2048 /* BLK16 operands, epilogue NONE, fp32 output, sizes vx_bsgemm_natural_sf_supported accepts: a_scales /
+                                  b_scales are the reference's u8 [K/16][M/2] and [K/16][N] (any alignment) instead of SF atoms */
 
 int vx_bsgemm(const vx_gemm_desc* desc, void* stream);
+
+/* Whether VX_GEMM_NATURAL_SF takes this product: one 128 x 128 tile per SM at most, K <= 1024, M even, K % 32 == 0. */
+int vx_bsgemm_natural_sf_supported(int64_t M, int64_t N, int64_t K);
 
 /* One linear of the reference's per-row-scaled lane: out f32 [M, N] = dequant(quantize(x)) . W^T (+ bias), i.e.
  * vx_quantize_pack(ROWSCALE) of the activation rows and vx_bsgemm (NONE / BIAS, fp32 out).  Replaces

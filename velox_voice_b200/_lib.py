@@ -61,6 +61,7 @@ EXPORTS = (
     "vx_power_mel_log_supported",
     "vx_power_mel_log",
     "vx_relpos_attention",
+    "vx_bsgemm_natural_sf_supported",
     "vx_bsgemm_residual_ln_supported",
     "vx_bsgemm_residual_ln",
     "vx_bsgemm_residual_ln2",
@@ -199,6 +200,8 @@ def load(build_if_missing: bool = True) -> C.CDLL:
         lib.vx_power_mel_log.argtypes = [vp, i64, i64, i64, vp, i64, i64, vp, vp, vp, i64, vp]
         lib.vx_relpos_attention.restype = i32
         lib.vx_relpos_attention.argtypes = [vp, vp, vp, i64, i32, i32, i64, vp, i64, vp]
+        lib.vx_bsgemm_natural_sf_supported.restype = i32
+        lib.vx_bsgemm_natural_sf_supported.argtypes = [i64, i64, i64]
         lib.vx_bsgemm_residual_ln_supported.restype = i32
         lib.vx_bsgemm_residual_ln_supported.argtypes = [i32, i64, i64]
         lib.vx_bsgemm_residual_ln.restype = i32

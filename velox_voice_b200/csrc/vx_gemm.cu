@@ -336,7 +336,9 @@ unsigned long long* g_trace_buffer = nullptr;
 //   1  bf16 through staged TMA stores, residual (if any) prefetched by TMA;
 //   2  FP4 re-quantized in the operands' own block format (MX32 for the 32-block kinds, NV16
 //      for the 16-block kinds);
-//   4  as 1, and the columns from quant_col0 on are also quantized (VX_GEMM_QUANT_TAIL).
+//   4  as 1, and the columns from quant_col0 on are also quantized (VX_GEMM_QUANT_TAIL);
+//   5  as 0, one tile per CTA, scale factors in the reference's natural layout (VX_GEMM_NATURAL_SF): the epilogue warps, which
+//      have nothing to do before the MMAs are through, write the atoms of all K stages into their staging buffers.
 template <int KIND, int EPI, int OUT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -394,6 +396,8 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   const int nslots = p.num_slots;
   const bool resident = p.b_resident != 0;
   const bool with_sf = !(FP8 || sf_unit);
+  constexpr bool NAT = OUT == 5;
+  const bool sf_ring = with_sf && !NAT;       // scale factors come with the stages
   const bool sfb_res = p.sfb_resident != 0;   // implies !resident && with_sf
   const bool owns_nb = resident || sfb_res;   // fixed n-block, B scale factors stay in TMEM
 
@@ -444,7 +448,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
       mbar_init(&sm.tmem_full[a], 1);
       mbar_init(&sm.tmem_empty[a], EPI_WARPS);
     }
-    mbar_init(&sm.b_full, 1);
+    mbar_init(&sm.b_full, NAT ? EPI_WARPS : 1);
     mbar_init(&sm.sfb_done, 1);
     for (int w = 0; w < 16; ++w) { mbar_init(&sm.res_full[0][w], 1); mbar_init(&sm.res_full[1][w], 1); }
     mbar_fence_init();
@@ -453,7 +457,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     if (tma_store) prefetch_tmap(&tmap_out);
     if (tma_residual) prefetch_tmap(&tmap_res);
   }
-  if (FP8 || p.N % BNT != 0) {
+  if (!NAT && (FP8 || p.N % BNT != 0)) {
     // Scale-factor tiles of B that lie beyond N are never loaded; they must read as zero
     // (their B rows are zero-filled by TMA, and 0 x NaN-scale would poison the accumulator).
     // With N a whole number of column blocks every tile exists and is loaded: nothing to clear
@@ -491,13 +495,13 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     // =========================== TMA producer ===========================
     if (lane == 0 && my_tiles > 0) {
       uint32_t s = 0, ph = 0;
-      const uint32_t sf_atom_bytes = with_sf ? static_cast<uint32_t>(APS * 512) : 0u;
+      const uint32_t sf_atom_bytes = sf_ring ? static_cast<uint32_t>(APS * 512) : 0u;
       const int64_t sf_stage = APS * 512;
       bool ok = true;
       // B tile (+ its scale factors) of n-block nb, K stage ks -> dst; returns bytes in flight
       auto load_b = [&](uint8_t* dst, int nb, int ks, uint64_t* bar) {
         tma_load_2d(dst, &tmap_b, ks * STAGE_ROW_BYTES, nb * BNT, bar);
-        if (with_sf && !sfb_res) {
+        if (sf_ring && !sfb_res) {
 #pragma unroll
           for (int rt = 0; rt < NRT; ++rt)
             if (nb * NRT + rt < n_sf_tiles)
@@ -507,7 +511,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
       };
       auto b_tx = [&](int nb) -> uint32_t {
         uint32_t t = B_TILE_BYTES;
-        if (with_sf && !sfb_res) {
+        if (sf_ring && !sfb_res) {
 #pragma unroll
           for (int rt = 0; rt < NRT; ++rt)
             if (nb * NRT + rt < n_sf_tiles) t += sf_atom_bytes;
@@ -552,7 +556,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
             const int ks = kg * G + u;
             uint8_t* dst = sm.arena + ring_off + (s * G + u) * slot_bytes;
             tma_load_2d(dst, &tmap_a, ks * STAGE_ROW_BYTES, mb * BM, &sm.full[s]);
-            if (with_sf) bulk_load(dst + TILE_BYTES, sfa_row + ks * sf_stage, APS * 512, &sm.full[s]);
+            if (sf_ring) bulk_load(dst + TILE_BYTES, sfa_row + ks * sf_stage, APS * 512, &sm.full[s]);
             if (!resident) load_b(dst + a_slot, nb, ks, &sm.full[s]);
           }
           if (++s == static_cast<uint32_t>(ngs)) { s = 0; ph ^= 1; }
@@ -615,6 +619,10 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
           for (int rt = 0; rt < NRT; ++rt)
             CP(col0 + a * SFB_COLS + rt * 4, desc(b_lo + b_sf_lo + (rt * APS + a) * 32, sf_hi));
       };
+      if constexpr (NAT) {
+        if (!mbar_wait<WAIT_CALL>(&sm.b_full, 0, p.status, 5)) ok = false;  // the atoms are written
+        tc_fence_after();
+      }
       if (resident) {
         if (!mbar_wait<WAIT_CALL>(&sm.b_full, 0, p.status, 5)) ok = false;
         tc_fence_after();
@@ -700,7 +708,14 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
             const uint32_t sfa_buf = tm_sfa + sfsel * 32;
             const uint32_t sfb_buf = tm_sfb + (owns_nb ? 0u : sfsel * sfb_alt);
             {
-              if (with_sf) {
+              if constexpr (NAT) {
+                const uint32_t a_lo = (smem_u32(sm.staging[0]) >> 4) + kg * (APS * 32), b_lo = a_lo + p.k_stages * (APS * 32);
+  #pragma unroll
+                for (int a = 0; a < APS; ++a) {
+                  CP(sfa_buf + a * 4, desc(a_lo + a * 32, sf_hi));
+                  CP(sfb_buf + a * SFB_COLS, desc(b_lo + a * 32, sf_hi));
+                }
+              } else if (with_sf) {
                 for (int u = 0; u < G; ++u) {
                   const uint32_t a_lo = a_lo0 + u * slot_lo;
   #pragma unroll
@@ -836,6 +851,56 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
 
     int mb = mb0, nb = nb0;
     const int col_base = WIDE && !GLU && !SEQ ? cc * 64 : cc * 32;  // first accumulator column of this warp
+    if constexpr (NAT) {
+      // Scale factors of this CTA's tile: byte (row, K block) of the natural layouts, [K/16][M/2] (a row pair shares one) and [K/16][N],
+      // to the atoms of stage ks: 4-byte words (row, four K blocks).  A warp takes the 128 rows of one operand and stage; lane l
+      // owns rows 4 l .. 4 l + 3, whose bytes of one K block it reads together where they are aligned.
+      static_assert(!NAT || (kind_vec4(KIND) && NRT == 1), "narrow tiles of a 16-block format");
+      const int nkb = static_cast<int>(p.K >> 4);
+      for (int un = ew; un < 2 * p.k_stages; un += EPI_WARPS) {
+        const bool is_b = un >= p.k_stages;
+        const int kb0 = (is_b ? un - p.k_stages : un) * 16;
+        const uint8_t* const base = is_b ? p.sfb : p.sfa;
+        const int64_t pitch = is_b ? p.N : p.M >> 1;                      // bytes of one K block
+        const int64_t at = is_b ? static_cast<int64_t>(nb0) * BNT + 4 * lane : static_cast<int64_t>(mb0) * (BM / 2) + 2 * lane;
+        const uint8_t* src = base + kb0 * pitch + at;
+        uint32_t v[16];
+        if (is_b && ((pitch | reinterpret_cast<uintptr_t>(base)) & 3) == 0) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v[k] = kb0 + k < nkb && at < pitch ? *reinterpret_cast<const uint32_t*>(src + k * pitch) : 0u;
+        } else if (is_b) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            v[k] = 0;
+            for (int i = 0; i < 4; ++i)
+              if (kb0 + k < nkb && at + i < pitch) v[k] |= static_cast<uint32_t>(src[k * pitch + i]) << (8 * i);
+          }
+        } else if (((pitch | reinterpret_cast<uintptr_t>(base)) & 1) == 0) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k)
+            v[k] = kb0 + k < nkb && at < pitch ? __byte_perm(*reinterpret_cast<const uint16_t*>(src + k * pitch), 0, 0x1100) : 0u;
+        } else {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const uint32_t lo = kb0 + k < nkb && at < pitch ? src[k * pitch] : 0u, hi = kb0 + k < nkb && at + 1 < pitch ? src[k * pitch + 1] : 0u;
+            v[k] = lo * 0x0101u | hi * 0x01010000u;
+          }
+        }
+        uint32_t* const dst = reinterpret_cast<uint32_t*>(sm.staging[0] + un * (APS * 512)) + ((4 * lane) & 31) * 4 + (lane >> 3);
+#pragma unroll
+        for (int a = 0; a < APS; ++a) {  // 4 x 4 bytes transposed
+          const uint32_t t0 = __byte_perm(v[4 * a], v[4 * a + 1], 0x5140), t1 = __byte_perm(v[4 * a + 2], v[4 * a + 3], 0x5140);
+          const uint32_t t2 = __byte_perm(v[4 * a], v[4 * a + 1], 0x7362), t3 = __byte_perm(v[4 * a + 2], v[4 * a + 3], 0x7362);
+          dst[a * 128] = __byte_perm(t0, t1, 0x5410);
+          dst[a * 128 + 4] = __byte_perm(t0, t1, 0x7632);
+          dst[a * 128 + 8] = __byte_perm(t2, t3, 0x5410);
+          dst[a * 128 + 12] = __byte_perm(t2, t3, 0x7632);
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.b_full);
+    }
     bool res_inflight = false;
     if constexpr (EPI == VX_EPI_BIAS_RESIDUAL) {
       if (tma_residual && my_tiles > 0 && has_work) {
@@ -1693,7 +1758,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, 
   // shared-memory plan: keep B resident when all of its K stages fit beside a useful ring
   constexpr int BNT = kind_bn(KIND);
   constexpr int APS = kind_vec4(KIND) ? 4 : 2;
-  const bool with_sf = KIND != KIND_FP8 && !p.sf_unit;
+  const bool with_sf = KIND != KIND_FP8 && !p.sf_unit && OUT != 5;
   p.a_slot_bytes = TILE_BYTES + (with_sf ? APS * 512 : 0);
   p.b_slot_bytes = BNT * STAGE_ROW_BYTES + (with_sf ? (BNT / 128) * APS * 512 : 0);
   // keep every slot 1024-byte aligned (128-byte swizzle atoms are 1 KB)
@@ -1773,6 +1838,18 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, 
   return 0;
 }
 
+// VX_GEMM_NATURAL_SF: one narrow tile per CTA, so that every scale is turned into atoms about once per column or row block, and a K whose
+// stages are all in flight at once.  It saves the relayout's launch and adds 1.2 us of loads in front of the MMAs.  Quantizer + product,
+// relayout launch / natural, rows x N x K: 64 x 256 x 512 11.8 / 9.4 us, 1,022 x 256 x 512 11.7 / 10.1, 3,800 x 200 x 512 12.2 / 10.5, 64 x 512 x 1024
+// 11.7 / 10.0, 3,800 x 512 x 1024 16.2 / 15.3; with K = 2048 and two loads per ring slot it gains nothing: 64 x 512 13.0 / 13.1, 130 x 512 13.8 / 14.2.
+constexpr int NAT_STAGES = ARENA_BYTES / (2 * TILE_BYTES);
+bool natural_sf_ok(int64_t M, int64_t N, int64_t K) {
+  if (M <= 0 || N <= 0 || K <= 0 || M % 2 != 0 || K % 32 != 0) return false;
+  const int64_t stages = (K + kStageK4 - 1) / kStageK4, mt = (M + BM - 1) / BM, nt = (N + 127) / 128;
+  static_assert(NAT_STAGES * 2 * 4 * 512 <= 16 * STAGING_BYTES, "the atoms lie in the staging buffers");
+  return stages <= NAT_STAGES && mt <= sm_count() && nt <= sm_count() && mt * nt <= sm_count();
+}
+
 template <int KIND, int EPI>
 int dispatch_out(int out, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to,
                  const CUtensorMap& tr, GemmParams& p, bool res, cudaStream_t st) {
@@ -1843,7 +1920,10 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
     return fail(-1, "operand rows must be 16-byte aligned and at least %lld bytes", (long long)row_bytes);
   if (!d->a_scales || !d->b_scales) return fail(-1, "a_scales and b_scales must not be NULL");
   if (fmt == VX_FMT_NV16 && (!d->a_amax || !d->b_amax)) return fail(-1, "NV16 needs a_amax and b_amax");
-  if (fmt_has_sf(fmt) && (!aligned16(d->a_scales) || !aligned16(d->b_scales)))
+  const bool natural = (d->flags & VX_GEMM_NATURAL_SF) != 0;
+  if (natural && (fmt != VX_FMT_BLK16_A || d->epilogue != VX_EPI_NONE || d->out_dtype != VX_F32 || (d->flags & VX_GEMM_WIDE_TILES) || !natural_sf_ok(M, N, K)))
+    return fail(-1, "VX_GEMM_NATURAL_SF: BLK16 operands, epilogue NONE, fp32 output, a size vx_bsgemm_natural_sf_supported accepts");
+  if (fmt_has_sf(fmt) && !natural && (!aligned16(d->a_scales) || !aligned16(d->b_scales)))
     return fail(-1, "SF atoms must be 16-byte aligned");
   const int epi = d->epilogue;
   if (epi < VX_EPI_NONE || epi > VX_EPI_BIAS_QKVPACK) return fail(-1, "unknown epilogue %d", epi);
@@ -1851,7 +1931,7 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
   const bool qkvpack = epi == VX_EPI_BIAS_QKVPACK;
   const bool out_heads = (d->flags & VX_GEMM_OUT_HEADS) != 0;
   constexpr int32_t kKnownFlags = VX_GEMM_DIRECT_STORE | VX_GEMM_STREAM_B | VX_GEMM_WIDE_TILES | VX_GEMM_NARROW_TILES |
-                                  VX_GEMM_OUT_HEADS | VX_GEMM_POS_F32 | VX_GEMM_CONST_B | VX_GEMM_QUANT_TAIL;
+                                  VX_GEMM_OUT_HEADS | VX_GEMM_POS_F32 | VX_GEMM_CONST_B | VX_GEMM_QUANT_TAIL | VX_GEMM_NATURAL_SF;
   if (d->flags & ~kKnownFlags) return fail(-1, "unknown bits in flags (0x%x)", d->flags & ~kKnownFlags);
   if (qkvpack && fmt == VX_FMT_ROWSCALE)
     return fail(-1, "BIAS_QKVPACK is not available for the per-row-scaled format (use a block-scaled format or FP8)");
@@ -1920,6 +2000,7 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
     // N = 128 MMAs read A from shared memory twice as often and that chain bounds the tile (144 vs 134 us at T = 90000).
     const bool swish_fp4 = epi == VX_EPI_BIAS_SWISH && d->out_dtype == VX_FP4 && d->out_fmt == (vec2 ? VX_FMT_MX32 : VX_FMT_NV16) && fmt != VX_FMT_ROWSCALE;
     if ((d->flags & VX_GEMM_NARROW_TILES) && epi != VX_EPI_BIAS_GLU && !swish_fp4) narrow = true;
+    if (natural) narrow = true;
     if (narrow) kind = vec2 ? KIND_FP4_VEC2_N128 : KIND_FP4_VEC4_N128;
   }
   const int BN = kind_bn(kind);
@@ -2058,6 +2139,7 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
     else if (d->out_dtype == VX_FP4 && !argmax && d->out_fmt == (vec2 ? VX_FMT_MX32 : VX_FMT_NV16))
       out_route = 2;
   }
+  if (natural) return launch<KIND_FP4_VEC4_N128, VX_EPI_NONE, 5>(ta, tb, to, tr, p, false, st);
   switch (kind) {
     case KIND_FP8: return dispatch_epi<KIND_FP8>(epi, out_route, ta, tb, to, tr, p, res, st);
     case KIND_FP4_VEC2: return dispatch_epi<KIND_FP4_VEC2>(epi, out_route, ta, tb, to, tr, p, res, st);
@@ -2066,6 +2148,8 @@ int vx_bsgemm(const vx_gemm_desc* d, void* stream) {
     default: return dispatch_epi<KIND_FP4_VEC4_N128>(epi, out_route, ta, tb, to, tr, p, res, st);
   }
 }
+
+int vx_bsgemm_natural_sf_supported(int64_t M, int64_t N, int64_t K) { return vx::natural_sf_ok(M, N, K) ? 1 : 0; }
 
 int vx_argmax_ids(const void* keys, int64_t M, int32_t* ids, float* max_out, void* stream) {
   using namespace vx;

@@ -29,7 +29,7 @@ namespace {
 
 #define VX_FUNCS(X)                                                                                                 \
   X(vx_last_error) X(vx_quantize_pack) X(vx_ln_quantize_pack) X(vx_ln2_quantize_pack) X(vx_amax) X(vx_bsgemm)        \
-  X(vx_bsgemm_residual_ln_supported) X(vx_bsgemm_residual_ln) X(vx_bsgemm_residual_ln2) X(vx_argmax_ids) X(vx_relpos_attention)   \
+  X(vx_bsgemm_natural_sf_supported) X(vx_bsgemm_residual_ln_supported) X(vx_bsgemm_residual_ln) X(vx_bsgemm_residual_ln2) X(vx_argmax_ids) X(vx_relpos_attention)   \
   X(vx_power_mel_log) X(vx_power_mel_log_supported) X(vx_sf_from_natural_pair) X(vx_rowscale_linear) X(vx_rowscale_linear_scratch) X(vx_ctc_topk_rows) X(vx_ctc_topk)        \
   X(vx_conformer_pass_supported) X(vx_conformer_pass_scratch) X(vx_conformer_pass)
 struct Api {
@@ -451,8 +451,9 @@ PyObject* py_rowscale_linear(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   VX_END
 }
 
-// blkscale_gemm(pack_a, pack_b, scale_a, scale_b) -> f32 [M, N] | None: the reference's per-16 block-scaled product.  The
-// tensor-core copies of both operands' scales live in one scratch block, made by one launch.
+// blkscale_gemm(pack_a, pack_b, scale_a, scale_b) -> f32 [M, N] | None: the reference's per-16 block-scaled product.  Up to one
+// tile per SM the GEMM takes the scales as they are; beyond, the tensor-core copies of both operands' scales live in one
+// scratch block, made by one launch.
 PyObject* py_blkscale_gemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   VX_BEGIN
   VX_ARGS(4)
@@ -470,20 +471,26 @@ PyObject* py_blkscale_gemm(PyObject*, PyObject* const* p, Py_ssize_t nargs) {
   at::Tensor out;
   {
     NoGil nogil;
-    const int64_t na = sf_bytes(VX_FMT_BLK16_A, M, K), nb = sf_bytes(VX_FMT_BLK16_B, N, K);
-    const at::Tensor scratch = empty({na + nb}, at::kByte, dev);
-    uint8_t* const sf = static_cast<uint8_t*>(scratch.data_ptr());
-    out = empty({M, N}, at::kFloat, dev);
-    check(g.vx_sf_from_natural_pair(VX_FMT_BLK16_A, sa.data_ptr(), M, sf, VX_FMT_BLK16_B, sb.data_ptr(), N, sf + na, K, stream()),
-          "vx_sf_from_natural_pair");
-    count();
     vx_gemm_desc d{};
+    at::Tensor scratch;
+    if (g.vx_bsgemm_natural_sf_supported(M, N, K)) {
+      d.flags = VX_GEMM_NATURAL_SF;
+      d.a_scales = sa.data_ptr(); d.b_scales = sb.data_ptr();
+    } else {
+      const int64_t na = sf_bytes(VX_FMT_BLK16_A, M, K), nb = sf_bytes(VX_FMT_BLK16_B, N, K);
+      scratch = empty({na + nb}, at::kByte, dev);
+      uint8_t* const sf = static_cast<uint8_t*>(scratch.data_ptr());
+      check(g.vx_sf_from_natural_pair(VX_FMT_BLK16_A, sa.data_ptr(), M, sf, VX_FMT_BLK16_B, sb.data_ptr(), N, sf + na, K, stream()),
+            "vx_sf_from_natural_pair");
+      count();
+      d.a_scales = sf; d.b_scales = sf + na;
+    }
+    out = empty({M, N}, at::kFloat, dev);
     d.struct_size = sizeof(d);
     d.fmt = VX_FMT_BLK16_A;
     d.M = M; d.N = N; d.K = K;
     d.a_codes = pa.data_ptr(); d.lda = pa.stride(0);
     d.b_codes = pb.data_ptr(); d.ldb = pb.stride(0);
-    d.a_scales = sf; d.b_scales = sf + na;
     d.epilogue = VX_EPI_NONE;
     d.out_dtype = VX_F32; d.out = out.data_ptr(); d.ldo = N;
     launch(d);

@@ -71,9 +71,10 @@ extern "C" int vx_blkscale_gemm_noalloc(const void* pack_a, const void* pack_b, 
   if (rc) return rc;
   uint8_t* sfa = scratch;
   uint8_t* sfb = scratch + VX_NOALLOC_SF_MAX_BYTES;
+  const bool natural = vx_bsgemm_natural_sf_supported(M, N, K) != 0;  // the GEMM takes the scales as they are: no scratch
   // the relayout clears the bytes it owns (padding rows / K groups must read as zero), so the
   // previous call's contents never leak into this one
-  rc = vx_sf_from_natural_pair(VX_FMT_BLK16_A, scale_a, M, sfa, VX_FMT_BLK16_B, scale_b, N, sfb, K, stream);
+  rc = natural ? 0 : vx_sf_from_natural_pair(VX_FMT_BLK16_A, scale_a, M, sfa, VX_FMT_BLK16_B, scale_b, N, sfb, K, stream);
   if (rc) return rc;
   vx_gemm_desc d = {};
   d.struct_size = static_cast<int32_t>(sizeof(vx_gemm_desc));
@@ -81,7 +82,8 @@ extern "C" int vx_blkscale_gemm_noalloc(const void* pack_a, const void* pack_b, 
   d.M = M; d.N = N; d.K = K;
   d.a_codes = pack_a; d.lda = K / 2;
   d.b_codes = pack_b; d.ldb = K / 2;
-  d.a_scales = sfa; d.b_scales = sfb;
+  d.a_scales = natural ? scale_a : sfa; d.b_scales = natural ? scale_b : sfb;
+  d.flags = natural ? VX_GEMM_NATURAL_SF : 0;
   d.epilogue = VX_EPI_NONE;
   d.out_dtype = VX_F32;
   d.out = out; d.ldo = N;
