@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "vx_common.cuh"
+#include "vx_ptx.cuh"
 #include "vx_quant_math.cuh"
 
 namespace vx {
@@ -126,9 +127,10 @@ __device__ __forceinline__ void swish_group8(const uint32_t (&r)[32], int g, con
       // (acc + bias) / 2 = fma(acc, 1/2, bias / 2) bit for bit; the caller's table holds bias / 2
       const uint64_t half2 = pack_f32x2(0.5f, 0.5f);
       if constexpr (BIAS) {
-        const float4 b = *reinterpret_cast<const float4*>(bias_s + 4 * q4);
-        za = fma_f32x2(za, half2, pack_f32x2(b.x, b.y));
-        zb = fma_f32x2(zb, half2, pack_f32x2(b.z, b.w));
+        uint64_t ba, bb;
+        ld_shared_pairs(smem_u32(bias_s) + 16 * q4, ba, bb);
+        za = fma_f32x2(za, half2, ba);
+        zb = fma_f32x2(zb, half2, bb);
       } else {
         za = mul_f32x2(za, half2);
         zb = mul_f32x2(zb, half2);
@@ -136,9 +138,10 @@ __device__ __forceinline__ void swish_group8(const uint32_t (&r)[32], int g, con
       swish4p_half(za, zb);
     } else {
       if constexpr (BIAS) {
-        const float4 b = *reinterpret_cast<const float4*>(bias_s + 4 * q4);
-        za = add_f32x2(za, pack_f32x2(b.x, b.y));
-        zb = add_f32x2(zb, pack_f32x2(b.z, b.w));
+        uint64_t ba, bb;
+        ld_shared_pairs(smem_u32(bias_s) + 16 * q4, ba, bb);
+        za = add_f32x2(za, ba);
+        zb = add_f32x2(zb, bb);
       }
       swish4p<false>(za, zb);
     }
@@ -189,10 +192,9 @@ __device__ __forceinline__ uint32_t encode_group8(const uint64_t (&sv)[16], int 
   return e2m1_pack8p<false, true>(v, NV16 && g >= 2 ? rcp1 : rcp0);
 }
 
+// ... in two steps: the Swish values of the chunk, and their scales and codes.
 template <bool NV16>
-__device__ __forceinline__ uint32_t swish_quant_chunk(const uint32_t (&r)[32], const float* bias_s, bool scale_acc,
-                                                      float g_ab, const Nv16Tensor& nv, const float* nv_tab, uint32_t (&w)[4]) {
-  uint64_t sv[16];
+__device__ __forceinline__ void swish_chunk(const uint32_t (&r)[32], const float* bias_s, bool scale_acc, float g_ab, uint64_t (&sv)[16]) {
   const uint64_t g2 = pack_f32x2(g_ab, g_ab);
   // (the bias test once per chunk, not once per four values: the epilogue is bound by instruction issue)
   if (bias_s) {
@@ -212,11 +214,21 @@ __device__ __forceinline__ uint32_t swish_quant_chunk(const uint32_t (&r)[32], c
       for (int j = 0; j < 4; ++j) sv[4 * g + j] = o[j];
     }
   }
+}
+template <bool NV16>
+__device__ __forceinline__ uint32_t quant_chunk(const uint64_t (&sv)[16], const Nv16Tensor& nv, const float* nv_tab, uint32_t (&w)[4]) {
   float rcp0, rcp1;
   const uint32_t sbytes = chunk_scales_p<NV16>(sv, nv, nv_tab, rcp0, rcp1);
 #pragma unroll
   for (int g = 0; g < 4; ++g) w[g] = encode_group8<NV16>(sv, g, rcp0, rcp1);
   return sbytes;
+}
+template <bool NV16>
+__device__ __forceinline__ uint32_t swish_quant_chunk(const uint32_t (&r)[32], const float* bias_s, bool scale_acc,
+                                                      float g_ab, const Nv16Tensor& nv, const float* nv_tab, uint32_t (&w)[4]) {
+  uint64_t sv[16];
+  swish_chunk<NV16>(r, bias_s, scale_acc, g_ab, sv);
+  return quant_chunk<NV16>(sv, nv, nv_tab, w);
 }
 
 // z += 32 bias values cached in shared memory (all lanes read the same words)

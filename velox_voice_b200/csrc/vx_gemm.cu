@@ -446,7 +446,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     }
     for (int a = 0; a < FP8_ACCS; ++a) {
       mbar_init(&sm.tmem_full[a], 1);
-      mbar_init(&sm.tmem_empty[a], EPI_WARPS);
+      mbar_init(&sm.tmem_empty[a], SWQ ? EPI_WARPS / 2 : EPI_WARPS);
     }
     mbar_init(&sm.b_full, NAT ? EPI_WARPS : 1);
     mbar_init(&sm.sfb_done, 1);
@@ -788,7 +788,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     const bool tr = tr_on && ew == 0 && lane == 0;
     uint32_t group = 0;  // FP8: rounds taken
     const uint32_t accs = UNITS ? p.accs : 1;
-    uint32_t es = 0, eph = 0;  // accumulator read next, parity of the wait for it
+    uint32_t es = SWQ ? static_cast<uint32_t>(cc >> 1) : 0u, eph = 0;  // accumulator read next, parity of the wait for it
     auto next_acc = [&] { if (++es == accs) { es = 0; eph ^= 1; } };
     bool ok = true;
     float g_ab = 1.0f, g_out = 1.0f;
@@ -850,7 +850,11 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
     };
 
     int mb = mb0, nb = nb0;
-    const int col_base = WIDE && !GLU && !SEQ ? cc * 64 : cc * 32;  // first accumulator column of this warp
+    const int col_base = (WIDE && !GLU && !SEQ) || SWQ ? cc * 64 : cc * 32;  // first accumulator column of this warp
+    // Swish + FP4 output: this thread's codes and scale bytes in the tile at row block 0, column block 0
+    uint8_t* const code0 = static_cast<uint8_t*>(p.out) + (q * 32 + lane) * p.ldo + (col_base >> 1);
+    uint8_t* const sf0 = p.out_sf + lane * 16 + q * 4 + (kind_vec4(KIND) ? cc * 512 : (cc >> 1) * 512 + (cc & 1) * 2);
+    const int64_t code_tile = BM * p.ldo;
     if constexpr (NAT) {
       // Scale factors of this CTA's tile: byte (row, K block) of the natural layouts, [K/16][M/2] (a row pair shares one) and [K/16][N],
       // to the atoms of stage ks: 4-byte words (row, four K blocks).  A warp takes the 128 rows of one operand and stage; lane l
@@ -919,7 +923,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         // (re)load this warp's bias values: lane i fetches the i-th column of each chunk
         __syncwarp();
         const int64_t c0 = static_cast<int64_t>(nb) * BNT + col_base + lane;
-        const int64_t c1 = GLU ? c0 + GATE_OFF : c0 + CH_STRIDE;
+        const int64_t c1 = GLU ? c0 + GATE_OFF : c0 + (SWQ ? 32 : CH_STRIDE);
         constexpr float BIAS_SCALE = SWQ && !kind_vec4(KIND) ? 0.5f : 1.0f;  // see swish_group8
         bias_w[lane] = BIAS_SCALE * (c0 < p.N ? __ldg(p.bias + c0) : 0.0f);
         bias_w[32 + lane] = BIAS_SCALE * (c1 < p.N ? __ldg(p.bias + c1) : 0.0f);
@@ -927,49 +931,66 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         bias_nb = nb;
       }
       if constexpr (SWQ) {
-        // FFN up-projection: accumulator -> bias + Swish -> E2M1 codes + scale factors, one
-        // 32-column chunk at a time (the second chunk of a wide tile is read from tensor memory
-        // only after the first is finished, so that one chunk's registers are live at a time;
-        // the MMAs of the next tile then run under the arithmetic of the second chunk)
-        const uint32_t acc_addr = lane_addr + TM_ACC0 + col_base;
+        // FFN up-projection: accumulator -> bias + Swish -> E2M1 codes + scale factors.  The warps of column groups 0 and 1 take the first
+        // half of every tile, the others the second: 64 adjacent columns each, as two chunks of 32 that are in registers one after the
+        // other.  Time follows the number of instructions (283 warp instructions per chunk at 0.58 per cycle and scheduler; without tanh the
+        // same 87 us), and a third of them were the waits, hand-overs and addresses of a chunk: once per two chunks now, and the codes of a
+        // row fill a sector.  90,000 x 512 x 2,048, one chunk of each half per warp / like this: 86.8 / 74.6 us (without the read of the second
+        // chunk under the codes of the first 85.8, with it but the bias read as float4 81.4), NV16 123.0 / 114.7; 5,000 rows 10.0 / 9.0.
         if (tr) trace_rec(p, 2, it, 0);
         const bool scale_acc = kind_vec4(KIND) && p.a_amax != nullptr;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {  // halves of the tile
-          ok = __all_sync(0xffffffffu, mbar_wait_spin<WAIT_CALL>(&sm.tmem_full[es], eph, p.status, 4));
-          if (!ok) break;
-          tc_fence_after();
-          if (tr && h == 0) trace_rec(p, 2, it, 1);
-          uint32_t r[32];
-          tc_ld_32x32b_x32(acc_addr + es * 128, r);
-          tc_wait_ld();
+        ok = __all_sync(0xffffffffu, mbar_wait_spin<WAIT_CALL>(&sm.tmem_full[es], eph, p.status, 4));
+        if (!ok) break;
+        tc_fence_after();
+        if (tr) trace_rec(p, 2, it, 1);
+        const uint32_t acc_addr = lane_addr + TM_ACC0 + es * 128 + (cc & 1) * 64;
+        uint8_t* const code = code0 + mb * code_tile + nb * (BNT / 2);
+        const bool cols_ok = static_cast<int64_t>(nb) * BNT + col_base < p.N, code_ok = cols_ok && row_ok;
+        constexpr bool NV = kind_vec4(KIND);
+        uint32_t sbytes = 0, w[4], r[32];
+        auto release = [&] {
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&sm.tmem_empty[es]);
-          next_acc();
-          if (tr && h == 0) trace_rec(p, 2, it, 2);
-          const int64_t out_col0 = static_cast<int64_t>(nb) * BNT + col_base + h * CH_STRIDE;
-          uint32_t w[4];
-          const uint32_t sb = swish_quant_chunk<kind_vec4(KIND)>(r, bias_base ? bias_base + h * 32 : nullptr, scale_acc, g_ab,
-                                                                 nv, nv_tab, w);
-          if (out_col0 < p.N) {
-            if (row_ok)
-              *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + row * p.ldo + (out_col0 >> 1)) =
-                  make_uint4(w[0], w[1], w[2], w[3]);
-            // rows of the last tile beyond M get zero scale factors (the SF atoms cover whole 128-row tiles)
-            const uint32_t sbw = row_ok ? sb : 0u;
-            const int64_t sf_row = (row >> 7) * p.out_sf_kg * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4;
-            if constexpr (!kind_vec4(KIND)) {
-              p.out_sf[sf_row + (out_col0 >> 7) * 512 + ((out_col0 >> 5) & 3)] = static_cast<uint8_t>(sbw);
-              if (p.out_scales && row_ok) p.out_scales[row * (p.N >> 5) + (out_col0 >> 5)] = static_cast<uint8_t>(sbw);
-            } else {
-              *reinterpret_cast<uint16_t*>(p.out_sf + sf_row + (out_col0 >> 6) * 512 + ((out_col0 >> 5) & 1) * 2) =
-                  static_cast<uint16_t>(sbw);
-              if (p.out_scales && row_ok)
-                *reinterpret_cast<uint16_t*>(p.out_scales + row * (p.N >> 4) + (out_col0 >> 4)) = static_cast<uint16_t>(sbw);
-            }
+        };
+        if constexpr (NV) {  // (too many registers live for the order below: 119 us like this, 138)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            tc_ld_32x32b_x32(acc_addr + c * 32, r);
+            tc_wait_ld();
+            if (c == 1) release();
+            const uint32_t sb = swish_quant_chunk<NV>(r, bias_base ? bias_base + c * 32 : nullptr, scale_acc, g_ab, nv, nv_tab, w);
+            if (code_ok) *reinterpret_cast<uint4*>(code + c * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+            sbytes |= sb << (16 * c);
           }
-          if (tr) trace_rec(p, 2, it, h == 0 ? 4 : 6);
+        } else {
+          uint64_t sv[16];
+          tc_ld_32x32b_x32(acc_addr, r);
+          tc_wait_ld();
+          swish_chunk<NV>(r, bias_base, scale_acc, g_ab, sv);
+          tc_ld_32x32b_x32(acc_addr + 32, r);  // comes in under the codes of the first chunk
+          sbytes = quant_chunk<NV>(sv, nv, nv_tab, w);
+          if (code_ok) *reinterpret_cast<uint4*>(code) = make_uint4(w[0], w[1], w[2], w[3]);
+          tc_wait_ld();
+          release();
+          swish_chunk<NV>(r, bias_base ? bias_base + 32 : nullptr, scale_acc, g_ab, sv);
+          sbytes |= quant_chunk<NV>(sv, nv, nv_tab, w) << 8;
+          if (code_ok) *reinterpret_cast<uint4*>(code + 16) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        if (tr) trace_rec(p, 2, it, 6);
+        es += 2;
+        if (es >= accs) { es -= accs; eph ^= 1; }
+        if (cols_ok) {
+          // rows of the last tile beyond M get zero scale factors (the SF atoms cover whole 128-row tiles)
+          const uint32_t sbw = row_ok ? sbytes : 0u;
+          uint8_t* const sf = sf0 + (mb * p.out_sf_kg + nb * (kind_vec4(KIND) ? 4 : 2)) * 512;
+          if constexpr (!kind_vec4(KIND)) *reinterpret_cast<uint16_t*>(sf) = static_cast<uint16_t>(sbw);
+          else *reinterpret_cast<uint32_t*>(sf) = sbw;
+          if (p.out_scales && row_ok) {  // and in the natural layout
+            const int64_t col = static_cast<int64_t>(nb) * BNT + col_base;
+            if constexpr (!kind_vec4(KIND)) *reinterpret_cast<uint16_t*>(p.out_scales + row * (p.N >> 5) + (col >> 5)) = static_cast<uint16_t>(sbw);
+            else *reinterpret_cast<uint32_t*>(p.out_scales + row * (p.N >> 4) + (col >> 4)) = sbw;
+          }
         }
         if (!ok) break;
         mb = mb_next;
