@@ -425,9 +425,10 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         uint64_t S = pack_f32x2(0.0f, 0.0f), Q = S;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const float* bs = sm.bias + k * 32 + piece[c] * 8;
-          const float4 b0 = *reinterpret_cast<const float4*>(bs), b1 = *reinterpret_cast<const float4*>(bs + 4);
-          const uint64_t bb[4] = {pack_f32x2(b0.x, b0.y), pack_f32x2(b0.z, b0.w), pack_f32x2(b1.x, b1.y), pack_f32x2(b1.z, b1.w)};
+          const uint32_t bs = smem_u32(sm.bias + k * 32 + piece[c] * 8);
+          uint64_t bb[4];
+          ld_shared_pairs(bs, bb[0], bb[1]);
+          ld_shared_pairs(bs + 16, bb[2], bb[3]);
           uint4* const slot = reinterpret_cast<uint4*>(stage_row + (((4 * t + piece[c]) ^ sw) << 4));
           const uint4 res = *slot;
           const uint32_t rw[4] = {res.x, res.y, res.z, res.w};
@@ -535,17 +536,18 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           uint64_t S = pack_f32x2(0.0f, 0.0f), Q = S;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const float4* ga = reinterpret_cast<const float4*>(sm.gamma + k * 32 + piece[c] * 8);
-            const float4* be = reinterpret_cast<const float4*>(sm.beta + k * 32 + piece[c] * 8);
+            const uint32_t ga = smem_u32(sm.gamma + k * 32 + piece[c] * 8), be = smem_u32(sm.beta + k * 32 + piece[c] * 8);
             uint32_t w[4];
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
-              const float4 gv = ga[hh], bv = be[hh];
+              uint64_t g0, g1, b0, b1;
+            ld_shared_pairs(ga + 16 * hh, g0, g1);
+            ld_shared_pairs(be + 16 * hh, b0, b1);
               const uint32_t w0 = xp[4 * c + 2 * hh], w1 = xp[4 * c + 2 * hh + 1];
               const uint64_t x0 = pack_f32x2(__uint_as_float(w0 << 16), __uint_as_float(w0 & 0xffff0000u));
               const uint64_t x1 = pack_f32x2(__uint_as_float(w1 << 16), __uint_as_float(w1 & 0xffff0000u));
-              const uint64_t y0 = fma_f32x2(fma_f32x2(x0, R2, N2), pack_f32x2(gv.x, gv.y), pack_f32x2(bv.x, bv.y));
-              const uint64_t y1 = fma_f32x2(fma_f32x2(x1, R2, N2), pack_f32x2(gv.z, gv.w), pack_f32x2(bv.z, bv.w));
+              const uint64_t y0 = fma_f32x2(fma_f32x2(x0, R2, N2), g0, b0);
+              const uint64_t y1 = fma_f32x2(fma_f32x2(x1, R2, N2), g1, b1);
               float a0, a1, a2, a3;
               unpack_f32x2(y0, a0, a1);
               unpack_f32x2(y1, a2, a3);
@@ -586,16 +588,17 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         float a[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const float4* ga = reinterpret_cast<const float4*>(gamma_q + k * 32 + piece[c] * 8);
-          const float4* be = reinterpret_cast<const float4*>(beta_q + k * 32 + piece[c] * 8);
+          const uint32_t ga = smem_u32(gamma_q + k * 32 + piece[c] * 8), be = smem_u32(beta_q + k * 32 + piece[c] * 8);
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
-            const float4 gv = ga[hh], bv = be[hh];
+            uint64_t g0, g1, b0, b1;
+            ld_shared_pairs(ga + 16 * hh, g0, g1);
+            ld_shared_pairs(be + 16 * hh, b0, b1);
             const uint32_t w0 = xp[4 * c + 2 * hh], w1 = xp[4 * c + 2 * hh + 1];
             const uint64_t x0 = pack_f32x2(__uint_as_float(w0 << 16), __uint_as_float(w0 & 0xffff0000u));
             const uint64_t x1 = pack_f32x2(__uint_as_float(w1 << 16), __uint_as_float(w1 & 0xffff0000u));
-            v[c][2 * hh] = fma_f32x2(fma_f32x2(x0, R2, N2), pack_f32x2(gv.x, gv.y), pack_f32x2(bv.x, bv.y));
-            v[c][2 * hh + 1] = fma_f32x2(fma_f32x2(x1, R2, N2), pack_f32x2(gv.z, gv.w), pack_f32x2(bv.z, bv.w));
+            v[c][2 * hh] = fma_f32x2(fma_f32x2(x0, R2, N2), g0, b0);
+            v[c][2 * hh + 1] = fma_f32x2(fma_f32x2(x1, R2, N2), g1, b1);
           }
           a[c] = amax8p(v[c]);
         }

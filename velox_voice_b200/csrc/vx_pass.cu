@@ -454,13 +454,14 @@ __global__ void __launch_bounds__(PS_THREADS, 1) conformer_pass_kernel(const __g
     // four LayerNorm outputs (values 4 hh .. of piece c) as two packed pairs
     auto normed = [&](const uint32_t (&xp)[16], int c, int hh, const float* ga, const float* be, uint64_t R2, uint64_t N2, uint64_t& y0,
                       uint64_t& y1) {
-      const float4 gv = *reinterpret_cast<const float4*>(ga + piece[c] * 8 + 4 * hh);
-      const float4 bv = *reinterpret_cast<const float4*>(be + piece[c] * 8 + 4 * hh);
+      uint64_t g0, g1, b0, b1;
+      ld_shared_pairs(smem_u32(ga + piece[c] * 8 + 4 * hh), g0, g1);
+      ld_shared_pairs(smem_u32(be + piece[c] * 8 + 4 * hh), b0, b1);
       const uint32_t w0 = xp[4 * c + 2 * hh], w1 = xp[4 * c + 2 * hh + 1];
       const uint64_t x0 = pack_f32x2(__uint_as_float(w0 << 16), __uint_as_float(w0 & 0xffff0000u));
       const uint64_t x1 = pack_f32x2(__uint_as_float(w1 << 16), __uint_as_float(w1 & 0xffff0000u));
-      y0 = fma_f32x2(fma_f32x2(x0, R2, N2), pack_f32x2(gv.x, gv.y), pack_f32x2(bv.x, bv.y));
-      y1 = fma_f32x2(fma_f32x2(x1, R2, N2), pack_f32x2(gv.z, gv.w), pack_f32x2(bv.z, bv.w));
+      y0 = fma_f32x2(fma_f32x2(x0, R2, N2), g0, b0);
+      y1 = fma_f32x2(fma_f32x2(x1, R2, N2), g1, b1);
     };
 
 #pragma unroll 1
@@ -581,9 +582,10 @@ __global__ void __launch_bounds__(PS_THREADS, 1) conformer_pass_kernel(const __g
             const uint64_t A2 = pack_f32x2(alpha, alpha);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-              const float* bs = par + g * 32 + piece[c] * 8;
-              const float4 b0 = *reinterpret_cast<const float4*>(bs), b1 = *reinterpret_cast<const float4*>(bs + 4);
-              const uint64_t bb[4] = {pack_f32x2(b0.x, b0.y), pack_f32x2(b0.z, b0.w), pack_f32x2(b1.x, b1.y), pack_f32x2(b1.z, b1.w)};
+              const uint32_t bs = smem_u32(par + g * 32 + piece[c] * 8);
+              uint64_t bb[4];
+              ld_shared_pairs(bs, bb[0], bb[1]);
+              ld_shared_pairs(bs + 16, bb[2], bb[3]);
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 const uint32_t rw = xp[4 * c + e];

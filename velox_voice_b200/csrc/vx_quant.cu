@@ -745,10 +745,11 @@ __global__ void __launch_bounds__(256, LN ? VX_R2_MIN_BLOCKS_LN : VX_R2_MIN_BLOC
         auto normalise = [&](int c) {
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
-            const float4 ga = gb_s[pass][0][c * 2 + hh][j];
-            const float4 be = gb_s[pass][1][c * 2 + hh][j];
-            v[c][2 * hh] = fma_f32x2(fma_f32x2(v[c][2 * hh], R2, N2), pack_f32x2(ga.x, ga.y), pack_f32x2(be.x, be.y));
-            v[c][2 * hh + 1] = fma_f32x2(fma_f32x2(v[c][2 * hh + 1], R2, N2), pack_f32x2(ga.z, ga.w), pack_f32x2(be.z, be.w));
+            uint64_t g0, g1, b0, b1;
+            ld_shared_pairs(smem_u32(&gb_s[pass][0][c * 2 + hh][j]), g0, g1);
+            ld_shared_pairs(smem_u32(&gb_s[pass][1][c * 2 + hh][j]), b0, b1);
+            v[c][2 * hh] = fma_f32x2(fma_f32x2(v[c][2 * hh], R2, N2), g0, b0);
+            v[c][2 * hh + 1] = fma_f32x2(fma_f32x2(v[c][2 * hh + 1], R2, N2), g1, b1);
           }
         };
         if (!(p.y && pass == 0)) {
