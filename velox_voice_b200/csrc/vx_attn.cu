@@ -29,7 +29,7 @@
 // row and step, 16 lanes per cycle and SM: 512 cycles per CTA and step; the MMAs take 400).  3,750 frames and 8 heads: 99 us
 // with one CTA per SM, P through shared memory and a maximum exchange between two warps per row (3,200 cycles per 128 x 128
 // tile); 62 us with two CTAs and P over S, where the round trip of a buffer -- P V, then the S behind it -- made the softmax
-// wait 340 cycles a step; 58 us with the maximum of the first 64 keys as reference, 60 us like this.  (The shared maximum in every
+// wait 340 cycles a step; 58 us with the maximum of the first 64 keys as reference, 60 with that of 128, 58 without a wait of its own for the buffer of P.  (The shared maximum in every
 // pair of steps: 70 us, the softmax then waits for the second S.)  Neither eight softmax warps per CTA in two independent groups (73 us) nor a
 // quarter of the exponentials as polynomials on the fp32 pipe (64 us) helped.
 // Every mbarrier wait is bounded.

@@ -387,11 +387,11 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   const int out_fmt = OUT == 2 || OUT == 4 ? static_cast<int>(kind_vec4(KIND) ? VX_FMT_NV16 : VX_FMT_MX32) : p.out_fmt;
   const bool tr_on = kPhaseTrace && p.trace != nullptr && blockIdx.x == 0;  // phase trace requested (CTA 0 only)
 
-  // The roles by a uniform warp index (warp_index) gain where registers or issue are short, and cost the others: captured calls in a
-  // row, per-lane against uniform, MX32: GLU 24,000 rows 15.3 and 13.9 us, residual 9.38 and 9.26, fold pack 63.6 and 62.0; but FFN-up
-  // (Swish, FP4) 26.0 and 26.7, arg-max 3,750 rows 17.5 and 17.9, fp32 result 1,537 x 2,048 6.50 and 6.87, plain bias 375 rows 4.04 and 4.15.
-  // (NV16: +4 to -10 % uniform, -5 % only for fp32 results of some sizes.)
-  constexpr bool LANE_ROLES = kind_pow2_scales(KIND) && (SWQ || EPI == VX_EPI_BIAS_ARGMAX || (EPI == VX_EPI_BIAS && OUT < 2));
+  // The roles by a uniform warp index (warp_index) gain where registers or issue are short, and cost some of the others: captured calls in a
+  // row, per-lane against uniform, MX32: FFN-up (Swish, FP4) 90,000 rows 74.6 and 70.0 us, 5,000 9.05 and 8.62, arg-max 90,000 rows 216.4 and 206.7, 3,750
+  // 17.0 and 16.4, GLU 24,000 rows 15.3 and 13.9, residual 9.38 and 9.26, fold pack 63.6 and 62.0; but plain bias 3,750 x 5,538 14.1 and 14.4, per-row
+  // format 1,537 rows 9.93 and 10.0, and for the rest of it +-1.5 %.  (NV16: +4 to -10 % uniform, -5 % only for fp32 results of some sizes.)
+  constexpr bool LANE_ROLES = kind_pow2_scales(KIND) && EPI == VX_EPI_BIAS && OUT < 2;
   const int warp = LANE_ROLES ? static_cast<int>(threadIdx.x >> 5) : warp_index();
   const int lane = threadIdx.x & 31;
   // (The waits below take no abort flag: a flag that the roles poll was built and measured -- the
@@ -966,7 +966,7 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
         // half of every tile, the others the second: 64 adjacent columns each, as two chunks of 32 that are in registers one after the
         // other.  Time follows the number of instructions (283 warp instructions per chunk at 0.58 per cycle and scheduler; without tanh the
         // same 87 us), and a third of them were the waits, hand-overs and addresses of a chunk: once per two chunks now, and the codes of a
-        // row fill a sector.  90,000 x 512 x 2,048, one chunk of each half per warp / like this: 86.8 / 74.6 us (without the read of the second
+        // row fill a sector.  90,000 x 512 x 2,048, one chunk of each half per warp / like this: 86.8 / 74.6 us and, with the uniform warp index, 70.1 (without the read of the second
         // chunk under the codes of the first 85.8, with it but the bias read as float4 81.4), NV16 123.0 / 114.7; 5,000 rows 10.0 / 9.0.
         if (tr) trace_rec(p, 2, it, 0);
         const bool scale_acc = kind_vec4(KIND) && p.a_amax != nullptr;

@@ -24,8 +24,8 @@
 // activations, 17 issues the MMAs (one elected lane), 18 and 19 load weights and the biases and LayerNorm parameters, which depend on
 // no layer and run ahead of them through rings of four and three slots.  Accumulators: a ring of three times 128 columns.
 //
-// Measured, whole greedy pass of 12 blocks, separate launches against this: 375 frames 752 us -> 579, 1,920 frames (the most for
-// clusters of eight) 838 -> 592, 4,000 frames (clusters of four) 988 -> 718, 4,200 frames 1,038 -> 760 (its twelve positional projections are launches of their own).  What bounds it now, of 92,000 cycles a
+// Measured, whole greedy pass of 12 blocks, separate launches against this: 375 frames 752 us -> 558, 1,920 frames (the most for
+// clusters of eight) 838 -> 571, 4,000 frames (clusters of four) 988 -> 695, 4,200 frames 1,038 -> 737 (its twelve positional projections are launches of their own).  What bounds it now, of 88,000 cycles a
 // block (47 us, clusters of eight): the hand-over of an operand, 4,000 a phase -- the release waits 1,750 for the stores, fence and loads take
 // 1,900 --, the issue of the MMAs, 500 to 700 cycles per stage of four, and the chain accumulator -> sums -> exchange -> quantize of
 // the four LayerNorms, 4,000 each.  Tried and not kept: operands pushed to the other CTAs' shared memory by st.async (630 us) or bulk
@@ -748,7 +748,7 @@ int vx_conformer_pass_supported(int fmt, int64_t d_model, int64_t ffn, int64_t c
          blocks <= PS_MAX_BLOCKS;
 }
 
-// One round of clusters of four.  4,200 frames: separate launches 1,038 us, one launch 760; a second round takes as long again, and
+// One round of clusters of four.  4,200 frames: separate launches 1,038 us (4,300 frames now 1,004), one launch 737; a second round takes as long again, and
 // the launches that pipeline over many row blocks are as fast (4,608 frames: 1,075 and about 1,450).
 int64_t vx_conformer_pass_frames(void) {
   return static_cast<int64_t>(vx::max_clusters<4>()) * vx::PS_BM;
