@@ -133,3 +133,14 @@ def test_what_writes_weights_does_not_trigger_the_next_launch():
     pair = text[text.index("int vx_sf_from_natural_pair("):]
     assert re.search(r"launch_dependent\(sf_relayout_kernel.*?side\[1\]\.words != 0 \? 1 : 0\)\)", pair, re.S)
     assert "vx_sf_from_natural_pair(fmt, scales, R, scales_sf, fmt, nullptr, 0, nullptr, K, stream)" in pair
+
+
+@pytest.mark.parametrize("name,kernel", [("vx_quant.cu", "ln_quant_kernel(const QuantParams p) {"), ("vx_quant.cu", "rows2_kernel(const QuantParams p) {")])
+def test_parameters_are_read_behind_the_wait(name, kernel):
+    """A library GEMM may have written a bias, a LayerNorm parameter or a filterbank, and triggers the launch behind it early: no address
+    of one is formed ahead of that launch's wait."""
+    text = source(name)
+    text = text[text.index(kernel):]
+    text = text[:re.search(r"\n}\n", text).end()]
+    ahead = text[:text.index("pdl_wait()")]
+    assert not re.search(r"\bp\.(bias|gamma2?|beta2?|mel)\b(?! \? 2 : 1)", ahead), (name, kernel)
