@@ -56,3 +56,22 @@ def test_layernorm_quantizers(fmt, K, M):
     if fmt == "mx32":
         assert stale(2, K, lambda p: ops.ln2_quantize(x, one, p[0], p[1], one, 1e-5, fmt, y=torch.empty_like(x)).codes) == 0
         assert stale(2, K, lambda p: ops.layernorm(x, p[0], p[1], 1e-5)) == 0
+
+
+@pytest.mark.parametrize("K", [512, 2048])
+@pytest.mark.parametrize("M", [100, 10000])
+def test_residual_layernorm_gemm(M, K):
+    from velox_voice_b200 import ops
+    from velox_voice_b200.linear import PackedLinear
+
+    lin = PackedLinear(0.05 * torch.randn(512, K, device="cuda"), torch.zeros(512, device="cuda"), "mx32")
+    a = ops.quantize(torch.randn(M, K, device="cuda").bfloat16(), "mx32")
+    res, one = torch.randn(M, 512, device="cuda").bfloat16(), torch.ones(512, device="cuda")
+
+    def call(bias=one, gamma=one, beta=one, **two):
+        lin.bias = bias
+        return lin.residual_ln(a, residual=res, gamma=gamma, beta=beta, eps=1e-5, alpha=1.0, **two)[1].codes
+
+    assert stale(1, 512, lambda p: call(bias=p[0])) == 0
+    assert stale(2, 512, lambda p: call(gamma=p[0], beta=p[1])) == 0
+    assert stale(2, 512, lambda p: call(gamma2=p[0], beta2=p[1])) == 0

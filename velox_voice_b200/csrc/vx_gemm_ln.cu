@@ -140,8 +140,8 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 
   // ---- set-up
   // Warp 0 makes the barriers and goes straight to its loads, as do the loader of B, the MMA issuer and the storer once the barriers exist
-  // (named barrier); they meet the others only at the end.  The epilogue needs the cluster's barrier: tensor memory, parameters, the
-  // peer's barriers.
+  // (named barrier); they meet the others only at the end.  The epilogue needs the cluster's barrier: tensor memory, the peer's
+  // barriers.
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap_b);
     for (int s = 0; s < LN_A_SLOTS; ++s) { mbar_init(&sm.full[s], 1); mbar_init(&sm.empty[s], 1); }
@@ -163,17 +163,6 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     tmem_relinquish();
   } else if (warp == 18) {
     if (lane == 0) { prefetch_tmap(&tmap_res); prefetch_tmap(&tmap_out); }
-  } else if (warp >= 2 && warp < 18) {
-    const int i = threadIdx.x - 64;  // constants of the model
-    if (i < LN_BN) {
-      sm.bias[i] = p.bias ? __ldg(p.bias + rank * LN_BN + i) : 0.0f;
-      sm.gamma[i] = __ldg(p.gamma + rank * LN_BN + i);
-      sm.beta[i] = __ldg(p.beta + rank * LN_BN + i);
-      if constexpr (LN2) {
-        sm.gamma2[i] = __ldg(p.gamma2 + rank * LN_BN + i);
-        sm.beta2[i] = __ldg(p.beta2 + rank * LN_BN + i);
-      }
-    }
   }
   __syncwarp();
   tc_fence_before();
@@ -181,7 +170,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   const bool epilogue_warp = warp >= 2 && warp < 18;
   constexpr int SETUP_THREADS = ln_threads(LN2) - 16 * 32;
   if (epilogue_warp) {
-    cluster_wait();  // tensor memory, parameters, and the peer's barriers before anything is sent to them
+    cluster_wait();  // tensor memory, and the peer's barriers before anything is sent to them
   } else if (warp == 0) {
     named_bar_arrive(1, SETUP_THREADS);
   } else {
@@ -393,6 +382,22 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     if (!paced && lane == 0 && my_tiles > 0) {
       mbar_expect_tx(&sm.res_full[sb], LN_STAGING);
       tma_load_2d(sm.staging[sb], &tmap_res, tile_col, mb * LN_BM + q * 32, &sm.res_full[sb]);
+    }
+    {
+      // biases and LayerNorm parameters, behind the wait, since the launch before may have written them, while the first stage comes in
+      const int c = threadIdx.x - 64;
+      if (c < LN_BN) {
+        const int n = static_cast<int>(rank) * LN_BN + c;
+        sm.bias[c] = p.bias ? p.bias[n] : 0.0f;
+        sm.gamma[c] = p.gamma[n];
+        sm.beta[c] = p.beta[n];
+        if constexpr (LN2) {
+          sm.gamma2[c] = p.gamma2[n];
+          sm.beta2[c] = p.beta2[n];
+        }
+      }
+      __syncwarp();
+      named_bar_sync(2, 16 * 32);
     }
     for (int i = 0; i < my_tiles && ok; ++i, mb += nclusters) {
       const int64_t row = static_cast<int64_t>(mb) * LN_BM + row_in;
