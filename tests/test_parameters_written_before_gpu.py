@@ -75,3 +75,14 @@ def test_residual_layernorm_gemm(M, K):
     assert stale(1, 512, lambda p: call(bias=p[0])) == 0
     assert stale(2, 512, lambda p: call(gamma=p[0], beta=p[1])) == 0
     assert stale(2, 512, lambda p: call(gamma2=p[0], beta2=p[1])) == 0
+
+
+@pytest.mark.parametrize("M,F", [(80, 257), (3, 257), (80, 256), (130, 257)])  # one copy, its remainder of three, word by word, the other kernel
+def test_filterbank(M, F):
+    from velox_voice_b200 import ops
+
+    spec = torch.randn(1000, F, dtype=torch.complex64, device="cuda")
+    zero, one = torch.zeros(M, device="cuda"), torch.ones(M, device="cuda")
+    assert stale(M, F, lambda p: ops.power_mel_log(spec, p, zero, one)) == 0
+    bank = torch.linspace(0.0, 1.0, M * F, device="cuda").view(M, F)
+    assert stale(2, M, lambda p: ops.power_mel_log(spec, bank, p[0], p[1])) == 0

@@ -116,13 +116,14 @@ __global__ void __launch_bounds__(MEL_THREADS, 1) power_mel_log_kernel(const Mel
     bar.abort_flag = 0;
     mbar_fence_init();
   }
+  pdl_wait();  // the launch before may have written the filterbank, too
   // the filterbank, zero-padded, into its resident swizzled tiles: element (n, k) of stage k / 32
   for (int64_t i = threadIdx.x; i < static_cast<int64_t>(p.stages) * p.n_pad * MEL_KS; i += blockDim.x) {
     const int kk = static_cast<int>(i % MEL_KS);
     const int n = static_cast<int>((i / MEL_KS) % p.n_pad);
     const int ks = static_cast<int>(i / (static_cast<int64_t>(MEL_KS) * p.n_pad));
     const int64_t k = static_cast<int64_t>(ks) * MEL_KS + kk;
-    const float v = (n < p.M && k < p.F) ? __ldg(p.mel + n * p.ld_mel + k) : 0.0f;
+    const float v = (n < p.M && k < p.F) ? p.mel[n * p.ld_mel + k] : 0.0f;
     *reinterpret_cast<float*>(bres + ks * b_stage_bytes + sw128(n, kk)) = v;
   }
   fence_proxy_async_smem();
@@ -134,7 +135,6 @@ __global__ void __launch_bounds__(MEL_THREADS, 1) power_mel_log_kernel(const Mel
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bar.tmem_base;
-  pdl_wait();  // the filterbank is a constant of the front-end; the spectrum and the output are not
 
   if (warp >= 4 && warp < 4 + MEL_LOADERS) {
     // =========================== loaders ===========================
@@ -279,7 +279,7 @@ constexpr int MT_MAX_F = 512 - MT_TM_A;
 
 struct MtBarriers {
   uint64_t raw_full[MT_RING_MAX], raw_empty[MT_RING_MAX];
-  uint64_t b_full[2], b_empty[2], acc_full[2], acc_empty[2];
+  uint64_t b_full[2], b_empty[2], acc_full[2], acc_empty[2], bank_full;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -327,14 +327,29 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
       mbar_init(&bar.acc_full[a], 1);
       mbar_init(&bar.acc_empty[a], 4);
     }
+    mbar_init(&bar.bank_full, 1);
     bar.abort_flag = 0;
     mbar_fence_init();
   }
-  // filterbank -> shared memory, rows of F | 1 words (an odd pitch: the column reads below are conflict-free)
+  // Filterbank -> shared memory, behind the wait: the launch before may have written it, too.  Rows of F | 1 words (an odd pitch: the column
+  // reads below are conflict-free); a dense bank of odd F lies like this already and comes in one copy.  64 frames right behind another call: 4.1 us with
+  // the filterbank read ahead of the wait, 7.7 behind it word by word, 5.8 like this, 1,000 frames 7.5 and 6.4; behind torch's rfft, which triggers
+  // nothing early, 64 frames 10.1 and 8.6, 3,750 14.6 and 12.9.
+  pdl_wait();
   const int pitch = F | 1;
   float* const bank_s = reinterpret_cast<float*>(base);
-  for (int n = warp; n < M; n += MT_THREADS / 32)
-    for (int k = lane; k < F; k += 32) cp_async4(smem_u32(bank_s + n * pitch + k), p.mel + n * p.ld_mel + k);
+  const bool one_copy = pitch == F && p.ld_mel == F && M * F >= 4 && (reinterpret_cast<uintptr_t>(p.mel) & 15) == 0;
+  if (one_copy) {
+    const int whole = (M * F) & ~3;
+    if (threadIdx.x == 0) {
+      mbar_expect_tx(&bar.bank_full, whole * 4u);
+      bulk_load(bank_s, p.mel, whole * 4u, &bar.bank_full);
+    }
+    if (threadIdx.x < static_cast<unsigned>(M * F - whole)) bank_s[whole + threadIdx.x] = p.mel[whole + threadIdx.x];
+  } else {
+    for (int n = warp; n < M; n += MT_THREADS / 32)
+      for (int k = lane; k < F; k += 32) cp_async4(smem_u32(bank_s + n * pitch + k), p.mel + n * p.ld_mel + k);
+  }
   if (warp == 4 + MT_XF) {
     tmem_alloc(&bar.tmem_base, 512);
     tmem_relinquish();
@@ -345,13 +360,26 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
   tc_fence_after();
   const uint32_t tmem_base = bar.tmem_base;
   // -> tensor memory: lane m of quadrant `warp` holds filterbank row m, zero beyond M and F
-  if (warp < 4) {
+  if (warp < 4 && (!one_copy || __all_sync(0xffffffffu, mbar_wait<true>(&bar.bank_full, 0, p.status, 17, abortp)))) {
     const int m = warp * 32 + lane;
     const uint32_t ta = tmem_base + MT_TM_A + (static_cast<uint32_t>(warp * 32) << 16);
-    for (int k0 = 0; k0 < 8 * ksteps; k0 += 8) {
+    const float* const src = bank_s + (m < M ? m : 0) * pitch;
+    int k0 = 0;
+#pragma unroll 4
+    for (; k0 + 8 <= F; k0 += 8) {
       float v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = m < M && k0 + j < F ? bank_s[m * pitch + k0 + j] : 0.0f;
+      for (int j = 0; j < 8; ++j) v[j] = src[k0 + j];
+      if (m >= M) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+      }
+      tc_st_32x32b_x8(ta + k0, v);
+    }
+    if (k0 < F) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = m < M && k0 + j < F ? src[k0 + j] : 0.0f;
       tc_st_32x32b_x8(ta + k0, v);
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -359,11 +387,13 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // operand tiles: the bins beyond F are never written, they must read as zero
-  for (uint32_t i = threadIdx.x; i < 2 * tile_bytes / 16; i += MT_THREADS) reinterpret_cast<uint4*>(tiles_s)[i] = make_uint4(0, 0, 0, 0);
+  // operand tiles: the bins beyond F, in the last stage, are never written, they must read as zero (rows of frames beyond T only reach columns
+  // that are not stored)
+  if (F % MEL_KS != 0)
+    for (uint32_t i = threadIdx.x; i < 2 * MT_N * 8; i += MT_THREADS)
+      reinterpret_cast<uint4*>(tiles_s + (i / (MT_N * 8)) * tile_bytes + (p.stages - 1) * (MT_N * 128))[i % (MT_N * 8)] = make_uint4(0, 0, 0, 0);
   fence_proxy_async_smem();
   __syncthreads();
-  pdl_wait();  // the filterbank is a constant of the front-end; the spectrum and the output are not
 
   // Tile i of this CTA covers frames [32 t, 32 t + 32), t = blockIdx.x + i gridDim.x, as up to four chunks of eight rows.
   auto chunks_of = [&](int64_t t0) { const int64_t left = p.T - t0; return left >= MT_N ? MT_N / MT_ROWS : static_cast<int>((left + MT_ROWS - 1) / MT_ROWS); };
