@@ -137,7 +137,7 @@ def test_what_writes_weights_does_not_trigger_the_next_launch():
 
 @pytest.mark.parametrize("name,kernel", [("vx_quant.cu", "ln_quant_kernel(const QuantParams p) {"), ("vx_quant.cu", "rows2_kernel(const QuantParams p) {"),
                                          ("vx_gemm_ln.cu", "bsgemm_residual_ln_kernel("), ("vx_mel.cu", "power_mel_log_kernel("),
-                                         ("vx_mel.cu", "power_mel_log_dense_kernel(")])
+                                         ("vx_mel.cu", "power_mel_log_dense_kernel("), ("vx_rowscale.cu", "rowscale_small_kernel(const RsParams p) {")])
 def test_parameters_are_read_behind_the_wait(name, kernel):
     """A library GEMM may have written a bias, a LayerNorm parameter or a filterbank, and triggers the launch behind it early: no address
     of one is formed ahead of that launch's wait."""

@@ -86,3 +86,12 @@ def test_filterbank(M, F):
     assert stale(M, F, lambda p: ops.power_mel_log(spec, p, zero, one)) == 0
     bank = torch.linspace(0.0, 1.0, M * F, device="cuda").view(M, F)
     assert stale(2, M, lambda p: ops.power_mel_log(spec, bank, p[0], p[1])) == 0
+
+
+@pytest.mark.parametrize("M", [1, 16, 300])
+def test_bias_of_the_per_row_lane(M):
+    from velox_voice_b200 import ops
+
+    x = torch.randn(M, 512, device="cuda")
+    wq, ws = ops.per_row_col_quantize(0.02 * torch.randn(2048, 512, device="cuda"))
+    assert stale(1, 2048, lambda p: ops.rowscale_linear(x, wq, ws, p[0])) == 0

@@ -52,11 +52,11 @@ bool pdl_enabled();
 // set-up (barriers, tensor memory, constant operands) overlap the predecessor's tail.
 //
 // What a kernel may read before its pdl_wait(): only what no kernel that triggers early (pdl_launch_dependents) wrote in
-// the launch before it, nor -- since a kernel may trigger before its own wait -- in the launches before that.  LayerNorm
-// parameters, biases and the filterbank come from torch kernels, which never trigger early.  Weights come from the
-// quantizers: those that pack weights (quant_kernel, and rows2_kernel when it writes natural-layout scales) and the relayout of
+// the launch before it, nor -- since a kernel may trigger before its own wait -- in the launches before that.  That leaves weights, which come from
+// the quantizers: those that pack weights (quant_kernel, and rows2_kernel when it writes natural-layout scales) and the relayout of
 // one operand's scales do not trigger, and the GEMMs read weights ahead only when the caller says that they are constants (VX_GEMM_CONST_B), not
-// for an operand that the previous launch may just have produced.
+// for an operand that the previous launch may just have produced.  Biases, LayerNorm parameters and filterbanks may be an fp32 result of a GEMM
+// that triggered early: they are read behind the wait.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                     Args&&... args) {

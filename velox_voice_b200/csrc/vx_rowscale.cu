@@ -80,14 +80,14 @@ __global__ void __launch_bounds__(RS_WARPS * 32) rowscale_small_kernel(const RsP
     wv[i] = c < chunks ? __ldg(reinterpret_cast<const uint4*>(wrow + c * 64)) : make_uint4(0, 0, 0, 0);
   }
   const int nc = n0 + 2 * t;  // this lane's two output columns
-  float col_scale[2], bias[2];
+  pdl_wait();
+  float col_scale[2], bias[2];  // (behind the wait: the launch before may have written the bias)
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int c = nc + i < p.N ? nc + i : p.N - 1;
     col_scale[i] = ue8m0_to_float(__ldg(p.ws + c));
     bias[i] = p.bias ? __ldg(p.bias + c) : 0.0f;
   }
-  pdl_wait();
 
   // ---- quantize: a warp per row (up to four rows: 2, 4 or 8 warps share one, every wpr-th 256-element chunk each), lane l
   // owns elements [8 l, 8 l + 8) of a chunk (as quant_kernel does)
