@@ -232,8 +232,21 @@ __device__ __forceinline__ uint32_t swish_quant_chunk(const uint32_t (&r)[32], c
 }
 
 // z += 32 bias values cached in shared memory (all lanes read the same words), two at a time: each half rounds like the scalar addition.
-// (Scalar additions of a float4: GLU of 90,000 x 512 x 1,024 37.8 us and 34.3 like this, FP8 q | k | v 129.9 and 126.2, FFN-down 68.6 and 67.8.)
+// (Scalar additions of a float4: GLU of 90,000 x 512 x 1,024 37.8 us and 34.3 like this, FP8 q | k | v 129.9 and 126.2, FFN-down 68.6 and 67.8,
+// fp32 results of 1,537 rows 6.50 and 6.20.)  PAIRS = false, one at a time, for the residual epilogue whose output is chosen at run time: there the pairs cost
+// registers of its long tail.  NVFP4 residual with fp32 output, 512 x 512, pairs / one at a time: 90,000 rows 74.4 and 63.7 us, 24,000 21.5 and 19.5, 1,537 6.27
+// and 5.99; MX32 1,537 rows 6.31 and 5.98, 90,000 61.7 and 62.8; FP8 with an fp32 residual 1,537 rows 16.3 and 15.9.
+template <bool PAIRS = true>
 __device__ __forceinline__ void add_bias32(float (&z)[32], const float* bias_s) {
+  if constexpr (!PAIRS) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      const float4 b = *reinterpret_cast<const float4*>(bias_s + i);
+      z[i] = __fadd_rn(z[i], b.x); z[i + 1] = __fadd_rn(z[i + 1], b.y);
+      z[i + 2] = __fadd_rn(z[i + 2], b.z); z[i + 3] = __fadd_rn(z[i + 3], b.w);
+    }
+    return;
+  }
   const uint32_t addr = smem_u32(bias_s);
 #pragma unroll
   for (int i = 0; i < 32; i += 4) {

@@ -182,7 +182,7 @@ struct ChunkOut {
                                                int lane) {
     if constexpr (EPI != VX_EPI_NONE) {
       if (bias_s) {
-        add_bias32(z, bias_s);
+        add_bias32<EPI != VX_EPI_BIAS_RESIDUAL || RES_TMA>(z, bias_s);
         if constexpr (EPI == VX_EPI_BIAS_GLU) add_bias32(gate, gate_s);
       }
     }
