@@ -87,6 +87,19 @@ def test_stores_are_complete_before_a_kernel_ends(name):
     assert text.rindex("tma_store_commit()") < last < text.index("tmem_dealloc(tmem_base", last)
 
 
+@pytest.mark.parametrize("name,kernel,storers", [("vx_gemm_ln.cu", "bsgemm_residual_ln_kernel(", 2), ("vx_gemm.cu", "bsgemm_kernel(", 1)])
+def test_every_role_that_stores_waits_for_its_writes(name, kernel, storers):
+    """Each role that hands blocks to the TMA ends with the full wait for them, not with that of another role."""
+    text = source(name)
+    text = text[text.index(kernel):]
+    text = text[:re.search(r"\n}\n", text).end()]
+    roles = [r for r in re.split(r"\n  } else\b[^\n]*{|\n  if \(warp == 0\) {", text) if "tma_store_commit()" in r]
+    assert len(roles) == storers
+    for role in roles:
+        role = role[:role.find("tmem_dealloc")]
+        assert role.rindex("tma_store_commit()") < role.rindex("tma_store_wait_all<0>()")
+
+
 @pytest.mark.parametrize("name,kernel,waits", [("vx_gemm.cu", "bsgemm_kernel(", r"warp != 0 \|\| my_tiles == 0"),
                                                ("vx_gemm_ln.cu", "bsgemm_residual_ln_kernel(", "!producer_thread"),
                                                ("vx_pass.cu", "conformer_pass_kernel(", "warp != PS_WARP_B")])

@@ -87,6 +87,24 @@ def test_fused_in_place_and_repeated(ops):
     assert torch.equal(q2.codes, q2_ref.codes) and torch.equal(q2.sf, q2_ref.sf)
 
 
+@pytest.mark.parametrize("K", [768, 2048])
+@pytest.mark.parametrize("M", [9472, 9473, 10000, 30000])  # 74 clusters of 128 rows: one tile each, one cluster with a second, several
+def test_fused_in_place_with_streamed_weights(ops, M, K):
+    """Weights that stream, out over the residual, again and again: x leaves by the warp that moves it, or by the epilogue's where each cluster has
+    one tile, and is whole when the next launch reads it."""
+    a, lin, res, gamma, beta = _case(M, K, seed=M + K)
+    qa = ops.quantize(a, "mx32")
+    x_ref, x = res.clone(), res.clone()
+    for alpha in (1.0, 0.5, 0.25, 0.5):
+        x_ref = lin(qa, residual=x_ref, alpha=alpha)
+    q_ref = ops.ln_quantize(x_ref, gamma, beta, 1e-5, "mx32")
+    for alpha in (1.0, 0.5, 0.25, 0.5):
+        got, q = lin.residual_ln(qa, residual=x, gamma=gamma, beta=beta, eps=1e-5, alpha=alpha, out=x)
+    assert got.data_ptr() == x.data_ptr()
+    assert torch.equal(x, x_ref)
+    assert torch.equal(q.codes, q_ref.codes) and torch.equal(q.sf, q_ref.sf)
+
+
 def test_fused_matches_the_oracle(ops):
     """x within the path's bound of the oracle GEMM + epilogue; codes and scales bit-exact against the oracle's
     LayerNorm (half-row summation order) + MX32 quantizer applied to the x the kernel stored."""

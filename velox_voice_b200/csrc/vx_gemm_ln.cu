@@ -7,11 +7,11 @@
 // factors of a block-scaled MMA in tensor memory.  So a CLUSTER OF TWO CTAs owns each block of 128 rows:
 // CTA r computes columns [256 r, 256 r + 256) with 128 x 256 x 64 MXF4 MMAs, and the two exchange the
 // per-row partial sums of the LayerNorm statistics through distributed shared memory (st.async with
-// mbarrier completion into a table double-buffered per tile, one barrier per lane quadrant).  Per CTA, 20 warps:
+// mbarrier completion into a table double-buffered per tile, one barrier per lane quadrant).  Per CTA, 20 warps (19 with two LayerNorms):
 //   warp 0      TMA producer: A tiles (128-byte swizzle) + scale-factor atoms into a ring; the CTA's half of B stays
 //               resident in shared memory when K <= 512;
 //   warp 18     otherwise streams B through a ring of its own;
-//   warp 19     where B streams, moves the residual and x blocks of the epilogue warps;
+//   warp 19     where B streams for more than one tile, moves the residual and x blocks of the epilogue warps (one LayerNorm only);
 //   warp 1      owns tensor memory, copies scale factors shared -> tensor memory and issues the MMAs;
 //   warps 2..17 epilogue, warp (q, g) = TMEM lane quadrant q, 32-column blocks 2 g and 2 g + 1 of the CTA:
 //     pass 1  accumulator -> + bias, alpha, residual (its 32 x 64 block prefetched by TMA into the warp's
@@ -132,10 +132,10 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   const bool resident = p.b_resident != 0;
   // Warp 19 moves the residual and x blocks, two of x at a time, or each epilogue warp its own, sixteen of x at a time.  The sixteen hold up
   // the loads of the operands (64 KB leave an SM at about 16 bytes a cycle, in front of the loads in the TMA's queue), which costs where
-  // operands stream: of 12,700 cycles a tile with K = 2048 the MMAs waited 3,000 for one stage of B.  One thread for sixteen blocks is
-  // slower where they don't, and nothing else than the epilogue bounds the kernel.  90,000 rows, captured calls in a row, own / paced:
-  // K = 2048 80.9 / 75.5 us, K = 512 53.8 / 56.0, two LayerNorms with K = 2048 88.7 / 88.8.
-  const bool paced = !LN2 && !resident;
+  // operands stream for a further tile: of 12,700 cycles a tile with K = 2048 the MMAs waited 3,000 for one stage of B.  One thread for sixteen
+  // blocks is slower where no loads follow: with resident weights, and with one tile per cluster.  Captured calls in a row, own / paced: K = 2048, 90,000 rows
+  // 79.8 / 72.7 us, 24,000 26.3 / 24.7, 3,750 10.25 / 10.6, 375 9.9 / 10.4; K = 1024, 3,750 rows 8.4 / 8.9; K = 512, 90,000 rows 50.7 / 53.6.
+  const bool paced = !LN2 && !resident && p.m_tiles > nclusters;
   const uint32_t ring_off = resident ? p.k_stages * LN_B_SLOT : LN_HB_SLOTS * LN_HB_SLOT;  // ring of A
 
   // ---- set-up
@@ -546,8 +546,8 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
               uint64_t g0, g1, b0, b1;
-            ld_shared_pairs(ga + 16 * hh, g0, g1);
-            ld_shared_pairs(be + 16 * hh, b0, b1);
+              ld_shared_pairs(ga + 16 * hh, g0, g1);
+              ld_shared_pairs(be + 16 * hh, b0, b1);
               const uint32_t w0 = xp[4 * c + 2 * hh], w1 = xp[4 * c + 2 * hh + 1];
               const uint64_t x0 = pack_f32x2(__uint_as_float(w0 << 16), __uint_as_float(w0 & 0xffff0000u));
               const uint64_t x1 = pack_f32x2(__uint_as_float(w1 << 16), __uint_as_float(w1 & 0xffff0000u));
