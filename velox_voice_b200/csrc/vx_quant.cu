@@ -22,6 +22,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "vx_common.cuh"
 #include "vx_ptx.cuh"
 #include "vx_quant_math.cuh"
@@ -891,10 +893,14 @@ bool launch_rows2(const QuantParams& p, bool ln, cudaStream_t st) {
   }
 }
 
-// max |x|.  Each thread keeps eight 16-byte loads in flight; dense tensors (ldx == K) are walked as one long row; one atomic
-// maximum per block (one per warp: 90,000 x 512 bf16 24.6 us, 20.5 like this; 24,000 x 512 12.4 and 8.3).  Bound by HBM.  ONE_BLOCK: a tensor small enough for one block, which then writes the result itself (no cleared accumulator).
+// max |x|.  Dense tensors (ldx == K) are walked as one long row.  A block of 256 threads takes 1,024 vectors, four a thread, all in flight at once; with the
+// eight blocks per SM that are resident, tensors beyond 34 MB are walked in strides, eight loads a turn.  One atomic maximum per warp up to one block per SM, per
+// block beyond (`warp_atomics` blocks): thousands of atomics on one address take microseconds (90,000 x 512 bf16 one per warp 24.6 us, per block 18.5),
+// a few hundred less than meeting in the block.  Bound by HBM.  ONE_BLOCK: a tensor small enough for one block, which then writes the result
+// itself (no cleared accumulator).
 template <typename T, bool ONE_BLOCK>
-__global__ void __launch_bounds__(ONE_BLOCK ? 1024 : 256) amax_kernel(const T* x, int64_t rows, int64_t row_vecs, int64_t ldx, float* out) {
+__global__ void __launch_bounds__(ONE_BLOCK ? 1024 : 256) amax_kernel(const T* x, int64_t rows, int64_t row_vecs, int64_t ldx, float* out,
+                                                                       int warp_atomics) {
   constexpr int EV = 16 / sizeof(T);  // elements per 16-byte vector
   pdl_launch_dependents();
   pdl_wait();
@@ -911,18 +917,18 @@ __global__ void __launch_bounds__(ONE_BLOCK ? 1024 : 256) amax_kernel(const T* x
   if (rows == 1) {
     const uint4* v = reinterpret_cast<const uint4*>(x);
     int64_t i = t0;
-    for (; i + 7 * step < row_vecs; i += 8 * step) {
-      uint4 u[8];
+    auto batch = [&](auto count, bool whole) {  // the loads of `count` vectors leave together
+      constexpr int C = decltype(count)::value;
+      uint4 u[C];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) u[j] = v[i + j * step];
+      for (int j = 0; j < C; ++j) u[j] = whole || i + j * step < row_vecs ? v[i + j * step] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) take(u[j]);
-    }
-    for (; i + 3 * step < row_vecs; i += 4 * step) {
-      const uint4 u0 = v[i], u1 = v[i + step], u2 = v[i + 2 * step], u3 = v[i + 3 * step];
-      take(u0); take(u1); take(u2); take(u3);
-    }
-    for (; i < row_vecs; i += step) take(v[i]);
+      for (int j = 0; j < C; ++j) take(u[j]);
+      i += C * step;
+    };
+    while (i + 7 * step < row_vecs) batch(std::integral_constant<int, 8>{}, true);
+    if (i + 3 * step < row_vecs) batch(std::integral_constant<int, 4>{}, true);
+    if (i < row_vecs) batch(std::integral_constant<int, 3>{}, false);
   } else {
     const int64_t total = rows * row_vecs;
     for (int64_t i = t0; i < total; i += step) {
@@ -931,6 +937,10 @@ __global__ void __launch_bounds__(ONE_BLOCK ? 1024 : 256) amax_kernel(const T* x
     }
   }
   a = warp_max(a);
+  if (!ONE_BLOCK && static_cast<int>(gridDim.x) <= warp_atomics) {
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned int*>(out), __float_as_uint(a));  // non-negative floats order like their bit patterns
+    return;
+  }
   __shared__ float part[32];
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = a;
   __syncthreads();
@@ -938,7 +948,7 @@ __global__ void __launch_bounds__(ONE_BLOCK ? 1024 : 256) amax_kernel(const T* x
     a = warp_max(ONE_BLOCK || threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0.0f);
     if (threadIdx.x == 0) {
       if constexpr (ONE_BLOCK) *out = a;
-      else atomicMax(reinterpret_cast<unsigned int*>(out), __float_as_uint(a));  // non-negative floats order like their bit patterns
+      else atomicMax(reinterpret_cast<unsigned int*>(out), __float_as_uint(a));
     }
   }
 }
@@ -1185,11 +1195,12 @@ int vx_amax(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, float
     return fail(-1, "x must be 16-byte aligned rows with K %% 8 == 0");
   const bool dense = ldx == K || M == 1;
   const int64_t rows = dense ? 1 : M, row_vecs = (dense ? M * K : K) * esz / 16, vecs = rows * row_vecs;
-  // One block up to 512 KB of dense rows, 32 vectors per thread: it needs no cleared accumulator (memset + blocks / one block, bf16 rows of
-  // 512: 160 rows 4.3 / 2.9 us, 375 5.8 / 4.3, 500 5.8 / 5.1).  Strided rows, walked one vector at a time, up to 128 KB.
+  // One block up to 512 KB of dense rows, 32 vectors per thread: it needs no cleared accumulator.  Memset + blocks / one block, bf16 rows of 512: 200
+  // rows 4.2 / 2.9 us, 300 4.2 to 5.2 / 3.4, 400 4.1 / 4.1, 500 4.4 to 5.8 / 4.6 captured (the two nodes round up to about 2 us each), called one by one 12.8 / 11.7
+  // at all of them.  Strided rows, walked one vector at a time, up to 128 KB.
   const bool one = vecs <= (rows == 1 ? 32768 : 8192);
   auto go = [&](auto* kernel, const auto* xt, int grid, int threads) {
-    return launch_dependent(kernel, dim3(grid), dim3(threads), 0, st, xt, rows, row_vecs, ldx, amax_out);
+    return launch_dependent(kernel, dim3(grid), dim3(threads), 0, st, xt, rows, row_vecs, ldx, amax_out, sm_count());
   };
   if (!one) VX_CUDA_OK(cudaMemsetAsync(amax_out, 0, sizeof(float), st));
   int64_t blocks = (vecs + 1023) / 1024;
