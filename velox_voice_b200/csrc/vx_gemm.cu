@@ -85,8 +85,9 @@ __host__ __device__ constexpr bool kind_vec4(int kind) { return kind == KIND_FP4
 // MX32 and the per-row-scaled format: every scale a power of two (see swish4p)
 __host__ __device__ constexpr bool kind_pow2_scales(int kind) { return kind == KIND_FP4_VEC2 || kind == KIND_FP4_VEC2_N128; }
 
-// Sixteen epilogue warps: warp (quadrant of tensor memory, column group) owns 32 rows x 64 columns of a wide tile (32 x 32 of a
-// narrow one), the same part of every tile.
+// (Sixteen epilogue warps in every kernel: warp (quadrant of tensor memory, column group) owns 32 rows x 64 columns of a wide tile, 32 x 32 of a
+// narrow one, the same part of every tile.)
+
 // Kernels with the sf_split plan (a run-time choice in all of them cost the others up to 7 %: FFN-down of 3,000 rows 7.2 -> 7.7 us).
 __host__ __device__ constexpr bool sf_split_kind(int kind, int epi) { return kind == KIND_FP4_VEC4 && epi == VX_EPI_BIAS_RESIDUAL; }
 
@@ -150,7 +151,7 @@ struct GemmParams {
   int* status;
 };
 
-// Operand arena, two plans:
+// Operand arena, three plans:
 //   streaming  slot s = [A tile 16K | SFA 2K | B tile 16K | SFB 2K], ARENA / 36K slots;
 //   B resident [B stage 0 .. k-1: tile 16K | SFB 2K] then slots [A tile 16K | SFA 2K];
 //   streaming, scale factors apart  slots [A tile | B tile], then two slots [SFA | SFB] (sf_split: three slots of a 16-block format's wide tile).
@@ -366,7 +367,8 @@ bsgemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   constexpr int GATE_OFF = BNT / 2;          // GLU: gate columns follow the value columns
   // Chunk-sequential reads of the wide tile: the second 32-column chunk of a warp is read only after the
   // first is finished, which halves the live accumulator registers (the kernel is capped at 96
-  // per thread).  The two chunks lie in different HALVES of the tile (columns [0, 128) and [128, 256)), and the halves are
+  // per thread).  The two chunks lie in different HALVES of the tile (columns [0, 128) and [128, 256); Swish + FP4 output: both in one half, and
+  // eight warps read each half), and the halves are
   // accumulators of their own in a ring of three (two where the scale factors leave no room, then both at once): each
   // is published and handed back by itself, so the MMAs of the next half run ahead of the epilogue by up to two, which takes
   // up the skew between the warps of a scheduler.  With one barrier for all 256 columns the 1,700 cycles of a K = 512

@@ -36,6 +36,8 @@ __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, st
 
 // 16 bytes of shared memory as two packed fp32 pairs.  (Read as a float4 and then paired, the four values are moved into aligned register
 // pairs one by one: FFN up-projection of 90,000 x 512 x 2,048, whose bias comes this way, 81.4 us and 74.5.)
+// It states no clobber of memory (up to 4 % in long residual and FP8 launches): the stores that fill a table are kept in front of it by the barrier or
+// __syncwarp() that follows them, which a volatile statement does not cross.
 __device__ __forceinline__ void ld_shared_pairs(uint32_t addr, uint64_t& a, uint64_t& b) {
   asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
 }
