@@ -179,7 +179,7 @@ bsgemm_residual_ln_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
   // The loaders wait for the previous launch behind what they may read ahead of it; their other lanes do not wait here at all: they
-  // would hold up the loading lane at the end of the branch (as they once did: no weight was read ahead, 90,000 rows x 512 56.5 us, 53.8 like
+  // would hold up the loading lane at the end of the branch (as they once did: no weight was read ahead, 90,000 rows x 512 56.5 us, 53.3 like
   // this).  The next launch is triggered behind the wait, by threads that have waited, as in vx_gemm.cu: its set-up and weights come in under
   // the last round, which leaves clusters idle (12 blocks, 24,000 frames: 2,650 us without, 2,577 like this).
   const bool producer_thread = (warp == 0 || warp == 18) && lane == 0 && my_tiles > 0;

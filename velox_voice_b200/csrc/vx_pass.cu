@@ -24,9 +24,9 @@
 // activations, 17 issues the MMAs (one elected lane), 18 and 19 load weights and the biases and LayerNorm parameters, which depend on
 // no layer and run ahead of them through rings of four and three slots.  Accumulators: a ring of three times 128 columns.
 //
-// Measured, whole greedy pass of 12 blocks, separate launches against this: 375 frames 752 us -> 558, 1,920 frames (the most for
-// clusters of eight) 838 -> 571, 4,000 frames (clusters of four) 988 -> 695, 4,200 frames 1,038 -> 737 (its twelve positional projections are launches of their own).  What bounds it now, of 88,000 cycles a
-// block (47 us, clusters of eight): the hand-over of an operand, 4,000 a phase -- the release waits 1,750 for the stores, fence and loads take
+// Measured, whole greedy pass of 12 blocks, captured, separate launches / this: 375 frames 632 / 550 us, 1,920 frames (the most for
+// clusters of eight) 773 / 564, 4,000 frames (clusters of four) 890 / 687, 4,200 frames 937 / 724 (its twelve positional projections are launches of their own).  What bounds
+// it now, of 88,000 cycles a block (45 us, clusters of eight): the hand-over of an operand, 4,000 a phase -- the release waits 1,750 for the stores, fence and loads take
 // 1,900 --, the issue of the MMAs, 500 to 700 cycles per stage of four, and the chain accumulator -> sums -> exchange -> quantize of
 // the four LayerNorms, 4,000 each.  Tried and not kept: operands pushed to the other CTAs' shared memory by st.async (630 us) or bulk
 // copies (590; shared memory leaves an SM at 14 to 16 bytes a cycle, what L2 delivers enters at 90), jobs of 64 columns for the
@@ -748,8 +748,8 @@ int vx_conformer_pass_supported(int fmt, int64_t d_model, int64_t ffn, int64_t c
          blocks <= PS_MAX_BLOCKS;
 }
 
-// One round of clusters of four.  4,200 frames: separate launches 1,038 us (4,300 frames now 1,004), one launch 737; a second round takes as long again, and
-// the launches that pipeline over many row blocks are as fast (4,608 frames: 1,075 and about 1,450).
+// One round of clusters of four.  Separate launches / one launch: 4,200 frames 937 / 724 us; a second round would take as long again, about 1,450 us, where the launches
+// that pipeline over many row blocks take 954 (4,608 frames).
 int64_t vx_conformer_pass_frames(void) {
   return static_cast<int64_t>(vx::max_clusters<4>()) * vx::PS_BM;
 }
