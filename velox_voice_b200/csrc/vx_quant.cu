@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(256, LN ? VX_R2_MIN_BLOCKS_LN : VX_R2_MIN_BLOC
     for (int d = 0; d < VX_R2_RING; ++d) mbar_init(&full_w[d], 1);
     mbar_fence_init();
   }
-  __syncwarp();
+  __syncthreads();
   pdl_wait();  // from here on the kernel touches what the previous kernels of the stream produced
   auto issue = [&](int slot, int u) {
     if (lane == 0) {
