@@ -30,3 +30,22 @@ def test_edges_match_the_oracle(T, F, M, offset):
     cu = lambda a: torch.from_numpy(a).cuda()
     out = ops.power_mel_log_tf32(flat[offset:].view(T, F), cu(bank), cu(mean), cu(istd)).cpu().numpy()
     assert np.abs(out - ML.power_mel_log_tf32(spec, bank, mean, istd)).max() < 2e-5
+
+
+# Where the filterbank passes through shared memory and how many chunks come in ahead of it: all slots of the ring (few mel rows, many bins), some, none (a bank that
+# reaches over the operand tiles); banks of odd and even pitch, off a 16-byte boundary, with columns between their rows
+@pytest.mark.parametrize("T,F,M", [(100, 447, 1), (32 * 148 * 2 + 5, 447, 2), (100, 447, 96), (47, 445, 90), (100, 257, 80), (24, 257, 128), (100, 255, 3), (100, 256, 80), (40, 3, 1), (40, 1, 2)])
+@pytest.mark.parametrize("form", ["dense", "shifted", "strided"])
+def test_places_of_the_filterbank(T, F, M, form):
+    from velox_voice_b200 import ops
+
+    rng = np.random.default_rng(T + F + M)
+    spec = ((rng.standard_normal((T, F)) + 1j * rng.standard_normal((T, F))) * 3.0).astype(np.complex64)
+    bank = rng.random((M, F)).astype(np.float32)
+    wide = torch.full((M * (F + 3) + 1,), float("nan"), device="cuda")
+    cu = {"dense": wide[: M * F].view(M, F), "shifted": wide[1 : M * F + 1].view(M, F), "strided": wide[: M * (F + 3)].view(M, F + 3)[:, :F]}[form]
+    cu.copy_(torch.from_numpy(bank))
+    zero, one = np.zeros(M, np.float32), np.ones(M, np.float32)
+    for _ in range(2):  # the second right behind the first
+        out = ops.power_mel_log_tf32(torch.from_numpy(spec).cuda(), cu, torch.from_numpy(zero).cuda(), torch.from_numpy(one).cuda())
+    assert np.abs(out.cpu().numpy() - ML.power_mel_log_tf32(spec, bank, zero, one)).max() < 2e-5  # as above

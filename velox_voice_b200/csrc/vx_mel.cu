@@ -51,6 +51,7 @@ struct MelParams {
   float* out;
   int64_t ldo;
   int n_pad, stages, tiles, ring;
+  int bank_off, early;  // dense kernel: where the filterbank passes through shared memory, ring slots in front of it
   int* status;
 };
 
@@ -305,7 +306,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* const base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  // [operand tiles: 2 x stages x 32 x 128 B][ring of raw chunks]; during set-up the filterbank passes through the same memory
+  // [operand tiles: 2 x stages x 32 x 128 B][ring of raw chunks]; during set-up the filterbank passes through the end of the memory
   uint8_t* const tiles_s = base;
   const uint32_t tile_bytes = static_cast<uint32_t>(p.stages) * MT_N * 128u;
   uint8_t* const ring = tiles_s + 2 * tile_bytes;
@@ -331,13 +332,25 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
     bar.abort_flag = 0;
     mbar_fence_init();
   }
+  // Tile i of this CTA covers frames [32 t, 32 t + 32), t = blockIdx.x + i gridDim.x, as up to four chunks of eight rows.
+  auto chunks_of = [&](int64_t t0) { const int64_t left = p.T - t0; return left >= MT_N ? MT_N / MT_ROWS : static_cast<int>((left + MT_ROWS - 1) / MT_ROWS); };
+  auto tile_frame = [&](int i) { return (static_cast<int64_t>(blockIdx.x) + static_cast<int64_t>(i) * gridDim.x) * MT_N; };
+  auto load_chunk = [&](int64_t row, uint32_t s) {
+    const int64_t rows = p.T - row < MT_ROWS ? p.T - row : MT_ROWS;
+    // (an odd number of rows, the end of the input only, may leave 8 bytes: the transform warp fetches them itself)
+    const uint32_t bytes = (static_cast<uint32_t>(rows) * row_bytes) & ~15u;
+    mbar_expect_tx(&bar.raw_full[s], bytes);
+    if (bytes) bulk_load(ring + s * chunk_bytes, p.spec + row * p.F, bytes, &bar.raw_full[s]);
+  };
+
   // Filterbank -> shared memory, behind the wait: the launch before may have written it, too.  Rows of F | 1 words (an odd pitch: the column
-  // reads below are conflict-free); a dense bank of odd F lies like this already and comes in one copy.  64 frames right behind another call: 4.1 us with
-  // the filterbank read ahead of the wait, 7.7 behind it word by word, 5.8 like this, 1,000 frames 7.5 and 6.4; behind torch's rfft, which triggers
-  // nothing early, 64 frames 10.1 and 8.6, 3,750 14.6 and 12.9.
+  // reads below are conflict-free); a dense bank of odd F lies like this already and comes in one copy.  It passes through the end of the memory, so that
+  // the chunks of the first tile whose slots lie in front of it come in meanwhile.  64 frames right behind another call: 4.1 us with
+  // the filterbank read ahead of the wait, 7.7 behind it word by word, 5.6 like this, 1,000 frames 7.5 and 6.2, 20,000 33.6 and 32.3; behind torch's rfft,
+  // which triggers nothing early, 64 frames 10.3 and 8.2, 3,750 14.6 and 12.3.
   pdl_wait();
   const int pitch = F | 1;
-  float* const bank_s = reinterpret_cast<float*>(base);
+  float* const bank_s = reinterpret_cast<float*>(base + p.bank_off);
   const bool one_copy = pitch == F && p.ld_mel == F && M * F >= 4 && (reinterpret_cast<uintptr_t>(p.mel) & 15) == 0;
   if (one_copy) {
     const int whole = (M * F) & ~3;
@@ -350,6 +363,9 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
     for (int n = warp; n < M; n += MT_THREADS / 32)
       for (int k = lane; k < F; k += 32) cp_async4(smem_u32(bank_s + n * pitch + k), p.mel + n * p.ld_mel + k);
   }
+  const int early = p.early < chunks_of(tile_frame(0)) ? p.early : chunks_of(tile_frame(0));
+  if (threadIdx.x == 0)
+    for (int c = 0; c < early; ++c) load_chunk(tile_frame(0) + c * MT_ROWS, c);
   if (warp == 4 + MT_XF) {
     tmem_alloc(&bar.tmem_base, 512);
     tmem_relinquish();
@@ -395,26 +411,17 @@ __global__ void __launch_bounds__(MT_THREADS, 1) power_mel_log_dense_kernel(cons
   fence_proxy_async_smem();
   __syncthreads();
 
-  // Tile i of this CTA covers frames [32 t, 32 t + 32), t = blockIdx.x + i gridDim.x, as up to four chunks of eight rows.
-  auto chunks_of = [&](int64_t t0) { const int64_t left = p.T - t0; return left >= MT_N ? MT_N / MT_ROWS : static_cast<int>((left + MT_ROWS - 1) / MT_ROWS); };
-  auto tile_frame = [&](int i) { return (static_cast<int64_t>(blockIdx.x) + static_cast<int64_t>(i) * gridDim.x) * MT_N; };
-
   if (warp == 4 + MT_XF + 1) {
     // =========================== producer ===========================
     if (lane == 0) {
-      uint32_t s = 0, ph = 0;
+      uint32_t s = early == p.ring ? 0 : early, ph = early == p.ring ? 1 : 0;
       bool ok = true;
       for (int i = 0; i < my_tiles && ok; ++i) {
         const int64_t t0 = tile_frame(i);
         const int nc = chunks_of(t0);
-        for (int c = 0; c < nc; ++c) {
+        for (int c = i == 0 ? early : 0; c < nc; ++c) {
           if (!mbar_wait<true>(&bar.raw_empty[s], ph ^ 1, p.status, 11, abortp)) { ok = false; break; }
-          const int64_t row = t0 + c * MT_ROWS;
-          const int64_t rows = p.T - row < MT_ROWS ? p.T - row : MT_ROWS;
-          // (an odd number of rows, the end of the input only, may leave 8 bytes: the transform warp fetches them itself)
-          const uint32_t bytes = (static_cast<uint32_t>(rows) * row_bytes) & ~15u;
-          mbar_expect_tx(&bar.raw_full[s], bytes);
-          if (bytes) bulk_load(ring + s * chunk_bytes, p.spec + row * p.F, bytes, &bar.raw_full[s]);
+          load_chunk(t0 + c * MT_ROWS, s);
           if (++s == static_cast<uint32_t>(p.ring)) { s = 0; ph ^= 1; }
         }
       }
@@ -608,7 +615,13 @@ extern "C" int vx_power_mel_log(const void* spec, int64_t T, int64_t F, int64_t 
     if (ld_spec == F && aligned16(spec) && M <= 128 && F <= MT_MAX_F && ring >= 2 && bank_bytes <= room) {
       p.ring = ring < MT_RING_MAX ? ring : MT_RING_MAX;
       p.tiles = static_cast<int>((T + MT_N - 1) / MT_N);
-      const size_t need = tiles_bytes + p.ring * chunk, bytes = need > bank_bytes ? need : bank_bytes;
+      const size_t need = tiles_bytes + p.ring * chunk;
+      size_t bytes = need > bank_bytes ? need : bank_bytes;
+      const size_t four = tiles_bytes + MT_N / MT_ROWS * chunk + bank_bytes;  // a tile's chunks in front of the filterbank, where that fits
+      if (four > bytes) bytes = four < room ? four : room;
+      p.bank_off = static_cast<int>((bytes - bank_bytes) & ~static_cast<size_t>(127));
+      const int64_t front = p.bank_off - static_cast<int64_t>(tiles_bytes - 1024);
+      p.early = front <= 0 ? 0 : static_cast<int>(front / static_cast<int64_t>(chunk) < p.ring ? front / static_cast<int64_t>(chunk) : p.ring);
       static std::atomic<uint64_t> dense_done{0};
       int dv = 0;
       VX_CUDA_OK(cudaGetDevice(&dv));
